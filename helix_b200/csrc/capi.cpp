@@ -247,22 +247,12 @@ int hbk_gemm_qkv_rope(const void* A, int lda, const void* W, int ldw, void* qkv,
   cudaFree(cs);
   return kret(e);
 }
-static int sample_impl(const float* logits, int ldl, const float* temperature, const uint64_t* seed, const int32_t* top_k,
-                       const float* top_p, int32_t* out, int B, int V) {
-  void* scratch = nullptr;
-  cudaError_t e = cudaMalloc(&scratch, hb::sample_scratch_bytes(B, V));
-  if (e != cudaSuccess) return kret(e);
-  e = hb::sample_tokens(0, logits, ldl, temperature, seed, out, B, V, scratch, top_k, top_p);
-  cudaError_t e2 = cudaDeviceSynchronize();
-  cudaFree(scratch);
-  return kret(e != cudaSuccess ? e : e2);
-}
 int hbk_sample(const float* logits, int ldl, const float* temperature, const uint64_t* seed, int32_t* out, int B, int V) {
-  return sample_impl(logits, ldl, temperature, seed, nullptr, nullptr, out, B, V);
+  return kret(hb::sample_tokens(0, logits, ldl, temperature, seed, out, B, V));
 }
 int hbk_sample_filtered(const float* logits, int ldl, const float* temperature, const uint64_t* seed, const int32_t* top_k,
                         const float* top_p, int32_t* out, int B, int V) {
-  return sample_impl(logits, ldl, temperature, seed, top_k, top_p, out, B, V);
+  return kret(hb::sample_tokens(0, logits, ldl, temperature, seed, out, B, V, top_k, top_p));
 }
 int hbk_apply_penalties(float* logits, int ldl, const int32_t* pen_off, const void* pen, int B, int V) {
   return kret(hb::apply_penalties(0, logits, ldl, pen_off, pen, B, V));

@@ -189,7 +189,6 @@ size_t Engine::workspace_bytes() const {
     b += al256((size_t)cfg_.max_seqs * d.vocab * 4);          // logits
     b += al256(attn_decode_workspace_floats(cfg_.max_seqs, d.heads, d.head_dim, 16) * 4);
     b += al256((size_t)cfg_.max_seqs * 4);                    // sampled
-    b += al256(sample_scratch_bytes(cfg_.max_seqs, d.vocab)); // argmax partials
     b += 2 * al256((size_t)cfg_.max_seqs * HB_MAX_LOGPROBS * 4);  // log-probability records of one step
     b += al256((size_t)(5 * d.layers + 1 + 9 * d.layers + 2) * sizeof(int));  // hand-over counters + dependency flags of the decode step
     b += al256(fused_counter_ints(d) * sizeof(int));              // tile arrival counters of the fused decode GEMMs
@@ -340,7 +339,6 @@ int Engine::alloc_runtime() {
     logits_ = (float*)take((size_t)cfg_.max_seqs * d.vocab * 4);
     dec_ws_ = (float*)take(attn_decode_workspace_floats(cfg_.max_seqs, d.heads, d.head_dim, 16) * 4);
     sampled_ = (int32_t*)take((size_t)cfg_.max_seqs * 4);
-    sample_ws_ = take(sample_scratch_bytes(cfg_.max_seqs, d.vocab));
     sig_ = (int*)take((size_t)(5 * d.layers + 1 + 9 * d.layers + 2) * sizeof(int));
     dep_ = sig_ + (5 * d.layers + 1);  // dependency flags of the decode chain follow the hand-over counters (one memset)
     {
@@ -727,7 +725,7 @@ int Engine::forward_llama(int T, int B, bool prefill, int max_seqlen, const Step
   return sample_step(B, L);
 }
 
-// penalties -> (top-k / top-p threshold) -> Gumbel-max / argmax -> log-probabilities, all on logits_[B, vocab]
+// penalties -> Gumbel-max / argmax (of the top-k / top-p survivors) -> log-probabilities, all on logits_[B, vocab]
 int Engine::sample_step(int B, const StepLayout& L) {
   const hb_model_desc& d = model_.d;
   const float* temp = (const float*)(d_step_ + L.temp);
@@ -737,9 +735,8 @@ int Engine::sample_step(int B, const StepLayout& L) {
   const bool filt = (step_flags_ & STEP_FILTER) != 0;
   if (step_flags_ & STEP_PENALTY)
     SPAN(3, 0.0, apply_penalties(stream_, logits_, d.vocab, (const int32_t*)(d_step_ + L.pen_off), d_step_ + L.pen, B, d.vocab));
-  SPAN(3, 4.0 * B * d.vocab, sample_tokens(stream_, logits_, d.vocab, temp, seed, sampled_, B, d.vocab, sample_ws_,
-                                           filt ? topk : nullptr, filt ? topp : nullptr));
-  launches_.fetch_add(filt ? 2 : 1, std::memory_order_relaxed);  // sample_tokens is 2 kernels (+1 threshold pass)
+  SPAN(3, 4.0 * B * d.vocab, sample_tokens(stream_, logits_, d.vocab, temp, seed, sampled_, B, d.vocab, filt ? topk : nullptr,
+                                           filt ? topp : nullptr));
   if (step_flags_ & STEP_LOGPROBS)
     SPAN(3, 4.0 * B * d.vocab, logprob_topk(stream_, logits_, d.vocab, d.vocab, sampled_, (const int32_t*)(d_step_ + L.lpw),
                                             lp_ids_, lp_vals_, B, HB_MAX_LOGPROBS));

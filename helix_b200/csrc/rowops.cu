@@ -290,35 +290,9 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {  // splitmix64 finaliser
   return z ^ (z >> 31);
 }
 
-constexpr int kSampleChunk = 4096;  // vocabulary columns per stage-1 block
-
 __device__ __forceinline__ void argmax_merge(float& best, int& bi, float ov, int oi) {
   if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
 }
-template <int NT>
-__device__ __forceinline__ void block_argmax(float& best, int& bi, float* sval, int* sidx) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    argmax_merge(best, bi, ov, oi);
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) { sval[w] = best; sidx[w] = bi; }
-  __syncthreads();
-  if (w == 0) {
-    best = (l < NT / 32) ? sval[l] : -INFINITY;
-    bi = (l < NT / 32) ? sidx[l] : 0x7fffffff;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      argmax_merge(best, bi, ov, oi);
-    }
-  }
-}
-
-// ---- top-k / top-p (nucleus) filtering: stage 0 finds, per row, the logit threshold below which tokens are dropped ----
 // float -> unsigned key that orders like the float (and back)
 __device__ __forceinline__ uint32_t fkey(float x) {
   const uint32_t u = __float_as_uint(x);
@@ -327,120 +301,290 @@ __device__ __forceinline__ uint32_t fkey(float x) {
 __device__ __forceinline__ float fkey_inv(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
-constexpr int kThrThreads = 1024;
-// block-wide sum of a (count, mass) pair; every thread gets the result; fixed summation tree -> deterministic
-__device__ __forceinline__ void block_sum2(unsigned long long& cnt, unsigned long long& mass, unsigned long long* sh) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    mass += __shfl_xor_sync(0xffffffffu, mass, o);
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();  // sh reuse across calls
-  if (l == 0) { sh[2 * w] = cnt; sh[2 * w + 1] = mass; }
-  __syncthreads();
-  cnt = sh[2 * l];
-  mass = sh[2 * l + 1];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    mass += __shfl_xor_sync(0xffffffffu, mass, o);
-  }
+
+// ---- rows of the vocabulary, one cluster of kVocCtas blocks per row ----
+// Both kernels below look at a row many times (bisection passes, arg-max rounds).  One block per row left most SMs idle and read
+// 0.5 MB through one SM's L1 per pass; here every block keeps an eighth of the row in shared memory, passes run on the slices and
+// what they find meets through distributed shared memory, one cluster barrier per pass.  Rows whose slices do not fit
+// (vocabularies above 400k) are read from global memory instead (SM = false).
+constexpr int kVocCtas = 8, kVocThreads = 512, kVocWarps = kVocThreads / 32;
+constexpr int kVocSmemFloats = 50000;  // largest slice kept on chip (200 KB)
+__host__ __device__ inline int voc_slice(int V) { return ((V + kVocCtas - 1) / kVocCtas + 3) & ~3; }
+
+__device__ __forceinline__ void voc_sync() {  // (the aligned barrier wants converged warps)
+  __syncwarp();
+  cluster_sync_all();
 }
-// One block per row. Result thr[b]: tokens with logit < thr[b] are excluded from sampling (-inf: keep all).
-//   top-k : the largest threshold that keeps >= k tokens (ties at the k-th value are all kept)
-//   top-p : applied to the top-k survivors: the smallest set of most-probable tokens whose softmax(logits/T) mass
-//           reaches p of the survivors' mass
-// Both are bisections over the ordered 32-bit key space (at most 32 passes over an L2-resident row each, usually ~18:
-// the search stops as soon as one more step cannot change the kept set).  Probability mass is accumulated in 2^-32 fixed
-// point so the result does not depend on summation order.
-__global__ void __launch_bounds__(kThrThreads)
-sample_threshold_kernel(const float* __restrict__ logits, int ldl, const float* __restrict__ temperature,
-                        const int32_t* __restrict__ top_k, const float* __restrict__ top_p, float* __restrict__ thr, int V) {
-  __shared__ unsigned long long sh[64];
-  __shared__ float smax[32];
-  pdl_launch_dependents();
-  pdl_wait();
-  const int b = blockIdx.x;
-  const float temp = temperature ? temperature[b] : 0.f;
-  const int k = top_k ? top_k[b] : 0;
-  const float p = top_p ? top_p[b] : 1.f;
-  const bool use_k = k > 0 && k < V, use_p = p > 0.f && p < 1.f;
-  if (!(temp > 0.f) || (!use_k && !use_p)) {  // greedy rows and unfiltered rows
-    if (threadIdx.x == 0) thr[b] = -INFINITY;
-    return;
-  }
-  const float* row = logits + (size_t)b * ldl;
-  // row max (for the softmax weights)
-  float mx = -INFINITY;
-  for (int v = threadIdx.x; v < V; v += kThrThreads) mx = fmaxf(mx, row[v]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = mx;
-  __syncthreads();
-  mx = smax[threadIdx.x & 31];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const float inv_t = 1.f / temp;
-  // (count, mass) of the tokens whose key is >= `key`
-  auto tally = [&](uint32_t key, unsigned long long& cnt, unsigned long long& mass) {
-    cnt = 0;
-    mass = 0;
-    for (int v = threadIdx.x; v < V; v += kThrThreads) {
-      const float x = row[v];
-      if (fkey(x) >= key) {
-        cnt += 1;
-        mass += (unsigned long long)(__expf((x - mx) * inv_t) * 4294967296.0f);
-      }
-    }
-    block_sum2(cnt, mass, sh);
-  };
-  unsigned long long lo = 0, hi = 1ull << 32;  // keys; invariant: keeping [lo, ..) is enough, keeping [hi, ..) is not
-  unsigned long long c_lo = V, c_hi = 0, m_lo = 0, c, m;
-  if (use_k) {
-    while (hi - lo > 1 && c_lo != (unsigned long long)k) {
-      const unsigned long long mid = (lo + hi) >> 1;
-      tally((uint32_t)mid, c, m);
-      if (c >= (unsigned long long)k) { lo = mid; c_lo = c; } else { hi = mid; c_hi = c; }
-    }
-  }
-  if (use_p) {
-    tally((uint32_t)lo, c_lo, m_lo);  // mass of the top-k survivors (of the whole row without top-k)
-    unsigned long long target = (unsigned long long)((double)p * (double)m_lo);
-    if (target < 1) target = 1;
-    hi = 1ull << 32;
-    c_hi = 0;
-    while (hi - lo > 1 && c_lo - c_hi > 1) {
-      const unsigned long long mid = (lo + hi) >> 1;
-      tally((uint32_t)mid, c, m);
-      if (m >= target) { lo = mid; c_lo = c; } else { hi = mid; c_hi = c; }
-    }
-  }
-  if (threadIdx.x == 0) thr[b] = lo == 0 ? -INFINITY : fkey_inv((uint32_t)lo);
+template <typename T>
+__device__ __forceinline__ T* cluster_ptr(T* p, uint32_t cta) {  // the same shared-memory object in another block of the cluster
+  uint64_t r;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t>(p)), "r"(cta));
+  return reinterpret_cast<T*>(r);
 }
 
-// stage 1: grid (chunks, B): per-chunk argmax of logits/T + Gumbel noise -> part[b][chunk]
-__global__ void __launch_bounds__(256)
-sample_stage1_kernel(const float* __restrict__ logits, int ldl, const float* __restrict__ temperature,
-                     const uint64_t* __restrict__ seed, const float* __restrict__ thr, float* __restrict__ part_val,
-                     int* __restrict__ part_idx, int V) {
-  __shared__ float sval[8];
-  __shared__ int sidx[8];
+// f(i, values, how many of them exist) for every group of four columns i .. i + 3 of a slice of n that a thread keeps; eight groups are
+// in flight per thread (one at a time left the load at the latency of eight round trips)
+template <typename F>
+__device__ __forceinline__ void load_slice(const float* __restrict__ src, int n, int tid, F&& f) {
+  constexpr int kAhead = 8, kStep = kVocThreads * 4;
+  const bool vec = ((uintptr_t)src & 15) == 0;
+  for (int i0 = tid * 4; i0 < n; i0 += kStep * kAhead) {
+    float v[kAhead][4];
+#pragma unroll
+    for (int g = 0; g < kAhead; ++g) {
+      const int i = i0 + g * kStep;
+      if (vec && i + 4 <= n) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(src + i));
+        v[g][0] = t.x; v[g][1] = t.y; v[g][2] = t.z; v[g][3] = t.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[g][e] = i + e < n ? __ldg(src + i + e) : 0.f;
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < kAhead; ++g) {
+      const int i = i0 + g * kStep;
+      if (i < n) f(i, v[g], min(4, n - i));
+    }
+  }
+}
+
+// ---- sampling: greedy / temperature (Gumbel-max), optionally from the top-k / top-p survivors ----
+// The threshold that separates the survivors is found on the ordered 32-bit keys:
+//   top-k : the largest key that keeps >= k tokens (ties at the k-th value are all kept)
+//   top-p : among the top-k survivors, the largest key whose tokens' softmax(logits/T) mass reaches p of the survivors' mass
+// Probability mass is accumulated in 2^-32 fixed point, so every sum is exact and independent of its order.  A pass compares a
+// slice with three keys inside the interval that still holds the answer; once the interval holds at most kFin tokens, block 0
+// gets them and finds the answer directly.
+// Measured (32 rows x 128256, mixed top-k / top-p): 1100 us with a block per row and up to 32 + 32 one-key passes, 73 us now.
+constexpr int kFin = 256;
+struct SampleShared {
+  unsigned long long part[2][5];  // this block's totals of a pass: counts (c1 | c2 << 32), c3, masses m1 .. m3
+  unsigned long long wred[kVocWarps][5];
+  uint32_t list[kFin];
+  unsigned long long mass[kFin];
+  float val[kVocWarps];
+  int idx[kVocWarps];
+  uint32_t n_list, result;
+  float best_val, row_max;
+  int best_idx;
+};
+
+template <bool SM>
+__global__ void __cluster_dims__(kVocCtas, 1, 1) __launch_bounds__(kVocThreads)
+sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict__ temperature, const uint64_t* __restrict__ seed,
+              const int32_t* __restrict__ top_k, const float* __restrict__ top_p, int32_t* __restrict__ out, int V) {
+  extern __shared__ __align__(16) uint32_t keys[];
+  __shared__ SampleShared sh;
   pdl_launch_dependents();
   pdl_wait();
-  const int b = blockIdx.y, chunk = blockIdx.x;
-  const float* row = logits + (size_t)b * ldl;
+  typedef unsigned long long u64;
+  const int b = blockIdx.x / kVocCtas, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = cluster_ctarank();
+  const int per = voc_slice(V), start = min(V, (int)rank * per), n = min(V, start + per) - start;
+  const float* row = logits + (size_t)b * ldl + start;
   const float temp = temperature ? temperature[b] : 0.f;
   const bool greedy = !(temp > 0.f);
   const float inv_t = greedy ? 1.f : 1.f / temp;
-  const uint64_t sd = seed ? seed[b] : 0;
-  const float floor_logit = (thr && !greedy) ? thr[b] : -INFINITY;  // top-k / top-p survivors only
+  const int k = top_k ? top_k[b] : 0;
+  const float p = top_p ? top_p[b] : 1.f;
+  const bool use_k = !greedy && k > 0 && k < V, use_p = !greedy && p > 0.f && p < 1.f;
+
+  if (tid == 0) sh.n_list = 0;
+  float mx = -INFINITY;
+  if constexpr (SM) {  // (entries behind the slice's end read as key 0, below every float's key)
+    load_slice(row, n, tid, [&](int i, const float (&f)[4], int have) {
+      uint32_t q[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        mx = fmaxf(mx, e < have ? f[e] : -INFINITY);
+        q[e] = e < have ? fkey(f[e]) : 0u;
+      }
+      *reinterpret_cast<uint4*>(keys + i) = make_uint4(q[0], q[1], q[2], q[3]);
+    });
+  } else if (use_k || use_p) {
+    for (int i = tid; i < n; i += kVocThreads) mx = fmaxf(mx, __ldg(row + i));
+  }
+  __syncthreads();
+  auto scan = [&](auto&& f) {  // f(key, index inside the slice)
+    if constexpr (SM) {
+      for (int i = tid * 4; i < n; i += kVocThreads * 4) {
+        const uint4 q = *reinterpret_cast<const uint4*>(keys + i);
+        f(q.x, i);
+        f(q.y, i + 1);
+        f(q.z, i + 2);
+        f(q.w, i + 3);
+      }
+    } else {
+      for (int i = tid; i < n; i += kVocThreads) f(fkey(__ldg(row + i)), i);
+    }
+  };
+
+  float floor_logit = -INFINITY;
+  if (use_k || use_p) {
+    // row maximum (for the softmax weights)
+    const uint32_t wm = __reduce_max_sync(0xffffffffu, fkey(mx));
+    if (lane == 0) sh.val[warp] = fkey_inv(wm);
+    __syncthreads();
+    mx = sh.val[lane & (kVocWarps - 1)];
+    mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(mx)));
+    if (tid == 0) sh.row_max = mx;
+    voc_sync();
+    mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(*cluster_ptr(&sh.row_max, lane & (kVocCtas - 1)))));
+
+    auto weight = [&](uint32_t key) -> u64 {
+      const float e = __expf((fkey_inv(key) - mx) * inv_t) * 4294967296.0f;
+      return e >= 0.f ? (u64)e : 0;  // a NaN logit carries no mass
+    };
+    int turn = 0;
+    // sums of the cluster's blocks, in every thread of every block
+    auto warp_total = [](u64 v) -> u64 {  // (a thread's share is below 2^58: three limbs, one hardware reduction each)
+      const u64 a = __reduce_add_sync(0xffffffffu, (uint32_t)v & 0xffffu), c = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 16) & 0x1fffffu),
+                d = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 37));
+      return a + (c << 16) + (d << 37);
+    };
+    auto cluster_sum = [&](u64 (&v)[5]) {
+#pragma unroll
+      for (int j = 0; j < 5; ++j) {
+        const u64 t = j == 0 ? (u64)__reduce_add_sync(0xffffffffu, (uint32_t)v[0]) | (u64)__reduce_add_sync(0xffffffffu, (uint32_t)(v[0] >> 32)) << 32
+                      : j == 1 ? (u64)__reduce_add_sync(0xffffffffu, (uint32_t)v[1]) : warp_total(v[j]);
+        if (lane == 0) sh.wred[warp][j] = t;
+      }
+      __syncthreads();
+      if (warp == 0) {
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+          u64 t = lane < kVocWarps ? sh.wred[lane][j] : 0;
+#pragma unroll
+          for (int o = kVocWarps / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+          if (lane == 0) sh.part[turn][j] = t;
+        }
+      }
+      voc_sync();
+#pragma unroll
+      for (int j = 0; j < 5; ++j) {
+        u64 t = *cluster_ptr(&sh.part[turn][j], lane & (kVocCtas - 1));
+#pragma unroll
+        for (int o = kVocCtas / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        v[j] = t;
+      }
+      turn ^= 1;  // (a slot is written again two passes later, behind the barrier that follows every read of it)
+    };
+    // the largest key whose tokens (those with keys >= it) reach `goal`: in number, or in mass (by_mass).  Keeping [lo, ..) is
+    // enough (c_lo tokens), keeping [hi, ..) is not (c_hi tokens of mass m_hi).
+    auto search = [&](bool by_mass, u64 goal, u64 lo, u64 c_lo) -> u64 {
+      u64 hi = 1ull << 32, c_hi = 0, m_hi = 0;
+      for (int pass = 0; hi - lo > 1 && c_lo - c_hi > (u64)kFin; ++pass) {
+        // Logits are spread more evenly over values than over keys (where half of all keys are exponents nothing has): the first
+        // pass looks a few temperatures below the maximum, the next ones divide the values between the bounds; from the eighth
+        // on the keys are divided, so at most 8 + 16 passes are needed.
+        const u64 d = hi - lo;
+        u64 t[3];
+        const float flo = fkey_inv((uint32_t)lo), fhi = fkey_inv((uint32_t)(hi - 1));
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const float at = pass == 0 ? mx - temp * (j == 0 ? 16.f : j == 1 ? 8.f : 4.f) : flo + (fhi - flo) * (0.25f * (j + 1));
+          const u64 by_key = lo + max(1ull, j == 0 ? d / 4 : j == 1 ? d / 2 : d / 4 * 3);
+          t[j] = (pass < 8 && at - at == 0.f) ? min(max((u64)fkey(at), lo + 1), hi - 1) : by_key;
+        }
+        t[1] = max(t[1], t[0]);
+        t[2] = max(t[2], t[1]);
+        u64 v[5] = {0, 0, 0, 0, 0};
+        const uint32_t t1 = (uint32_t)t[0], t2 = (uint32_t)t[1], t3 = (uint32_t)t[2];
+        if (by_mass) {
+          scan([&](uint32_t q, int) {
+            if (q < t1) return;
+            const u64 w = weight(q);
+            v[0] += q >= t2 ? 0x100000001ull : 1ull;
+            v[2] += w;
+            if (q >= t2) v[3] += w;
+            if (q >= t3) { v[1] += 1; v[4] += w; }
+          });
+        } else {
+          uint32_t c1 = 0, c2 = 0, c3 = 0;
+          scan([&](uint32_t q, int) {
+            c1 += q >= t1;
+            c2 += q >= t2;
+            c3 += q >= t3;
+          });
+          v[0] = c1 | (u64)c2 << 32;
+          v[1] = c3;
+        }
+        cluster_sum(v);
+        const u64 c[3] = {v[0] & 0xffffffffull, v[0] >> 32, v[1]}, m[3] = {v[2], v[3], v[4]};
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          if ((by_mass ? m[j] : c[j]) >= goal) {
+            lo = t[j];
+            c_lo = c[j];
+          } else {
+            hi = t[j];
+            c_hi = c[j];
+            m_hi = m[j];
+            break;
+          }
+        }
+      }
+      if (hi - lo <= 1) return lo;
+      // few tokens left: block 0 decides
+      scan([&](uint32_t q, int) {
+        if (q < lo || (u64)q >= hi || q == 0) return;
+        cluster_ptr(sh.list, 0)[atomicAdd(cluster_ptr(&sh.n_list, 0), 1u)] = q;
+      });
+      voc_sync();
+      if (rank == 0) {
+        const int nl = (int)sh.n_list;
+        for (int i = tid; i < nl; i += kVocThreads) sh.mass[i] = weight(sh.list[i]);
+        __syncthreads();
+        const int cand = tid >> 1;
+        const uint32_t key = cand < nl ? sh.list[cand] : 0u;
+        u64 c = 0, m = 0;
+        for (int j = tid & 1; j < nl; j += 2)
+          if (sh.list[j] >= key) {
+            c += 1;
+            m += sh.mass[j];
+          }
+        c += __shfl_xor_sync(0xffffffffu, c, 1);
+        m += __shfl_xor_sync(0xffffffffu, m, 1);
+        const bool ok = cand < nl && (by_mass ? m_hi + m : c_hi + c) >= goal;
+        const uint32_t wk = __reduce_max_sync(0xffffffffu, ok ? key : 0u);
+        if (lane == 0) sh.idx[warp] = (int)wk;
+        __syncthreads();
+        if (warp == 0) {
+          const uint32_t r = __reduce_max_sync(0xffffffffu, (uint32_t)sh.idx[lane & (kVocWarps - 1)]);
+          if (lane < kVocCtas) *cluster_ptr(&sh.result, lane) = r;
+          if (lane == 0) sh.n_list = 0;
+        }
+      }
+      voc_sync();
+      return sh.result > lo ? sh.result : lo;
+    };
+    u64 lo = 0;
+    if (use_k) lo = search(false, (u64)k, 0, (u64)V);
+    if (use_p) {
+      u64 v[5] = {0, 0, 0, 0, 0};  // tokens and mass of the top-k survivors (of the whole row without top-k)
+      scan([&](uint32_t q, int i) {
+        if (i < n && q >= lo) {
+          v[0] += 1;
+          v[2] += weight(q);
+        }
+      });
+      cluster_sum(v);
+      u64 target = (u64)((double)p * (double)v[2]);
+      if (target < 1) target = 1;
+      lo = search(true, target, lo, v[0]);
+    }
+    if (lo > 0) floor_logit = fkey_inv((uint32_t)lo);
+  }
+
   float best = -INFINITY;
   int bi = 0x7fffffff;
-  const int v_end = min(V, (chunk + 1) * kSampleChunk);
-  for (int v = chunk * kSampleChunk + threadIdx.x; v < v_end; v += 256) {
-    const float raw = row[v];
-    if (raw < floor_logit) continue;
+  const uint64_t sd = seed ? seed[b] : 0;
+  scan([&](uint32_t q, int i) {
+    if (i >= n) return;
+    const float raw = fkey_inv(q);
+    if (raw < floor_logit) return;
+    const int v = start + i;
     float x = raw * inv_t;
     if (!greedy) {
       const uint64_t h = mix64(sd ^ (0xD1B54A32D192ED03ull * (uint64_t)(v + 1)));
@@ -451,31 +595,29 @@ sample_stage1_kernel(const float* __restrict__ logits, int ldl, const float* __r
       const float u = ((float)(h >> 41) + 0.5f) * (1.0f / 8388608.0f);
       x += -__logf(-logf(u));
     }
-    if (x > best || (x == best && v < bi)) { best = x; bi = v; }
-  }
-  block_argmax<256>(best, bi, sval, sidx);
-  if (threadIdx.x == 0) {
-    part_val[b * gridDim.x + chunk] = best;
-    part_idx[b * gridDim.x + chunk] = bi;
-  }
-}
-// stage 2: one warp per row merges the chunk winners (lowest index wins ties, as in stage 1)
-__global__ void __launch_bounds__(32)
-sample_stage2_kernel(const float* __restrict__ part_val, const int* __restrict__ part_idx, int32_t* __restrict__ out,
-                     int chunks) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int b = blockIdx.x;
-  float best = -INFINITY;
-  int bi = 0x7fffffff;
-  for (int c = threadIdx.x; c < chunks; c += 32) argmax_merge(best, bi, part_val[b * chunks + c], part_idx[b * chunks + c]);
+    argmax_merge(best, bi, x, v);
+  });
+  // lowest index wins ties, in whatever order the blocks' winners are merged
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, o);
     const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
     argmax_merge(best, bi, ov, oi);
   }
-  if (threadIdx.x == 0) out[b] = bi < 0x7fffffff ? bi : 0;  // all-NaN row: emit a valid id, never an out-of-range one
+  __syncthreads();
+  if (lane == 0) { sh.val[warp] = best; sh.idx[warp] = bi; }
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < kVocWarps; ++w) argmax_merge(best, bi, sh.val[w], sh.idx[w]);
+    sh.best_val = best;
+    sh.best_idx = bi;
+  }
+  voc_sync();
+  if (rank == 0 && tid == 0) {
+    for (int c = 1; c < kVocCtas; ++c) argmax_merge(best, bi, *cluster_ptr(&sh.best_val, c), *cluster_ptr(&sh.best_idx, c));
+    out[b] = bi < 0x7fffffff ? bi : 0;  // all-NaN row: emit a valid id, never an out-of-range one
+  }
+  voc_sync();  // no block's shared memory goes away while block 0 reads it
 }
 
 // ---- OpenAI presence / frequency penalties: logits[b, tok] -= val for the (tok, val) entries of row b ----
@@ -495,63 +637,170 @@ apply_penalties_kernel(float* __restrict__ logits, int ldl, const int32_t* __res
 }
 
 // ---- log-probabilities of the sampled token and of the width-1 most likely tokens (descending, lowest id on ties) ----
-constexpr int kLpThreads = 1024;
-__global__ void __launch_bounds__(kLpThreads)
+// Every block picks the width-1 best of its slice (a thread remembers the best of its own entries; after a round only the entries
+// of the thread that owned the winner are looked at again, by its whole warp), block 0 merges the eight short lists by rank.
+// Measured (32 rows x 128256, width 6): 69 us with a block per row that read it once per pick, 16 us now.
+constexpr int kLpMax = 32;  // picks per merge; wider records take several
+struct LpShared {
+  uint32_t wkey[2][kVocWarps];
+  int widx[2][kVocWarps];
+  uint32_t top_key[kLpMax];
+  int top_idx[kLpMax];
+  uint32_t all_key[kVocCtas * kLpMax];
+  int all_idx[kVocCtas * kLpMax];
+  float red[kVocWarps];
+  float part_max, part_sum;
+  uint32_t last_key;
+  int last_idx;
+};
+template <bool SM>
+__global__ void __cluster_dims__(kVocCtas, 1, 1) __launch_bounds__(kVocThreads)
 logprob_topk_kernel(const float* __restrict__ logits, int ldl, int V, const int32_t* __restrict__ sampled,
-                    const int32_t* __restrict__ width, int32_t* __restrict__ out_ids, float* __restrict__ out_lp,
-                    int max_width) {
-  __shared__ float sval[kLpThreads / 32];
-  __shared__ int sidx[kLpThreads / 32];
-  __shared__ float red[kLpThreads / 32];
-  __shared__ float s_bv;
-  __shared__ int s_bi;
+                    const int32_t* __restrict__ width, int32_t* __restrict__ out_ids, float* __restrict__ out_lp, int max_width) {
+  extern __shared__ __align__(16) float slice[];
+  __shared__ LpShared sh;
   pdl_launch_dependents();
   pdl_wait();
-  const int b = blockIdx.x;
+  const int b = blockIdx.x / kVocCtas, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int w = min(width[b], max_width);
-  if (w <= 0) return;
+  if (w <= 0) return;  // (the whole cluster)
+  const int picks = min(w - 1, kLpMax);
+  const uint32_t rank = cluster_ctarank();
+  const int per = voc_slice(V), start = min(V, (int)rank * per), n = min(V, start + per) - start;
   const float* row = logits + (size_t)b * ldl;
-  float best = -INFINITY;
+  const float* src = row + start;
+  constexpr int kStep = kVocThreads * 4;  // a thread's entries: columns 4 tid .. 4 tid + 3 of every kStep
+  float mx = -INFINITY;
+  uint32_t bk = 0;  // best of this thread's entries in the order (value descending, index ascending); NaN is never picked, zeros tie
   int bi = 0x7fffffff;
-  for (int v = threadIdx.x; v < V; v += kLpThreads) argmax_merge(best, bi, row[v], v);
-  block_argmax<kLpThreads>(best, bi, sval, sidx);
-  if (threadIdx.x == 0) { s_bv = best; s_bi = bi; }
-  __syncthreads();
-  const float mx = s_bv;
+  auto as_key = [](float x) -> uint32_t {
+    const float y = x + 0.f;
+    return y == y ? fkey(y) : 0u;
+  };
+  load_slice(src, n, tid, [&](int i, const float (&f)[4], int have) {
+    float4 v = make_float4(f[0], have > 1 ? f[1] : -INFINITY, have > 2 ? f[2] : -INFINITY, have > 3 ? f[3] : -INFINITY);
+    if (SM) *reinterpret_cast<float4*>(slice + i) = v;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (e >= have) break;
+      mx = fmaxf(mx, f[e]);
+      const uint32_t q = as_key(f[e]);
+      if (q > bk) { bk = q; bi = start + i + e; }
+    }
+  });
+  // the best entry of thread t0 behind (key, index), found by its whole warp
+  auto next_best = [&](int t0, uint32_t after_key, int after_idx, uint32_t& k_out, int& i_out) {
+    uint32_t k1 = 0;
+    int i1 = 0x7fffffff;
+    for (int i = t0 * 4 + (lane & 3) + (lane >> 2) * kStep; i < n; i += 8 * kStep) {
+      const uint32_t q = as_key(SM ? slice[i] : __ldg(src + i));
+      if (q > after_key || (q == after_key && start + i <= after_idx)) continue;
+      if (q > k1) { k1 = q; i1 = start + i; }
+    }
+    __syncwarp();
+    k_out = __reduce_max_sync(0xffffffffu, k1);
+    i_out = __reduce_min_sync(0xffffffffu, k1 == k_out ? i1 : 0x7fffffff);
+  };
+  auto block_max = [&](float v) {
+    v = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(v)));
+    if (lane == 0) sh.red[warp] = v;
+    __syncthreads();
+    return fkey_inv(__reduce_max_sync(0xffffffffu, fkey(sh.red[lane & (kVocWarps - 1)])));
+  };
+  mx = block_max(mx);
+  if (tid == 0) sh.part_max = mx;
+  voc_sync();
+  mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(*cluster_ptr(&sh.part_max, lane & (kVocCtas - 1)))));
   float se = 0.f;
-  for (int v = threadIdx.x; v < V; v += kLpThreads) se += expf(row[v] - mx);
-  se = block_sum<kLpThreads>(se, red);
-  const float lse = mx + logf(se);
+  if constexpr (SM) {
+#pragma unroll 4
+    for (int i = tid * 4; i < n; i += kStep) {
+      const float4 v = *reinterpret_cast<const float4*>(slice + i);
+      se += (expf(v.x - mx) + expf(v.y - mx)) + (expf(v.z - mx) + expf(v.w - mx));
+    }
+  } else {
+    for (int i0 = tid * 4; i0 < n; i0 += kStep)
+      for (int i = i0; i < min(n, i0 + 4); ++i) se += expf(__ldg(src + i) - mx);
+  }
+  se = warp_sum(se);
+  if (lane == 0) sh.red[warp] = se;
+  __syncthreads();
+  if (warp == 0) {
+    se = warp_sum(lane < kVocWarps ? sh.red[lane] : 0.f);
+    if (lane == 0) sh.part_sum = se;
+  }
+  voc_sync();
+  float sum = 0.f;
+  for (int c = 0; c < kVocCtas; ++c) sum += *cluster_ptr(&sh.part_sum, c);
+  const float lse = mx + logf(sum);
   int32_t* ids = out_ids + (size_t)b * max_width;
   float* lps = out_lp + (size_t)b * max_width;
-  if (threadIdx.x == 0) {
+  if (rank == 0 && tid == 0) {
     const int t = sampled[b];
     ids[0] = t;
     lps[0] = (t >= 0 && t < V) ? row[t] - lse : -INFINITY;
   }
-  float pv = s_bv;   // the j-th most likely token in the order (value desc, id asc); j = 1 is the argmax found above
-  int pi = s_bi;
-  for (int j = 1; j < w; ++j) {
-    if (threadIdx.x == 0) { ids[j] = pi; lps[j] = pv - lse; }
-    if (j + 1 == w) break;
-    best = -INFINITY;
-    bi = 0x7fffffff;
-    for (int v = threadIdx.x; v < V; v += kLpThreads) {
-      const float x = row[v];
-      if (x < pv || (x == pv && v > pi)) argmax_merge(best, bi, x, v);  // strictly after the previous pick
+  for (int base = 0; base < w - 1; base += kLpMax) {
+    const int picks = min(w - 1 - base, kLpMax);
+    if (base > 0) {  // (a thread's own best may have been picked or lie behind the last pick: look again)
+      for (int l = 0; l < 32; ++l) {
+        uint32_t k1;
+        int i1;
+        next_best(warp * 32 + l, sh.last_key, sh.last_idx, k1, i1);
+        if (lane == l) { bk = k1; bi = i1; }
+      }
     }
-    __syncthreads();  // sval/sidx reuse
-    block_argmax<kLpThreads>(best, bi, sval, sidx);
-    if (threadIdx.x == 0) { s_bv = best; s_bi = bi; }
-    __syncthreads();
-    pv = s_bv;
-    pi = s_bi;
-    if (pi == 0x7fffffff) {  // fewer than `w` finite logits in the row
-      if (threadIdx.x == 0)
-        for (int k = j + 1; k < w; ++k) { ids[k] = -1; lps[k] = -INFINITY; }
-      break;
+    for (int r = 0; r < picks; ++r) {
+      const uint32_t wk = __reduce_max_sync(0xffffffffu, bk);
+      const int wi = __reduce_min_sync(0xffffffffu, bk == wk ? bi : 0x7fffffff);
+      if (lane == 0) { sh.wkey[r & 1][warp] = wk; sh.widx[r & 1][warp] = wi; }
+      __syncthreads();
+      const uint32_t ck = sh.wkey[r & 1][lane & (kVocWarps - 1)];
+      const int ci = sh.widx[r & 1][lane & (kVocWarps - 1)];
+      const uint32_t gk = __reduce_max_sync(0xffffffffu, ck);
+      const int gi = __reduce_min_sync(0xffffffffu, ck == gk ? ci : 0x7fffffff);
+      if (tid == 0) { sh.top_key[r] = gk; sh.top_idx[r] = gi; }
+      const uint32_t mine = __ballot_sync(0xffffffffu, bi == gi && gi != 0x7fffffff);
+      if (mine) {
+        uint32_t k1;
+        int i1;
+        next_best(warp * 32 + __ffs(mine) - 1, gk, gi, k1, i1);
+        if (mine >> lane & 1) { bk = k1; bi = i1; }
+      }
     }
+    voc_sync();
+    if (rank == 0) {
+      const int all = kVocCtas * picks;
+      for (int e = tid; e < all; e += kVocThreads) {
+        sh.all_key[e] = cluster_ptr(sh.top_key, e / picks)[e % picks];
+        sh.all_idx[e] = cluster_ptr(sh.top_idx, e / picks)[e % picks];
+      }
+      __syncthreads();
+      for (int e = tid; e < all; e += kVocThreads) {
+        const uint32_t q = sh.all_key[e];
+        const int i = sh.all_idx[e];
+        int better = 0;
+        for (int j = 0; j < all; ++j) {
+          const uint32_t oq = sh.all_key[j];
+          const int oi = sh.all_idx[j];
+          better += oq > q || (oq == q && (oi < i || (oi == i && j < e)));
+        }
+        if (better < picks) {
+          const int at = base + better;
+          const bool none = i == 0x7fffffff;  // fewer than `w` tokens to name
+          ids[1 + at] = none && at > 0 ? -1 : i;
+          lps[1 + at] = none ? (at > 0 ? -INFINITY : mx - lse) : fkey_inv(q) - lse;
+        }
+        if (better == picks - 1)
+          for (int c = 0; c < kVocCtas; ++c) {
+            *cluster_ptr(&sh.last_key, c) = q;
+            *cluster_ptr(&sh.last_idx, c) = i;
+          }
+      }
+    }
+    voc_sync();
   }
+  voc_sync();  // no block's shared memory goes away while another one reads it
 }
 
 __global__ void __launch_bounds__(kRowThreads)
@@ -620,26 +869,24 @@ cudaError_t rope_kv_write(cudaStream_t s, bf16* qkv, const int32_t* positions, c
                                                          Hkv, D, page_size);
   return cudaGetLastError();
 }
-size_t sample_scratch_bytes(int B, int V) { return (size_t)B * ((V + kSampleChunk - 1) / kSampleChunk) * 8 + (size_t)B * 4; }
-
-cudaError_t sample_tokens(cudaStream_t s, const float* logits, int ldl, const float* temperature, const uint64_t* seed,
-                          int32_t* out, int B, int V, void* scratch, const int32_t* top_k, const float* top_p) {
-  if (B <= 0) return cudaSuccess;
-  const int chunks = (V + kSampleChunk - 1) / kSampleChunk;
-  float* pv = static_cast<float*>(scratch);
-  int* pi = reinterpret_cast<int*>(pv + (size_t)B * chunks);
-  float* thr = nullptr;
-  cudaError_t e;
-  if (temperature && (top_k || top_p)) {  // rows that ask for neither leave the kernel at once
-    thr = reinterpret_cast<float*>(pi + (size_t)B * chunks);
-    e = launch_k(sample_threshold_kernel, dim3(B), dim3(kThrThreads), 0, s, true, logits, ldl, temperature, top_k, top_p,
-                 thr, V);
+namespace {
+// dynamic shared memory of the vocabulary kernels: a slice when it fits, nothing otherwise (the SM = false instances).  The opt-in is
+// per device and costs well under a microsecond, so it rides with every launch: callers need no initialisation call.
+template <typename K, typename... Args>
+cudaError_t launch_voc(K* on_chip, K* in_memory, cudaStream_t s, int B, int V, Args... args) {
+  const size_t floats = (size_t)voc_slice(V);
+  const bool fits = floats <= (size_t)kVocSmemFloats;
+  if (fits) {
+    const cudaError_t e = cudaFuncSetAttribute(on_chip, cudaFuncAttributeMaxDynamicSharedMemorySize, kVocSmemFloats * 4);
     if (e != cudaSuccess) return e;
   }
-  e = launch_k(sample_stage1_kernel, dim3(chunks, B), dim3(256), 0, s, true, logits, ldl, temperature, seed,
-               (const float*)thr, pv, pi, V);
-  if (e != cudaSuccess) return e;
-  return launch_k(sample_stage2_kernel, dim3(B), dim3(32), 0, s, true, (const float*)pv, (const int*)pi, out, chunks);
+  return launch_k(fits ? on_chip : in_memory, dim3(B * kVocCtas), dim3(kVocThreads), fits ? floats * 4 : 0, s, true, args...);
+}
+}  // namespace
+cudaError_t sample_tokens(cudaStream_t s, const float* logits, int ldl, const float* temperature, const uint64_t* seed,
+                          int32_t* out, int B, int V, const int32_t* top_k, const float* top_p) {
+  if (B <= 0) return cudaSuccess;
+  return launch_voc(sample_kernel<true>, sample_kernel<false>, s, B, V, logits, ldl, temperature, seed, top_k, top_p, out, V);
 }
 cudaError_t apply_penalties(cudaStream_t s, float* logits, int ldl, const int32_t* pen_off, const void* pen, int B, int V) {
   if (B <= 0) return cudaSuccess;
@@ -648,8 +895,8 @@ cudaError_t apply_penalties(cudaStream_t s, float* logits, int ldl, const int32_
 cudaError_t logprob_topk(cudaStream_t s, const float* logits, int ldl, int V, const int32_t* sampled, const int32_t* width,
                          int32_t* out_ids, float* out_lp, int B, int max_width) {
   if (B <= 0) return cudaSuccess;
-  return launch_k(logprob_topk_kernel, dim3(B), dim3(kLpThreads), 0, s, true, logits, ldl, V, sampled, width, out_ids,
-                  out_lp, max_width);
+  return launch_voc(logprob_topk_kernel<true>, logprob_topk_kernel<false>, s, B, V, logits, ldl, V, sampled, width, out_ids, out_lp,
+                    max_width);
 }
 cudaError_t cls_pool_l2(cudaStream_t s, const bf16* x, const int32_t* first_row, float* out, int B, int H) {
   if (B <= 0) return cudaSuccess;
