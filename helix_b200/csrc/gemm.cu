@@ -265,6 +265,13 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t aphase = (it >> 1) & 1;
       const int m0 = mi * TILE_M + (int)cta_rank * BLOCK_M;
       const int n_out0 = ni * OUT_BN;
+      if constexpr (kResid) {  // the first residual chunk travels while the products finish
+        if (leader && grp < NCHUNK) {
+          tma_store_wait_read<0>();
+          mbar_arrive_expect_tx(my_resid_bar, kStagingBytes);
+          tma_load_2d(buf, &map_r, my_resid_bar, n_out0 + grp * CHUNK_COLS, m0, kEvictFirst);
+        }
+      }
       mbar_wait(&tmem_full[as], aphase);
       tc_fence_after();
       const uint32_t t_tile = tmem_base + as * BN + (static_cast<uint32_t>(q * 32) << 16);
@@ -361,8 +368,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll 1
       for (int c = grp; c < NCHUNK; c += 2) {
         if (leader) {
-          tma_store_wait_read<0>();  // this group's previous store is done reading `buf`
-          if (kResid) {
+          if (!kResid || c != grp) tma_store_wait_read<0>();  // this group's previous store is done reading `buf`
+          if (kResid && c != grp) {
             mbar_arrive_expect_tx(my_resid_bar, kStagingBytes);
             tma_load_2d(buf, &map_r, my_resid_bar, n_out0 + c * CHUNK_COLS, m0, kEvictFirst);
           }
@@ -555,23 +562,48 @@ bool use_pair() {  // HB_GEMM_2CTA=0 falls back to single-CTA tiles (A/B measure
 
 template <int EPI>
 cudaError_t launch_epi(cudaStream_t stream, const GemmArgs& g, int num_sms) {
-  int bn = g.block_n;
+  constexpr bool kWideOnly = EPI == EPI_SWIGLU || EPI == EPI_GEGLU || EPI == EPI_CLAMPGLU || EPI == EPI_ROPE;
+  const bool pairs = use_pair() && !g.m_tile_group;
+  int bn = g.block_n, cg = 1;
   if (bn == 0) {
-    // Fill the machine: prefer 256-wide tiles when there are at least ~2 waves of them.
-    const int num_m = (g.M + BLOCK_M - 1) / BLOCK_M;
-    bn = 256;
-    while (bn > 64 && (long)num_m * ((g.N + bn - 1) / bn) < 2L * num_sms) bn >>= 1;
+    // The tile shape whose waves end first.  Per shape: us per 64-deep k block of one tile, the least a wave takes (its epilogue, when K
+    // is short) and the part of a launch that does not depend on K, fitted to runs on random operands:
+    //                          256 x 256 pair  256 x 128 pair  128 x 256  128 x 128  128 x 64
+    //   512 x 4096 x 14336 (R)       73.6            59.1         88.1       71.8     112.9 us
+    //  1100 x 4096 x 14336 (R)      178.4           186.1        106.3      130.6     250.5
+    //  1280 x 4096 x  4096 (R)       71.0            45.1         62.9       54.2      76.0
+    //  6000 x 10304 x 2048          199.6           228.4        202.5      263.9     415.8
+    //   600 x  768 x   768 (R)       12.3            10.2         12.3        9.1       8.2
+    // 13400 x 3072 x   768 (gelu)    63.6            79.3         72.6       83.2     124.9
+    // (R: residual epilogue.)  Narrow tiles read more operand bytes from L2 per product (24 KB per SM and block for 128 x 64, 32 KB for
+    // four times the products in a pair's 256 x 256), wide ones leave SMs without a tile.  The rule before, "halve the width until there
+    // are two waves", took 128 x 64 for the first, third and fifth line.  Every shape walks K in order: a row's result does not
+    // depend on the choice.
+    struct Shape { int bn, cg; double kb, floor, fixed; };
+    static constexpr Shape shapes[] = {{256, 2, 0.36, 5.6, 8.5}, {128, 2, 0.235, 3.4, 8.0}, {256, 1, 0.42, 6.0, 7.0}, {128, 1, 0.28, 3.9, 6.5}, {64, 1, 0.235, 3.1, 6.0}};
+    const int num_kb = (g.K + BLOCK_K - 1) / BLOCK_K;
+    double best = 1e30;
+    for (const Shape& t : shapes) {
+      if ((t.cg == 2 && (!pairs || num_sms < 2)) || (kWideOnly && t.bn != 256)) continue;
+      const long tiles = (long)((g.M + BLOCK_M * t.cg - 1) / (BLOCK_M * t.cg)) * ((g.N + t.bn - 1) / t.bn);
+      const long workers = std::max(1, num_sms / t.cg);
+      const double us = (double)((tiles + workers - 1) / workers) * std::max(num_kb * t.kb, t.floor) + t.fixed;
+      if (us < best) { best = us; bn = t.bn; cg = t.cg; }
+    }
+  } else if (bn == 256 && pairs && (long)((g.M + 255) / 256) * ((g.N + 255) / 256) >= num_sms / 2) {
+    cg = 2;  // a width asked for: CTA pairs once the problem has at least a wave of them
   }
-  switch (bn) {
-    case 256:
-      // CTA pairs (256 x 256 tiles) once the problem has at least a wave of them
-      if (use_pair() && !g.m_tile_group && (long)((g.M + 255) / 256) * ((g.N + 255) / 256) >= num_sms / 2) return launch_cfg<256, EPI, 2>(stream, g, num_sms);
-      return launch_cfg<256, EPI, 1>(stream, g, num_sms);
-    case 128:
-      if constexpr (EPI != EPI_SWIGLU && EPI != EPI_GEGLU && EPI != EPI_CLAMPGLU && EPI != EPI_ROPE) return launch_cfg<128, EPI, 1>(stream, g, num_sms);
+  switch (bn * 10 + cg) {
+    case 2562: return launch_cfg<256, EPI, 2>(stream, g, num_sms);
+    case 2561: return launch_cfg<256, EPI, 1>(stream, g, num_sms);
+    case 1282:
+      if constexpr (!kWideOnly) return launch_cfg<128, EPI, 2>(stream, g, num_sms);
       return cudaErrorInvalidValue;
-    case 64:
-      if constexpr (EPI != EPI_SWIGLU && EPI != EPI_GEGLU && EPI != EPI_CLAMPGLU && EPI != EPI_ROPE) return launch_cfg<64, EPI, 1>(stream, g, num_sms);
+    case 1281:
+      if constexpr (!kWideOnly) return launch_cfg<128, EPI, 1>(stream, g, num_sms);
+      return cudaErrorInvalidValue;
+    case 641:
+      if constexpr (!kWideOnly) return launch_cfg<64, EPI, 1>(stream, g, num_sms);
       return cudaErrorInvalidValue;
     default: return cudaErrorInvalidValue;
   }
@@ -590,6 +622,7 @@ cudaError_t set_attr_epi() {
   if ((e = set_attr<256, EPI, 2>()) != cudaSuccess) return e;
   if ((e = set_attr<256, EPI, 1>()) != cudaSuccess) return e;
   if constexpr (EPI != EPI_SWIGLU && EPI != EPI_GEGLU && EPI != EPI_CLAMPGLU && EPI != EPI_ROPE) {
+    if ((e = set_attr<128, EPI, 2>()) != cudaSuccess) return e;
     if ((e = set_attr<128, EPI, 1>()) != cudaSuccess) return e;
     return set_attr<64, EPI, 1>();
   }
@@ -641,19 +674,19 @@ cudaError_t gemm_bf16_tn(cudaStream_t stream, const GemmArgs& g) {
     case EPI_SWIGLU: {
       if (g.N % 256) return cudaErrorInvalidValue;
       GemmArgs h = g;
-      h.block_n = 256;
+      h.block_n = 0;  // (these tiles are 256 columns wide whatever is asked for)
       return launch_epi<EPI_SWIGLU>(stream, h, sms);
     }
     case EPI_GEGLU: {
       if (g.N % 256) return cudaErrorInvalidValue;
       GemmArgs h = g;
-      h.block_n = 256;
+      h.block_n = 0;  // (these tiles are 256 columns wide whatever is asked for)
       return launch_epi<EPI_GEGLU>(stream, h, sms);
     }
     case EPI_CLAMPGLU: {
       if (g.N % 256) return cudaErrorInvalidValue;
       GemmArgs h = g;
-      h.block_n = 256;
+      h.block_n = 0;  // (these tiles are 256 columns wide whatever is asked for)
       return launch_epi<EPI_CLAMPGLU>(stream, h, sms);
     }
     case EPI_F32: return launch_epi<EPI_F32>(stream, g, sms);
@@ -665,7 +698,7 @@ cudaError_t gemm_bf16_tn(cudaStream_t stream, const GemmArgs& g) {
       if ((g.N % 256) || !r.out || !r.cs || (r.D != 64 && r.D != 128) || g.N != (r.Hq + 2 * r.Hkv) * r.D || (r.ldc % 8)) return cudaErrorInvalidValue;
       if (r.slots && (!r.k_cache || !r.v_cache || r.page_size <= 0)) return cudaErrorInvalidValue;
       GemmArgs h = g;
-      h.block_n = 256;
+      h.block_n = 0;
       return launch_epi<EPI_ROPE>(stream, h, sms);
     }
   }
