@@ -42,12 +42,19 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 __global__ void __launch_bounds__(256)
 sum_slabs_kernel(const float* __restrict__ ws, const uint8_t* __restrict__ segs, float* __restrict__ out, int ldo, int M,
-                 int N) {
+                 int N, bf16* __restrict__ relu2) {
   pdl_launch_dependents();
   pdl_wait();
   const int m = blockIdx.y;
   const int n = blockIdx.x * 256 + threadIdx.x;
-  if (n < N) out[(size_t)m * ldo + n] = slab_sum(ws, segs, M, N, m, n);
+  if (n >= N) return;
+  const float v = slab_sum(ws, segs, M, N, m, n);
+  if (relu2) {
+    const float r = fmaxf(v, 0.f);
+    relu2[(size_t)m * N + n] = __float2bfloat16(r * r);
+  } else {
+    out[(size_t)m * ldo + n] = v;
+  }
 }
 
 // grid (Hq + 2*Hkv, M): one block per (head, token); D/2 threads, one rotary pair each.
@@ -223,8 +230,8 @@ cudaError_t dec_embed_prep(cudaStream_t s, const int32_t* tokens, const bf16* ta
   if (M <= 0) return cudaSuccess;
   return launch_k(embed_prep_kernel, dim3(M), dim3(128), 0, s, true, tokens, table, gain, x, xg, ss_out, H);
 }
-cudaError_t dec_sum_slabs(cudaStream_t s, const float* ws, const SkinnyPlan& p, float* out, int ldo, int M, int N) {
-  return launch_k(sum_slabs_kernel, dim3((N + 255) / 256, M), dim3(256), 0, s, true, ws, p.seg_count, out, ldo, M, N);
+cudaError_t dec_sum_slabs(cudaStream_t s, const float* ws, const SkinnyPlan& p, float* out, int ldo, int M, int N, bf16* relu2) {
+  return launch_k(sum_slabs_kernel, dim3((N + 255) / 256, M), dim3(256), 0, s, true, ws, p.seg_count, out, ldo, M, N, relu2);
 }
 cudaError_t dec_qkv_rope_kvwrite(cudaStream_t s, const float* ws, const SkinnyPlan& p, bf16* qkv_out,
                                  const int32_t* positions, const int32_t* slot_mapping, const float* inv_freq,

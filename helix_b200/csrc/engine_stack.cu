@@ -639,7 +639,8 @@ bool Engine::stack_tc(int N, int K, int lda, int ldc) const {
   return !model_.sd.compute_f32 && !simt_only && K % 8 == 0 && lda % 8 == 0 && K >= 64 && N >= 64 && ldc % 4 == 0;
 }
 
-int Engine::stack_gemm(const float* A, const bf16* A16, int lda, const void* Wt, int N, int K, float* C, int ldc, int M, const void* bias) {
+int Engine::stack_gemm(const float* A, const bf16* A16, int lda, const void* Wt, int N, int K, float* C, int ldc, int M, const void* bias, bf16* relu2,
+                       bool* relu2_done) {
   const bool f32 = model_.sd.compute_f32 != 0;
   static const bool simt_only = [] { const char* e = getenv("HB_STACK_SIMT"); return e && atoi(e) != 0; }();  // A/B and bring-up
   const double flops = 2.0 * M * N * K;
@@ -652,7 +653,8 @@ int Engine::stack_gemm(const float* A, const bf16* A16, int lda, const void* Wt,
     CU(gemm_skinny_plan(N, K, &plan));
     if (gemm_skinny_ws_floats(plan, M, N) <= stack_skinny_floats(model_)) {
       SPAN(4, 2.0 * N * K + 2.0 * M * K + 4.0 * M * N, gemm_skinny(stream_, plan, A16, lda, (const bf16*)Wt, K, skinny_ws_, M, N, K));
-      SPAN(3, 8.0 * M * N, dec_sum_slabs(stream_, skinny_ws_, plan, C, ldc, M, N));
+      SPAN(3, 8.0 * M * N, dec_sum_slabs(stream_, skinny_ws_, plan, C, ldc, M, N, relu2));
+      if (relu2) *relu2_done = true;
       return HB_OK;
     }
   }
@@ -899,9 +901,10 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       GemmArgs g{ff_in16, W, (const bf16*)w_up, W, mo16, F, nullptr, 0, nullptr, T, F, W, EPI_RELU2, 0};
       SPAN(0, 2.0 * T * F * W, gemm_bf16_tn(stream_, g));
     } else {
-      int rc = stack_gemm(ff_in, ff_in16, W, w_up, F, W, k.p1, k.ld1, T);
+      bool squared = false;  // the sum of the few-token product's slabs has already applied it
+      int rc = stack_gemm(ff_in, ff_in16, W, w_up, F, W, k.p1, k.ld1, T, nullptr, stack_tc(W, F, F, W) ? mo16 : nullptr, &squared);
       if (rc != HB_OK) return rc;
-      SPAN(3, 10.0 * T * F, relu2_rows(stream_, k.p1, k.ld1, k.mo, mo16, T, F));
+      if (!squared) SPAN(3, 10.0 * T * F, relu2_rows(stream_, k.p1, k.ld1, k.mo, mo16, T, F));
     }
     return stack_gemm(k.mo, mo16, F, w_down, W, F, out, W, T);
   };
@@ -1045,9 +1048,14 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       ca.out = k.cv; ca.ldo = k.ldcv;
       ca.state = state_; ca.slot_stride = (long)model_.state_floats; ca.tail_off = w.tail_off;
       ca.cu = cu; ca.first_pos = first; ca.slots = sslot; ca.seq_of = seqof; ca.T = T; ca.B = B; ca.C = C;
-      SPAN(3, 4.0 * T * C * (l.conv_taps + 1), short_conv(stream_, ca));
-      SPAN(3, 8.0 * B * C * l.conv_taps, conv_tails(stream_, ca));
-      SPAN(3, 12.0 * T * H, ssm_steps(stream_, k.p1, k.ld1, w.off_a, w.a_dt, f32, k.ab, k.ldab, T, H));
+      const bool fused = short_conv_fused(ca);
+      if (fused) {
+        ca.single = T == B;  // (no entry is empty)
+        ca.off_dt = w.off_a; ca.H = H; ca.a_dt = w.a_dt; ca.ab = k.ab; ca.ldab = k.ldab;
+      }
+      SPAN(3, 4.0 * T * C * (l.conv_taps + 1) + 12.0 * T * H, short_conv(stream_, ca));
+      if (!ca.single) SPAN(3, 8.0 * B * C * l.conv_taps, conv_tails(stream_, ca));
+      if (!fused) SPAN(3, 12.0 * T * H, ssm_steps(stream_, k.p1, k.ld1, w.off_a, w.a_dt, f32, k.ab, k.ldab, T, H));
       LinRecArgs ra{};
       ra.q = k.cv; ra.ldq = k.ldcv; ra.q_off = inner + G * N;
       ra.k = k.cv; ra.ldk = k.ldcv; ra.k_off = inner;
@@ -1143,8 +1151,9 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
         ca.out = k.cv; ca.ldo = k.ldcv;
         ca.state = state_; ca.slot_stride = (long)model_.state_floats; ca.tail_off = w.tail_off;
         ca.cu = cu; ca.first_pos = first; ca.slots = sslot; ca.seq_of = seqof; ca.T = T; ca.B = B; ca.C = C;
+        ca.single = T == B && short_conv_fused(ca);
         SPAN(3, 4.0 * T * C * (l.conv_taps + 1), short_conv(stream_, ca));
-        SPAN(3, 8.0 * B * C * l.conv_taps, conv_tails(stream_, ca));
+        if (!ca.single) SPAN(3, 8.0 * B * C * l.conv_taps, conv_tails(stream_, ca));
         pa.p = k.cv; pa.ldp = k.ldcv; pa.q_off = 0; pa.k_off = H * Dk; pa.v_off = (H + G) * Dk;
       }
       // an entry-wise output gate or a second mixer: the attention output passes one more kernel on its way to the output

@@ -274,7 +274,8 @@ int gemm_skinny_max_segs(int N, int K, int sms);  // pure host arithmetic (memor
 cudaError_t gemm_skinny(cudaStream_t stream, const SkinnyPlan& plan, const bf16* X, int ldx, const bf16* W, int ldw,
                         float* ws, int M, int N, int K, const StreamSig* sig = nullptr, const SkinnyEpi* epi = nullptr);
 // consumers of the slabs (each sums the slabs in fixed order, then applies its fused epilogue)
-cudaError_t dec_sum_slabs(cudaStream_t s, const float* ws, const SkinnyPlan& p, float* out, int ldo, int M, int N);
+// relu2 given: relu(sum)^2 as dense bf16 rows there instead of the sums in out
+cudaError_t dec_sum_slabs(cudaStream_t s, const float* ws, const SkinnyPlan& p, float* out, int ldo, int M, int N, bf16* relu2 = nullptr);
 // the dec_* kernels below take an optional DepSig; *ctas (when given) receives the number of CTAs that will report
 cudaError_t dec_qkv_rope_kvwrite(cudaStream_t s, const float* ws, const SkinnyPlan& p, bf16* qkv_out,
                                  const int32_t* positions, const int32_t* slot_mapping, const float* inv_freq,
@@ -554,8 +555,13 @@ struct ConvArgs {
   float* state; long slot_stride; size_t tail_off;
   const int32_t* cu; const int32_t* first_pos; const int32_t* slots; const int32_t* seq_of;
   int T, B, C;
+  // Where short_conv_fused says so, one launch may also do
+  bool single = false;  // what conv_tails does, when every entry is exactly one token;
+  // ab given: what ssm_steps does for the same rows (on `in` with these arguments)
+  int off_dt = 0, H = 0; const void* a_dt = nullptr; float* ab = nullptr; long ldab = 0;
 };
 cudaError_t short_conv(cudaStream_t s, const ConvArgs& a);
+bool short_conv_fused(const ConvArgs& a);
 cudaError_t conv_tails(cudaStream_t s, const ConvArgs& a);
 // State-space step sizes: dt = softplus(p[t, off_dt + h] + dt_bias[h]); ab[t, h] = exp(-exp(A_log[h]) dt), ab[t, H + h] = dt
 // (a_dt = [A_log (H) | dt_bias (H) | ...] of the weight type)

@@ -235,6 +235,8 @@ __global__ void __launch_bounds__(256) postnorm_vec_kernel(const float* x, const
                                                            const WT* __restrict__ w, float alpha, float off, float eps,
                                                            float* out, bf16* __restrict__ outb, int W, int add_x) {
   __shared__ float red[32];
+  pdl_launch_dependents();
+  pdl_wait();
   const int r = blockIdx.x;
   const size_t src = row_index ? (size_t)row_index[r] : (size_t)r;
   const int nv = W / 4;
@@ -1053,9 +1055,11 @@ static cudaError_t postnorm_launch(cudaStream_t s, const float* x, const int32_t
   if (W % 4 == 0 && W <= 4 * 256 * kPnChunks && (!y || ldy % 4 == 0) && ((uintptr_t)x & 15) == 0 && ((uintptr_t)y & 15) == 0 &&
       ((uintptr_t)out & 15) == 0 && ((uintptr_t)outb & 7) == 0) {
     if (f32)
-      postnorm_vec_kernel<float><<<rows, 256, 0, s>>>(x, idx, y, ldy, (const float*)bias, (const float*)w, alpha, off, eps, out, outb, W, add_x);
+      return launch_k(postnorm_vec_kernel<float>, dim3(rows), dim3(256), 0, s, true, x, idx, y, ldy, (const float*)bias, (const float*)w, alpha, off, eps, out, outb, W,
+                      add_x);
     else
-      postnorm_vec_kernel<bf16><<<rows, 256, 0, s>>>(x, idx, y, ldy, (const bf16*)bias, (const bf16*)w, alpha, off, eps, out, outb, W, add_x);
+      return launch_k(postnorm_vec_kernel<bf16>, dim3(rows), dim3(256), 0, s, true, x, idx, y, ldy, (const bf16*)bias, (const bf16*)w, alpha, off, eps, out, outb, W,
+                      add_x);
     return KERR();
   }
   const size_t smem = (size_t)(W + 32) * 4;

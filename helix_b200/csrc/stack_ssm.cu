@@ -26,6 +26,14 @@ namespace {
 
 __device__ __forceinline__ float softplus_(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 
+template <typename WT>
+__device__ __forceinline__ void ssm_step(const float* __restrict__ p, long ldp, int off_dt, const WT* __restrict__ a_dt, float* __restrict__ ab, long ldab,
+                                         int t, int H, int h) {
+  const float dt = softplus_(p[(size_t)t * ldp + off_dt + h] + ldf<WT>(a_dt, H + h));
+  ab[(size_t)t * ldab + h] = expf(-expf(ldf<WT>(a_dt, h)) * dt);
+  ab[(size_t)t * ldab + H + h] = dt;
+}
+
 // ------------------------------------------------------------------ short convolutions
 template <typename WT>
 __global__ void __launch_bounds__(256) short_conv_kernel(ConvArgs a) {
@@ -52,13 +60,22 @@ __global__ void __launch_bounds__(256) short_conv_kernel(ConvArgs a) {
 // The same for rows whose pieces start on 16-byte boundaries and up to four taps: thread = four neighbouring channels x kConvRun
 // consecutive tokens, the last TAPS - 1 inputs in registers, so a row is read once per run instead of once per tap.  A run may
 // cross entries: the window is refilled (from the slot or with zeros) wherever an entry starts.
+// Steps of a few tokens take runs of one token: a run of eight then was eight dependent chains (entry, slot, tail) in a row, 14 us for 16
+// tokens of 16 entries against 4 now; where every entry is a single token the same thread also moves the slot's inputs on.
 constexpr int kConvRun = 8;
 __device__ __forceinline__ float4 f4add(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
-template <typename WT, int TAPS>
+template <typename WT, int TAPS, int RUN>
 __global__ void __launch_bounds__(128) short_conv_run_kernel(ConvArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tb = blockIdx.y * RUN;
+  if (a.ab && blockIdx.x == gridDim.x - 1) {  // the last column of blocks makes the run's step sizes
+    for (int e = threadIdx.x; e < RUN * a.H; e += blockDim.x)
+      if (tb + e / a.H < a.T) ssm_step<WT>(a.in, a.ldi, a.off_dt, (const WT*)a.a_dt, a.ab, a.ldab, tb + e / a.H, a.H, e % a.H);
+    return;
+  }
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (c >= a.C) return;
-  const int tb = blockIdx.y * kConvRun;
   float w[4][TAPS];
 #pragma unroll
   for (int e = 0; e < 4; ++e)
@@ -76,9 +93,9 @@ __global__ void __launch_bounds__(128) short_conv_run_kernel(ConvArgs a) {
   float4 win[TAPS > 1 ? TAPS - 1 : 1];
   int t0 = 0, t1 = -1;
   bool fresh = false;
-  const float* tail = nullptr;
+  float* tail = nullptr;
 #pragma unroll
-  for (int tt = 0; tt < kConvRun; ++tt) {
+  for (int tt = 0; tt < RUN; ++tt) {
     const int t = tb + tt;
     if (t >= a.T) break;
     bool refill = tt == 0;
@@ -116,6 +133,10 @@ __global__ void __launch_bounds__(128) short_conv_run_kernel(ConvArgs a) {
 #pragma unroll
     for (int j = 0; j + 1 < TAPS - 1; ++j) win[j] = win[j + 1];
     if (TAPS > 1) win[TAPS - 2] = x;
+    if (a.single) {  // the entry's only token: the window is what conv_tails would store
+#pragma unroll
+      for (int j = 0; j < TAPS - 1; ++j) *reinterpret_cast<float4*>(tail + (size_t)j * a.C + c) = win[j];
+    }
   }
 }
 
@@ -150,10 +171,7 @@ __global__ void ssm_steps_kernel(const float* __restrict__ p, long ldp, int off_
                                  long ldab, int T, int H) {
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long)T * H) return;
-  const int t = (int)(idx / H), h = (int)(idx % H);
-  const float dt = softplus_(p[(size_t)t * ldp + off_dt + h] + ldf<WT>(a_dt, H + h));
-  ab[(size_t)t * ldab + h] = expf(-expf(ldf<WT>(a_dt, h)) * dt);
-  ab[(size_t)t * ldab + H + h] = dt;
+  ssm_step<WT>(p, ldp, off_dt, a_dt, ab, ldab, (int)(idx / H), H, (int)(idx % H));
 }
 
 // One warp per (entry, head).  The step m -> max(m + f, i) is the pair (f, i); two steps compose to
@@ -225,6 +243,8 @@ __global__ void __launch_bounds__(DKP * 2, 512 / DKP) lin_recurrence_kernel(LinR
   constexpr int KS = DKP / 16, BC = 32 * NC;
   constexpr int per_tok = 2 * DKP + BC + 4, stage_floats = kRecTch * per_tok;
   extern __shared__ __align__(16) float sm[];  // 2 stages | partial outputs [kRecTch][KS][BC] | partial n . q [kRecTch][KS]
+  pdl_launch_dependents();
+  pdl_wait();
   float* obuf = sm + 2 * stage_floats;
   float* nbuf = obuf + kRecTch * KS * BC;
   const int b = blockIdx.x, h = blockIdx.y, kvh = h / (a.H / a.G);
@@ -377,8 +397,7 @@ cudaError_t launch_rec(cudaStream_t s, const LinRecArgs& a) {
   constexpr int KS = DKP / 16, BC = 32 * NC, kRecTch = 16 / NC;
   const size_t smem = (size_t)(2 * kRecTch * (2 * DKP + BC + 4) + kRecTch * KS * BC + kRecTch * KS) * 4;
   dim3 grid(a.B, a.H, (a.Dv + BC - 1) / BC);
-  lin_recurrence_kernel<DKP, NC><<<grid, DKP * 2, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_k(lin_recurrence_kernel<DKP, NC>, grid, dim3(DKP * 2), smem, s, true, a);
 }
 
 // ------------------------------------------------------------------ read-outs
@@ -468,6 +487,8 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
                                                                    const WT* __restrict__ w, float eps, int parts, float* __restrict__ out,
                                                                    bf16* __restrict__ outb, int n, int gate_last) {
   __shared__ float red[32];
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.y, part = blockIdx.x, len = n / parts, c0 = part * len;
   const float* ys = y + (size_t)t * ldy + c0;
   const float* zs = z ? z + (size_t)t * ldz + c0 : nullptr;
@@ -590,6 +611,8 @@ __global__ void __launch_bounds__(256) parallel_step_vec_kernel(const float* x, 
                                                                 float* __restrict__ h1, bf16* __restrict__ h1b, float* __restrict__ h2,
                                                                 bf16* __restrict__ h2b, int W, const ParScale sc) {
   __shared__ float red[32];
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t r = blockIdx.x;
   const float* xs = x + (row_index ? (size_t)row_index[r] : r) * W;
   float4 v[CH];
@@ -669,19 +692,28 @@ cudaError_t stack_ssm_init() {
   return cudaSuccess;
 }
 
+bool short_conv_fused(const ConvArgs& a) {
+  return a.taps <= 4 && a.T <= 65535 && ((a.C | (int)a.ldi | a.off | (int)a.ldo | (int)a.slot_stride | (int)a.tail_off) & 3) == 0 &&
+         ((uintptr_t)a.in & 15) == 0 && ((uintptr_t)a.out & 15) == 0 && ((uintptr_t)a.state & 15) == 0;
+}
 cudaError_t short_conv(cudaStream_t s, const ConvArgs& a) {
   if (a.T <= 0 || a.C <= 0) return cudaSuccess;
   if (a.taps < 1 || a.taps - 1 > kMaxConvTail) return cudaErrorInvalidValue;
-  const bool vec = a.taps <= 4 && ((a.C | (int)a.ldi | a.off | (int)a.ldo | (int)a.slot_stride | (int)a.tail_off) & 3) == 0 &&
-                   ((uintptr_t)a.in & 15) == 0 && ((uintptr_t)a.out & 15) == 0 && ((uintptr_t)a.state & 15) == 0;
-  if (vec) {
-    dim3 g((a.C / 4 + 127) / 128, (a.T + kConvRun - 1) / kConvRun);
-#define HB_CONV(WT, TP) short_conv_run_kernel<WT, TP><<<g, 128, 0, s>>>(a)
-    if (a.f32) { if (a.taps == 1) HB_CONV(float, 1); else if (a.taps == 2) HB_CONV(float, 2); else if (a.taps == 3) HB_CONV(float, 3); else HB_CONV(float, 4); }
-    else { if (a.taps == 1) HB_CONV(bf16, 1); else if (a.taps == 2) HB_CONV(bf16, 2); else if (a.taps == 3) HB_CONV(bf16, 3); else HB_CONV(bf16, 4); }
+  if (short_conv_fused(a)) {
+    const int across = (a.C / 4 + 127) / 128;
+    // runs of one token until runs of eight give every SM two blocks (or where the tails ride along)
+    const bool one = a.single || (long)across * ((a.T + kConvRun - 1) / kConvRun) < 2 * 148;
+    const dim3 g(across + (a.ab ? 1 : 0), one ? a.T : (a.T + kConvRun - 1) / kConvRun);
+#define HB_CONV_T(WT, TP) return one ? launch_k(short_conv_run_kernel<WT, TP, 1>, g, dim3(128), 0, s, true, a) : launch_k(short_conv_run_kernel<WT, TP, kConvRun>, g, dim3(128), 0, s, true, a)
+#define HB_CONV(TP) do { if (a.f32) HB_CONV_T(float, TP); else HB_CONV_T(bf16, TP); } while (0)
+    if (a.taps == 1) HB_CONV(1);
+    if (a.taps == 2) HB_CONV(2);
+    if (a.taps == 3) HB_CONV(3);
+    HB_CONV(4);
 #undef HB_CONV
-    return cudaGetLastError();
+#undef HB_CONV_T
   }
+  if (a.single || a.ab) return cudaErrorInvalidValue;
   dim3 grid((a.C + 255) / 256, a.T);
   if (a.f32) short_conv_kernel<float><<<grid, 256, 0, s>>>(a);
   else short_conv_kernel<bf16><<<grid, 256, 0, s>>>(a);
@@ -751,7 +783,8 @@ cudaError_t gated_group_norm(cudaStream_t s, const float* y, long ldy, const flo
   dim3 grid(parts, T);
   const int len = n / parts;
   if (len % 4 == 0 && len <= 8192 && ((ldy | ldz) & 3) == 0 && (((uintptr_t)y | (uintptr_t)z | (uintptr_t)out) & 15) == 0 && (((uintptr_t)outb | (uintptr_t)zb) & 7) == 0) {
-#define HB_GGN(WT, CH) gated_group_norm_vec_kernel<WT, CH><<<grid, 256, 0, s>>>(y, ldy, z, zb, ldz, (const WT*)w, eps, parts, out, outb, n, gate_last)
+#define HB_GGN(WT, CH) \
+  return launch_k(gated_group_norm_vec_kernel<WT, CH>, grid, dim3(256), 0, s, true, y, ldy, z, zb, ldz, (const WT*)w, eps, parts, out, outb, n, (int)gate_last)
 #define HB_GGN_T(CH) do { if (f32) HB_GGN(float, CH); else HB_GGN(bf16, CH); } while (0)
     if (len <= 1024) HB_GGN_T(1);
     else if (len <= 2048) HB_GGN_T(2);
@@ -759,7 +792,6 @@ cudaError_t gated_group_norm(cudaStream_t s, const float* y, long ldy, const flo
     else HB_GGN_T(8);
 #undef HB_GGN_T
 #undef HB_GGN
-    return cudaGetLastError();
   }
   if (zb) return cudaErrorInvalidValue;
   if (f32) gated_group_norm_kernel<float><<<grid, 256, 0, s>>>(y, ldy, z, ldz, (const float*)w, eps, parts, out, outb, n, gate_last);
@@ -784,15 +816,14 @@ cudaError_t parallel_step(cudaStream_t s, const float* x, const int32_t* row_ind
   const uintptr_t al = (uintptr_t)x | (uintptr_t)y | (uintptr_t)y2 | (uintptr_t)bias | (uintptr_t)w1 | (uintptr_t)w2 | (uintptr_t)x_out | (uintptr_t)h1 |
                        (uintptr_t)h1b | (uintptr_t)h2 | (uintptr_t)h2b | (uintptr_t)sc.s1 | (uintptr_t)sc.s2 | (uintptr_t)sc.rows;
   if (W % 4 == 0 && W <= 4 * 256 * kParChunks && (al & 15) == 0 && sc.top_k <= kParTop) {
-#define HB_PAR(WT, CH)                                                                                                                      \
-  parallel_step_vec_kernel<WT, CH><<<rows, 256, 0, s>>>(x, row_index, y, y2, (const WT*)bias, bias_scale, (const WT*)w1, (const WT*)w2, eps, \
-                                                        x_out, h1, h1b, h2, h2b, W, sc)
+#define HB_PAR(WT, CH)                                                                                                                   \
+  return launch_k(parallel_step_vec_kernel<WT, CH>, dim3(rows), dim3(256), 0, s, true, x, row_index, y, y2, (const WT*)bias, bias_scale, \
+                  (const WT*)w1, (const WT*)w2, eps, x_out, h1, h1b, h2, h2b, W, sc)
     if (W <= 1024) { if (f32) HB_PAR(float, 1); else HB_PAR(bf16, 1); }
     else if (W <= 2048) { if (f32) HB_PAR(float, 2); else HB_PAR(bf16, 2); }
     else if (W <= 4096) { if (f32) HB_PAR(float, 4); else HB_PAR(bf16, 4); }
     else { if (f32) HB_PAR(float, 8); else HB_PAR(bf16, 8); }
 #undef HB_PAR
-    return cudaGetLastError();
   }
   if ((size_t)W * 4 > 200 * 1024) return cudaErrorInvalidValue;
   const size_t smem = (size_t)W * 4;
