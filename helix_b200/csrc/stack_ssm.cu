@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(256) short_conv_kernel(ConvArgs a) {
 // consecutive tokens, the last TAPS - 1 inputs in registers, so a row is read once per run instead of once per tap.  A run may
 // cross entries: the window is refilled (from the slot or with zeros) wherever an entry starts.
 // Steps of a few tokens take runs of one token: a run of eight then was eight dependent chains (entry, slot, tail) in a row, 14 us for 16
-// tokens of 16 entries against 4 now; where every entry is a single token the same thread also moves the slot's inputs on.
+// tokens of 16 entries against 5 now; where every entry is a single token the same thread also moves the slot's inputs on.
 constexpr int kConvRun = 8;
 __device__ __forceinline__ float4 f4add(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 template <typename WT, int TAPS, int RUN>
