@@ -10,17 +10,17 @@
 // hm, hh with fp32 accumulation, so what is dropped is below 2^-24 of the factors.  The small products come first, and for A the
 // second half of hh has an accumulator of its own, because the tensor pipe's accumulators round toward zero: only the last steps
 // do so at the sum's full size.  Products of decays are formed in 64 bits; the state and the sum of an output's two parts are
-// formed in registers, once per 128 tokens where the token-by-token kernel rounds the state at rounds the state at every token.  Relative
-// errors against 64 bits, that kernel / this one: state 7.2e-8 / 6.4e-8, outputs 1.1e-7 / 1.3e-7 at a model's decays, outputs
-// 4.2e-7 / 2.3e-7 and state 4.7e-7 / 1.6e-7 over 2048 tokens of slow decays.
+// formed in registers, once per 128 tokens where the token-by-token kernel rounds the state at every token.  Relative errors
+// against 64 bits, that kernel / this one: state 7.2e-8 / 6.4e-8, outputs 1.1e-7 / 1.3e-7 at a model's decays, outputs 4.2e-7 /
+// 2.3e-7 and state 4.7e-7 / 1.6e-7 over 2048 tokens of slow decays.
 //
 // Bound by the threads that split operands and by the tensor pipe (six passes).  One CTA per (entry, head, 64 value columns) walks the
 // entry's chunks; an entry that starts at position 0 starts from zeros.
 //   warp 16   : all products: A | S^T q | W V | U = K^T Vw, in this order
 //   warps 0-15: thread (row r = 32 (warp & 3) + lane, quarter qf = warp >> 2).  While the products of a chunk run they split the next
 //               chunk's q (into TMEM: the A operand of two products) and v; k, whose tile U's product still reads, comes last.
-// TMEM columns: [U (64) | S^T q, then W V (64), both together A's second accumulator | q terms (3 x 64) | A (128), then W terms (3 x 64)].  Shared memory: k terms, v terms, one
-// set of tiles that holds S's terms for S^T q and then the weighted v's terms for U.
+// TMEM columns: [U (64) | S^T q, then W V (64), both together A's second accumulator | q terms (3 x 64) | A (128), then W terms
+// (3 x 64)].  Shared memory: k terms, v terms, one set of tiles that holds S's terms for S^T q and then the weighted v's for U.
 // Measured (11k tokens in 8 sequences, 64 heads, 128 x 64 states): 1650 us token by token, 575 us here.
 // A NaN or an infinity among the inputs reaches every row of its chunk and head (earlier ones of the same sequence too).
 // Waits are bounded: one that runs out marks the launch as failed (the host reads the flag behind the step), and the block runs
