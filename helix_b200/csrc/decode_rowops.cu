@@ -13,8 +13,18 @@ namespace {
 __device__ __forceinline__ float slab_sum(const float* __restrict__ ws, const uint8_t* __restrict__ segs, int M, int N,
                                           int m, int n) {
   const int ns = segs[n >> 7];
+  const float* p = ws + (size_t)m * N + n;
+  const size_t step = (size_t)M * N;
   float acc = 0.f;
-  for (int s = 0; s < ns; ++s) acc += ws[((size_t)s * M + m) * N + n];
+  int s = 0;
+  for (; s + 8 <= ns; s += 8) {  // (in slab order, eight loads in flight: small products are cut into up to sixteen slabs)
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = p[(s + e) * step];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc += v[e];
+  }
+  for (; s < ns; ++s) acc += p[s * step];
   return acc;
 }
 // block-wide entry / exit of a kernel in the decode chain (ptx.cuh dep_*)

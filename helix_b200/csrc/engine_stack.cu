@@ -1069,6 +1069,7 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       ra.cu = cu; ra.first_pos = first; ra.slots = sslot;
       ra.B = B; ra.H = H; ra.G = G; ra.Dk = N; ra.Dv = Dv;
       ra.error = kernel_error_;
+      ra.single = T == B;
       // Portions of 64 tokens and more on average go chunk by chunk, where any part of a chunk costs a whole one: 16 sequences x 32 heads
       // of 128 x 64 states take 65 us there for 32 to 128 tokens, token by token 39 us for 32, 53 for 48, 163 for 120.
       if (!f32 && T >= 64 * B && rec_chunk_ok(ra)) SPAN(6, 4.0 * T * H * N * Dv, rec_chunk(stream_, ra));
@@ -1101,6 +1102,7 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       ra.state = state_; ra.slot_stride = (long)model_.state_floats; ra.s_off = w.state_off;
       ra.cu = cu; ra.first_pos = first; ra.slots = sslot;
       ra.B = B; ra.H = H; ra.G = H; ra.Dk = Dk; ra.Dv = Dv;
+      ra.single = T == B;
       SPAN(6, 4.0 * T * H * Dk * Dv, lin_recurrence(stream_, ra));
       SPAN(3, 16.0 * T * H * Dv, gated_group_norm(stream_, k.ctx, k.ldctx, k.p1 + w.off_g, k.ld1, w.hnorm, f32, sd.norm_eps, 1, mo_f32, mo16, T, H * Dv,
                                                   true));

@@ -598,6 +598,7 @@ struct LinRecArgs {
   int B, H, G, Dk, Dv;
   const float* head_decay = nullptr;
   int silu = 0;
+  bool single = false;  // every entry is exactly one token
 };
 cudaError_t lin_recurrence(cudaStream_t s, const LinRecArgs& a);
 // The same without normaliser, constant decays and activations, chunk by chunk on the tensor cores with operands in three bf16 terms
