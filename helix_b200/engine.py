@@ -5,6 +5,7 @@ for a slot's ``gpu_index`` / ``model_memory_requirement``, load a model, start t
 submit / poll token ids (chat) or call ``embed`` (RAG ingest).
 """
 import ctypes as C
+import struct
 from dataclasses import dataclass, field, asdict
 
 import numpy as np
@@ -14,6 +15,10 @@ from ._lib import EngineCfg, LayerDescC, ModelDescC, SamplingC, SeqFeedC, StackD
 
 CAPTURE_STEP_LOGITS = 1
 CAPTURE_PROMPT_LOGITS = 2
+
+
+_FEED = struct.Struct("@QPiPi0P")  # hb_seq_feed
+assert _FEED.size == C.sizeof(SeqFeedC)
 
 
 class HBError(RuntimeError):
@@ -432,17 +437,31 @@ class Engine:
 
     def seq_step(self, entries):
         """entries: [(seq id, tokens, want positions)] -> fp32 [sum(len(want)), vocab]; ONE engine step over all entries."""
-        keep, arr = [], (SeqFeedC * len(entries))()
-        rows = 0
-        for i, (sid, toks, want) in enumerate(entries):
-            t = np.ascontiguousarray(toks, dtype=np.int32)
-            w = np.ascontiguousarray(want, dtype=np.int32)
-            keep += [t, w]
-            arr[i] = SeqFeedC(sid, t.ctypes.data, t.size, w.ctypes.data if w.size else None, w.size)
-            rows += w.size
+        # one array of all tokens, one of all wanted positions, the descriptors packed behind them: arrays and structures made entry by
+        # entry took longer than the launches of a decoding step (16 entries: 65 us, 18 now)
+        n = len(entries)
+        toks, want, counts = [], [], []
+        for _, t, w in entries:
+            if type(t) is not np.ndarray or t.dtype != np.int32 or t.ndim != 1:
+                t = np.ascontiguousarray(t, dtype=np.int32).ravel()
+            if type(w) is not list or (w and type(w[0]) is not int):
+                w = np.ascontiguousarray(w, dtype=np.int32).ravel().tolist()
+            toks.append(t)
+            want += w
+            counts.append(len(w))
+        flat = np.concatenate(toks) if n else np.zeros(0, np.int32)
+        want = np.array(want, dtype=np.int32)
+        rows, feeds = want.size, bytearray(n * _FEED.size)
+        at_t, at_w = flat.ctypes.data, want.ctypes.data
+        for i in range(n):
+            nt, nw = toks[i].size, counts[i]
+            _FEED.pack_into(feeds, i * _FEED.size, entries[i][0], at_t, nt, at_w if nw else 0, nw)
+            at_t += 4 * nt
+            at_w += 4 * nw
+        arr = (SeqFeedC * n).from_buffer(feeds)
         out = np.empty((rows, self.desc.vocab), dtype=np.float32)
         got = C.c_int32()
-        self._ck(self._l.hb_seq_step(self._h, arr, len(entries), out.ctypes.data if rows else None, out.size, C.byref(got)))
+        self._ck(self._l.hb_seq_step(self._h, arr, n, out.ctypes.data if rows else None, out.size, C.byref(got)))
         return out
 
     # ---- embeddings
