@@ -293,13 +293,19 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {  // splitmix64 finaliser
 __device__ __forceinline__ void argmax_merge(float& best, int& bi, float ov, int oi) {
   if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
 }
-// float -> unsigned key that orders like the float (and back)
+// float -> unsigned key that orders like the float (and back); NaN is key 0, below every number, and key 0 is a NaN.  (The bits
+// change type in asm: the compiler may turn integer operations on a float's sign into float ones, which lose a NaN's bits.)
 __device__ __forceinline__ uint32_t fkey(float x) {
-  const uint32_t u = __float_as_uint(x);
+  uint32_t u;
+  asm("mov.b32 %0, %1;" : "=r"(u) : "f"(x));
+  if (x != x) return 0u;
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 __device__ __forceinline__ float fkey_inv(uint32_t k) {
-  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+  const uint32_t u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
+  float x;
+  asm("mov.b32 %0, %1;" : "=f"(x) : "r"(u));
+  return x;
 }
 
 // ---- rows of the vocabulary, one cluster of kVocCtas blocks per row ----
@@ -582,6 +588,7 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
   const uint64_t sd = seed ? seed[b] : 0;
   scan([&](uint32_t q, int i) {
     if (i >= n) return;
+    if (q == 0) return;  // a NaN is never drawn
     const float raw = fkey_inv(q);
     if (raw < floor_logit) return;
     const int v = start + i;

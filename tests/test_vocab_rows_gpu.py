@@ -81,10 +81,8 @@ def test_greedy_and_top_k_rows(V):
             seed = torch.arange(B, device="cuda", dtype=torch.int64) * 77 + s
             assert L.hbk_sample_filtered(p(x), ld, p(temp), p(seed), p(topk), None, p(out), B, V) == 0
             torch.cuda.synchronize()
-            for b in range(B):
-                if b == 3:
-                    continue  # (a NaN counts as one of the k)
-                kth = np.sort(rows[b])[::-1][min(k, V) - 1]
+            for b in range(B):  # (a NaN is below every number)
+                kth = np.sort(np.where(np.isnan(rows[b]), -np.inf, rows[b]))[::-1][min(k, V) - 1]
                 assert rows[b][int(out[b])] >= kth
 
 
@@ -108,3 +106,21 @@ def test_nucleus_rows(V, top_k):
         assert L.hbk_sample_filtered(p(x), V, p(temp), p(seed), p(tk), p(tp), p(out), B, V) == 0
         torch.cuda.synchronize()
         assert set(out.tolist()) == set(int(i) for i in at[:keep])  # the rarest survivor: missed with probability < 0.95^256
+
+
+@pytest.mark.parametrize("filtered", [False, True])
+@pytest.mark.parametrize("V", [8, 1000])
+def test_nan_logits_are_never_drawn(V, filtered):
+    """All but three logits of every row are NaN: whatever the noise, one of the three is drawn."""
+    L = hb.lib()
+    B = 256
+    x = torch.full((B, V), float("nan"), device="cuda")
+    keep = [0, V // 2, V - 1]
+    x[:, keep] = torch.tensor([0.5, -1.0, 0.0], device="cuda")
+    temp = torch.full((B,), 2.0, device="cuda")
+    tk = torch.full((B,), V - 1, device="cuda", dtype=torch.int32) if filtered else None
+    seed = torch.arange(B, device="cuda", dtype=torch.int64) * 7919
+    out = torch.empty(B, device="cuda", dtype=torch.int32)
+    assert L.hbk_sample_filtered(p(x), V, p(temp), p(seed), p(tk), None, p(out), B, V) == 0
+    torch.cuda.synchronize()
+    assert set(out.tolist()) == set(keep)
