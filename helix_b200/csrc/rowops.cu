@@ -362,9 +362,11 @@ __device__ __forceinline__ void load_slice(const float* __restrict__ src, int n,
 // Probability mass is accumulated in 2^-32 fixed point, so every sum is exact and independent of its order.  A pass compares a
 // slice with three keys inside the interval that still holds the answer; once the interval holds at most kFin tokens, block 0
 // gets them and finds the answer directly.
-// Measured (32 rows x 128256, mixed top-k / top-p): 1100 us with a block per row and up to 32 + 32 one-key passes, 73 us now.
-constexpr int kFin = 256;
+// Measured (32 rows x 128256, mixed top-k / top-p): 1100 us with a block per row and up to 32 + 32 one-key passes, 62 us now.
+constexpr int kFin = 256, kBins = 128;
 struct SampleShared {
+  uint32_t hist[2][3][kBins];  // this block's tokens per value bin, the low 16 bits of their masses, the rest
+  unsigned long long tot_c[kBins], tot_m[kBins];
   unsigned long long part[2][5];  // this block's totals of a pass: counts (c1 | c2 << 32), c3, masses m1 .. m3
   unsigned long long wred[kVocWarps][5];
   uint32_t list[kFin];
@@ -479,12 +481,90 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
     // the largest key whose tokens (those with keys >= it) reach `goal`: in number, or in mass (by_mass).  Keeping [lo, ..) is
     // enough (c_lo tokens), keeping [hi, ..) is not (c_hi tokens of mass m_hi).
     auto search = [&](bool by_mass, u64 goal, u64 lo, u64 c_lo) -> u64 {
-      u64 hi = 1ull << 32, c_hi = 0, m_hi = 0;
+      u64 hi = (u64)fkey(mx) + 1, c_hi = 0, m_hi = 0;  // (nothing is above the maximum)
       for (int pass = 0; hi - lo > 1 && c_lo - c_hi > (u64)kFin; ++pass) {
         // Logits are spread more evenly over values than over keys (where half of all keys are exponents nothing has): the first
         // pass looks a few temperatures below the maximum, the next ones divide the values between the bounds; from the eighth
         // on the keys are divided, so at most 8 + 16 passes are needed.
         const u64 d = hi - lo;
+        // A mass between two finite values: the tokens go into kBins equal bins of values at once, and the bin that holds the answer is
+        // the next interval (a threshold in the bulk of the vocabulary needs two such passes instead of five or six of three keys,
+        // which weigh nearly as many tokens each: rows of top_p 0.95 85 -> 69 us; counting is cheap, so top-k stays with the keys).
+        // Slices beyond shared memory, whose sums could leave 32 bits, and intervals that no longer split take the keys below.
+        if constexpr (SM) {
+          const float b_lo = fkey_inv((uint32_t)lo), b_hi = fkey_inv((uint32_t)(hi - 1)), scale = (float)kBins / (b_hi - b_lo);
+          if (by_mass && pass > 0 && pass < 8 && lo > 0 && scale > 0.f && scale < 1e30f && b_lo - b_lo == 0.f) {
+            auto bin_of = [&](uint32_t q) { return min(kBins - 1, (int)((fkey_inv(q) - b_lo) * scale)); };
+            uint32_t (&hist)[3][kBins] = sh.hist[turn];
+            for (int e = tid; e < 3 * kBins; e += kVocThreads) (&hist[0][0])[e] = 0;
+            __syncthreads();
+            scan([&](uint32_t q, int) {
+              if (q < (uint32_t)lo || (u64)q >= hi) return;
+              const int at = bin_of(q);
+              atomicAdd(&hist[0][at], 1u);
+              const u64 w = weight(q);
+              atomicAdd(&hist[1][at], (uint32_t)w & 0xffffu);
+              atomicAdd(&hist[2][at], (uint32_t)(w >> 16));
+            });
+            voc_sync();
+            for (int e = tid; e < kBins; e += kVocThreads) {
+              u64 c = 0, m = 0;
+#pragma unroll
+              for (int r = 0; r < kVocCtas; ++r) {
+                uint32_t (&o)[3][kBins] = *cluster_ptr(&hist, r);
+                c += o[0][e];
+                m += o[1][e] + ((u64)o[2][e] << 16);
+              }
+              sh.tot_c[e] = c;
+              sh.tot_m[e] = m;
+            }
+            __syncthreads();
+            turn ^= 1;  // (zeroed again two passes later, behind the barrier that follows every read of it)
+            u64 c4[4], m4[4], c_up = 0, m_up = 0;  // a lane's four bins, then everything above them
+#pragma unroll
+            for (int e = 3; e >= 0; --e) {
+              c4[e] = c_up += sh.tot_c[lane * 4 + e];
+              m4[e] = m_up += sh.tot_m[lane * 4 + e];
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+              const u64 c = __shfl_down_sync(0xffffffffu, c_up, o), m = __shfl_down_sync(0xffffffffu, m_up, o);
+              if (lane + o < 32) { c_up += c; m_up += m; }
+            }
+            u64 c_above = __shfl_down_sync(0xffffffffu, c_up, 1), m_above = __shfl_down_sync(0xffffffffu, m_up, 1);
+            if (lane == 31) c_above = m_above = 0;
+            c_above += c_hi;
+            m_above += m_hi;
+            int best = -1;  // the highest bin that reaches the goal together with everything above it
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (m4[e] + m_above >= goal) best = lane * 4 + e;
+            best = __reduce_max_sync(0xffffffffu, best);
+            if (best >= 0) {
+              const int src = best >> 2, e = best & 3;
+              const u64 c_in = __shfl_sync(0xffffffffu, (e == 0 ? c4[0] : e == 1 ? c4[1] : e == 2 ? c4[2] : c4[3]) + c_above, src);
+              const u64 c_out = __shfl_sync(0xffffffffu, (e == 0 ? c4[1] : e == 1 ? c4[2] : e == 2 ? c4[3] : 0ull) + c_above, src);
+              const u64 m_out = __shfl_sync(0xffffffffu, (e == 0 ? m4[1] : e == 1 ? m4[2] : e == 2 ? m4[3] : 0ull) + m_above, src);
+              auto first_in = [&](int bin) {  // the smallest key of the interval whose bin is at least this one (hi: none)
+                u64 a = lo, z = hi;
+                while (a < z) {
+                  const u64 mid = (a + z) >> 1;
+                  if (bin_of((uint32_t)mid) >= bin) z = mid; else a = mid + 1;
+                }
+                return a;
+              };
+              const u64 n_lo = best == 0 ? lo : first_in(best), n_hi = best == kBins - 1 ? hi : first_in(best + 1);
+              if (n_lo > lo || n_hi < hi) {
+                lo = n_lo;
+                c_lo = c_in;
+                hi = n_hi;
+                c_hi = c_out;
+                m_hi = m_out;
+                continue;
+              }
+            }
+          }
+        }
         u64 t[3];
         const float flo = fkey_inv((uint32_t)lo), fhi = fkey_inv((uint32_t)(hi - 1));
 #pragma unroll
