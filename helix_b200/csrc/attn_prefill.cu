@@ -82,7 +82,7 @@ struct ACfg {
   static constexpr bool STAGE_O = SRC != KV_EXPANDED;
   static constexpr int O_STAGE_BYTES = 32 * DV * 2;  // per softmax warp
   static constexpr int BAR_BYTES = 1024;            // barriers + TMEM pointer, padded so the staging area stays 1024-aligned
-  static constexpr int ORDER_BYTES = 2 * 512;       // kMaxRows entries of the item order
+  static constexpr int ORDER_BYTES = SRC == KV_PACKED ? 2 * 512 : 0;       // kMaxRows entries of the item order
   static constexpr int SMEM = 2 * Q_BYTES + STAGES * (K_BYTES + V_BYTES) + 1024 + BAR_BYTES + (STAGE_O ? 8 * O_STAGE_BYTES : 0) + ORDER_BYTES;
   static constexpr int SUBK = DK / 64, SUBV = DV / 64;  // 64-column swizzle sub-tiles per row
   static_assert(SMEM <= 227 * 1024, "shared memory");
@@ -123,9 +123,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     int max_pages, int Hkv, int chunk, int sink, const float* __restrict__ head_gate, int ldg,
                     int window, float cap_in, float cap_out, const bf16* __restrict__ sink_w,
                     const __grid_constant__ CUtensorMap map_qr, const __grid_constant__ CUtensorMap map_kr,
-                    const __grid_constant__ AttnRuns runs, int vdim) {
+                    const __grid_constant__ AttnRuns runs, int vdim, int sort_rows) {
   using C = ACfg<DK, DV, SRC>;
-  constexpr bool PAGED = SRC == KV_PAGED, EXPANDED = SRC == KV_EXPANDED;
+  constexpr bool PAGED = SRC == KV_PAGED, EXPANDED = SRC == KV_EXPANDED, SORTED = SRC == KV_PACKED;
   constexpr int KST = C::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -185,70 +185,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     it.n1 = it.act1 ? (causal ? min(kv_tiles, (it.q_off + it.q0 + 2 * BQ - 1) / BKV + 1) : kv_tiles) - it.j_lo : 0;
     it.n = max(it.n0, it.n1);
   };
-  // Order of the items: rows (q pair, sequence) by falling number of kv tiles, a row's heads side by side (they share keys), dealt to
-  // the CTAs forth and back (round r of CTA c is item r G + c, or r G + G - 1 - c in odd rounds).  Every CTA sorts the rows itself
-  // (ranks by counting, under a microsecond).  With sequences of unequal length the plain order, q pair by q pair with a slot
-  // for every sequence whether it has that pair or not, left the longest-loaded CTA 24 to 30 % above the mean (6 prompts of 300
-  // to 3000 tokens: 231 tile times of a mean of 187, now 191; 64 chunks of 64 to 512: 74 of 57, now 60).  Measured: 250 -> 232 us and 70.6 -> 63.9 us.
-  // More rows than kMaxRows (or sequences than fit the packed entry) keep the plain order.
-  if (B <= 256 && max_q_pairs <= 255) {
-    uint32_t* keys = reinterpret_cast<uint32_t*>(sK);            // scratch over the K ring (nothing has been loaded yet)
-    uint16_t* ids = reinterpret_cast<uint16_t*>(keys + kMaxRows);
-    const int b = threadIdx.x;
-    Item it;
-    int pairs = 0;
-    if (b < B) {
-      set_seq(it, b);
-      pairs = min(max_q_pairs, max(0, (it.len + QPAIR - 1) / QPAIR));
-    }
-    int upto = pairs;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, upto, o);
-      if (lane >= o) upto += v;
-    }
-    if (lane == 31) s_rows[1 + warp] = upto;
-    __syncthreads();
-    int before = 0, rows = 0;
-    for (int w = 0; w < kThreads / 32; ++w) {
-      if (w < warp) before += s_rows[1 + w];
-      rows += s_rows[1 + w];
-    }
-    if (rows <= kMaxRows) {
-      for (int qp = 0; qp < pairs; ++qp) {
-        const int r = before + upto - pairs + qp;
-        set_pair(it, qp);
-        keys[r] = (uint32_t)(it.n + 2) * kMaxRows + (kMaxRows - 1 - r);
-        ids[r] = (uint16_t)(qp << 8 | b);
-      }
-      __syncthreads();
-      for (int r = threadIdx.x; r < rows; r += kThreads) {
-        const uint32_t key = keys[r];
-        int rank = 0;
-        for (int i = 0; i < rows; ++i) rank += keys[i] > key;
-        s_order[rank] = ids[r];
-      }
-      fence_proxy_async_smem();  // the scratch becomes a target of asynchronous copies
-    }
-    if (threadIdx.x == 0) s_rows[0] = rows <= kMaxRows ? rows : -1;
-  } else if (threadIdx.x == 0) {
-    s_rows[0] = -1;
-  }
-  __syncthreads();
-  const int rows = s_rows[0];
-  const int num_items = (rows >= 0 ? rows : max_q_pairs * B) * Hq;
-  auto item_index = [&](int round) { return round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x); };
-  auto get_item = [&](int idx) {
-    Item it;
-    const int row = idx / Hq;
-    it.h = idx - row * Hq;
-    it.kvh = it.h / group;
-    const int id = rows >= 0 ? s_order[row] : 0;
-    set_seq(it, rows >= 0 ? id & 255 : row % B);
-    set_pair(it, rows >= 0 ? id >> 8 : max_q_pairs - 1 - row / B);
-    return it;
-  };
-
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_k);
@@ -278,10 +214,85 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     tmem_alloc(tmem_ptr, 512);
     tmem_relinquish();
   }
+  // Order of the items: rows (q pair, sequence) by falling number of kv tiles, a row's heads side by side (they share keys), dealt to
+  // the CTAs forth and back (round r of CTA c is item r G + c, or r G + G - 1 - c in odd rounds).  Every CTA sorts the rows itself
+  // (ranks by counting, about a microsecond).  With sequences of unequal length the plain order, q pair by q pair with a slot
+  // for every sequence whether it has that pair or not, left the longest-loaded CTA 24 to 30 % above the mean (6 prompts of 300
+  // to 3000 tokens: 231 tile times of a mean of 187, now 191; 64 chunks of 64 to 512: 74 of 57, now 60).  Measured: 250 -> 233 us and 70.8 -> 62.6 us.
+  // Plain order: launches whose sequences have about equal lengths or whose items fill one round (sort_rows == 0; the sort only cost
+  // its microsecond: 12.3 -> 13.3 us), more rows than kMaxRows, more sequences than fit the packed entry, and, at compile time,
+  // keys from a page pool or an expanded run: portions of a long context are level already, and two of 777 rows over 6000
+  // positions took 204 us with the choice in the item loop, 199 us without.
+  if (SORTED && sort_rows && B <= 256 && max_q_pairs <= 255) {
+    uint32_t* keys = reinterpret_cast<uint32_t*>(sK);            // scratch over the K ring (nothing has been loaded yet)
+    uint16_t* ids = reinterpret_cast<uint16_t*>(keys + kMaxRows);
+    const int b = threadIdx.x;
+    Item it;
+    int pairs = 0;
+    if (b < B) {
+      set_seq(it, b);
+      pairs = min(max_q_pairs, max(0, (it.len + QPAIR - 1) / QPAIR));
+    }
+    int upto = pairs;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    if (lane == 31) s_rows[1 + warp] = upto;
+    __syncthreads();
+    int before = 0, rows = 0;
+    for (int w = 0; w < kThreads / 32; ++w) {
+      if (w < warp) before += s_rows[1 + w];
+      rows += s_rows[1 + w];
+    }
+    if (rows <= kMaxRows) {
+      for (int qp = 0; qp < pairs; ++qp) {
+        const int r = before + upto - pairs + qp;
+        set_pair(it, qp);
+        keys[r] = (uint32_t)(3 * it.n + min(it.n0, it.n1) + 6) * kMaxRows + (kMaxRows - 1 - r);  // (a lone q tile takes about 3/4 of a pair's time)
+        ids[r] = (uint16_t)(qp << 8 | b);
+      }
+      __syncthreads();
+      for (int r = threadIdx.x; r < rows; r += kThreads) {
+        const uint32_t key = keys[r];
+        int rank = 0;
+        for (int i = 0; i < rows; ++i) rank += keys[i] > key;
+        s_order[rank] = ids[r];
+      }
+      fence_proxy_async_smem();  // the scratch becomes a target of asynchronous copies
+    }
+    if (threadIdx.x == 0) s_rows[0] = rows <= kMaxRows ? rows : -1;
+  } else if (SORTED && threadIdx.x == 0) {
+    s_rows[0] = -1;
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);  // warp-uniform for the compiler too
+  const int rows = SORTED ? s_rows[0] : -1;
+  const int num_items = (rows >= 0 ? rows : max_q_pairs * B) * Hq;
+  auto item_index = [&](int round) { return round * (int)gridDim.x + ((rows >= 0 && (round & 1)) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x); };
+  auto get_item = [&](int idx) {
+    Item it;
+    int b, qp;
+    if (rows >= 0) {
+      const int row = idx / Hq;
+      it.h = idx - row * Hq;
+      b = s_order[row] & 255;
+      qp = s_order[row] >> 8;
+    } else {
+      const int per_qp = B * Hq;
+      const int rem = idx % per_qp;
+      qp = max_q_pairs - 1 - idx / per_qp;  // latest q rows first, one "round" per q pair index
+      b = rem / Hq;
+      it.h = rem % Hq;
+    }
+    it.kvh = it.h / group;
+    set_seq(it, b);
+    set_pair(it, qp);
+    return it;
+  };
 
   // The two single-thread roles run their loops and barrier waits with the WHOLE warp converged and only predicate the
   // TMA / tcgen05 instructions on an elect.sync leader: issuing them under `if (lane == 0)` measured slower (the tensor pipe
@@ -690,12 +701,14 @@ cudaError_t launch_p(cudaStream_t stream, const AttnPrefillArgs& a) {
   const int max_q_pairs = (a.max_seqlen + QPAIR - 1) / QPAIR;
   const long long items = (long long)max_q_pairs * a.B * a.Hq;
   const int grid = (int)std::min<long long>(items, effective_sms(num_sms));  // hb_engine_cfg.sm_budget
+  // uneven lengths: a tenth of the (sequence, position) slots or more stay empty
+  const int sort_rows = !PAGED && a.B > 1 && items > grid && 10.0 * a.T < 9.0 * (double)a.B * a.max_seqlen;
   const float scale_log2 = a.scale * 1.4426950408889634f;
   kern<<<grid, kThreads, C::SMEM, stream>>>(mq, mk, mv, mo, a.out, a.ldo, a.cu_seqlens, a.B, a.Hq, a.Hq / a.Hkv, a.causal,
                                             scale_log2, max_q_pairs, a.kv_lens, a.page_table, a.max_pages, a.Hkv,
                                             paged_only(a.block_mask, PAGED), a.unit_sink, a.head_gate, a.ldg,
                                             paged_only(a.window, PAGED), a.softcap > 0.f ? a.scale / a.softcap : 0.f,
-                                            a.softcap > 0.f ? a.softcap * 1.4426950408889634f : 0.f, a.sink, mq, mk, AttnRuns{}, D);
+                                            a.softcap > 0.f ? a.softcap * 1.4426950408889634f : 0.f, a.sink, mq, mk, AttnRuns{}, D, sort_rows);
   return cudaGetLastError();
 }
 
@@ -721,7 +734,7 @@ cudaError_t launch_expanded(cudaStream_t stream, const AttnExpandedArgs& a) {
   const int grid = (int)std::min<long long>(items, effective_sms(num_sms));
   kern<<<grid, kThreads, C::SMEM, stream>>>(mq, mk, mv, mq, a.out, a.ldo, nullptr, a.runs.n, a.H, 1, 1, a.scale * 1.4426950408889634f,
                                             max_q_pairs, nullptr, nullptr, 0, a.H, 0, 0, a.head_gate, a.ldg, a.window, 0.f, 0.f, a.sink,
-                                            mqr, mkr, a.runs, a.vdim);
+                                            mqr, mkr, a.runs, a.vdim, 0);
   return cudaGetLastError();
 }
 
