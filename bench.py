@@ -205,7 +205,7 @@ def hf_session(m, torch, prompt_len, decode):
 
 def host_threads():
     """All host cores for the BLAS behind numpy / torch, whatever the launcher exported (torch.distributed.run sets
-    OMP_NUM_THREADS=1, which made the r01 reference arm single-threaded at N >= 2)."""
+    OMP_NUM_THREADS=1, which makes numpy's BLAS single-threaded at N >= 2)."""
     n = os.cpu_count() or 1
     for k in ("OMP_NUM_THREADS", "OPENBLAS_NUM_THREADS", "MKL_NUM_THREADS"):
         os.environ[k] = str(n)

@@ -216,7 +216,7 @@ def test_replica_broadcast_two_gpus():
     starts empty, receives rank 0's arena by ncclBroadcast over NVLink and then generates exactly rank 0's tokens."""
     import torch
     if torch.cuda.device_count() < 2:
-        pytest.skip("needs 2 GPUs (gpurun --gpus 2)")
+        pytest.skip("needs 2 GPUs")
     d = configs.tiny_llama(layers=2, head_dim=64, vocab=1000)
     uid = replica_unique_id()
     engines = [hb.Engine(hb.EngineConfig(device=i, max_seqs=2, max_ctx=128, max_batched_tokens=128)) for i in range(2)]

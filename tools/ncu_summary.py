@@ -1,7 +1,7 @@
 #!/usr/bin/env python
-"""Summarise ncu outputs brought back in gpurun_out/ into small text files under profiles/ (tracked).
-  python tools/ncu_summary.py launches gpurun_out/r01_launches.csv profiles/r01_launches_summary.txt
-  python tools/ncu_summary.py raw gpurun_out/r01_prof_gemm.ncu-rep profiles/r01_gemm_ncu.txt
+"""Summarise ncu outputs into small text files under profiles/ (tracked).
+  python tools/ncu_summary.py launches launches.csv profiles/launches_summary.txt
+  python tools/ncu_summary.py raw gemm.ncu-rep profiles/gemm_ncu.txt
 """
 import collections
 import csv

@@ -2,7 +2,7 @@
 """Optional same-box comparator: vLLM (the image ships 0.22; the reference pins 0.11.2) on the bench
 workload with dummy (random) weights.  Informational only — not the reference arm, not a parity oracle.
 
-    python tools/vllm_compare.py > profiles/r01_vllm_compare.json
+    python tools/vllm_compare.py > vllm_compare.json
 """
 import json
 import os
