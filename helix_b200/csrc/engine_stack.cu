@@ -408,7 +408,6 @@ int Engine::alloc_runtime_stack() {
   CU(stack_ssm_init());
   CU(stack_streams_init());
   CU(stack_lightning_init());
-  CU(stack_chunk_init());
   CU(attn_latent_init());
   if (!sd.compute_f32) {  // stream-K plans allocate on first use of a shape: make them now, not inside a graph capture
     SmLimitScope sm_scope(cfg_.sm_budget);
@@ -1057,7 +1056,7 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       SPAN(3, 4.0 * T * C * (l.conv_taps + 1) + 12.0 * T * H, short_conv(stream_, ca));
       if (!ca.single) SPAN(3, 8.0 * B * C * l.conv_taps, conv_tails(stream_, ca));
       if (!fused) SPAN(3, 12.0 * T * H, ssm_steps(stream_, k.p1, k.ld1, w.off_a, w.a_dt, f32, k.ab, k.ldab, T, H));
-      RecChunkArgs ra{};
+      LinRecArgs ra{};
       ra.q = k.cv; ra.ldq = k.ldcv; ra.q_off = inner + G * N;
       ra.k = k.cv; ra.ldk = k.ldcv; ra.k_off = inner;
       ra.v = k.cv; ra.ldv = k.ldcv; ra.v_off = 0;
@@ -1068,12 +1067,8 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       ra.state = state_; ra.slot_stride = (long)model_.state_floats; ra.s_off = w.state_off; ra.n_off = 0;
       ra.cu = cu; ra.first_pos = first; ra.slots = sslot;
       ra.B = B; ra.H = H; ra.G = G; ra.Dk = N; ra.Dv = Dv;
-      ra.error = kernel_error_;
       ra.single = T == B;
-      // Portions of 64 tokens and more on average go chunk by chunk, where any part of a chunk costs a whole one: 16 sequences x 32 heads
-      // of 128 x 64 states take 65 us there for 32 to 128 tokens, token by token 39 us for 32, 53 for 48, 163 for 120.
-      if (!f32 && T >= 64 * B && rec_chunk_ok(ra)) SPAN(6, 4.0 * T * H * N * Dv, rec_chunk(stream_, ra));
-      else SPAN(6, 4.0 * T * H * N * Dv, lin_recurrence(stream_, ra));
+      SPAN(6, 4.0 * T * H * N * Dv, lin_recurrence(stream_, ra));
       SPAN(3, 16.0 * T * inner, gated_group_norm(stream_, k.ctx, k.ldctx, k.p1 + w.off_g, k.ld1, w.hnorm, f32, sd.norm_eps, l.norm_groups, mo_f32,
                                                  mo16, T, inner));
     } else if (l.mixer == HB_MIXER_MLSTM) {

@@ -601,14 +601,6 @@ struct LinRecArgs {
   bool single = false;  // every entry is exactly one token
 };
 cudaError_t lin_recurrence(cudaStream_t s, const LinRecArgs& a);
-// The same without normaliser, constant decays and activations, chunk by chunk on the tensor cores with operands in three bf16 terms
-// (stack_chunk.cu): for long portions.  error: a word that the host can read; set to 1 when a wait inside the kernel ran out.
-struct RecChunkArgs : LinRecArgs {
-  int* error = nullptr;
-};
-bool rec_chunk_ok(const RecChunkArgs& a);
-cudaError_t stack_chunk_init();
-cudaError_t rec_chunk(cudaStream_t s, const RecChunkArgs& a);
 // S_t = decay_h S_(t-1) + k_t v_t^T, out_t = S_t^T q_t on the tensor cores, chunk by chunk (stack_lightning.cu): q, k [T, H * Dk] and
 // v [T, H * Dv] are bf16 columns (behind their activations) of rows of stride ld, out fp32, the state as for lin_recurrence.
 // error: a word that the host can read; set to 1 when a wait inside the kernel ran out (results are then void).

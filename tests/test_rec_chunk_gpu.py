@@ -1,5 +1,5 @@
-"""State-space layers over portions that the chunked tensor-core recurrence takes, at the edges of its chunks, channel steps, value slices
-and portions, against the float64 oracle, and against the same tokens fed one by one (the token-by-token kernel)."""
+"""State-space layers over portions of one to many chunks of 128 tokens, ragged ones among them, at head and state sizes from narrow to wide,
+against the float64 oracle, and against the same tokens fed one by one."""
 import numpy as np
 import pytest
 
