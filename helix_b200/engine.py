@@ -5,6 +5,7 @@ for a slot's ``gpu_index`` / ``model_memory_requirement``, load a model, start t
 submit / poll token ids (chat) or call ``embed`` (RAG ingest).
 """
 import ctypes as C
+import operator
 import struct
 from dataclasses import dataclass, field, asdict
 
@@ -440,12 +441,13 @@ class Engine:
         # one array of all tokens, one of all wanted positions, the descriptors packed behind them: arrays and structures made entry by
         # entry took longer than the launches of a decoding step (16 entries: 65 us, 18 now)
         n = len(entries)
-        toks, want, counts = [], [], []
-        for _, t, w in entries:
+        ids, toks, want, counts = [], [], [], []
+        for sid, t, w in entries:
             if type(t) is not np.ndarray or t.dtype != np.int32 or t.ndim != 1:
                 t = np.ascontiguousarray(t, dtype=np.int32).ravel()
             if type(w) is not list or (w and type(w[0]) is not int):
                 w = np.ascontiguousarray(w, dtype=np.int32).ravel().tolist()
+            ids.append(operator.index(sid) & 0xFFFFFFFFFFFFFFFF)
             toks.append(t)
             want += w
             counts.append(len(w))
@@ -455,7 +457,7 @@ class Engine:
         at_t, at_w = flat.ctypes.data, want.ctypes.data
         for i in range(n):
             nt, nw = toks[i].size, counts[i]
-            _FEED.pack_into(feeds, i * _FEED.size, entries[i][0], at_t, nt, at_w if nw else 0, nw)
+            _FEED.pack_into(feeds, i * _FEED.size, ids[i], at_t, nt, at_w if nw else 0, nw)
             at_t += 4 * nt
             at_w += 4 * nw
         arr = (SeqFeedC * n).from_buffer(feeds)
