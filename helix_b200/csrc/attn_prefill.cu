@@ -82,8 +82,9 @@ struct ACfg {
   static constexpr bool STAGE_O = SRC != KV_EXPANDED;
   static constexpr int O_STAGE_BYTES = 32 * DV * 2;  // per softmax warp
   static constexpr int BAR_BYTES = 1024;            // barriers + TMEM pointer, padded so the staging area stays 1024-aligned
-  static constexpr int ORDER_BYTES = SRC == KV_PACKED ? 2 * 512 : 0;       // kMaxRows entries of the item order
-  static constexpr int SMEM = 2 * Q_BYTES + STAGES * (K_BYTES + V_BYTES) + 1024 + BAR_BYTES + (STAGE_O ? 8 * O_STAGE_BYTES : 0) + ORDER_BYTES;
+  static constexpr int SMEM = 2 * Q_BYTES + STAGES * (K_BYTES + V_BYTES) + 1024 + BAR_BYTES + (STAGE_O ? 8 * O_STAGE_BYTES : 0);
+  static constexpr int SMEM_SORTED = SMEM + 2 * kMaxRows;  // the item order behind it
+  static_assert(SRC != KV_PACKED || SMEM_SORTED <= 227 * 1024, "shared memory");
   static constexpr int SUBK = DK / 64, SUBV = DV / 64;  // 64-column swizzle sub-tiles per row
   static_assert(SMEM <= 227 * 1024, "shared memory");
 };
@@ -113,7 +114,7 @@ struct ACfg {
 //                [row0, row0 + kv) of the expanded buffers).  A q / k row has DK / 64 sub-tiles: the head's unrotated part in
 //                all but the last, the rotated part (shared by all heads on the key side) in the last; parts that are no
 //                multiple of 64 wide are zero-filled by the tensor maps.
-template <int DK, int DV, int SRC, int POLY>
+template <int DK, int DV, int SRC, int POLY, bool SORTED>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
@@ -123,9 +124,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     int max_pages, int Hkv, int chunk, int sink, const float* __restrict__ head_gate, int ldg,
                     int window, float cap_in, float cap_out, const bf16* __restrict__ sink_w,
                     const __grid_constant__ CUtensorMap map_qr, const __grid_constant__ CUtensorMap map_kr,
-                    const __grid_constant__ AttnRuns runs, int vdim, int sort_rows) {
+                    const __grid_constant__ AttnRuns runs, int vdim) {
   using C = ACfg<DK, DV, SRC>;
-  constexpr bool PAGED = SRC == KV_PAGED, EXPANDED = SRC == KV_EXPANDED, SORTED = SRC == KV_PACKED;
+  constexpr bool PAGED = SRC == KV_PAGED, EXPANDED = SRC == KV_EXPANDED;
   constexpr int KST = C::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -214,16 +215,15 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     tmem_alloc(tmem_ptr, 512);
     tmem_relinquish();
   }
-  // Order of the items: rows (q pair, sequence) by falling number of kv tiles, a row's heads side by side (they share keys), dealt to
-  // the CTAs forth and back (round r of CTA c is item r G + c, or r G + G - 1 - c in odd rounds).  Every CTA sorts the rows itself
+  // Order of the items (SORTED): rows (q pair, sequence) by falling number of kv tiles, a row's heads side by side (they share keys), dealt
+  // to the CTAs forth and back (round r of CTA c is item r G + c, or r G + G - 1 - c in odd rounds).  Every CTA sorts the rows itself
   // (ranks by counting, about a microsecond).  With sequences of unequal length the plain order, q pair by q pair with a slot
   // for every sequence whether it has that pair or not, left the longest-loaded CTA 24 to 30 % above the mean (6 prompts of 300
   // to 3000 tokens: 231 tile times of a mean of 187, now 191; 64 chunks of 64 to 512: 74 of 57, now 60).  Measured: 250 -> 233 us and 70.8 -> 62.6 us.
-  // Plain order: launches whose sequences have about equal lengths or whose items fill one round (sort_rows == 0; the sort only cost
-  // its microsecond: 12.3 -> 13.3 us), more rows than kMaxRows, more sequences than fit the packed entry, and, at compile time,
-  // keys from a page pool or an expanded run: portions of a long context are level already, and two of 777 rows over 6000
-  // positions took 204 us with the choice in the item loop, 199 us without.
-  if (SORTED && sort_rows && B <= 256 && max_q_pairs <= 255) {
+  // Everything else runs the kernel with the plain walk: launches whose sequences have about equal lengths or whose items fill one round
+  // (the sort only cost its microsecond: 12.3 -> 13.3 us), and keys from a page pool or an expanded run (portions of a long context
+  // are level already).  The plain order also stands in where a launch turns out to have more rows than kMaxRows.
+  if constexpr (SORTED) {
     uint32_t* keys = reinterpret_cast<uint32_t*>(sK);            // scratch over the K ring (nothing has been loaded yet)
     uint16_t* ids = reinterpret_cast<uint16_t*>(keys + kMaxRows);
     const int b = threadIdx.x;
@@ -263,31 +263,36 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       fence_proxy_async_smem();  // the scratch becomes a target of asynchronous copies
     }
     if (threadIdx.x == 0) s_rows[0] = rows <= kMaxRows ? rows : -1;
-  } else if (SORTED && threadIdx.x == 0) {
-    s_rows[0] = -1;
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);  // warp-uniform for the compiler too
   const int rows = SORTED ? s_rows[0] : -1;
-  const int num_items = (rows >= 0 ? rows : max_q_pairs * B) * Hq;
-  auto item_index = [&](int round) { return round * (int)gridDim.x + ((rows >= 0 && (round & 1)) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x); };
+  const int num_items = (SORTED && rows >= 0 ? rows : max_q_pairs * B) * Hq;
+  auto next_item = [&](int idx, int round) {
+    if constexpr (SORTED) {
+      if (rows >= 0) return round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+    }
+    return idx + (int)gridDim.x;
+  };
   auto get_item = [&](int idx) {
     Item it;
-    int b, qp;
-    if (rows >= 0) {
-      const int row = idx / Hq;
-      it.h = idx - row * Hq;
-      b = s_order[row] & 255;
-      qp = s_order[row] >> 8;
-    } else {
-      const int per_qp = B * Hq;
-      const int rem = idx % per_qp;
-      qp = max_q_pairs - 1 - idx / per_qp;  // latest q rows first, one "round" per q pair index
-      b = rem / Hq;
-      it.h = rem % Hq;
+    if constexpr (SORTED) {
+      if (rows >= 0) {
+        const int row = idx / Hq;
+        it.h = idx - row * Hq;
+        it.kvh = it.h / group;
+        set_seq(it, s_order[row] & 255);
+        set_pair(it, s_order[row] >> 8);
+        return it;
+      }
     }
+    const int per_qp = B * Hq;
+    const int qp = max_q_pairs - 1 - idx / per_qp;  // latest q rows first, one "round" per q pair index
+    const int rem = idx % per_qp;
+    const int b = rem / Hq;
+    it.h = rem % Hq;
     it.kvh = it.h / group;
     set_seq(it, b);
     set_pair(it, qp);
@@ -301,7 +306,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const bool leader = elect_one_sync();
     {
       int kt = 0, qi = 0;  // running kv-tile / item counters: barrier phases continue across items
-      for (int round = 0, idx = item_index(0); idx < num_items; idx = item_index(++round)) {
+      for (int round = 0, idx = blockIdx.x; idx < num_items; idx = next_item(idx, ++round)) {
         const Item it = get_item(idx);
         if (!it.valid) continue;
         mbar_wait(q_empty, (qi & 1) ^ 1);  // every S MMA of the previous item has retired: the Q pair buffer is free
@@ -433,7 +438,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       v_advance();
       if (FAST || has_k) k_advance();
     };
-    for (int round = 0, idx = item_index(0); idx < num_items; idx = item_index(++round)) {
+    for (int round = 0, idx = blockIdx.x; idx < num_items; idx = next_item(idx, ++round)) {
       const Item it = get_item(idx);
       if (!it.valid) continue;
       const int nt = t == 0 ? it.n0 : it.n1, n = it.n;
@@ -467,7 +472,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const uint32_t lane_sel = static_cast<uint32_t>(qd * 32) << 16;
     const uint32_t tO = tmem_base + lane_sel + 256 + t * 128;
     int jt = 0;  // kv tiles this warpgroup has processed so far (S buffer and barrier phases)
-    for (int round = 0, idx = item_index(0); idx < num_items; idx = item_index(++round)) {
+    for (int round = 0, idx = blockIdx.x; idx < num_items; idx = next_item(idx, ++round)) {
       const Item it = get_item(idx);
       if (!it.valid) continue;
       const int nt = t == 0 ? it.n0 : it.n1;
@@ -675,7 +680,23 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 }
 
 inline int paged_only(int v, bool paged) { return paged ? v : 0; }
-template <int D, bool PAGED, int POLY>
+int device_sms() {
+  static int num_sms = 0;
+  if (num_sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
+  return num_sms;
+}
+// packed launches that sort their items: uneven lengths (a tenth of the (sequence, position) slots or more stay empty), more items than
+// SMs, and indices that fit the order's entries
+bool sorts_items(const AttnPrefillArgs& a) {
+  const int max_q_pairs = (a.max_seqlen + QPAIR - 1) / QPAIR;
+  return a.B > 1 && a.B <= 256 && max_q_pairs <= 255 && (long long)max_q_pairs * a.B * a.Hq > effective_sms(device_sms()) &&
+         10.0 * a.T < 9.0 * (double)a.B * a.max_seqlen;
+}
+template <int D, bool PAGED, int POLY, bool SORTED>
 cudaError_t launch_p(cudaStream_t stream, const AttnPrefillArgs& a) {
   constexpr int SRC = PAGED ? KV_PAGED : KV_PACKED;
   using C = ACfg<D, D, SRC>;
@@ -691,24 +712,16 @@ cudaError_t launch_p(cudaStream_t stream, const AttnPrefillArgs& a) {
     if (!make_tmap_2d(&mk, a.k, TM_BF16, (uint64_t)a.Hkv * D, (uint64_t)a.T, (uint64_t)a.ldk * 2, 64, BKV)) return cudaErrorInvalidValue;
     if (!make_tmap_2d(&mv, a.v, TM_BF16, (uint64_t)a.Hkv * D, (uint64_t)a.T, (uint64_t)a.ldv * 2, 64, BKV)) return cudaErrorInvalidValue;
   }
-  auto kern = attn_prefill_kernel<D, D, SRC, POLY>;
-  static int num_sms = 0;
-  if (num_sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-  }
+  auto kern = attn_prefill_kernel<D, D, SRC, POLY, SORTED>;
   const int max_q_pairs = (a.max_seqlen + QPAIR - 1) / QPAIR;
   const long long items = (long long)max_q_pairs * a.B * a.Hq;
-  const int grid = (int)std::min<long long>(items, effective_sms(num_sms));  // hb_engine_cfg.sm_budget
-  // uneven lengths: a tenth of the (sequence, position) slots or more stay empty
-  const int sort_rows = !PAGED && a.B > 1 && items > grid && 10.0 * a.T < 9.0 * (double)a.B * a.max_seqlen;
+  const int grid = (int)std::min<long long>(items, effective_sms(device_sms()));  // hb_engine_cfg.sm_budget
   const float scale_log2 = a.scale * 1.4426950408889634f;
-  kern<<<grid, kThreads, C::SMEM, stream>>>(mq, mk, mv, mo, a.out, a.ldo, a.cu_seqlens, a.B, a.Hq, a.Hq / a.Hkv, a.causal,
+  kern<<<grid, kThreads, SORTED ? C::SMEM_SORTED : C::SMEM, stream>>>(mq, mk, mv, mo, a.out, a.ldo, a.cu_seqlens, a.B, a.Hq, a.Hq / a.Hkv, a.causal,
                                             scale_log2, max_q_pairs, a.kv_lens, a.page_table, a.max_pages, a.Hkv,
                                             paged_only(a.block_mask, PAGED), a.unit_sink, a.head_gate, a.ldg,
                                             paged_only(a.window, PAGED), a.softcap > 0.f ? a.scale / a.softcap : 0.f,
-                                            a.softcap > 0.f ? a.softcap * 1.4426950408889634f : 0.f, a.sink, mq, mk, AttnRuns{}, D, sort_rows);
+                                            a.softcap > 0.f ? a.softcap * 1.4426950408889634f : 0.f, a.sink, mq, mk, AttnRuns{}, D);
   return cudaGetLastError();
 }
 
@@ -723,7 +736,7 @@ cudaError_t launch_expanded(cudaStream_t stream, const AttnExpandedArgs& a) {
   if (!make_tmap_3d(&mk, a.k, TM_BF16, a.nope, H, rows, (uint64_t)a.nope * 2, (uint64_t)a.ldkv * 2, 64, 1, BKV)) return cudaErrorInvalidValue;
   if (!make_tmap_3d(&mv, a.v, TM_BF16, a.vdim, H, rows, (uint64_t)a.vdim * 2, (uint64_t)a.ldkv * 2, 64, 1, BKV)) return cudaErrorInvalidValue;
   if (!make_tmap_2d(&mkr, a.k_rot, TM_BF16, a.rot, rows, (uint64_t)a.ldkr * 2, 64, BKV)) return cudaErrorInvalidValue;
-  auto kern = attn_prefill_kernel<DK, DV, KV_EXPANDED, 2>;
+  auto kern = attn_prefill_kernel<DK, DV, KV_EXPANDED, 2, false>;
   int longest = 0;
   for (int i = 0; i < a.runs.n; ++i) longest = std::max(longest, a.runs.len[i]);
   const int max_q_pairs = (longest + QPAIR - 1) / QPAIR;
@@ -734,7 +747,7 @@ cudaError_t launch_expanded(cudaStream_t stream, const AttnExpandedArgs& a) {
   const int grid = (int)std::min<long long>(items, effective_sms(num_sms));
   kern<<<grid, kThreads, C::SMEM, stream>>>(mq, mk, mv, mq, a.out, a.ldo, nullptr, a.runs.n, a.H, 1, 1, a.scale * 1.4426950408889634f,
                                             max_q_pairs, nullptr, nullptr, 0, a.H, 0, 0, a.head_gate, a.ldg, a.window, 0.f, 0.f, a.sink,
-                                            mqr, mkr, a.runs, a.vdim, 0);
+                                            mqr, mkr, a.runs, a.vdim);
   return cudaGetLastError();
 }
 
@@ -779,27 +792,28 @@ int poly_pairs(int D) {
   (void)D;
   return 2;  // measured on B200 (two issuers, 64-wide kv tiles), 0 / 2 / 4 of 8: D=128 1107 / 1171 / 1139, D=64 476 / 501 / 489 TFLOP/s
 }
-template <int D, bool PAGED>
+template <int D, bool PAGED, bool SORTED>
 cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a) {
   switch (poly_pairs(D)) {
-    case 0: return launch_p<D, PAGED, 0>(stream, a);
-    case 4: return launch_p<D, PAGED, 4>(stream, a);
-    default: return launch_p<D, PAGED, 2>(stream, a);
+    case 0: return launch_p<D, PAGED, 0, SORTED>(stream, a);
+    case 4: return launch_p<D, PAGED, 4, SORTED>(stream, a);
+    default: return launch_p<D, PAGED, 2, SORTED>(stream, a);
   }
 }
 
 cudaError_t attn_prefill_init() {
   cudaError_t e;
-#define HB_ATTR1(D_, P_, Y_)                                                                                         \
-  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<D_, D_, P_, Y_>, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
-                                ACfg<D_, D_, P_>::SMEM)) != cudaSuccess)                                             \
+#define HB_ATTR1(D_, P_, Y_, S_)                                                                                     \
+  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<D_, D_, P_, Y_, S_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                S_ ? ACfg<D_, D_, P_>::SMEM_SORTED : ACfg<D_, D_, P_>::SMEM)) != cudaSuccess)         \
     return e;
-#define HB_ATTR(D_, P_) HB_ATTR1(D_, P_, 0) HB_ATTR1(D_, P_, 2) HB_ATTR1(D_, P_, 4)
-  HB_ATTR(128, KV_PACKED) HB_ATTR(128, KV_PAGED) HB_ATTR(64, KV_PACKED) HB_ATTR(64, KV_PAGED)
+#define HB_ATTR(D_, P_, S_) HB_ATTR1(D_, P_, 0, S_) HB_ATTR1(D_, P_, 2, S_) HB_ATTR1(D_, P_, 4, S_)
+  HB_ATTR(128, KV_PACKED, false) HB_ATTR(128, KV_PACKED, true) HB_ATTR(128, KV_PAGED, false)
+  HB_ATTR(64, KV_PACKED, false) HB_ATTR(64, KV_PACKED, true) HB_ATTR(64, KV_PAGED, false)
 #undef HB_ATTR
 #undef HB_ATTR1
 #define HB_ATTRX(K_, V_)                                                                                                  \
-  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<K_, V_, KV_EXPANDED, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<K_, V_, KV_EXPANDED, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                 ACfg<K_, V_, KV_EXPANDED>::SMEM)) != cudaSuccess)                                        \
     return e;
   HB_ATTRX(128, 64) HB_ATTRX(128, 128) HB_ATTRX(192, 64) HB_ATTRX(192, 128)
@@ -816,12 +830,13 @@ cudaError_t attn_prefill(cudaStream_t stream, const AttnPrefillArgs& a) {
   if (a.window < 0 || (a.window > 0 && (!paged || !a.causal || a.block_mask > 0))) return cudaErrorInvalidValue;
   if (paged) {
     if (!a.v_cache || !a.page_table || !a.kv_lens || a.max_pages <= 0 || a.num_pages <= 0 || a.page_size != 64) return cudaErrorInvalidValue;
-    if (a.D == 128) return launch<128, true>(stream, a);
-    if (a.D == 64) return launch<64, true>(stream, a);
+    if (a.D == 128) return launch<128, true, false>(stream, a);
+    if (a.D == 64) return launch<64, true, false>(stream, a);
     return cudaErrorInvalidValue;
   }
-  if (a.D == 128) return launch<128, false>(stream, a);
-  if (a.D == 64) return launch<64, false>(stream, a);
+  const bool sorted = sorts_items(a);
+  if (a.D == 128) return sorted ? launch<128, false, true>(stream, a) : launch<128, false, false>(stream, a);
+  if (a.D == 64) return sorted ? launch<64, false, true>(stream, a) : launch<64, false, false>(stream, a);
   return cudaErrorInvalidValue;
 }
 
