@@ -247,12 +247,23 @@ int hbk_gemm_qkv_rope(const void* A, int lda, const void* W, int ldw, void* qkv,
   cudaFree(cs);
   return kret(e);
 }
+static int sample_impl(const float* logits, int ldl, const float* temperature, const uint64_t* seed, const int32_t* top_k,
+                       const float* top_p, int32_t* out, int B, int V) {
+  void* scratch = nullptr;  // (from the device's pool, in stream order: the call does not wait)
+  if (B > 0 && V > 0 && hb::sample_two_stage(B, V, temperature && (top_k || top_p))) {
+    const cudaError_t e = cudaMallocAsync(&scratch, hb::sample_scratch_bytes(B, V), 0);
+    if (e != cudaSuccess) return kret(e);
+  }
+  const cudaError_t e = hb::sample_tokens(0, logits, ldl, temperature, seed, out, B, V, scratch, top_k, top_p);
+  const cudaError_t e2 = scratch ? cudaFreeAsync(scratch, 0) : cudaSuccess;
+  return kret(e != cudaSuccess ? e : e2);
+}
 int hbk_sample(const float* logits, int ldl, const float* temperature, const uint64_t* seed, int32_t* out, int B, int V) {
-  return kret(hb::sample_tokens(0, logits, ldl, temperature, seed, out, B, V));
+  return sample_impl(logits, ldl, temperature, seed, nullptr, nullptr, out, B, V);
 }
 int hbk_sample_filtered(const float* logits, int ldl, const float* temperature, const uint64_t* seed, const int32_t* top_k,
                         const float* top_p, int32_t* out, int B, int V) {
-  return kret(hb::sample_tokens(0, logits, ldl, temperature, seed, out, B, V, top_k, top_p));
+  return sample_impl(logits, ldl, temperature, seed, top_k, top_p, out, B, V);
 }
 int hbk_apply_penalties(float* logits, int ldl, const int32_t* pen_off, const void* pen, int B, int V) {
   return kret(hb::apply_penalties(0, logits, ldl, pen_off, pen, B, V));

@@ -189,6 +189,7 @@ size_t Engine::workspace_bytes() const {
     b += al256((size_t)cfg_.max_seqs * d.vocab * 4);          // logits
     b += al256(attn_decode_workspace_floats(cfg_.max_seqs, d.heads, d.head_dim, 16) * 4);
     b += al256((size_t)cfg_.max_seqs * 4);                    // sampled
+    b += al256(sample_scratch_bytes(cfg_.max_seqs, d.vocab)); // argmax partials
     b += 2 * al256((size_t)cfg_.max_seqs * HB_MAX_LOGPROBS * 4);  // log-probability records of one step
     b += al256((size_t)(5 * d.layers + 1 + 9 * d.layers + 2) * sizeof(int));  // hand-over counters + dependency flags of the decode step
     b += al256(fused_counter_ints(d) * sizeof(int));              // tile arrival counters of the fused decode GEMMs
@@ -339,6 +340,7 @@ int Engine::alloc_runtime() {
     logits_ = (float*)take((size_t)cfg_.max_seqs * d.vocab * 4);
     dec_ws_ = (float*)take(attn_decode_workspace_floats(cfg_.max_seqs, d.heads, d.head_dim, 16) * 4);
     sampled_ = (int32_t*)take((size_t)cfg_.max_seqs * 4);
+    sample_ws_ = take(sample_scratch_bytes(cfg_.max_seqs, d.vocab));
     sig_ = (int*)take((size_t)(5 * d.layers + 1 + 9 * d.layers + 2) * sizeof(int));
     dep_ = sig_ + (5 * d.layers + 1);  // dependency flags of the decode chain follow the hand-over counters (one memset)
     {
@@ -735,8 +737,9 @@ int Engine::sample_step(int B, const StepLayout& L) {
   const bool filt = (step_flags_ & STEP_FILTER) != 0;
   if (step_flags_ & STEP_PENALTY)
     SPAN(3, 0.0, apply_penalties(stream_, logits_, d.vocab, (const int32_t*)(d_step_ + L.pen_off), d_step_ + L.pen, B, d.vocab));
-  SPAN(3, 4.0 * B * d.vocab, sample_tokens(stream_, logits_, d.vocab, temp, seed, sampled_, B, d.vocab, filt ? topk : nullptr,
-                                           filt ? topp : nullptr));
+  SPAN(3, 4.0 * B * d.vocab, sample_tokens(stream_, logits_, d.vocab, temp, seed, sampled_, B, d.vocab, sample_ws_,
+                                           filt ? topk : nullptr, filt ? topp : nullptr));
+  if (sample_two_stage(B, d.vocab, filt)) launches_.fetch_add(1, std::memory_order_relaxed);  // two kernels behind one call
   if (step_flags_ & STEP_LOGPROBS)
     SPAN(3, 4.0 * B * d.vocab, logprob_topk(stream_, logits_, d.vocab, d.vocab, sampled_, (const int32_t*)(d_step_ + L.lpw),
                                             lp_ids_, lp_vals_, B, HB_MAX_LOGPROBS));

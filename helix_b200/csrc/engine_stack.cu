@@ -388,6 +388,7 @@ size_t Engine::workspace_bytes_stack() const {
   b += al256(T * (size_t)up8(mo) * 4) + al256(T * (size_t)up8(mo) * 2);   // mo, mo16
   b += al256((size_t)cfg_.max_seqs * sd.vocab * 4);                   // logits
   b += al256((size_t)cfg_.max_seqs * 4);                              // sampled
+  b += al256(sample_scratch_bytes(cfg_.max_seqs, sd.vocab));
   b += 2 * al256((size_t)cfg_.max_seqs * HB_MAX_LOGPROBS * 4);
   if (!sd.compute_f32) b += al256(stack_skinny_floats(model_) * 4) + al256(T * (size_t)up8(n2) * 2) + al256(T * (size_t)up8(cx) * 2);
   {
@@ -547,6 +548,7 @@ int Engine::alloc_runtime_stack() {
   sk_.mo16 = (bf16*)take(T * (size_t)sk_.ldmo * 2);
   logits_ = (float*)take((size_t)cfg_.max_seqs * sd.vocab * 4);
   sampled_ = (int32_t*)take((size_t)cfg_.max_seqs * 4);
+  sample_ws_ = take(sample_scratch_bytes(cfg_.max_seqs, sd.vocab));
   lp_ids_ = (int32_t*)take((size_t)cfg_.max_seqs * HB_MAX_LOGPROBS * 4);
   lp_vals_ = (float*)take((size_t)cfg_.max_seqs * HB_MAX_LOGPROBS * 4);
   skinny_ws_ = sd.compute_f32 ? nullptr : (float*)take(stack_skinny_floats(model_) * 4);

@@ -99,8 +99,10 @@ cudaError_t rope_table(cudaStream_t s, const int32_t* positions, const float* in
 // Greedy / Gumbel-max sampling over fp32 logits[B,V]: out[b] = argmax_v(logits[b,v]/temp[b] + g(seed[b],v)),
 // temp[b] <= 0 -> pure argmax (lowest index wins ties).
 cudaError_t sample_tokens(cudaStream_t s, const float* logits, int ldl, const float* temperature, const uint64_t* seed,
-                          int32_t* out, int B, int V, const int32_t* top_k = nullptr,
+                          int32_t* out, int B, int V, void* scratch, const int32_t* top_k = nullptr,
                           const float* top_p = nullptr);  // per-row top-k (<=0 off) / top-p (outside (0,1) off), sampled rows only
+bool sample_two_stage(int B, int V, bool filtered);  // sample_tokens is two kernels and needs the scratch below (else one, without)
+size_t sample_scratch_bytes(int B, int V);
 // logits[b, tok] -= val for the entries {int32 tok; float val} [pen_off[b], pen_off[b+1]) of row b (distinct tokens per row)
 cudaError_t apply_penalties(cudaStream_t s, float* logits, int ldl, const int32_t* pen_off, const void* pen, int B, int V);
 // rows with width[b] > 0: out_ids/out_lp[b][0] = sampled token and its log-softmax, [1..width) = most likely tokens (desc)

@@ -293,6 +293,88 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {  // splitmix64 finaliser
 __device__ __forceinline__ void argmax_merge(float& best, int& bi, float ov, int oi) {
   if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
 }
+// standard Gumbel noise of (seed, column)
+__device__ __forceinline__ float gumbel(uint64_t sd, int v) {
+  const uint64_t h = mix64(sd ^ (0xD1B54A32D192ED03ull * (uint64_t)(v + 1)));
+  // 23 random bits + 0.5: every value is exact in fp32 and u stays strictly inside (0,1) — with 24 bits the
+  // "+0.5f" rounds the top half of the range up and u == 1.0 made the noise +inf (a uniformly random token won
+  // once per 2^24 draws, ~0.8 % of sampled tokens at a 128k vocabulary).  The inner log is the accurate one: the
+  // fast-math log has an absolute error comparable to log(1 - 2^-24).
+  const float u = ((float)(h >> 41) + 0.5f) * (1.0f / 8388608.0f);
+  return -__logf(-logf(u));
+}
+template <int NT>
+__device__ __forceinline__ void block_argmax(float& best, int& bi, float* sval, int* sidx) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    argmax_merge(best, bi, ov, oi);
+  }
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) { sval[w] = best; sidx[w] = bi; }
+  __syncthreads();
+  if (w == 0) {
+    best = (l < NT / 32) ? sval[l] : -INFINITY;
+    bi = (l < NT / 32) ? sidx[l] : 0x7fffffff;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      argmax_merge(best, bi, ov, oi);
+    }
+  }
+}
+
+// ---- sampling without filters: one look at every logit, in two launches ----
+// stage 1: grid (chunks, B): per-chunk argmax of logits/T + Gumbel noise -> part[b][chunk]
+constexpr int kSampleChunk = 4096;  // vocabulary columns per stage-1 block
+__global__ void __launch_bounds__(256)
+sample_stage1_kernel(const float* __restrict__ logits, int ldl, const float* __restrict__ temperature,
+                     const uint64_t* __restrict__ seed, float* __restrict__ part_val, int* __restrict__ part_idx, int V) {
+  __shared__ float sval[8];
+  __shared__ int sidx[8];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int b = blockIdx.y, chunk = blockIdx.x;
+  const float* row = logits + (size_t)b * ldl;
+  const float temp = temperature ? temperature[b] : 0.f;
+  const bool greedy = !(temp > 0.f);
+  const float inv_t = greedy ? 1.f : 1.f / temp;
+  const uint64_t sd = seed ? seed[b] : 0;
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  const int v_end = min(V, (chunk + 1) * kSampleChunk);
+  for (int v = chunk * kSampleChunk + threadIdx.x; v < v_end; v += 256) {
+    float x = row[v] * inv_t;
+    if (!greedy) x += gumbel(sd, v);
+    argmax_merge(best, bi, x, v);
+  }
+  block_argmax<256>(best, bi, sval, sidx);
+  if (threadIdx.x == 0) {
+    part_val[b * gridDim.x + chunk] = best;
+    part_idx[b * gridDim.x + chunk] = bi;
+  }
+}
+// stage 2: one warp per row merges the chunk winners (lowest index wins ties, as in stage 1)
+__global__ void __launch_bounds__(32)
+sample_stage2_kernel(const float* __restrict__ part_val, const int* __restrict__ part_idx, int32_t* __restrict__ out,
+                     int chunks) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int b = blockIdx.x;
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  for (int c = threadIdx.x; c < chunks; c += 32) argmax_merge(best, bi, part_val[b * chunks + c], part_idx[b * chunks + c]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    argmax_merge(best, bi, ov, oi);
+  }
+  if (threadIdx.x == 0) out[b] = bi < 0x7fffffff ? bi : 0;  // all-NaN row: emit a valid id, never an out-of-range one
+}
+
 // float -> unsigned key that orders like the float (and back); NaN is key 0, below every number, and key 0 is a NaN.  (The bits
 // change type in asm: the compiler may turn integer operations on a float's sign into float ones, which lose a NaN's bits.)
 __device__ __forceinline__ uint32_t fkey(float x) {
@@ -673,15 +755,7 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
     if (raw < floor_logit) return;
     const int v = start + i;
     float x = raw * inv_t;
-    if (!greedy) {
-      const uint64_t h = mix64(sd ^ (0xD1B54A32D192ED03ull * (uint64_t)(v + 1)));
-      // 23 random bits + 0.5: every value is exact in fp32 and u stays strictly inside (0,1) — with 24 bits the
-      // "+0.5f" rounds the top half of the range up and u == 1.0 made the noise +inf (a uniformly random token won
-      // once per 2^24 draws, ~0.8 % of sampled tokens at a 128k vocabulary).  The inner log is the accurate one: the
-      // fast-math log has an absolute error comparable to log(1 - 2^-24).
-      const float u = ((float)(h >> 41) + 0.5f) * (1.0f / 8388608.0f);
-      x += -__logf(-logf(u));
-    }
+    if (!greedy) x += gumbel(sd, v);
     argmax_merge(best, bi, x, v);
   });
   // lowest index wins ties, in whatever order the blocks' winners are merged
@@ -970,9 +1044,25 @@ cudaError_t launch_voc(K* on_chip, K* in_memory, cudaStream_t s, int B, int V, A
   return launch_k(fits ? on_chip : in_memory, dim3(B * kVocCtas), dim3(kVocThreads), fits ? floats * 4 : 0, s, true, args...);
 }
 }  // namespace
+// Rows without filters are looked at once, so nothing is gained by keeping them on chip: two launches over chunks of the row, with room
+// for the chunks' winners, unless the clusters of few short rows are through sooner.  Us, clusters | two launches: 32 rows of
+// 32768, temperature 8.6 | 9.7, 64 rows of 32768 15.8 | 12.4, greedy 10.8 | 7.3, 256 rows of 8192 34 | 12.5, greedy 28 | 7.2, 1 row
+// of 128256 12.6 | 7.5, 256 rows of 128256 140 | 93, greedy 71 | 42.
+bool sample_two_stage(int B, int V, bool filtered) { return !filtered && !(B <= 32 && V <= 32768); }
+size_t sample_scratch_bytes(int B, int V) { return (size_t)B * ((V + kSampleChunk - 1) / kSampleChunk) * 8; }
+
 cudaError_t sample_tokens(cudaStream_t s, const float* logits, int ldl, const float* temperature, const uint64_t* seed,
-                          int32_t* out, int B, int V, const int32_t* top_k, const float* top_p) {
+                          int32_t* out, int B, int V, void* scratch, const int32_t* top_k, const float* top_p) {
   if (B <= 0) return cudaSuccess;
+  if (V <= 0) return cudaErrorInvalidValue;
+  if (sample_two_stage(B, V, temperature && (top_k || top_p))) {
+    const int chunks = (V + kSampleChunk - 1) / kSampleChunk;
+    float* pv = static_cast<float*>(scratch);
+    int* pi = reinterpret_cast<int*>(pv + (size_t)B * chunks);
+    const cudaError_t e = launch_k(sample_stage1_kernel, dim3(chunks, B), dim3(256), 0, s, true, logits, ldl, temperature, seed, pv, pi, V);
+    if (e != cudaSuccess) return e;
+    return launch_k(sample_stage2_kernel, dim3(B), dim3(32), 0, s, true, (const float*)pv, (const int*)pi, out, chunks);
+  }
   return launch_voc(sample_kernel<true>, sample_kernel<false>, s, B, V, logits, ldl, temperature, seed, top_k, top_p, out, V);
 }
 cudaError_t apply_penalties(cudaStream_t s, float* logits, int ldl, const int32_t* pen_off, const void* pen, int B, int V) {

@@ -124,3 +124,27 @@ def test_nan_logits_are_never_drawn(V, filtered):
     assert L.hbk_sample_filtered(p(x), V, p(temp), p(seed), p(tk), None, p(out), B, V) == 0
     torch.cuda.synchronize()
     assert set(out.tolist()) == set(keep)
+
+
+@pytest.mark.parametrize("B,V", [(32, 32768), (33, 32768), (32, 32769), (1, 40000), (40, 1), (40, 4095), (40, 4096), (40, 8193), (200, 1000), (3, 400009)])
+def test_rows_without_filters_take_the_same_tokens_either_way(B, V):
+    """Rows without filters go through two launches over chunks or, few short ones and those of filtered steps, through a cluster per row:
+    the same noise and the same order of ties, so the same tokens."""
+    L = hb.lib()
+    x = rows_of(V, V + 1, B + V, max(B, 6))
+    B = x.shape[0]
+    temp = torch.tensor([0.0 if b % 3 == 0 else 0.7 for b in range(B)], device="cuda")
+    seed = torch.arange(B, device="cuda", dtype=torch.int64) * 104729
+    no_k, no_p = torch.zeros(B, device="cuda", dtype=torch.int32), torch.ones(B, device="cuda")
+    a, b = torch.full((B,), -1, device="cuda", dtype=torch.int32), torch.full((B,), -1, device="cuda", dtype=torch.int32)
+    assert L.hbk_sample(p(x), V + 1, p(temp), p(seed), p(a), B, V) == 0
+    assert L.hbk_sample_filtered(p(x), V + 1, p(temp), p(seed), p(no_k), p(no_p), p(b), B, V) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(a, b) and (a >= 0).all() and (a < V).all()
+
+
+def test_no_columns_are_refused():
+    L = hb.lib()
+    out = torch.zeros(2, device="cuda", dtype=torch.int32)
+    x = torch.zeros(2, device="cuda")
+    assert L.hbk_sample(p(x), 1, None, None, p(out), 2, 0) != 0
