@@ -270,7 +270,7 @@ int hbk_apply_penalties(float* logits, int ldl, const int32_t* pen_off, const vo
 }
 int hbk_logprob_topk(const float* logits, int ldl, int V, const int32_t* sampled, const int32_t* width, int32_t* out_ids,
                      float* out_lp, int B, int max_width) {
-  return kret(hb::logprob_topk(0, logits, ldl, V, sampled, width, out_ids, out_lp, B, max_width));
+  return kret(hb::logprob_topk(0, logits, ldl, V, sampled, width, out_ids, out_lp, B, max_width, max_width));
 }
 int hbk_cls_pool_l2(const void* x, const int32_t* first_row, float* out, int B, int H) {
   return kret(hb::cls_pool_l2(0, (const hb::bf16*)x, first_row, out, B, H));

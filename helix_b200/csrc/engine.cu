@@ -742,7 +742,7 @@ int Engine::sample_step(int B, const StepLayout& L) {
   if (sample_two_stage(B, d.vocab, filt)) launches_.fetch_add(1, std::memory_order_relaxed);  // two kernels behind one call
   if (step_flags_ & STEP_LOGPROBS)
     SPAN(3, 4.0 * B * d.vocab, logprob_topk(stream_, logits_, d.vocab, d.vocab, sampled_, (const int32_t*)(d_step_ + L.lpw),
-                                            lp_ids_, lp_vals_, B, HB_MAX_LOGPROBS));
+                                            lp_ids_, lp_vals_, B, HB_MAX_LOGPROBS, (step_flags_ & STEP_WIDE_RECORDS) ? HB_MAX_LOGPROBS : 2));
   return HB_OK;
 }
 
@@ -1237,6 +1237,7 @@ size_t Engine::fill_sampling(Request* const* batch, int B, const StepLayout& L, 
     lpw[i] = std::max(0, std::min(r->sp.logprobs, (int)HB_MAX_LOGPROBS));
     if (wants_filter(r->sp, model_.d.vocab)) step_flags_ |= STEP_FILTER;
     if (lpw[i] > 0) step_flags_ |= STEP_LOGPROBS;
+    if (lpw[i] > 2) step_flags_ |= STEP_WIDE_RECORDS;
     pen_off[i] = (int32_t)n;
     if (r->sp.presence_penalty != 0.f || r->sp.frequency_penalty != 0.f) {
       step_flags_ |= STEP_PENALTY;

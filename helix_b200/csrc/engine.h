@@ -54,7 +54,7 @@ struct Request {
 struct StepLayout {
   size_t tokens, positions, slots, cu, last, ctx, pt, temp, seed, topk, topp, lpw, pen_off, sslot, first, seqof, rows, prev, pen, total;
 };
-enum StepFlags : int { STEP_FILTER = 1, STEP_PENALTY = 2, STEP_LOGPROBS = 4 };
+enum StepFlags : int { STEP_FILTER = 1, STEP_PENALTY = 2, STEP_LOGPROBS = 4, STEP_WIDE_RECORDS = 8 /* of more than two tokens */ };
 
 class Engine {
  public:

@@ -390,21 +390,27 @@ __device__ __forceinline__ float fkey_inv(uint32_t k) {
   return x;
 }
 
-// ---- rows of the vocabulary, one cluster of kVocCtas blocks per row ----
-// Both kernels below look at a row many times (bisection passes, arg-max rounds).  One block per row left most SMs idle and read
-// 0.5 MB through one SM's L1 per pass; here every block keeps an eighth of the row in shared memory, passes run on the slices and
-// what they find meets through distributed shared memory, one cluster barrier per pass.  Rows whose slices do not fit
-// (vocabularies above 400k) are read from global memory instead (SM = false).
-constexpr int kVocCtas = 8, kVocThreads = 512, kVocWarps = kVocThreads / 32;
-constexpr int kVocSmemFloats = 50000;  // largest slice kept on chip (200 KB)
-__host__ __device__ inline int voc_slice(int V) { return ((V + kVocCtas - 1) / kVocCtas + 3) & ~3; }
+// ---- rows of the vocabulary, one cluster of NC blocks per row ----
+// Both kernels below look at a row many times (bisection passes, arg-max rounds).  Reading 0.5 MB through one SM's L1 per pass left most
+// SMs idle; here every block keeps its part of the row in shared memory, passes run on the parts and what they find meets through
+// distributed shared memory, one cluster barrier per pass.  Rows whose eighths do not fit (vocabularies above 400k) are read
+// from global memory instead (SM = false).
+constexpr int kVocThreads = 512, kVocWarps = kVocThreads / 32;
+constexpr int kVocSmemFloats = 50000;  // largest part kept on chip (200 KB)
+__host__ __device__ inline int voc_slice(int V, int ctas) { return ((V + ctas - 1) / ctas + 3) & ~3; }
 
-__device__ __forceinline__ void voc_sync() {  // (the aligned barrier wants converged warps)
-  __syncwarp();
-  cluster_sync_all();
+template <int NC>
+__device__ __forceinline__ void voc_sync() {
+  if constexpr (NC == 1) {
+    __syncthreads();
+  } else {  // (the aligned barrier wants converged warps)
+    __syncwarp();
+    cluster_sync_all();
+  }
 }
-template <typename T>
+template <int NC, typename T>
 __device__ __forceinline__ T* cluster_ptr(T* p, uint32_t cta) {  // the same shared-memory object in another block of the cluster
+  if constexpr (NC == 1) return p;
   uint64_t r;
   asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t>(p)), "r"(cta));
   return reinterpret_cast<T*>(r);
@@ -442,7 +448,7 @@ __device__ __forceinline__ void load_slice(const float* __restrict__ src, int n,
 //   top-k : the largest key that keeps >= k tokens (ties at the k-th value are all kept)
 //   top-p : among the top-k survivors, the largest key whose tokens' softmax(logits/T) mass reaches p of the survivors' mass
 // Probability mass is accumulated in 2^-32 fixed point, so every sum is exact and independent of its order.  A pass compares a
-// slice with three keys inside the interval that still holds the answer; once the interval holds at most kFin tokens, block 0
+// part with three keys inside the interval that still holds the answer; once the interval holds at most kFin tokens, block 0
 // gets them and finds the answer directly.
 // Measured (32 rows x 128256, mixed top-k / top-p): 1100 us with a block per row and up to 32 + 32 one-key passes, 62 us now.
 constexpr int kFin = 256, kBins = 128;
@@ -460,8 +466,8 @@ struct SampleShared {
   int best_idx;
 };
 
-template <bool SM>
-__global__ void __cluster_dims__(kVocCtas, 1, 1) __launch_bounds__(kVocThreads)
+template <int NC, bool SM>
+__global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(kVocThreads)
 sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict__ temperature, const uint64_t* __restrict__ seed,
               const int32_t* __restrict__ top_k, const float* __restrict__ top_p, int32_t* __restrict__ out, int V) {
   extern __shared__ __align__(16) uint32_t keys[];
@@ -469,9 +475,9 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
   pdl_launch_dependents();
   pdl_wait();
   typedef unsigned long long u64;
-  const int b = blockIdx.x / kVocCtas, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int b = blockIdx.x / NC, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
-  const int per = voc_slice(V), start = min(V, (int)rank * per), n = min(V, start + per) - start;
+  const int per = voc_slice(V, NC), start = min(V, (int)rank * per), n = min(V, start + per) - start;
   const float* row = logits + (size_t)b * ldl + start;
   const float temp = temperature ? temperature[b] : 0.f;
   const bool greedy = !(temp > 0.f);
@@ -519,8 +525,8 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
     mx = sh.val[lane & (kVocWarps - 1)];
     mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(mx)));
     if (tid == 0) sh.row_max = mx;
-    voc_sync();
-    mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(*cluster_ptr(&sh.row_max, lane & (kVocCtas - 1)))));
+    voc_sync<NC>();
+    mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(*cluster_ptr<NC>(&sh.row_max, lane & (NC - 1)))));
 
     auto weight = [&](uint32_t key) -> u64 {
       const float e = __expf((fkey_inv(key) - mx) * inv_t) * 4294967296.0f;
@@ -550,12 +556,12 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
           if (lane == 0) sh.part[turn][j] = t;
         }
       }
-      voc_sync();
+      voc_sync<NC>();
 #pragma unroll
       for (int j = 0; j < 5; ++j) {
-        u64 t = *cluster_ptr(&sh.part[turn][j], lane & (kVocCtas - 1));
+        u64 t = *cluster_ptr<NC>(&sh.part[turn][j], lane & (NC - 1));
 #pragma unroll
-        for (int o = kVocCtas / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        for (int o = NC / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
         v[j] = t;
       }
       turn ^= 1;  // (a slot is written again two passes later, behind the barrier that follows every read of it)
@@ -588,12 +594,12 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
               atomicAdd(&hist[1][at], (uint32_t)w & 0xffffu);
               atomicAdd(&hist[2][at], (uint32_t)(w >> 16));
             });
-            voc_sync();
+            voc_sync<NC>();
             for (int e = tid; e < kBins; e += kVocThreads) {
               u64 c = 0, m = 0;
 #pragma unroll
-              for (int r = 0; r < kVocCtas; ++r) {
-                uint32_t (&o)[3][kBins] = *cluster_ptr(&hist, r);
+              for (int r = 0; r < NC; ++r) {
+                uint32_t (&o)[3][kBins] = *cluster_ptr<NC>(&hist, r);
                 c += o[0][e];
                 m += o[1][e] + ((u64)o[2][e] << 16);
               }
@@ -697,9 +703,9 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
       // few tokens left: block 0 decides
       scan([&](uint32_t q, int) {
         if (q < lo || (u64)q >= hi || q == 0) return;
-        cluster_ptr(sh.list, 0)[atomicAdd(cluster_ptr(&sh.n_list, 0), 1u)] = q;
+        cluster_ptr<NC>(sh.list, 0)[atomicAdd(cluster_ptr<NC>(&sh.n_list, 0), 1u)] = q;
       });
-      voc_sync();
+      voc_sync<NC>();
       if (rank == 0) {
         const int nl = (int)sh.n_list;
         for (int i = tid; i < nl; i += kVocThreads) sh.mass[i] = weight(sh.list[i]);
@@ -720,11 +726,11 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
         __syncthreads();
         if (warp == 0) {
           const uint32_t r = __reduce_max_sync(0xffffffffu, (uint32_t)sh.idx[lane & (kVocWarps - 1)]);
-          if (lane < kVocCtas) *cluster_ptr(&sh.result, lane) = r;
+          if (lane < NC) *cluster_ptr<NC>(&sh.result, lane) = r;
           if (lane == 0) sh.n_list = 0;
         }
       }
-      voc_sync();
+      voc_sync<NC>();
       return sh.result > lo ? sh.result : lo;
     };
     u64 lo = 0;
@@ -773,12 +779,12 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
     sh.best_val = best;
     sh.best_idx = bi;
   }
-  voc_sync();
+  voc_sync<NC>();
   if (rank == 0 && tid == 0) {
-    for (int c = 1; c < kVocCtas; ++c) argmax_merge(best, bi, *cluster_ptr(&sh.best_val, c), *cluster_ptr(&sh.best_idx, c));
+    for (int c = 1; c < NC; ++c) argmax_merge(best, bi, *cluster_ptr<NC>(&sh.best_val, c), *cluster_ptr<NC>(&sh.best_idx, c));
     out[b] = bi < 0x7fffffff ? bi : 0;  // all-NaN row: emit a valid id, never an out-of-range one
   }
-  voc_sync();  // no block's shared memory goes away while block 0 reads it
+  voc_sync<NC>();  // no block's shared memory goes away while block 0 reads it
 }
 
 // ---- OpenAI presence / frequency penalties: logits[b, tok] -= val for the (tok, val) entries of row b ----
@@ -798,36 +804,97 @@ apply_penalties_kernel(float* __restrict__ logits, int ldl, const int32_t* __res
 }
 
 // ---- log-probabilities of the sampled token and of the width-1 most likely tokens (descending, lowest id on ties) ----
-// Every block picks the width-1 best of its slice (a thread remembers the best of its own entries; after a round only the entries
-// of the thread that owned the winner are looked at again, by its whole warp), block 0 merges the eight short lists by rank.
+// One block per row that reads it twice and once more per further pick: for narrow records (logprob_topk below).
+constexpr int kLpThreads = 1024;
+__global__ void __launch_bounds__(kLpThreads)
+logprob_row_kernel(const float* __restrict__ logits, int ldl, int V, const int32_t* __restrict__ sampled,
+                    const int32_t* __restrict__ width, int32_t* __restrict__ out_ids, float* __restrict__ out_lp,
+                    int max_width) {
+  __shared__ float sval[kLpThreads / 32];
+  __shared__ int sidx[kLpThreads / 32];
+  __shared__ float red[kLpThreads / 32];
+  __shared__ float s_bv;
+  __shared__ int s_bi;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int b = blockIdx.x;
+  const int w = min(width[b], max_width);
+  if (w <= 0) return;
+  const float* row = logits + (size_t)b * ldl;
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  for (int v = threadIdx.x; v < V; v += kLpThreads) argmax_merge(best, bi, row[v], v);
+  block_argmax<kLpThreads>(best, bi, sval, sidx);
+  if (threadIdx.x == 0) { s_bv = best; s_bi = bi; }
+  __syncthreads();
+  const float mx = s_bv;
+  float se = 0.f;
+  for (int v = threadIdx.x; v < V; v += kLpThreads) se += expf(row[v] - mx);
+  se = block_sum<kLpThreads>(se, red);
+  const float lse = mx + logf(se);
+  int32_t* ids = out_ids + (size_t)b * max_width;
+  float* lps = out_lp + (size_t)b * max_width;
+  if (threadIdx.x == 0) {
+    const int t = sampled[b];
+    ids[0] = t;
+    lps[0] = (t >= 0 && t < V) ? row[t] - lse : -INFINITY;
+  }
+  float pv = s_bv;   // the j-th most likely token in the order (value desc, id asc); j = 1 is the argmax found above
+  int pi = s_bi;
+  for (int j = 1; j < w; ++j) {
+    if (threadIdx.x == 0) { ids[j] = pi; lps[j] = pv - lse; }
+    if (j + 1 == w) break;
+    best = -INFINITY;
+    bi = 0x7fffffff;
+    for (int v = threadIdx.x; v < V; v += kLpThreads) {
+      const float x = row[v];
+      if (x < pv || (x == pv && v > pi)) argmax_merge(best, bi, x, v);  // strictly after the previous pick
+    }
+    __syncthreads();  // sval/sidx reuse
+    block_argmax<kLpThreads>(best, bi, sval, sidx);
+    if (threadIdx.x == 0) { s_bv = best; s_bi = bi; }
+    __syncthreads();
+    pv = s_bv;
+    pi = s_bi;
+    if (pi == 0x7fffffff) {  // fewer than `w` finite logits in the row
+      if (threadIdx.x == 0)
+        for (int k = j + 1; k < w; ++k) { ids[k] = -1; lps[k] = -INFINITY; }
+      break;
+    }
+  }
+}
+
+// The same, a row shared by NC blocks.
+// Every block picks the width-1 best of its part (a thread remembers the best of its own entries; after a round only the entries
+// of the thread that owned the winner are looked at again, by its whole warp), block 0 merges the short lists by rank.
 // Measured (32 rows x 128256, width 6): 69 us with a block per row that read it once per pick, 16 us now.
 constexpr int kLpMax = 32;  // picks per merge; wider records take several
+template <int NC>
 struct LpShared {
   uint32_t wkey[2][kVocWarps];
   int widx[2][kVocWarps];
   uint32_t top_key[kLpMax];
   int top_idx[kLpMax];
-  uint32_t all_key[kVocCtas * kLpMax];
-  int all_idx[kVocCtas * kLpMax];
+  uint32_t all_key[NC * kLpMax];
+  int all_idx[NC * kLpMax];
   float red[kVocWarps];
   float part_max, part_sum;
   uint32_t last_key;
   int last_idx;
 };
-template <bool SM>
-__global__ void __cluster_dims__(kVocCtas, 1, 1) __launch_bounds__(kVocThreads)
+template <int NC, bool SM>
+__global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(kVocThreads)
 logprob_topk_kernel(const float* __restrict__ logits, int ldl, int V, const int32_t* __restrict__ sampled,
                     const int32_t* __restrict__ width, int32_t* __restrict__ out_ids, float* __restrict__ out_lp, int max_width) {
   extern __shared__ __align__(16) float slice[];
-  __shared__ LpShared sh;
+  __shared__ LpShared<NC> sh;
   pdl_launch_dependents();
   pdl_wait();
-  const int b = blockIdx.x / kVocCtas, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int b = blockIdx.x / NC, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int w = min(width[b], max_width);
   if (w <= 0) return;  // (the whole cluster)
-  const int picks = min(w - 1, kLpMax);
   const uint32_t rank = cluster_ctarank();
-  const int per = voc_slice(V), start = min(V, (int)rank * per), n = min(V, start + per) - start;
+  const int per = voc_slice(V, NC), start = min(V, (int)rank * per), n = min(V, start + per) - start;
   const float* row = logits + (size_t)b * ldl;
   const float* src = row + start;
   constexpr int kStep = kVocThreads * 4;  // a thread's entries: columns 4 tid .. 4 tid + 3 of every kStep
@@ -870,8 +937,8 @@ logprob_topk_kernel(const float* __restrict__ logits, int ldl, int V, const int3
   };
   mx = block_max(mx);
   if (tid == 0) sh.part_max = mx;
-  voc_sync();
-  mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(*cluster_ptr(&sh.part_max, lane & (kVocCtas - 1)))));
+  voc_sync<NC>();
+  mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(*cluster_ptr<NC>(&sh.part_max, lane & (NC - 1)))));
   float se = 0.f;
   if constexpr (SM) {
 #pragma unroll 4
@@ -890,9 +957,9 @@ logprob_topk_kernel(const float* __restrict__ logits, int ldl, int V, const int3
     se = warp_sum(lane < kVocWarps ? sh.red[lane] : 0.f);
     if (lane == 0) sh.part_sum = se;
   }
-  voc_sync();
+  voc_sync<NC>();
   float sum = 0.f;
-  for (int c = 0; c < kVocCtas; ++c) sum += *cluster_ptr(&sh.part_sum, c);
+  for (int c = 0; c < NC; ++c) sum += *cluster_ptr<NC>(&sh.part_sum, c);
   const float lse = mx + logf(sum);
   int32_t* ids = out_ids + (size_t)b * max_width;
   float* lps = out_lp + (size_t)b * max_width;
@@ -929,12 +996,12 @@ logprob_topk_kernel(const float* __restrict__ logits, int ldl, int V, const int3
         if (mine >> lane & 1) { bk = k1; bi = i1; }
       }
     }
-    voc_sync();
+    voc_sync<NC>();
     if (rank == 0) {
-      const int all = kVocCtas * picks;
+      const int all = NC * picks;
       for (int e = tid; e < all; e += kVocThreads) {
-        sh.all_key[e] = cluster_ptr(sh.top_key, e / picks)[e % picks];
-        sh.all_idx[e] = cluster_ptr(sh.top_idx, e / picks)[e % picks];
+        sh.all_key[e] = cluster_ptr<NC>(sh.top_key, e / picks)[e % picks];
+        sh.all_idx[e] = cluster_ptr<NC>(sh.top_idx, e / picks)[e % picks];
       }
       __syncthreads();
       for (int e = tid; e < all; e += kVocThreads) {
@@ -953,15 +1020,15 @@ logprob_topk_kernel(const float* __restrict__ logits, int ldl, int V, const int3
           lps[1 + at] = none ? (at > 0 ? -INFINITY : mx - lse) : fkey_inv(q) - lse;
         }
         if (better == picks - 1)
-          for (int c = 0; c < kVocCtas; ++c) {
-            *cluster_ptr(&sh.last_key, c) = q;
-            *cluster_ptr(&sh.last_idx, c) = i;
+          for (int c = 0; c < NC; ++c) {
+            *cluster_ptr<NC>(&sh.last_key, c) = q;
+            *cluster_ptr<NC>(&sh.last_idx, c) = i;
           }
       }
     }
-    voc_sync();
+    voc_sync<NC>();
   }
-  voc_sync();  // no block's shared memory goes away while another one reads it
+  voc_sync<NC>();  // no block's shared memory goes away while another one reads it
 }
 
 __global__ void __launch_bounds__(kRowThreads)
@@ -1031,31 +1098,53 @@ cudaError_t rope_kv_write(cudaStream_t s, bf16* qkv, const int32_t* positions, c
   return cudaGetLastError();
 }
 namespace {
-// dynamic shared memory of the vocabulary kernels: a slice when it fits, nothing otherwise (the SM = false instances).  The opt-in is
-// per device and costs well under a microsecond, so it rides with every launch: callers need no initialisation call.
+// Dynamic shared memory of the vocabulary kernels: a part of the row when it fits, nothing otherwise.  The opt-in is per device and
+// costs well under a microsecond, so it rides with every launch: callers need no initialisation call.
 template <typename K, typename... Args>
-cudaError_t launch_voc(K* on_chip, K* in_memory, cudaStream_t s, int B, int V, Args... args) {
-  const size_t floats = (size_t)voc_slice(V);
-  const bool fits = floats <= (size_t)kVocSmemFloats;
-  if (fits) {
-    const cudaError_t e = cudaFuncSetAttribute(on_chip, cudaFuncAttributeMaxDynamicSharedMemorySize, kVocSmemFloats * 4);
+cudaError_t launch_voc(K* kernel, int ctas, bool on_chip, cudaStream_t s, int B, int V, Args... args) {
+  if (on_chip) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kVocSmemFloats * 4);
     if (e != cudaSuccess) return e;
   }
-  return launch_k(fits ? on_chip : in_memory, dim3(B * kVocCtas), dim3(kVocThreads), fits ? floats * 4 : 0, s, true, args...);
+  return launch_k(kernel, dim3(B * ctas), dim3(kVocThreads), on_chip ? (size_t)voc_slice(V, ctas) * 4 : 0, s, true, args...);
 }
+// Blocks per row: one up to `whole` columns; else as many (at most `most`) as let the machine hold every row's blocks at once (33
+// clusters of eight), but enough that two blocks fit an SM (parts of 25000 columns).  Every shape gives the same tokens.  Us with 1 / 2 / 4 / 8 blocks per row:
+//   top_p 0.95   48 rows of 32768  57 / 49 / 42 / 65     128 of 16384  50 / 39 / 62 / 116    256 of 8192    34 / 57 / 97 / 200
+//   width 6      48 rows of 50000   - / 14 / 13 / 25     128 of 32768  12 / 13 / 24 / 47     256 of 8192   8.5 / 18 / 38 / 87
+//   top_p 0.95   32 rows of 128256  - /  - / 66 / 72      96 of 65536   - / 126 / 97 / 148   256 of 128256  - /  - / 510 / 512
+// (clusters of eight run 33 at a time whatever their size, which left 256 rows of 1000 to 8192 columns at 20 to 50 % of the speed
+// of the block per row that these kernels had replaced).
+int voc_ctas(int B, int V, int whole, int most) {
+  if (V <= whole) return 1;
+  int ctas = most;
+  while (ctas > 1 && (long)B * ctas > 264) ctas /= 2;
+  while (ctas < 8 && voc_slice(V, ctas) > 25000) ctas *= 2;
+  return ctas;
+}
+#define HB_VOC(KERNEL, CTAS, ...)                                                             \
+  do {                                                                                        \
+    const int ctas = (CTAS);                                                                  \
+    if (voc_slice(V, ctas) > kVocSmemFloats) return launch_voc(KERNEL<8, false>, 8, false, s, B, V, __VA_ARGS__); \
+    if (ctas == 1) return launch_voc(KERNEL<1, true>, 1, true, s, B, V, __VA_ARGS__);         \
+    if (ctas == 2) return launch_voc(KERNEL<2, true>, 2, true, s, B, V, __VA_ARGS__);         \
+    if (ctas == 4) return launch_voc(KERNEL<4, true>, 4, true, s, B, V, __VA_ARGS__);         \
+    return launch_voc(KERNEL<8, true>, 8, true, s, B, V, __VA_ARGS__);                        \
+  } while (0)
 }  // namespace
 // Rows without filters are looked at once, so nothing is gained by keeping them on chip: two launches over chunks of the row, with room
 // for the chunks' winners, unless the clusters of few short rows are through sooner.  Us, clusters | two launches: 32 rows of
 // 32768, temperature 8.6 | 9.7, 64 rows of 32768 15.8 | 12.4, greedy 10.8 | 7.3, 256 rows of 8192 34 | 12.5, greedy 28 | 7.2, 1 row
-// of 128256 12.6 | 7.5, 256 rows of 128256 140 | 93, greedy 71 | 42.
-bool sample_two_stage(int B, int V, bool filtered) { return !filtered && !(B <= 32 && V <= 32768); }
+// of 128256 12.6 | 7.5, 256 rows of 128256 140 | 93, greedy 71 | 42; 1 row of 65536 7.4 | 7.5, greedy 5.6 | 7.5, 16 rows 12.1 | 8.6.
+bool sample_two_stage(int B, int V, bool filtered) { return !filtered && !(B <= 33 && V <= (B <= 4 ? 65536 : 32768)); }
 size_t sample_scratch_bytes(int B, int V) { return (size_t)B * ((V + kSampleChunk - 1) / kSampleChunk) * 8; }
 
 cudaError_t sample_tokens(cudaStream_t s, const float* logits, int ldl, const float* temperature, const uint64_t* seed,
                           int32_t* out, int B, int V, void* scratch, const int32_t* top_k, const float* top_p) {
   if (B <= 0) return cudaSuccess;
   if (V <= 0) return cudaErrorInvalidValue;
-  if (sample_two_stage(B, V, temperature && (top_k || top_p))) {
+  const bool filtered = temperature && (top_k || top_p);
+  if (sample_two_stage(B, V, filtered)) {
     const int chunks = (V + kSampleChunk - 1) / kSampleChunk;
     float* pv = static_cast<float*>(scratch);
     int* pi = reinterpret_cast<int*>(pv + (size_t)B * chunks);
@@ -1063,18 +1152,25 @@ cudaError_t sample_tokens(cudaStream_t s, const float* logits, int ldl, const fl
     if (e != cudaSuccess) return e;
     return launch_k(sample_stage2_kernel, dim3(B), dim3(32), 0, s, true, (const float*)pv, (const int*)pi, out, chunks);
   }
-  return launch_voc(sample_kernel<true>, sample_kernel<false>, s, B, V, logits, ldl, temperature, seed, top_k, top_p, out, V);
+  HB_VOC(sample_kernel, filtered ? voc_ctas(B, V, 8192, 8) : 8, logits, ldl, temperature, seed, top_k, top_p, out, V);
 }
 cudaError_t apply_penalties(cudaStream_t s, float* logits, int ldl, const int32_t* pen_off, const void* pen, int B, int V) {
   if (B <= 0) return cudaSuccess;
   return launch_k(apply_penalties_kernel, dim3(B), dim3(256), 0, s, true, logits, ldl, pen_off, (const int2*)pen, V);
 }
 cudaError_t logprob_topk(cudaStream_t s, const float* logits, int ldl, int V, const int32_t* sampled, const int32_t* width,
-                         int32_t* out_ids, float* out_lp, int B, int max_width) {
+                         int32_t* out_ids, float* out_lp, int B, int max_width, int widest) {
   if (B <= 0) return cudaSuccess;
-  return launch_voc(logprob_topk_kernel<true>, logprob_topk_kernel<false>, s, B, V, logits, ldl, V, sampled, width, out_ids, out_lp,
-                    max_width);
+  // Narrow records are two reads of the row (three of width 3) and stay with a block per row, except few long rows, which clusters read
+  // sooner.  Us, block per row | clusters: width 2, 64 rows of 128256 19.8 | 23.4, 256 of 128256 47 | 89, 128 of 8192 4.5 | 5.9, 1 of
+  // 128256 15.9 | 8.9, 32 of 100000 13.5 | 11.9; width 1, 32 of 65536 9.6 | 8.0, 32 of 32768 6.4 | 7.2.
+  const int part = voc_slice(V, 8);
+  const bool few = part > kVocSmemFloats || B <= (part <= 25000 ? 33 : 16);
+  if ((widest <= 2 && !(few && V > (widest <= 1 ? 32768 : 65536))) || (widest == 3 && B > 128))
+    return launch_k(logprob_row_kernel, dim3(B), dim3(kLpThreads), 0, s, true, logits, ldl, V, sampled, width, out_ids, out_lp, max_width);
+  HB_VOC(logprob_topk_kernel, voc_ctas(B, V, 32768, V <= 65536 ? 4 : 8), logits, ldl, V, sampled, width, out_ids, out_lp, max_width);
 }
+#undef HB_VOC
 cudaError_t cls_pool_l2(cudaStream_t s, const bf16* x, const int32_t* first_row, float* out, int B, int H) {
   if (B <= 0) return cudaSuccess;
   cls_pool_l2_kernel<<<B, kRowThreads, 0, s>>>(x, first_row, out, H);

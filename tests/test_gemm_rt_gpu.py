@@ -9,7 +9,7 @@ from helix_b200 import engine as E
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("width,ff", [(64, 128), (100, 36), (260, 516), (1024, 4096)])
+@pytest.mark.parametrize("width,ff", [(64, 128), (68, 64), (100, 36), (260, 516), (1024, 4096)])
 def test_rows_do_not_depend_on_the_batch(width, ff):
     vocab = 132
     d = E.StackDesc(width=width, vocab=vocab, compute_f32=1, norm_eps=1e-6, norm_place=E.NORM_PARALLEL, embed_norm=1, plain_gains=1, tie_head=1,

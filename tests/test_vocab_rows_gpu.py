@@ -28,19 +28,21 @@ def rows_of(V, ld, seed, B=6):
 
 
 @pytest.mark.parametrize("V", SIZES)
-@pytest.mark.parametrize("width", [1, 2, 21, 70])
-def test_logprob_records(V, width):
+@pytest.mark.parametrize("width", [1, 2, 3, 21, 70])
+@pytest.mark.parametrize("B", [6, 130])  # (records of up to three tokens of that many rows: a block per row)
+def test_logprob_records(V, width, B):
     L = hb.lib()
     ld = V + 3
-    x = rows_of(V, ld, V + width)
-    B = x.shape[0]
+    if B * ld > 2 ** 24:
+        pytest.skip("as many rows of shorter vocabularies")
+    x = rows_of(V, ld, V + width, B)
     sampled = torch.tensor([(7 * b) % V for b in range(B)], device="cuda", dtype=torch.int32)
-    wid = torch.tensor([width, width, width, width, width, 0], device="cuda", dtype=torch.int32)
+    wid = torch.tensor([width] * 5 + [0] * (B - 5), device="cuda", dtype=torch.int32)
     ids = torch.full((B, width), -7, device="cuda", dtype=torch.int32)
     lps = torch.full((B, width), 5.0, device="cuda")
     assert L.hbk_logprob_topk(p(x), ld, V, p(sampled), p(wid), p(ids), p(lps), B, width) == 0
     torch.cuda.synchronize()
-    assert (ids[5] == -7).all() and (lps[5] == 5.0).all()
+    assert (ids[5:] == -7).all() and (lps[5:] == 5.0).all()
     for b in range(5):
         row = x[b, :V].cpu().double().numpy()
         lse_row = row if b != 3 else None
@@ -126,7 +128,7 @@ def test_nan_logits_are_never_drawn(V, filtered):
     assert set(out.tolist()) == set(keep)
 
 
-@pytest.mark.parametrize("B,V", [(32, 32768), (33, 32768), (32, 32769), (1, 40000), (40, 1), (40, 4095), (40, 4096), (40, 8193), (200, 1000), (3, 400009)])
+@pytest.mark.parametrize("B,V", [(32, 32768), (33, 32768), (32, 32769), (34, 32768), (5, 32769), (4, 65537), (4, 65536), (40, 1), (40, 4095), (40, 4096), (40, 8193), (200, 1000), (3, 400009)])
 def test_rows_without_filters_take_the_same_tokens_either_way(B, V):
     """Rows without filters go through two launches over chunks or, few short ones and those of filtered steps, through a cluster per row:
     the same noise and the same order of ties, so the same tokens."""
@@ -148,3 +150,31 @@ def test_no_columns_are_refused():
     out = torch.zeros(2, device="cuda", dtype=torch.int32)
     x = torch.zeros(2, device="cuda")
     assert L.hbk_sample(p(x), 1, None, None, p(out), 2, 0) != 0
+
+
+@pytest.mark.parametrize("B,V", [(48, 8192), (48, 8193), (48, 32769), (48, 100000), (48, 100001), (48, 200001), (48, 400009), (108, 16387), (108, 50000),
+                                 (108, 50001), (204, 16387), (204, 25001), (204, 128256)])
+def test_many_rows_equal_few(B, V):
+    """Rows beside many others are shared by one, two, four or eight blocks, beside few by eight (or one): the same tokens and the same
+    alternatives, whatever the number of blocks."""
+    L = hb.lib()
+    width = 6
+    x = rows_of(V, V + 3, 7 * V, B)
+    x[:, V // 3] += 9.0
+    f = lambda v, t: torch.tensor(v, device="cuda", dtype=t)  # noqa: E731
+    temp, seed = f([0.8, 0.5, 1.3, 0.0] * (B // 4), torch.float32), torch.arange(B, device="cuda", dtype=torch.int64) * 15485863
+    topk, topp = f([0, 40, 700, 3, 0, 5000] * (B // 6), torch.int32), f([0.95, 1.0, 0.6] * (B // 3), torch.float32)
+    tok = [torch.full((B,), -1, device="cuda", dtype=torch.int32) for _ in range(2)]
+    ids = [torch.full((B, width), -7, device="cuda", dtype=torch.int32) for _ in range(2)]
+    lps = [torch.zeros((B, width), device="cuda") for _ in range(2)]
+    wid = torch.full((B,), width, device="cuda", dtype=torch.int32)
+    for k, step in ((0, B), (1, 12)):
+        for r in range(0, B, step):
+            at = lambda t: t[r:].data_ptr()  # noqa: E731
+            assert L.hbk_sample_filtered(at(x), V + 3, at(temp), at(seed), at(topk), at(topp), at(tok[k]), step, V) == 0
+            assert L.hbk_logprob_topk(at(x), V + 3, V, at(tok[k]), at(wid), at(ids[k]), at(lps[k]), step, width) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(tok[0], tok[1]) and (tok[0] >= 0).all() and (tok[0] < V).all()
+    assert torch.equal(ids[0], ids[1])
+    # two orders of V positive fp32 terms in trees of at most V / 512 + 20 steps; the rest is one subtraction of values below 64
+    np.testing.assert_allclose(lps[0].cpu().numpy(), lps[1].cpu().numpy(), rtol=0, atol=2.0 ** -24 * (V / 512 + 20) + 2.0 ** -17)
