@@ -1004,7 +1004,7 @@ cudaError_t stack_ops_init() {
 cudaError_t gemm_rt(cudaStream_t s, const GemmRtArgs& a) {
   if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.batch <= 0) return cudaErrorInvalidValue;
   // Two parts of K or fewer leave half of a tile's threads without work: 1000 x 4096 x 32 17 us there, 28 on tiles, x 64 29 / 33, x 96 39 / 39.
-  // (By K alone, so that a row's bits do not depend on M; single rows of 64 terms would take 3.4 us on tiles, 6.2 there.)
+  // (By K alone, so that a row's bits do not depend on M; single rows of 64 terms would take 4.2 us on tiles, 6.3 there.)
   const bool pieces = a.K > 64 && a.w_sk == 1 && ((a.K | a.lda | a.a_bs | a.w_sn | a.w_bs) & 3) == 0 && (((uintptr_t)a.A | (uintptr_t)a.W) & 15) == 0;
   if (a.f32 && pieces && (a.M + 15) / 16 <= 65535) {
     if (a.M <= 2) return launch_rt_tile<2, 32, 2, 1, 32, 4>(s, a);
