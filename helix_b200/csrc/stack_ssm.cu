@@ -778,7 +778,7 @@ cudaError_t short_conv(cudaStream_t s, const ConvArgs& a) {
   if (short_conv_fused(a)) {
     const int across = (a.C / 4 + 127) / 128;
     // runs of one token until runs of eight give every SM two blocks (or where the tails ride along)
-    const bool one = a.single || (long)across * ((a.T + kConvRun - 1) / kConvRun) < 2 * 148;
+    const bool one = a.single || (long)across * ((a.T + kConvRun - 1) / kConvRun) < 2 * effective_sms(148);
     const dim3 g(across + (a.ab ? 1 : 0), one ? a.T : (a.T + kConvRun - 1) / kConvRun);
 #define HB_CONV_T(WT, TP) return one ? launch_k(short_conv_run_kernel<WT, TP, 1>, g, dim3(128), 0, s, true, a) : launch_k(short_conv_run_kernel<WT, TP, kConvRun>, g, dim3(128), 0, s, true, a)
 #define HB_CONV(TP) do { if (a.f32) HB_CONV_T(float, TP); else HB_CONV_T(bf16, TP); } while (0)
