@@ -220,9 +220,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   // (ranks by counting, about a microsecond).  With sequences of unequal length the plain order, q pair by q pair with a slot
   // for every sequence whether it has that pair or not, left the longest-loaded CTA 24 to 30 % above the mean (6 prompts of 300
   // to 3000 tokens: 231 tile times of a mean of 187, now 191; 64 chunks of 64 to 512: 74 of 57, now 60).  Measured: 250 -> 233 us and 70.8 -> 62.6 us.
-  // Everything else runs the kernel with the plain walk: launches whose sequences have about equal lengths or whose items fill one round
-  // (the sort only cost its microsecond: 12.3 -> 13.3 us), and keys from a page pool or an expanded run (portions of a long context
-  // are level already).  The plain order also stands in where a launch turns out to have more rows than kMaxRows.
+  // Everything else runs the kernel with the plain walk: launches whose sequences are short or of about equal lengths (sorts_items below), and
+  // keys from a page pool or an expanded run (portions of a long context are level already).  The plain order also stands in where a
+  // launch turns out to have more rows than kMaxRows.
   if constexpr (SORTED) {
     uint32_t* keys = reinterpret_cast<uint32_t*>(sK);            // scratch over the K ring (nothing has been loaded yet)
     uint16_t* ids = reinterpret_cast<uint16_t*>(keys + kMaxRows);
@@ -274,7 +274,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     if constexpr (SORTED) {
       if (rows >= 0) return round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
     }
-    return idx + (int)gridDim.x;
+    return (int)((unsigned)idx + gridDim.x);  // (as a signed sum it took four more registers, spilled, than `idx += gridDim.x` does)
   };
   auto get_item = [&](int idx) {
     Item it;
@@ -689,12 +689,20 @@ int device_sms() {
   }
   return num_sms;
 }
-// packed launches that sort their items: uneven lengths (a tenth of the (sequence, position) slots or more stay empty), more items than
-// SMs, and indices that fit the order's entries
+// Packed launches that sort their items: those whose q pairs differ enough for the order to matter, by what the host knows of the lengths
+// (us plain / sorted, 12 heads of 64 or 32 of 128 columns):
+//   - sequences of two q pairs and more, of a kv tile and more on average (200 sequences of 25 to 200 tokens 195 / 209, one of 300 beside 199 of
+//     50 138 / 149);
+//   - empty (sequence, position) slots: a tenth of all, a fifth where the longest has only two or three pairs (16 sequences of 375 to 500
+//     62 / 66, of 1125 to 1500 129 / 122);
+//   - more items than SMs, twice as many there (3 sequences of 37 to 300 12.4 / 14.5, of 75 to 600 20.3 / 20.5, of 187 to 1500 53 / 31).
+// Gains are 20 % on average over such launches.  The indices have to fit the order's entries.
 bool sorts_items(const AttnPrefillArgs& a) {
   const int max_q_pairs = (a.max_seqlen + QPAIR - 1) / QPAIR;
-  return a.B > 1 && a.B <= 256 && max_q_pairs <= 255 && (long long)max_q_pairs * a.B * a.Hq > effective_sms(device_sms()) &&
-         10.0 * a.T < 9.0 * (double)a.B * a.max_seqlen;
+  if (a.B <= 1 || a.B > 256 || max_q_pairs < 2 || max_q_pairs > 255 || a.T < (long long)BKV * a.B) return false;
+  const bool short_ones = max_q_pairs <= 3;
+  return (long long)max_q_pairs * a.B * a.Hq > (short_ones ? 2ll : 1ll) * effective_sms(device_sms()) &&
+         a.T < (short_ones ? 0.8 : 0.9) * (double)a.B * a.max_seqlen;
 }
 template <int D, bool PAGED, int POLY, bool SORTED>
 cudaError_t launch_p(cudaStream_t stream, const AttnPrefillArgs& a) {

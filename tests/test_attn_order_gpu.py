@@ -1,5 +1,5 @@
-"""Prefill attention at the edges of its item order: as many rows (q pairs of all sequences) as the sorted order holds and one more, more
-sequences than its entries name, empty sequences, one row, fewer items than blocks."""
+"""Prefill attention at the edges of its item order: as many rows (q pairs of all sequences) as the sorted order holds and one more, as many
+sequences as its entries name and one more, empty sequences among sorted ones, one row, fewer items than blocks."""
 import math
 
 import pytest
@@ -13,7 +13,8 @@ BF = torch.bfloat16
 LENS = {
     "one": [1], "fewer_items_than_blocks": [300, 40], "uneven": [3, 700, 256, 257, 90, 1025, 511, 64], "empty_ones": [0, 130, 0, 600, 0],
     "rows_512": [256] * 128 + [512] * 64 + [513] * 64 + [512] * 32, "rows_513": [1] * 200 + [1800] * 39 + [129], "sequences_256": [33] * 255 + [500],
-    "sequences_257": [33] * 256 + [500],
+    "sequences_257": [33] * 256 + [500], "rows_512_exactly": [1] * 200 + [1800] * 39, "sequences_256_sorted": [65] * 255 + [1500],
+    "sequences_257_long": [65] * 256 + [1500], "empty_ones_sorted": [0, 130, 0, 1100, 0, 900, 257, 300],
 }
 
 
