@@ -257,6 +257,10 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     uint8_t* const my_row = buf + row * 128;
     uint64_t* const my_resid_bar = &resid_bar[grp];
     uint32_t resid_phase = 0;
+    // A CTA with one tile has its first residual chunk travel while the products finish: 700 x 4096 x 4096 28.7 -> 27.5 us, 512 x 768 x 3072
+    // 16.3 -> 15.6.  With more tiles that load crowds the next tile's operands (4096 x 4096 x 4096 115.1 -> 117.0, 2048 x 8192 x 2048
+    // 64.7 -> 65.9), so there every chunk is asked for when its buffer is free.
+    const bool early = kResid && num_tiles <= tile_workers;
     int it = 0;
     for (int t = tile_worker; t < num_tiles; t += tile_workers, ++it) {
       int mi, ni;
@@ -265,9 +269,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       const uint32_t aphase = (it >> 1) & 1;
       const int m0 = mi * TILE_M + (int)cta_rank * BLOCK_M;
       const int n_out0 = ni * OUT_BN;
-      if constexpr (kResid) {  // the first residual chunk travels while the products finish
-        if (leader && grp < NCHUNK) {
-          tma_store_wait_read<0>();
+      if constexpr (kResid) {
+        if (early && leader && grp < NCHUNK) {
           mbar_arrive_expect_tx(my_resid_bar, kStagingBytes);
           tma_load_2d(buf, &map_r, my_resid_bar, n_out0 + grp * CHUNK_COLS, m0, kEvictFirst);
         }
@@ -368,8 +371,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll 1
       for (int c = grp; c < NCHUNK; c += 2) {
         if (leader) {
-          if (!kResid || c != grp) tma_store_wait_read<0>();  // this group's previous store is done reading `buf`
-          if (kResid && c != grp) {
+          if (!early || c != grp) tma_store_wait_read<0>();  // this group's previous store is done reading `buf`
+          if (kResid && (!early || c != grp)) {
             mbar_arrive_expect_tx(my_resid_bar, kStagingBytes);
             tma_load_2d(buf, &map_r, my_resid_bar, n_out0 + c * CHUNK_COLS, m0, kEvictFirst);
           }
@@ -577,7 +580,7 @@ cudaError_t launch_epi(cudaStream_t stream, const GemmArgs& g, int num_sms) {
     // 13400 x 3072 x   768 (gelu)    63.6            79.3         72.6       83.2     124.9
     // (R: residual epilogue.)  Narrow tiles read more operand bytes from L2 per product (24 KB per SM and block for 128 x 64, 32 KB for
     // four times the products in a pair's 256 x 256), wide ones leave SMs without a tile.  The rule before, "halve the width until there
-    // are two waves", took 128 x 64 for the first, third and fifth line.  Every shape walks K in order: a row's result does not
+    // are two waves", took 128 x 64 for the first, second and fifth line.  Every shape walks K in order: a row's result does not
     // depend on the choice.
     struct Shape { int bn, cg; double kb, floor, fixed; };
     static constexpr Shape shapes[] = {{256, 2, 0.36, 5.6, 8.5}, {128, 2, 0.235, 3.4, 8.0}, {256, 1, 0.42, 6.0, 7.0}, {128, 1, 0.28, 3.9, 6.5}, {64, 1, 0.235, 3.1, 6.0}};
