@@ -462,8 +462,10 @@ __global__ void lin_step_kernel(LinRecArgs a) {
     *reinterpret_cast<float2*>(a.out + (size_t)t * a.ldo + (size_t)h * a.Dv + j0) = make_float2(fmaf(skip, vv.x, o.x * a.q_scale), fmaf(skip, vv.y, o.y * a.q_scale));
   }
 }
+// Heads of up to 32 value columns leave half of a block's lanes idle: beside thousands of others they stay with the kernel above, whose blocks
+// are 32 columns wide there (256 sequences x 32 heads of 128 x 24 states 76 us there, 80 here; 64 x 64 heads 37 / 35.5, 16 x 8 6.2 / 3.2).
 bool lin_step_ok(const LinRecArgs& a) {
-  return a.single && !a.nq && a.Dk % 4 == 0 && a.Dv % 2 == 0 && ((a.ldq | a.ldk | (long)a.q_off | (long)a.k_off) & 3) == 0 &&
+  return a.single && !a.nq && (a.Dv > 32 || (long)a.B * a.H <= 4096) && a.Dk % 4 == 0 && a.Dv % 2 == 0 && ((a.ldq | a.ldk | (long)a.q_off | (long)a.k_off) & 3) == 0 &&
          ((a.ldv | a.ldo | a.slot_stride | (long)a.v_off | (long)a.s_off) & 1) == 0 && (((uintptr_t)a.q | (uintptr_t)a.k) & 15) == 0 &&
          (((uintptr_t)a.v | (uintptr_t)a.out | (uintptr_t)a.state) & 7) == 0;
 }

@@ -34,3 +34,23 @@ def test_single_tokens(kind, dim, vdim):
                 got[i].append(r)
         for a, b in zip(got, want):
             assert np.array_equal(np.stack(a), b)
+
+
+def test_narrow_heads_beside_thousands():
+    """Heads of up to 32 columns leave the single-token kernel beside more than 4096 (sequence, head) pairs: 66 sequences x 64 heads in one step give
+    the bits of the same sequences in two steps of 33."""
+    l = E.LayerDesc(mixer=E.MIXER_MAMBA2, heads=64, vdim=6, dim=8, kv_heads=4, norm_groups=1, conv_taps=1)
+    d = E.StackDesc(width=64, vocab=128, layers=[l], compute_f32=1, norm_eps=1e-5, norm_place=E.NORM_PARALLEL, embed_norm=1, plain_gains=1, tie_head=1)
+    rng = np.random.default_rng(1)
+    first, then = rng.integers(0, 128, (66, 2)).tolist(), rng.integers(0, 128, (66, 2)).tolist()
+    got = []
+    with hb.Engine(hb.EngineConfig(max_seqs=66, max_ctx=64, max_batched_tokens=256, kv_pool_tokens=66 * 64)) as e:
+        e.load_random(d, 12)
+        for parts in ([slice(0, 66)], [slice(0, 33), slice(33, 66)]):
+            ids = [e.seq_open() for _ in first]
+            e.seq_step([(s, t, []) for s, t in zip(ids, first)])
+            rows = [np.concatenate([e.seq_step([(s, [t[k]], [0]) for s, t in zip(ids[p], then[p])]) for p in parts]) for k in range(2)]
+            for s in ids:
+                e.seq_close(s)
+            got.append(np.stack(rows))
+    assert np.isfinite(got[0]).all() and np.array_equal(got[0], got[1])
