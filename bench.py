@@ -14,7 +14,7 @@ cache.  tokens = sessions * (seq + decode).
                  scheduler's least-active rule (replica.route_least_active == pickBestWarmSlot), 256/N per GPU
   cpu_baseline / --impl reference : CPU stand-in for the reference's llama.cpp CPU path (cannot run offline): the numpy
                  oracle port on all host threads (pinned with threadpoolctl), bounded sample; --cpu-impl hf switches to
-                 HF transformers on torch CPU, which measured 30x slower on the GPU box (profiles/r02c_reference_hf.json)
+                 HF transformers on torch CPU, which measured 30x slower on a B200's host (profiles/r02c_reference_hf.json)
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference] [--workload llama8b|bge|pack|risepel|lurepel|latanex|funudra|kamivik|pupalix]
 """
