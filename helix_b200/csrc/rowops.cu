@@ -577,7 +577,7 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
         const u64 d = hi - lo;
         // A mass between two finite values: the tokens go into kBins equal bins of values at once, and the bin that holds the answer is
         // the next interval (a threshold in the bulk of the vocabulary needs two such passes instead of five or six of three keys,
-        // which weigh nearly as many tokens each: rows of top_p 0.95 85 -> 69 us; counting is cheap, so top-k stays with the keys).
+        // which weigh nearly as many tokens each: rows of top_p 0.95 85 -> 70 us; counting is cheap, so top-k stays with the keys).
         // Slices beyond shared memory, whose sums could leave 32 bits, and intervals that no longer split take the keys below.
         if constexpr (SM) {
           const float b_lo = fkey_inv((uint32_t)lo), b_hi = fkey_inv((uint32_t)(hi - 1)), scale = (float)kBins / (b_hi - b_lo);

@@ -64,7 +64,8 @@ __global__ void __launch_bounds__(256) gemm_rt_kernel(const float* __restrict__ 
 }
 
 // The same product for fp32 operands whose rows along k are 16-byte pieces (every product of the exact mode at sizes that are multiples
-// of four): bound by the FMA pipe and shared-memory reads for prompts and by the weights' bytes for single tokens, where the kernel
+// of four and of more than 64 terms): for prompts bound by the FMA pipe and, at one block per SM, by the latency of its shared-memory reads
+// (30 of 72 TFLOP/s; which of the two is not settled), for single tokens by the weights' bytes, where the kernel
 // above was bound by scalar loads with no copies in flight and one thread per sum of K terms.
 // K is cut into kRtParts equal parts; a group of threads per part keeps its own stages of cp.async copies and the groups' sums
 // are added in order of k at the end; inside a part even and odd k have a sum each (packed FMAs on register pairs as they are
