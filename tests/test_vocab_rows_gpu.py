@@ -27,14 +27,11 @@ def rows_of(V, ld, seed, B=6):
     return x
 
 
-@pytest.mark.parametrize("V", SIZES)
+@pytest.mark.parametrize("V,B", [(v, 6) for v in SIZES] + [(v, 130) for v in SIZES[:-1]])  # (130: records of three tokens on a block per row too)
 @pytest.mark.parametrize("width", [1, 2, 3, 21, 70])
-@pytest.mark.parametrize("B", [6, 130])  # (records of up to three tokens of that many rows: a block per row)
 def test_logprob_records(V, width, B):
     L = hb.lib()
     ld = V + 3
-    if B * ld > 2 ** 24:
-        pytest.skip("as many rows of shorter vocabularies")
     x = rows_of(V, ld, V + width, B)
     sampled = torch.tensor([(7 * b) % V for b in range(B)], device="cuda", dtype=torch.int32)
     wid = torch.tensor([width] * 5 + [0] * (B - 5), device="cuda", dtype=torch.int32)
