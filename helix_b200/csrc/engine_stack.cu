@@ -999,7 +999,7 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
     ra.skip = nullptr; ra.f32 = f32; ra.q_scale = 1.0f / sqrtf((float)q.D);
     ra.state = state_; ra.slot_stride = (long)model_.state_floats; ra.s_off = q.state_off; ra.n_off = q.n_off;
     ra.cu = cu; ra.first_pos = first; ra.slots = sslot;
-    ra.B = B; ra.H = q.H; ra.G = q.H; ra.Dk = q.D; ra.Dv = q.Dv;
+    ra.T = T; ra.B = B; ra.H = q.H; ra.G = q.H; ra.Dk = q.D; ra.Dv = q.Dv;
     SPAN(6, 4.0 * T * q.H * q.D * q.Dv, lin_recurrence(stream_, ra));
     SPAN(3, 16.0 * T * q.H * q.Dv, memory_readout(stream_, k.ctx, k.ldctx, k.ab + 3 * q.H, k.ldab, k.ab, k.ldab, k.p1 + q.off_g, ldin, q.hnorm, f32,
                                                   sd.norm_eps, scale, out_f32, mo16, ldout, col0, T, q.H, q.Dv));
@@ -1068,7 +1068,7 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       ra.skip = (const uint8_t*)w.a_dt + (size_t)2 * H * model_.elem; ra.f32 = f32; ra.q_scale = 1.f;
       ra.state = state_; ra.slot_stride = (long)model_.state_floats; ra.s_off = w.state_off; ra.n_off = 0;
       ra.cu = cu; ra.first_pos = first; ra.slots = sslot;
-      ra.B = B; ra.H = H; ra.G = G; ra.Dk = N; ra.Dv = Dv;
+      ra.T = T; ra.B = B; ra.H = H; ra.G = G; ra.Dk = N; ra.Dv = Dv;
       ra.single = T == B;
       SPAN(6, 4.0 * T * H * N * Dv, lin_recurrence(stream_, ra));
       SPAN(3, 16.0 * T * inner, gated_group_norm(stream_, k.ctx, k.ldctx, k.p1 + w.off_g, k.ld1, w.hnorm, f32, sd.norm_eps, l.norm_groups, mo_f32,
@@ -1098,7 +1098,7 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       ra.f32 = f32; ra.q_scale = 1.f;
       ra.state = state_; ra.slot_stride = (long)model_.state_floats; ra.s_off = w.state_off;
       ra.cu = cu; ra.first_pos = first; ra.slots = sslot;
-      ra.B = B; ra.H = H; ra.G = H; ra.Dk = Dk; ra.Dv = Dv;
+      ra.T = T; ra.B = B; ra.H = H; ra.G = H; ra.Dk = Dk; ra.Dv = Dv;
       ra.single = T == B;
       SPAN(6, 4.0 * T * H * Dk * Dv, lin_recurrence(stream_, ra));
       SPAN(3, 16.0 * T * H * Dv, gated_group_norm(stream_, k.ctx, k.ldctx, k.p1 + w.off_g, k.ld1, w.hnorm, f32, sd.norm_eps, 1, mo_f32, mo16, T, H * Dv,

@@ -601,6 +601,7 @@ struct LinRecArgs {
   const float* head_decay = nullptr;
   int silu = 0;
   bool single = false;  // every entry is exactly one token
+  int T = 0;            // tokens of all entries
 };
 cudaError_t lin_recurrence(cudaStream_t s, const LinRecArgs& a);
 // S_t = decay_h S_(t-1) + k_t v_t^T, out_t = S_t^T q_t on the tensor cores, chunk by chunk (stack_lightning.cu): q, k [T, H * Dk] and

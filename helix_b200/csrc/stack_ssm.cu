@@ -4,7 +4,7 @@
 //
 // Both recurrences have one scalar decay per head and token,
 //   S_t = a_t S_(t-1) + b_t k_t v_t^T,   o_t = S_t^T q_t            (S [dim][vdim] fp32 per head and sequence)
-// and run on one kernel (lin_recurrence):
+// and run on the kernels behind lin_recurrence:
 //   state-space layer:  a = exp(-exp(A) dt), b = dt, k = B, q = C, v = x, o += D x       (ssm_steps makes a, b)
 //   matrix memory:      a = exp(f + m' - m), b = exp(i - m) with the running maximum m = max(f + m', i) of the log gates
 //                       (exp_gate_scan: a warp scan over the tokens of an entry, since m -> max(m + f, i) composes
@@ -12,10 +12,12 @@
 // Step entries are runs of tokens [first, first + n) of sequences whose state lives in their slot; an entry that starts at
 // position 0 starts from zeros inside the kernels (m from 0), so a slot needs no clearing when it changes hands.
 // Everything here is fp32; every sum has a fixed order per output element.
+#include <limits.h>
 #include <math.h>
 #include <stdlib.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "kernels.h"
 #include "launch.h"
@@ -233,7 +235,7 @@ template <int N> __device__ __forceinline__ void cpa_wait() { asm volatile("cp.a
 // state columns in registers (lane = NC neighbouring columns; pairs of neighbouring channels as packed f32x2 operands, so one
 // instruction serves two state elements, and one 16-byte broadcast read of q or k feeds 4 NC of them).  Tokens are staged
 // 16 / NC at a time through a cp.async double buffer (q | k | the block's v columns | a, b); every warp leaves its partial dot
-// products in shared memory and the block adds them in warp order once per stage.  The block of the first column slice also
+// products (sums of eight channels, added) in shared memory and the block adds them pair by pair once per stage.  The block of the first column slice also
 // carries the normaliser vector: lane l of warp w keeps channel 16 w + (l & 15), the 16 lanes' products are added by a
 // butterfly.
 template <int DKP, int NC>
@@ -330,12 +332,11 @@ __global__ void __launch_bounds__(DKP * 2, 512 / DKP) lin_recurrence_kernel(LinR
       const float2 dab = hd ? hab : *reinterpret_cast<const float2*>(tk + 2 * DKP + BC);
       const float da = dab.x, db = dab.y;
       const float2 da2 = make_float2(da, da);
-      float2 bv2[NC], oa[NC];
+      float2 bv2[NC], oa[NC], ob[NC];  // channels 0 .. 7 and 8 .. 15 of the warp's have a sum each
 #pragma unroll
       for (int e = 0; e < NC; ++e) {
         const float bv = db * tk[2 * DKP + lane * NC + e];
         bv2[e] = make_float2(bv, bv);
-        oa[e] = make_float2(0.f, 0.f);
       }
       const float4* q4 = reinterpret_cast<const float4*>(tk + i0);
       const float4* k4 = reinterpret_cast<const float4*>(tk + DKP + i0);
@@ -345,14 +346,15 @@ __global__ void __launch_bounds__(DKP * 2, 512 / DKP) lin_recurrence_kernel(LinR
         const float2 k01 = make_float2(k.x, k.y), k23 = make_float2(k.z, k.w), q01 = make_float2(q.x, q.y), q23 = make_float2(q.z, q.w);
 #pragma unroll
         for (int e = 0; e < NC; ++e) {
+          float2& o = i < 2 ? oa[e] : ob[e];
           S[e][2 * i] = __ffma2_rn(da2, S[e][2 * i], __fmul2_rn(k01, bv2[e]));
-          oa[e] = __ffma2_rn(S[e][2 * i], q01, oa[e]);
+          o = i % 2 == 0 ? __fmul2_rn(S[e][2 * i], q01) : __ffma2_rn(S[e][2 * i], q01, o);
           S[e][2 * i + 1] = __ffma2_rn(da2, S[e][2 * i + 1], __fmul2_rn(k23, bv2[e]));
-          oa[e] = __ffma2_rn(S[e][2 * i + 1], q23, oa[e]);
+          o = __ffma2_rn(S[e][2 * i + 1], q23, o);
         }
       }
 #pragma unroll
-      for (int e = 0; e < NC; ++e) obuf[(tt * KS + w) * BC + lane * NC + e] = oa[e].x + oa[e].y;
+      for (int e = 0; e < NC; ++e) obuf[(tt * KS + w) * BC + lane * NC + e] = (oa[e].x + oa[e].y) + (ob[e].x + ob[e].y);
       if (do_n) {
         nreg = fmaf(da, nreg, db * tk[DKP + nch]);
         float pn = nreg * tk[nch];
@@ -364,9 +366,14 @@ __global__ void __launch_bounds__(DKP * 2, 512 / DKP) lin_recurrence_kernel(LinR
     __syncthreads();
     for (int e = threadIdx.x; e < nt * BC; e += blockDim.x) {
       const int tt = e / BC, c = e % BC;
-      float o = 0.f;
+      float part[KS];
 #pragma unroll
-      for (int ww = 0; ww < KS; ++ww) o += obuf[(tt * KS + ww) * BC + c];
+      for (int ww = 0; ww < KS; ++ww) part[ww] = obuf[(tt * KS + ww) * BC + c];
+#pragma unroll
+      for (int st = 1; st < KS; st *= 2)
+#pragma unroll
+        for (int ww = 0; ww < KS; ww += 2 * st) part[ww] += part[ww + st];
+      const float o = part[0];
       if (c0 + c < a.Dv) a.out[(size_t)(tc + tt) * a.ldo + (size_t)h * a.Dv + c0 + c] = fmaf(skip, base[tt * per_tok + 2 * DKP + c], o * a.q_scale);
     }
     if (do_n) {
@@ -392,12 +399,215 @@ __global__ void __launch_bounds__(DKP * 2, 512 / DKP) lin_recurrence_kernel(LinR
   if (do_n && lane < 16 && nch < Dk) *nst = nreg;
 }
 
+// Portions without a normaliser: the same arithmetic (state elements, channel sums of eight, their sums pair by pair: the same bits as the
+// kernel above and the single-token one) in larger pieces.  A lane keeps CH channels of kPortionCols neighbouring columns, LS = DKP / CH lanes
+// share the columns.  What bounds it is the rate of packed products with three different operands (2.3 cycles each on a quarter of an SM, so
+// 220 per token for a block of 128 x 64 states), and close behind shared memory: a read hands a lane 16 bytes, 512 a warp, at 128 bytes a cycle
+// whoever shares the address, so q and k have to serve four columns each (two columns per lane, as above, take 84 cycles per warp and token,
+// four 45).  Tokens go in pairs, so that the 8 sums of a lane fold over the LS lanes with all of them useful and one
+// token's products cover the other's shuffles; one barrier per 16 tokens, no partial sums in shared memory.  Entries are taken longest first.
+// Prompts of 700 to 2048 tokens, 8 sequences x 64 heads of 128 x 64 states: 1670 -> 1030 us (320 cycles per token and head on a full SM, 430 before);
+// one sequence of 2048 723 -> 383; 32 heads of 64 x 64, 8 sequences 237 -> 125.
+constexpr int kPortionCols = 4;
+// Sums of r[0 .. CNT) over LS lanes, neighbours first: while a lane has several it gives half of them away, so that lane s ends up with the sum `at`.
+template <int CNT, int X, int LS, int M>
+__device__ __forceinline__ void fold_lanes(float (&r)[M], int s, int& at) {
+  if constexpr (X < LS) {
+    if constexpr (CNT > 1) {
+      constexpr int half = CNT / 2;
+      const bool up = s & X;
+      at += up ? half : 0;
+#pragma unroll
+      for (int e = 0; e < half; ++e) {
+        const float give = up ? r[e] : r[e + half], mine = up ? r[e + half] : r[e];
+        r[e] = mine + __shfl_xor_sync(0xffffffffu, give, X);
+      }
+      fold_lanes<half, 2 * X, LS>(r, s, at);
+    } else {
+      r[0] += __shfl_xor_sync(0xffffffffu, r[0], X);
+      fold_lanes<1, 2 * X, LS>(r, s, at);
+    }
+  }
+}
+template <int DKP, int CH, int W, int MB>
+__global__ void __launch_bounds__(32 * W, MB) lin_portion_kernel(LinRecArgs a) {
+  constexpr int NC = kPortionCols;
+  constexpr int LS = DKP / CH, CW = 32 / LS * NC, BC = W * CW, kTok = 16, NB = CH / 8, NT = 32 * W;
+  constexpr int PS = LS + (CH == 8 ? 4 : 2), QS = CH * PS;  // float4 between pieces, floats of a row
+  constexpr int per_tok = 2 * QS + BC + 4, stage_floats = kTok * per_tok;
+  extern __shared__ __align__(16) float sm[];  // 2 stages
+  __shared__ int s_len[128], s_b;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int per_entry = a.H * ((a.Dv + BC - 1) / BC), rest = blockIdx.x % per_entry, h = rest % a.H, c0 = rest / a.H * BC;
+  int b = blockIdx.x / per_entry;
+  if (a.B > 1 && a.B <= 128) {
+    for (int e = threadIdx.x; e < a.B; e += NT) s_len[e] = a.cu[e + 1] - a.cu[e];
+    __syncthreads();
+    for (int e = threadIdx.x; e < a.B; e += NT) {
+      const int n = s_len[e];
+      int rank = 0;
+      for (int i = 0; i < a.B; ++i) rank += s_len[i] > n || (s_len[i] == n && i < e);
+      if (rank == b) s_b = e;
+    }
+    __syncthreads();
+    b = s_b;
+  }
+  const int kvh = h / (a.H / a.G), t0 = a.cu[b], t1 = a.cu[b + 1];
+  if (t1 <= t0) return;
+  const int s = lane % LS, cl = w * CW + lane / LS * NC, j0 = c0 + cl, ch0 = s * CH;
+  float* st = a.state + (size_t)a.slots[b] * a.slot_stride + a.s_off + (size_t)h * a.Dk * a.Dv + (size_t)ch0 * a.Dv + j0;
+  const bool hd = a.head_decay != nullptr;
+  const float2 hab = make_float2(hd ? a.head_decay[h] : 0.f, 1.f);
+  if (a.Dk < DKP || a.Dv % BC != 0) {  // padded channels and columns read zeros
+    for (int e = threadIdx.x; e < 2 * stage_floats; e += NT) sm[e] = 0.f;
+    __syncthreads();
+  }
+  // Rows of q and k in shared memory: [4-channel piece of a lane's CH][lane of LS], so that a read of 16 bytes covers all banks.  Warp w
+  // stages the tokens w, w + W, ...; a lane one piece of q and of k (DKP / 128 of them), and v or the decay
+  const float* gq = a.q + (size_t)(t0 + w) * a.ldq + a.q_off + (size_t)kvh * a.Dk + lane * 4;
+  const float* gk = a.k + (size_t)(t0 + w) * a.ldk + a.k_off + (size_t)kvh * a.Dk + lane * 4;
+  const float* gv = a.v + (size_t)(t0 + w) * a.ldv + a.v_off + (size_t)h * a.Dv + c0 + lane * 4;
+  const float* gd = a.ab + (size_t)(t0 + w) * a.ldab + (lane & 1) * a.H + h;
+  const long dq = W * a.ldq, dk = W * a.ldk, dv = W * a.ldv, dd = W * a.ldab;
+  const bool in_v = lane * 4 < BC && c0 + lane * 4 < a.Dv;
+  auto issue = [&](int tc, int stage) {
+    const int nt = min(kTok, t1 - tc);
+    float* dst = sm + stage * stage_floats + w * per_tok;
+#pragma unroll
+    for (int r = 0; r < kTok / W; ++r) {
+      if (w + r * W < nt) {
+#pragma unroll
+        for (int p = 0; p < (DKP + 127) / 128; ++p) {
+          const int i = lane * 4 + p * 128, at = (i % CH / 4 * PS + i / CH) * 4;
+          if (i < a.Dk) {
+            cpa16(dst + at, gq + p * 128);
+            cpa16(dst + QS + at, gk + p * 128);
+          }
+        }
+        if (in_v) cpa16(dst + 2 * QS + lane * 4, gv);
+        if (!hd && lane >= 30) cpa4(dst + 2 * QS + BC + lane - 30, gd);
+      }
+      gq += dq; gk += dk; gv += dv; gd += dd;
+      dst += W * per_tok;
+    }
+    cpa_commit();
+  };
+  issue(t0, 0);
+  float2 S[NC][CH / 2];
+  const bool fresh = a.first_pos[b] == 0;
+#pragma unroll
+  for (int i = 0; i < CH / 2; ++i)
+#pragma unroll
+    for (int e = 0; e < NC; e += 4) {
+      const bool in = !fresh && ch0 + 2 * i < a.Dk && j0 + e < a.Dv;  // (Dk and Dv are multiples of four)
+      const float4 x = in ? *reinterpret_cast<const float4*>(st + (size_t)(2 * i) * a.Dv + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 y = in ? *reinterpret_cast<const float4*>(st + (size_t)(2 * i + 1) * a.Dv + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+      S[e][i] = make_float2(x.x, y.x);
+      S[e + 1][i] = make_float2(x.y, y.y);
+      S[e + 2][i] = make_float2(x.z, y.z);
+      S[e + 3][i] = make_float2(x.w, y.w);
+    }
+  const float skip = a.skip ? (a.f32 ? ((const float*)a.skip)[h] : __bfloat162float(((const bf16*)a.skip)[h])) : 0.f;
+  float* out = a.out + (size_t)h * a.Dv + j0;
+  // N neighbouring tokens of a stage
+  auto tokens = [&](const float* tk, size_t row, auto count) {
+    constexpr int N = decltype(count)::value;
+    float r[N * NC];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const float2 dab = hd ? hab : *reinterpret_cast<const float2*>(tk + u * per_tok + 2 * QS + BC);
+      const float2 da2 = make_float2(dab.x, dab.x);
+      float2 bv2[NC];
+#pragma unroll
+      for (int e = 0; e < NC; e += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(tk + u * per_tok + 2 * QS + cl + e);
+        const float bv[4] = {dab.y * v.x, dab.y * v.y, dab.y * v.z, dab.y * v.w};
+#pragma unroll
+        for (int f = 0; f < 4; ++f) bv2[e + f] = make_float2(bv[f], bv[f]);
+      }
+      const float4* q4 = reinterpret_cast<const float4*>(tk + u * per_tok) + s;
+      const float4* k4 = reinterpret_cast<const float4*>(tk + u * per_tok + QS) + s;
+#pragma unroll
+      for (int n = 0; n < NB; ++n) {
+        float2 oa[NC];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float4 q = q4[(2 * n + i) * PS], k = k4[(2 * n + i) * PS];
+          const float2 k01 = make_float2(k.x, k.y), k23 = make_float2(k.z, k.w), q01 = make_float2(q.x, q.y), q23 = make_float2(q.z, q.w);
+#pragma unroll
+          for (int e = 0; e < NC; ++e) {
+            float2& sa = S[e][n * 4 + 2 * i];
+            float2& sb = S[e][n * 4 + 2 * i + 1];
+            sa = __ffma2_rn(da2, sa, __fmul2_rn(k01, bv2[e]));
+            oa[e] = i == 0 ? __fmul2_rn(sa, q01) : __ffma2_rn(sa, q01, oa[e]);
+            sb = __ffma2_rn(da2, sb, __fmul2_rn(k23, bv2[e]));
+            oa[e] = __ffma2_rn(sb, q23, oa[e]);
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < NC; ++e) r[u * NC + e] = n == 0 ? oa[e].x + oa[e].y : r[u * NC + e] + (oa[e].x + oa[e].y);
+      }
+    }
+    int at = 0;  // (token, column) of the sum that this lane keeps
+    fold_lanes<N * NC, 1, LS>(r, s, at);
+    static_assert(N * NC <= LS, "one sum per lane");
+    const int u = at / NC, e = at % NC;
+    if (s < N * NC && j0 + e < a.Dv) out[(row + u) * a.ldo + e] = fmaf(skip, tk[u * per_tok + 2 * QS + cl + e], r[0] * a.q_scale);
+  };
+  int stage = 0;
+  for (int tc = t0; tc < t1; tc += kTok, stage ^= 1) {
+    const int nt = min(kTok, t1 - tc);
+    cpa_wait<0>();
+    __syncthreads();  // the stage has landed, and everybody is done with the other one
+    if (tc + kTok < t1) issue(tc + kTok, stage ^ 1);
+    float* base = sm + stage * stage_floats;
+    if (a.silu) {  // activations of the staged q | k | v, once per stage
+      for (int e = threadIdx.x; e < nt * (2 * QS + BC); e += NT) {
+        float& z = base[e / (2 * QS + BC) * per_tok + e % (2 * QS + BC)];
+        z = z * sigmoidf_(z);
+      }
+      __syncthreads();
+    }
+    int tt = 0;
+#pragma unroll 1
+    for (; tt + 2 <= nt; tt += 2) tokens(base + tt * per_tok, (size_t)(tc + tt), std::integral_constant<int, 2>());
+    if (tt < nt) tokens(base + tt * per_tok, (size_t)(tc + tt), std::integral_constant<int, 1>());
+  }
+#pragma unroll
+  for (int i = 0; i < CH / 2; ++i)
+#pragma unroll
+    for (int e = 0; e < NC; e += 4) {
+      if (ch0 + 2 * i >= a.Dk || j0 + e >= a.Dv) continue;
+      *reinterpret_cast<float4*>(st + (size_t)(2 * i) * a.Dv + e) = make_float4(S[e][i].x, S[e + 1][i].x, S[e + 2][i].x, S[e + 3][i].x);
+      *reinterpret_cast<float4*>(st + (size_t)(2 * i + 1) * a.Dv + e) = make_float4(S[e][i].y, S[e + 1][i].y, S[e + 2][i].y, S[e + 3][i].y);
+    }
+}
+// (portions of up to eight tokens on average are bound by the state's bytes, which the smaller pieces above have more of in flight: 32 sequences of 5 to
+// 10 tokens x 32 heads of 128 x 64 states 31 us there, 33 here)
+bool lin_portion_ok(const LinRecArgs& a) {
+  return !a.nq && a.T > 8 * a.B && a.Dk > 32 && a.Dv > 32 && ((a.Dk | a.Dv | (int)a.ldq | (int)a.ldk | (int)a.ldv | a.q_off | a.k_off | a.v_off) & 3) == 0 &&
+         ((a.slot_stride | (long)a.s_off) & 3) == 0 && (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.state) & 15) == 0;
+}
+template <int DKP, int CH, int W>
+constexpr int portion_cols() { return W * (32 / (DKP / CH)) * kPortionCols; }
+template <int DKP, int CH, int W>
+constexpr int portion_smem() { return 2 * 16 * (2 * CH * (DKP / CH + (CH == 8 ? 4 : 2)) + portion_cols<DKP, CH, W>() + 4) * 4; }
+template <int DKP, int CH, int W, int MB>
+cudaError_t launch_portion(cudaStream_t s, const LinRecArgs& a) {
+  constexpr int BC = portion_cols<DKP, CH, W>();
+  const long blocks = (long)a.B * a.H * ((a.Dv + BC - 1) / BC);
+  if (blocks > INT_MAX) return cudaErrorInvalidValue;
+  return launch_k(lin_portion_kernel<DKP, CH, W, MB>, dim3((unsigned)blocks), dim3(32 * W), portion_smem<DKP, CH, W>(), s, true, a);
+}
+
 // The same for entries of one token (decoding): bound by the state's bytes, 32 KB in and out per block of a 128 x 64 state.  Everything a
 // block needs is loaded at once (the staging above spent a round trip on the state, one on the token and three barriers): 16
 // sequences x 32 heads 12.2 -> 9.1 us.  Warp w has key channels 16 w .. 16 w + 15, a lane two neighbouring columns; the
 // arithmetic and its order are those of the kernel above, so both give the same bits.
 __global__ void lin_step_kernel(LinRecArgs a) {
-  __shared__ float obuf[16][64];
+  __shared__ __align__(8) float obuf[16][64];
   pdl_launch_dependents();
   pdl_wait();
   const int b = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * 64, kvh = h / (a.H / a.G);
@@ -430,9 +640,9 @@ __global__ void lin_step_kernel(LinRecArgs a) {
     act(vv.x);
     act(vv.y);
   }
-  // columns j0 (x) and j0 + 1 (y); even and odd channels have a sum each
+  // columns j0 (x) and j0 + 1 (y); even and odd channels of eight have a sum each
   const float bx = db * vv.x, by = db * vv.y;
-  float2 ox = make_float2(0.f, 0.f), oy = ox;
+  float2 ox[2], oy[2];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const float kk[4] = {k4[i].x, k4[i].y, k4[i].z, k4[i].w}, qq[4] = {q4[i].x, q4[i].y, q4[i].z, q4[i].w};
@@ -441,24 +651,34 @@ __global__ void lin_step_kernel(LinRecArgs a) {
       float2& s = S[4 * i + e];
       s.x = __fmaf_rn(da, s.x, __fmul_rn(kk[e], bx));
       s.y = __fmaf_rn(da, s.y, __fmul_rn(kk[e], by));
-      (e & 1 ? ox.y : ox.x) = __fmaf_rn(s.x, qq[e], e & 1 ? ox.y : ox.x);
-      (e & 1 ? oy.y : oy.x) = __fmaf_rn(s.y, qq[e], e & 1 ? oy.y : oy.x);
+      float& sx = e & 1 ? ox[i / 2].y : ox[i / 2].x;
+      float& sy = e & 1 ? oy[i / 2].y : oy[i / 2].x;
+      sx = i % 2 == 0 && e < 2 ? __fmul_rn(s.x, qq[e]) : __fmaf_rn(s.x, qq[e], sx);
+      sy = i % 2 == 0 && e < 2 ? __fmul_rn(s.y, qq[e]) : __fmaf_rn(s.y, qq[e], sy);
     }
   }
 #pragma unroll
   for (int i = 0; i < 16; ++i)
     if (cols && i0 + i < a.Dk) *reinterpret_cast<float2*>(st + (size_t)i * a.Dv) = S[i];
-  obuf[w][lane * 2] = ox.x + ox.y;
-  obuf[w][lane * 2 + 1] = oy.x + oy.y;
+  obuf[w][lane * 2] = (ox[0].x + ox[0].y) + (ox[1].x + ox[1].y);
+  obuf[w][lane * 2 + 1] = (oy[0].x + oy[0].y) + (oy[1].x + oy[1].y);
   __syncthreads();
   const int warps = blockDim.x >> 5;
   if (w == 0 && cols) {
     const float skip = a.skip ? (a.f32 ? ((const float*)a.skip)[h] : __bfloat162float(((const bf16*)a.skip)[h])) : 0.f;
-    float2 o = make_float2(0.f, 0.f);
-    for (int ww = 0; ww < warps; ++ww) {
-      o.x += obuf[ww][lane * 2];
-      o.y += obuf[ww][lane * 2 + 1];
+    float2 part[16];
+#pragma unroll
+    for (int ww = 0; ww < 16; ++ww) part[ww] = ww < warps ? *reinterpret_cast<const float2*>(&obuf[ww][lane * 2]) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int st = 1; st < 16; st *= 2) {
+      if (st >= warps) break;
+#pragma unroll
+      for (int ww = 0; ww < 16; ww += 2 * st) {
+        part[ww].x += part[ww + st].x;
+        part[ww].y += part[ww + st].y;
+      }
     }
+    const float2 o = part[0];
     *reinterpret_cast<float2*>(a.out + (size_t)t * a.ldo + (size_t)h * a.Dv + j0) = make_float2(fmaf(skip, vv.x, o.x * a.q_scale), fmaf(skip, vv.y, o.y * a.q_scale));
   }
 }
@@ -764,6 +984,11 @@ cudaError_t stack_ssm_init() {
   HB_SMEM((lin_recurrence_kernel<64, 2>), 96 * 1024);
   HB_SMEM((lin_recurrence_kernel<128, 2>), 128 * 1024);
   HB_SMEM((lin_recurrence_kernel<256, 2>), 200 * 1024);
+  HB_SMEM((lin_portion_kernel<64, 8, 4, 5>), (portion_smem<64, 8, 4>()));
+  HB_SMEM((lin_portion_kernel<128, 8, 4, 5>), (portion_smem<128, 8, 4>()));
+  HB_SMEM((lin_portion_kernel<128, 16, 4, 4>), (portion_smem<128, 16, 4>()));
+  HB_SMEM((lin_portion_kernel<256, 16, 4, 4>), (portion_smem<256, 16, 4>()));
+  HB_SMEM((lin_portion_kernel<256, 16, 8, 2>), (portion_smem<256, 16, 8>()));
   HB_SMEM(parallel_step_kernel<float>, 200 * 1024);
   HB_SMEM(parallel_step_kernel<bf16>, 200 * 1024);
 #undef HB_SMEM
@@ -826,6 +1051,14 @@ cudaError_t lin_recurrence(cudaStream_t s, const LinRecArgs& a) {
   if (a.B <= 0) return cudaSuccess;
   if (a.G <= 0 || a.H % a.G || a.Dk > 256 || a.Dk <= 0) return cudaErrorInvalidValue;
   if (lin_step_ok(a)) return launch_k(lin_step_kernel, dim3(a.B, a.H, (a.Dv + 63) / 64), dim3((a.Dk + 15) / 16 * 32), 0, s, true, a);
+  if (lin_portion_ok(a)) {
+    // narrower blocks where the wide ones are no more than the SMs (us wide / narrow: one sequence of 2048 tokens x 64 heads of 128 x 64 states
+    // 492 / 383, four of 500 to 1000 316 / 361; 32 heads of 256 x 40 125 / 92)
+    const bool few = (long)a.B * a.H * ((a.Dv + 63) / 64) <= effective_sms(148);
+    if (a.Dk <= 64) return launch_portion<64, 8, 4, 5>(s, a);
+    if (a.Dk <= 128) return few ? launch_portion<128, 8, 4, 5>(s, a) : launch_portion<128, 16, 4, 4>(s, a);
+    return few ? launch_portion<256, 16, 4, 4>(s, a) : launch_portion<256, 16, 8, 2>(s, a);
+  }
   // two columns per lane (blocks of 64 columns) halve the shared-memory reads per product; heads of up to 32 value columns
   // keep one.  HB_REC_COLS=1 forces the narrow blocks (A/B measurements)
   // (the arithmetic per column is the same either way, so the choice never shows in a result; narrow blocks for small grids
