@@ -293,16 +293,17 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {  // splitmix64 finaliser
 __device__ __forceinline__ void argmax_merge(float& best, int& bi, float ov, int oi) {
   if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
 }
-// standard Gumbel noise of (seed, column)
-__device__ __forceinline__ float gumbel(uint64_t sd, int v) {
+// standard Gumbel noise of (seed, column): -log(-log u) of a uniform u
+__device__ __forceinline__ float gumbel_uniform(uint64_t sd, int v) {
   const uint64_t h = mix64(sd ^ (0xD1B54A32D192ED03ull * (uint64_t)(v + 1)));
   // 23 random bits + 0.5: every value is exact in fp32 and u stays strictly inside (0,1) — with 24 bits the
   // "+0.5f" rounds the top half of the range up and u == 1.0 made the noise +inf (a uniformly random token won
-  // once per 2^24 draws, ~0.8 % of sampled tokens at a 128k vocabulary).  The inner log is the accurate one: the
-  // fast-math log has an absolute error comparable to log(1 - 2^-24).
-  const float u = ((float)(h >> 41) + 0.5f) * (1.0f / 8388608.0f);
-  return -__logf(-logf(u));
+  // once per 2^24 draws, ~0.8 % of sampled tokens at a 128k vocabulary).
+  return ((float)(h >> 41) + 0.5f) * (1.0f / 8388608.0f);
 }
+// The inner log is the accurate one: the fast-math log has an absolute error comparable to log(1 - 2^-24).
+__device__ __forceinline__ float gumbel_of(float u) { return -__logf(-logf(u)); }
+__device__ __forceinline__ float gumbel(uint64_t sd, int v) { return gumbel_of(gumbel_uniform(sd, v)); }
 template <int NT>
 __device__ __forceinline__ void block_argmax(float& best, int& bi, float* sval, int* sidx) {
 #pragma unroll
@@ -447,30 +448,41 @@ __device__ __forceinline__ void load_slice(const float* __restrict__ src, int n,
 // The threshold that separates the survivors is found on the ordered 32-bit keys:
 //   top-k : the largest key that keeps >= k tokens (ties at the k-th value are all kept)
 //   top-p : among the top-k survivors, the largest key whose tokens' softmax(logits/T) mass reaches p of the survivors' mass
-// Probability mass is accumulated in 2^-32 fixed point, so every sum is exact and independent of its order.  A pass compares a
-// part with three keys inside the interval that still holds the answer; once the interval holds at most kFin tokens, block 0
-// gets them and finds the answer directly.
-// Measured (32 rows x 128256, mixed top-k / top-p): 1100 us with a block per row and up to 32 + 32 one-key passes, 62 us now.
-constexpr int kFin = 256, kBins = 128;
-struct SampleShared {
-  uint32_t hist[2][3][kBins];  // this block's tokens per value bin, the low 16 bits of their masses, the rest
-  unsigned long long tot_c[kBins], tot_m[kBins];
+// Probability mass is accumulated in 2^-32 fixed point, so every sum is exact and independent of its order.
+// One pass counts the tokens in kBins bins of values and sums the mass.  The counts give top-k's bin, and with each bin's mean weight an
+// estimate of where the mass of top-p is reached, good to a few dozen tokens; a second pass sums the mass above a bracket around it exactly
+// and hands the bracket's tokens, at most kFin, to block 0, which ranks them and checks that the answer is among them.  Where it is not
+// (or the bins are no use: infinite maxima, hundreds of equal logits) the keys are searched by halves.  What is left of the time: the load, these two
+// passes and the draw over 32 tokens a thread each, and seven cluster barriers.
+// Measured (us, with passes of three keys or 128 bins of masses | now): 32 rows of 128256, kinds of filters mixed 60 | 32, top_p 0.95 68 | 35, top_k 40 25 | 21;
+// 1 row 38 | 23; 64 rows of 32768 35 | 23.  The bins cost two barriers before anything is known, so rows whose first pass of keys had left next to
+// nothing are a little slower (temperature 0.1, top_p 0.8, 64 rows of 32768 18 | 21; of 128256 53 | 50).
+constexpr int kFin = 1024, kBins = 4096, kHeavy = 512;
+constexpr float kReach = 80.f;  // tokens on either side of the estimate
+struct alignas(16) SampleShared {
+  uint32_t hist[kBins];  // tokens per bin: this block's, then the cluster's; afterwards the warps' queues of survivors
+  uint32_t heavy[kHeavy];  // mass of the highest bins, in units of 2^-20: this block's, then (a float) the cluster's
   unsigned long long part[2][5];  // this block's totals of a pass: counts (c1 | c2 << 32), c3, masses m1 .. m3
   unsigned long long wred[kVocWarps][5];
-  uint32_t list[kFin];
-  unsigned long long mass[kFin];
-  float val[kVocWarps];
-  int idx[kVocWarps];
+  unsigned long long post[2][8];  // the blocks' shares of a sum
+  alignas(16) uint32_t list[kFin];
+  uint32_t sorted[256];
+  float val[kVocWarps], top[8];  // (the blocks' maxima, at the end their best values)
+  int idx[kVocWarps], top_idx[8];
+  uint32_t warp_c[kVocWarps];
+  float warp_m[kVocWarps], reach;
+  int bin[2];        // bracket: its lowest and highest bin, the tokens from the lowest up and above the highest
+  uint32_t upto[2];
+  unsigned long long top_mass;
   uint32_t n_list, result;
-  float best_val, row_max;
-  int best_idx;
 };
+constexpr int kQueue = kBins / kVocWarps;  // survivors that a warp collects before it draws for 32 of them
 
 template <int NC, bool SM>
-__global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(kVocThreads)
-sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict__ temperature, const uint64_t* __restrict__ seed,
+__global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(kVocThreads, 2)
+sample_cluster_kernel(const float* __restrict__ logits, int ldl, const float* __restrict__ temperature, const uint64_t* __restrict__ seed,
               const int32_t* __restrict__ top_k, const float* __restrict__ top_p, int32_t* __restrict__ out, int V) {
-  extern __shared__ __align__(16) uint32_t keys[];
+  extern __shared__ __align__(16) float slice[];
   __shared__ SampleShared sh;
   pdl_launch_dependents();
   pdl_wait();
@@ -484,53 +496,84 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
   const float inv_t = greedy ? 1.f : 1.f / temp;
   const int k = top_k ? top_k[b] : 0;
   const float p = top_p ? top_p[b] : 1.f;
-  const bool use_k = !greedy && k > 0 && k < V, use_p = !greedy && p > 0.f && p < 1.f;
+  const bool use_k = !greedy && k > 0 && k < V, use_p = !greedy && p > 0.f && p < 1.f, filters = use_k || use_p;
+
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  const uint64_t sd = seed ? seed[b] : 0;
+  auto draw = [&](float raw, int i) {
+    const int v = start + i;
+    float x = raw * inv_t;
+    if (!greedy) x += gumbel(sd, v);
+    argmax_merge(best, bi, x, v);
+  };
+  // The same for every token of a part.  -log(-log u) <= -log(1 - u), one fast logarithm: where not even that (and a thousandth, far
+  // above the rounding of both) reaches what the warp has found so far, which is soon true of nearly all, the exact noise is not needed.
+  float bar = -INFINITY;
+  auto draw_over = [&](const float (&raw)[4], int i, int have) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (e >= have || raw[e] != raw[e]) continue;  // a NaN is never drawn
+      if (greedy) {
+        argmax_merge(best, bi, raw[e], start + i + e);
+      } else {
+        const float u = gumbel_uniform(sd, start + i + e), x = raw[e] * inv_t;
+        if (!(x + (1e-3f - __logf(1.f - u)) < bar)) argmax_merge(best, bi, x + gumbel_of(u), start + i + e);
+      }
+    }
+    bar = fmaxf(bar, best);
+  };
+  auto share_bar = [&] { bar = fkey_inv(__reduce_max_sync(__activemask(), fkey(bar))); };
 
   if (tid == 0) sh.n_list = 0;
+  if constexpr (NC > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // (this block runs: others may write to it)
   float mx = -INFINITY;
-  if constexpr (SM) {  // (entries behind the slice's end read as key 0, below every float's key)
+  if constexpr (SM) {  // (entries behind the slice's end read as NaN)
     load_slice(row, n, tid, [&](int i, const float (&f)[4], int have) {
-      uint32_t q[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        mx = fmaxf(mx, e < have ? f[e] : -INFINITY);
-        q[e] = e < have ? fkey(f[e]) : 0u;
+      if (!filters) {
+        draw_over(f, i, have);
+        share_bar();
+        return;
       }
-      *reinterpret_cast<uint4*>(keys + i) = make_uint4(q[0], q[1], q[2], q[3]);
+      const float none = __int_as_float(0x7fffffff);
+      const float4 v = make_float4(f[0], have > 1 ? f[1] : none, have > 2 ? f[2] : none, have > 3 ? f[3] : none);
+      mx = fmaxf(fmaxf(mx, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
+      *reinterpret_cast<float4*>(slice + i) = v;
     });
-  } else if (use_k || use_p) {
+  } else if (filters) {
     for (int i = tid; i < n; i += kVocThreads) mx = fmaxf(mx, __ldg(row + i));
   }
   __syncthreads();
-  auto scan = [&](auto&& f) {  // f(key, index inside the slice)
+  if constexpr (NC > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  auto scan = [&](auto&& f) {  // f(logit)
     if constexpr (SM) {
       for (int i = tid * 4; i < n; i += kVocThreads * 4) {
-        const uint4 q = *reinterpret_cast<const uint4*>(keys + i);
-        f(q.x, i);
-        f(q.y, i + 1);
-        f(q.z, i + 2);
-        f(q.w, i + 3);
+        const float4 q = *reinterpret_cast<const float4*>(slice + i);
+        f(q.x);
+        f(q.y);
+        f(q.z);
+        f(q.w);
       }
     } else {
-      for (int i = tid; i < n; i += kVocThreads) f(fkey(__ldg(row + i)), i);
+      for (int i = tid; i < n; i += kVocThreads) f(__ldg(row + i));
     }
   };
 
   float floor_logit = -INFINITY;
-  if (use_k || use_p) {
+  if (filters) {
     // row maximum (for the softmax weights)
     const uint32_t wm = __reduce_max_sync(0xffffffffu, fkey(mx));
     if (lane == 0) sh.val[warp] = fkey_inv(wm);
     __syncthreads();
     mx = sh.val[lane & (kVocWarps - 1)];
     mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(mx)));
-    if (tid == 0) sh.row_max = mx;
+    if (tid < NC) cluster_ptr<NC>(sh.top, tid)[rank] = mx;
     voc_sync<NC>();
-    mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(*cluster_ptr<NC>(&sh.row_max, lane & (NC - 1)))));
+    mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(sh.top[lane & (NC - 1)])));
 
-    auto weight = [&](uint32_t key) -> u64 {
-      const float e = __expf((fkey_inv(key) - mx) * inv_t) * 4294967296.0f;
-      return e >= 0.f ? (u64)e : 0;  // a NaN logit carries no mass
+    auto weight_at = [&](float x) -> u64 {
+      const float e = __expf((x - mx) * inv_t) * 4294967296.0f;
+      return e >= 0.f ? (u64)__float2uint_rz(e) + (e >= 4294967296.0f) : 0;  // (2^32 at the maximum itself; a NaN logit carries no mass)
     };
     int turn = 0;
     // sums of the cluster's blocks, in every thread of every block
@@ -538,6 +581,24 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
       const u64 a = __reduce_add_sync(0xffffffffu, (uint32_t)v & 0xffffu), c = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 16) & 0x1fffffu),
                 d = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 37));
       return a + (c << 16) + (d << 37);
+    };
+    int at_post = 0;
+    auto cluster_add = [&](u64 v) -> u64 {
+      v = warp_total(v);
+      if (lane == 0) sh.wred[warp][0] = v;
+      __syncthreads();
+      if (warp == 0) {
+        u64 t = lane < kVocWarps ? sh.wred[lane][0] : 0;
+#pragma unroll
+        for (int o = kVocWarps / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane < NC) cluster_ptr<NC>(sh.post[at_post], lane)[rank] = t;
+      }
+      voc_sync<NC>();
+      u64 t = 0;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) t += sh.post[at_post][c];
+      at_post ^= 1;  // (a slot is written again two sums later, behind the barrier that follows every read of it)
+      return t;
     };
     auto cluster_sum = [&](u64 (&v)[5]) {
 #pragma unroll
@@ -566,25 +627,524 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
       }
       turn ^= 1;  // (a slot is written again two passes later, behind the barrier that follows every read of it)
     };
-    // the largest key whose tokens (those with keys >= it) reach `goal`: in number, or in mass (by_mass).  Keeping [lo, ..) is
+    // Block 0: the largest key of its list whose tokens, with c_hi tokens of mass m_hi above the list, reach `goal` in number or in mass;
+    // `both`: goal in number first, then p of the mass of the tokens that this keeps.  Every block gets the answer (0: there is none).
+    // The list is sorted (falling), its masses summed up along the way.
+    auto decide = [&](bool by_mass, u64 goal, u64 c_hi, u64 m_hi, bool both) -> uint32_t {
+      if (rank == 0) {
+        const int nl = (int)sh.n_list, len = nl <= 256 ? 256 : nl <= 512 ? 512 : kFin;
+        const uint32_t* list = sh.list;
+        for (int i = nl + tid; i < len; i += kVocThreads) sh.list[i] = 0u;
+        if (tid < 256) sh.sorted[tid] = 0u;
+        if (tid == 0) sh.idx[0] = 0;
+        __syncthreads();
+        if (len == 256) {  // two threads per entry count the entries before it
+          const int at = tid >> 1;
+          const uint32_t key = sh.list[at];
+          uint32_t before = 0;
+#pragma unroll 4
+          for (int j = tid & 1; j < (nl + 3) / 4; j += 2) {
+            const uint4 q = *reinterpret_cast<const uint4*>(sh.list + 4 * j);
+            before += (q.x > key) + (q.y > key) + (q.z > key) + (q.w > key);
+            before += (q.x == key && 4 * j < at) + (q.y == key && 4 * j + 1 < at) + (q.z == key && 4 * j + 2 < at) + (q.w == key && 4 * j + 3 < at);
+          }
+          before += __shfl_xor_sync(0xffffffffu, before, 1);
+          if ((tid & 1) == 0 && key != 0) sh.sorted[before] = key;
+          list = sh.sorted;
+        } else {
+          for (int m = 2; m <= len; m *= 2)
+            for (int j = m / 2; j > 0; j /= 2) {
+              const int i = 2 * tid - (tid & (j - 1));
+              if (tid < len / 2) {
+                const uint32_t x = sh.list[i], y = sh.list[i + j];
+                if ((i & m) == 0 ? x < y : x > y) {
+                  sh.list[i] = y;
+                  sh.list[i + j] = x;
+                }
+              }
+              if (j > 32 || (j == 1 && m > 32)) __syncthreads();  // (pairs up to 32 apart stay inside a warp's 64 entries)
+              else __syncwarp();
+            }
+        }
+        __syncthreads();
+        const bool in = tid < len / 2;
+        const uint32_t k0 = in ? list[2 * tid] : 0u, k1 = in ? list[2 * tid + 1] : 0u;
+        const u64 w0 = k0 ? weight_at(fkey_inv(k0)) : 0, w1 = k1 ? weight_at(fkey_inv(k1)) : 0;
+        u64 upto = w0 + w1;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const u64 t = __shfl_up_sync(0xffffffffu, upto, o);
+          if (lane >= o) upto += t;
+        }
+        if (lane == 31) sh.wred[warp][0] = upto;
+        __syncthreads();
+        for (int w = 0; w < warp; ++w) upto += sh.wred[w][0];
+        const u64 m1 = upto, m0 = upto - w1, before = m0 - w0;
+        auto first = [&](u64 want) {  // the entry at which the mass reaches `want`
+          if (k0 && m_hi + m0 >= want && m_hi + before < want) sh.idx[0] = (int)k0;
+          if (k1 && m_hi + m1 >= want && m_hi + m0 < want) sh.idx[0] = (int)k1;
+          __syncthreads();
+        };
+        if (by_mass) {
+          first(goal);
+        } else if (goal > c_hi && goal - c_hi <= (u64)nl) {
+          const uint32_t kth = list[goal - c_hi - 1];
+          if (!both) {
+            if (tid == 0) sh.idx[0] = (int)kth;
+            __syncthreads();
+          } else {
+            const uint32_t k2 = 2 * tid + 2 < len ? list[2 * tid + 2] : 0u;
+            if (in && k0 >= kth && k1 < kth) sh.top_mass = m0;
+            if (in && k1 >= kth && k2 < kth) sh.top_mass = m1;
+            if (tid == 0) sh.idx[0] = (int)kth;  // (no mass at all: all of them)
+            __syncthreads();
+            first(max((u64)1, (u64)((double)p * (double)sh.top_mass)));
+          }
+        }
+        if (tid < NC) *cluster_ptr<NC>(&sh.result, tid) = (uint32_t)sh.idx[0];
+        if (tid == 0) sh.n_list = 0;
+      }
+      voc_sync<NC>();
+      return sh.result;
+    };
+    auto list_token = [&](uint32_t q) { cluster_ptr<NC>(sh.list, 0)[atomicAdd(cluster_ptr<NC>(&sh.n_list, 0), 1u)] = q; };
+    // Without bins: the largest key whose tokens (those with keys >= it) reach `goal`: in number, or in mass (by_mass).  Keeping [lo, ..) is
     // enough (c_lo tokens), keeping [hi, ..) is not (c_hi tokens of mass m_hi).
     auto search = [&](bool by_mass, u64 goal, u64 lo, u64 c_lo) -> u64 {
       u64 hi = (u64)fkey(mx) + 1, c_hi = 0, m_hi = 0;  // (nothing is above the maximum)
-      for (int pass = 0; hi - lo > 1 && c_lo - c_hi > (u64)kFin; ++pass) {
+      for (int pass = 0; hi - lo > 1 && c_lo - c_hi > 256; ++pass) {
         // Logits are spread more evenly over values than over keys (where half of all keys are exponents nothing has): the first
         // pass looks a few temperatures below the maximum, the next ones divide the values between the bounds; from the eighth
         // on the keys are divided, so at most 8 + 16 passes are needed.
         const u64 d = hi - lo;
-        // A mass between two finite values: the tokens go into kBins equal bins of values at once, and the bin that holds the answer is
+        u64 t[3];
+        const float flo = fkey_inv((uint32_t)lo), fhi = fkey_inv((uint32_t)(hi - 1));
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const float at = pass == 0 ? mx - temp * (j == 0 ? 16.f : j == 1 ? 8.f : 4.f) : flo + (fhi - flo) * (0.25f * (j + 1));
+          const u64 by_key = lo + max(1ull, j == 0 ? d / 4 : j == 1 ? d / 2 : d / 4 * 3);
+          t[j] = (pass < 8 && at - at == 0.f) ? min(max((u64)fkey(at), lo + 1), hi - 1) : by_key;
+        }
+        t[1] = max(t[1], t[0]);
+        t[2] = max(t[2], t[1]);
+        u64 v[5] = {0, 0, 0, 0, 0};
+        const uint32_t t1 = (uint32_t)t[0], t2 = (uint32_t)t[1], t3 = (uint32_t)t[2];
+        if (by_mass) {
+          scan([&](float x) {
+            const uint32_t q = fkey(x);
+            if (q < t1) return;
+            const u64 w = weight_at(x);
+            v[0] += q >= t2 ? 0x100000001ull : 1ull;
+            v[2] += w;
+            if (q >= t2) v[3] += w;
+            if (q >= t3) { v[1] += 1; v[4] += w; }
+          });
+        } else {
+          uint32_t c1 = 0, c2 = 0, c3 = 0;
+          scan([&](float x) {
+            const uint32_t q = fkey(x);
+            c1 += q >= t1;
+            c2 += q >= t2;
+            c3 += q >= t3;
+          });
+          v[0] = c1 | (u64)c2 << 32;
+          v[1] = c3;
+        }
+        cluster_sum(v);
+        const u64 c[3] = {v[0] & 0xffffffffull, v[0] >> 32, v[1]}, m[3] = {v[2], v[3], v[4]};
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          if ((by_mass ? m[j] : c[j]) >= goal) {
+            lo = t[j];
+            c_lo = c[j];
+          } else {
+            hi = t[j];
+            c_hi = c[j];
+            m_hi = m[j];
+            break;
+          }
+        }
+      }
+      if (hi - lo <= 1) return lo;
+      // few tokens left: block 0 decides
+      scan([&](float x) {
+        const uint32_t q = fkey(x);
+        if (q != 0 && q >= lo && (u64)q < hi) list_token(q);
+      });
+      voc_sync<NC>();
+      return max((u64)decide(by_mass, goal, c_hi, m_hi, false), lo);
+    };
+    // ---- bins
+    const float width = fmaxf(16.f, 22.5f * temp);  // tokens further below the maximum than 22.2 T weigh nothing
+    const float scale = (float)kBins / width, shift = (width - mx) * scale;
+    auto bin_of = [&](float x) { return (int)min(__float2uint_rz(fmaf(x, scale, shift)), (unsigned)kBins - 1); };  // (0, not counted: NaN and what weighs nothing)
+    // (the second bound keeps a bin's edge within 1.1 bins of where it should be; below it lies -inf too, and no maximum is a NaN)
+    const bool binned = V > kFin && fabsf(mx) * scale < 8388608.f;
+    u64 total = 0;
+    uint32_t tokens = 0, above[8], c_next = 0;  // tokens in the bins; those in this thread's eight bins and everything above each; above all eight
+    float above_m[8], m_next = 0.f;  // and an estimate of their mass
+    if (binned) {
+      for (int e = tid * 4; e < kBins; e += kVocThreads * 4) *reinterpret_cast<uint4*>(sh.hist + e) = make_uint4(0, 0, 0, 0);
+      sh.heavy[tid] = 0;
+      __syncthreads();
+      u64 m = 0;
+      const bool weigh = use_p && !use_k;
+      if (weigh) {
+        scan([&](float x) {
+          const int at = bin_of(x);
+          if (at == 0) return;
+          atomicAdd(&sh.hist[at], 1u);
+          const u64 w = weight_at(x);
+          m += w;
+          if (at >= kBins - kHeavy) atomicAdd(&sh.heavy[at - (kBins - kHeavy)], (uint32_t)(w >> 12));
+        });
+      } else {
+        scan([&](float x) {
+          const int at = bin_of(x);
+          if (at > 0) atomicAdd(&sh.hist[at], 1u);
+        });
+      }
+      total = cluster_add(m);
+      if constexpr (NC > 1) {  // block r adds up the r-th part of the bins and hands it to everybody
+        for (int e = rank * (kBins / NC) + tid; e < (int)(rank + 1) * (kBins / NC); e += kVocThreads) {
+          uint32_t c = 0;
+#pragma unroll
+          for (int r = 0; r < NC; ++r) c += cluster_ptr<NC>(sh.hist, r)[e];
+#pragma unroll
+          for (int r = 0; r < NC; ++r) cluster_ptr<NC>(sh.hist, r)[e] = c;
+        }
+      }
+      if (weigh && tid < kHeavy / NC) {
+        const int e = rank * (kHeavy / NC) + tid;
+        float hm = 0.f;
+#pragma unroll
+        for (int r = 0; r < NC; ++r) hm += (float)cluster_ptr<NC>(sh.heavy, r)[e];
+#pragma unroll
+        for (int r = 0; r < NC; ++r) cluster_ptr<NC>(sh.heavy, r)[e] = __float_as_uint(hm * 4096.f);
+      }
+      voc_sync<NC>();
+      static_assert(kBins == 8 * kVocThreads && kHeavy == kVocThreads, "eight bins per thread");
+      const bool heavy = tid >= (kBins - kHeavy) / 8;  // (whole warps)
+      uint32_t h[8], c = 0;
+      float sm = 0.f;
+      *reinterpret_cast<uint4*>(h) = *reinterpret_cast<const uint4*>(sh.hist + tid * 8);
+      *reinterpret_cast<uint4*>(h + 4) = *reinterpret_cast<const uint4*>(sh.hist + tid * 8 + 4);
+#pragma unroll
+      for (int e = 7; e >= 0; --e) {
+        const int at = tid * 8 + e;
+        c += h[e];
+        if (heavy && weigh) sm += __uint_as_float(sh.heavy[at - (kBins - kHeavy)]);
+        else sm += (float)h[e] * __expf((((float)at + 0.5f) / scale - width) * inv_t) * 4294967296.0f;
+        above[e] = c;
+        above_m[e] = sm;
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t oc = __shfl_down_sync(0xffffffffu, c, o);
+        const float om = __shfl_down_sync(0xffffffffu, sm, o);
+        if (lane + o < 32) { c += oc; sm += om; }
+      }
+      if (lane == 0) { sh.warp_c[warp] = c; sh.warp_m[warp] = sm; }
+      c_next = __shfl_down_sync(0xffffffffu, c, 1);
+      m_next = __shfl_down_sync(0xffffffffu, sm, 1);
+      if (lane == 31) { c_next = 0; m_next = 0.f; }
+      __syncthreads();
+      // the warps above this one; the estimate's bias (values sit anywhere in a bin) goes by what is known: the total, and the heavy bins' share
+      uint32_t wc = lane < kVocWarps ? sh.warp_c[lane] : 0;
+      const float wm2 = lane < kVocWarps ? sh.warp_m[lane] : 0.f;
+      constexpr int kLight = (kBins - kHeavy) / 256;  // warps of the other bins
+      float all_heavy = lane >= kLight ? wm2 : 0.f, all_light = lane < kLight ? wm2 : 0.f, later = lane > warp ? wm2 : 0.f;
+      uint32_t wc_later = lane > warp ? wc : 0;
+      wc_later = __reduce_add_sync(0xffffffffu, wc_later);
+      tokens = __reduce_add_sync(0xffffffffu, wc);
+      if (!heavy) later = lane > warp && lane < kLight ? wm2 : 0.f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        all_heavy += __shfl_xor_sync(0xffffffffu, all_heavy, o);
+        all_light += __shfl_xor_sync(0xffffffffu, all_light, o);
+        later += __shfl_xor_sync(0xffffffffu, later, o);
+      }
+      const float bias = weigh && all_light > 0.f ? fmaxf(((float)total - all_heavy) / all_light, 0.f) : 1.f;
+      c_next += wc_later;
+      m_next += later;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) { above[e] += c_next; above_m[e] += m_next; }
+      if (!heavy) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) above_m[e] = fmaf(bias, above_m[e], all_heavy);
+        m_next = fmaf(bias, m_next, all_heavy);
+      }
+    }
+    // the bin that reaches `goal` tokens with everything above it -> sh.bin[s], the tokens with or without it -> sh.upto[s]
+    auto locate = [&](int s, uint32_t goal, bool with) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const uint32_t more = e == 7 ? c_next : above[(e + 1) & 7];
+        if (above[e] >= goal && more < goal) {
+          sh.bin[s] = tid * 8 + e;
+          sh.upto[s] = with ? above[e] : more;
+        }
+      }
+    };
+    // The bins' answer to `goal`, 0: none.  `both`: the top-k threshold (goal tokens), then top-p's among its survivors.
+    auto bracket = [&](bool by_mass, u64 goal, bool both) -> u64 {
+      if (tokens == 0 || (!by_mass && goal > tokens)) return 0;
+      if (by_mass) {
+        if (tid == 0) sh.reach = (float)tokens;
+        __syncthreads();
+        const float g = (float)goal;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const uint32_t more = e == 7 ? c_next : above[(e + 1) & 7];
+          const float more_m = e == 7 ? m_next : above_m[(e + 1) & 7];
+          if (above_m[e] >= g && more_m < g) sh.reach = (float)more + (float)(above[e] - more) * ((g - more_m) / (above_m[e] - more_m));
+        }
+        __syncthreads();
+        const float at = sh.reach;
+        locate(0, min(tokens, (uint32_t)(at + kReach)), true);
+        locate(1, (uint32_t)fmaxf(1.f, at - kReach), false);
+      } else {
+        locate(0, (uint32_t)goal, true);
+        locate(1, both ? 1u : (uint32_t)goal, false);
+      }
+      __syncthreads();
+      const int b_lo = sh.bin[0], b_hi = sh.bin[1];
+      const uint32_t c_hi = sh.upto[1];
+      if (sh.upto[0] - c_hi > (uint32_t)kFin) return 0;
+      u64 m_hi = 0;
+      if (by_mass) {
+        scan([&](float x) {
+          const int at = bin_of(x);
+          if (at < b_lo) return;
+          if (at <= b_hi) list_token(fkey(x));
+          else m_hi += weight_at(x);
+        });
+        m_hi = cluster_add(m_hi);
+      } else {
+        scan([&](float x) {
+          const int at = bin_of(x);
+          if (at >= b_lo && at <= b_hi) list_token(fkey(x));
+        });
+        voc_sync<NC>();
+      }
+      return decide(by_mass, goal, c_hi, m_hi, both);
+    };
+    u64 lo = 0;
+    bool done = false;
+    if (use_k) {
+      if (binned) {
+        lo = bracket(false, (u64)k, use_p);
+        done = lo > 0;
+        if (lo == 0 && use_p) lo = bracket(false, (u64)k, false);
+      }
+      if (lo == 0) lo = search(false, (u64)k, 0, (u64)V);
+    }
+    if (use_p && !done) {
+      u64 count = V;
+      if (use_k || !binned) {
+        u64 v[5] = {0, 0, 0, 0, 0};  // tokens and mass of the top-k survivors (of the whole row without top-k)
+        scan([&](float x) {
+          if (x == x && fkey(x) >= lo) {
+            v[0] += 1;
+            v[2] += weight_at(x);
+          }
+        });
+        cluster_sum(v);
+        count = v[0];
+        total = v[2];
+      }
+      u64 target = (u64)((double)p * (double)total);
+      if (target < 1) target = 1;
+      const u64 found = binned ? bracket(true, target, false) : 0;
+      lo = found > 0 ? max(found, lo) : search(true, target, lo, count);
+    }
+    if (lo > 0) floor_logit = fkey_inv((uint32_t)lo);
+  }
+
+  if constexpr (SM) {
+    if (filters) {
+      // Few tokens of a filtered row are drawn for: every warp collects its survivors and draws for 32 at a time
+      uint32_t* queue = sh.hist + warp * kQueue;
+      int held = 0;
+      __syncthreads();  // (the counts are read by every warp)
+      for (int i0 = warp * 128; i0 < n; i0 += kVocThreads * 4) {
+        const int i = i0 + lane * 4;
+        const float none = __int_as_float(0x7fffffff);
+        const float4 q4 = i < n ? *reinterpret_cast<const float4*>(slice + i) : make_float4(none, none, none, none);
+        const float q[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t who = __ballot_sync(0xffffffffu, q[e] >= floor_logit);
+          if (q[e] >= floor_logit) queue[held + __popc(who & ((1u << lane) - 1))] = i + e;
+          held += __popc(who);
+        }
+        __syncwarp();
+        while (held >= 32) {
+          held -= 32;
+          const int at = queue[held + lane];
+          draw(slice[at], at);
+        }
+        __syncwarp();
+      }
+      if (lane < held) {
+        const int at = queue[lane];
+        draw(slice[at], at);
+      }
+      __syncwarp();
+    }
+  } else {
+    for (int i = tid; i < n; i += kVocThreads) {
+      const float x = __ldg(row + i);
+      if (x >= floor_logit) draw(x, i);
+    }
+    __syncwarp();
+  }
+  // lowest index wins ties, in whatever order the blocks' winners are merged
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    argmax_merge(best, bi, ov, oi);
+  }
+  __syncthreads();
+  if (lane == 0) { sh.val[warp] = best; sh.idx[warp] = bi; }
+  __syncthreads();
+  if (warp == 0) {
+    best = sh.val[lane & (kVocWarps - 1)];
+    bi = sh.idx[lane & (kVocWarps - 1)];
+#pragma unroll
+    for (int o = kVocWarps / 2; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      argmax_merge(best, bi, ov, oi);
+    }
+    if (lane == 0) {
+      cluster_ptr<NC>(sh.top, 0)[rank] = best;
+      cluster_ptr<NC>(sh.top_idx, 0)[rank] = bi;
+    }
+  }
+  voc_sync<NC>();
+  if (rank == 0 && tid == 0) {
+    for (int c = 1; c < NC; ++c) argmax_merge(best, bi, sh.top[c], sh.top_idx[c]);
+    out[b] = bi < 0x7fffffff ? bi : 0;  // all-NaN row: emit a valid id, never an out-of-range one
+  }
+}
+
+// The same for short rows, a block each, whose search by masses and counts of the keys ends within a few passes that cost next to nothing
+// (us there | with clusters' bins, 128 rows of 8192: top_k 40 15 | 17, top_p 0.5 17 | 19): a pass compares the row with three keys inside the
+// interval that still holds the answer, or sorts it into 128 bins of masses; the last 256 tokens are ranked directly.
+constexpr int kRowFin = 256, kRowBins = 128;
+struct SampleRowShared {
+  uint32_t hist[2][3][kRowBins];  // tokens per value bin, the low 16 bits of their masses, the rest
+  unsigned long long tot_c[kRowBins], tot_m[kRowBins];
+  unsigned long long part[2][5];  // totals of a pass: counts (c1 | c2 << 32), c3, masses m1 .. m3
+  unsigned long long wred[kVocWarps][5];
+  uint32_t list[kRowFin];
+  unsigned long long mass[kRowFin];
+  float val[kVocWarps];
+  int idx[kVocWarps];
+  uint32_t n_list, result;
+};
+
+__global__ void __launch_bounds__(kVocThreads)
+sample_row_kernel(const float* __restrict__ logits, int ldl, const float* __restrict__ temperature, const uint64_t* __restrict__ seed,
+              const int32_t* __restrict__ top_k, const float* __restrict__ top_p, int32_t* __restrict__ out, int V) {
+  extern __shared__ __align__(16) uint32_t keys[];
+  __shared__ SampleRowShared sh;
+  pdl_launch_dependents();
+  pdl_wait();
+  typedef unsigned long long u64;
+  const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const float* row = logits + (size_t)b * ldl;
+  const float temp = temperature ? temperature[b] : 0.f;
+  const bool greedy = !(temp > 0.f);
+  const float inv_t = greedy ? 1.f : 1.f / temp;
+  const int k = top_k ? top_k[b] : 0;
+  const float p = top_p ? top_p[b] : 1.f;
+  const bool use_k = !greedy && k > 0 && k < V, use_p = !greedy && p > 0.f && p < 1.f;
+
+  if (tid == 0) sh.n_list = 0;
+  float mx = -INFINITY;
+  load_slice(row, V, tid, [&](int i, const float (&f)[4], int have) {  // (entries behind the row's end read as key 0, below every float's key)
+    uint32_t q[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      mx = fmaxf(mx, e < have ? f[e] : -INFINITY);
+      q[e] = e < have ? fkey(f[e]) : 0u;
+    }
+    *reinterpret_cast<uint4*>(keys + i) = make_uint4(q[0], q[1], q[2], q[3]);
+  });
+  __syncthreads();
+  auto scan = [&](auto&& f) {  // f(key, column)
+    for (int i = tid * 4; i < V; i += kVocThreads * 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(keys + i);
+      f(q.x, i);
+      f(q.y, i + 1);
+      f(q.z, i + 2);
+      f(q.w, i + 3);
+    }
+  };
+
+  float floor_logit = -INFINITY;
+  if (use_k || use_p) {
+    // row maximum (for the softmax weights)
+    const uint32_t wm = __reduce_max_sync(0xffffffffu, fkey(mx));
+    if (lane == 0) sh.val[warp] = fkey_inv(wm);
+    __syncthreads();
+    mx = sh.val[lane & (kVocWarps - 1)];
+    mx = fkey_inv(__reduce_max_sync(0xffffffffu, fkey(mx)));
+    auto weight = [&](uint32_t key) -> u64 {
+      const float e = __expf((fkey_inv(key) - mx) * inv_t) * 4294967296.0f;
+      return e >= 0.f ? (u64)e : 0;  // a NaN logit carries no mass
+    };
+    int turn = 0;
+    // sums of the block's threads, in every thread
+    auto warp_total = [](u64 v) -> u64 {  // (a thread's share is below 2^58: three limbs, one hardware reduction each)
+      const u64 a = __reduce_add_sync(0xffffffffu, (uint32_t)v & 0xffffu), c = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 16) & 0x1fffffu),
+                d = __reduce_add_sync(0xffffffffu, (uint32_t)(v >> 37));
+      return a + (c << 16) + (d << 37);
+    };
+    auto block_sum5 = [&](u64 (&v)[5]) {
+#pragma unroll
+      for (int j = 0; j < 5; ++j) {
+        const u64 t = j == 0 ? (u64)__reduce_add_sync(0xffffffffu, (uint32_t)v[0]) | (u64)__reduce_add_sync(0xffffffffu, (uint32_t)(v[0] >> 32)) << 32
+                      : j == 1 ? (u64)__reduce_add_sync(0xffffffffu, (uint32_t)v[1]) : warp_total(v[j]);
+        if (lane == 0) sh.wred[warp][j] = t;
+      }
+      __syncthreads();
+      if (warp == 0) {
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+          u64 t = lane < kVocWarps ? sh.wred[lane][j] : 0;
+#pragma unroll
+          for (int o = kVocWarps / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+          if (lane == 0) sh.part[turn][j] = t;
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 5; ++j) v[j] = sh.part[turn][j];
+      turn ^= 1;  // (a slot is written again two passes later, behind the barrier that follows every read of it)
+    };
+    // the largest key whose tokens (those with keys >= it) reach `goal`: in number, or in mass (by_mass).  Keeping [lo, ..) is
+    // enough (c_lo tokens), keeping [hi, ..) is not (c_hi tokens of mass m_hi).
+    auto search = [&](bool by_mass, u64 goal, u64 lo, u64 c_lo) -> u64 {
+      u64 hi = (u64)fkey(mx) + 1, c_hi = 0, m_hi = 0;  // (nothing is above the maximum)
+      for (int pass = 0; hi - lo > 1 && c_lo - c_hi > (u64)kRowFin; ++pass) {
+        // Logits are spread more evenly over values than over keys (where half of all keys are exponents nothing has): the first
+        // pass looks a few temperatures below the maximum, the next ones divide the values between the bounds; from the eighth
+        // on the keys are divided, so at most 8 + 16 passes are needed.
+        const u64 d = hi - lo;
+        // A mass between two finite values: the tokens go into kRowBins equal bins of values at once, and the bin that holds the answer is
         // the next interval (a threshold in the bulk of the vocabulary needs two such passes instead of five or six of three keys,
         // which weigh nearly as many tokens each: rows of top_p 0.95 85 -> 70 us; counting is cheap, so top-k stays with the keys).
-        // Slices beyond shared memory, whose sums could leave 32 bits, and intervals that no longer split take the keys below.
-        if constexpr (SM) {
-          const float b_lo = fkey_inv((uint32_t)lo), b_hi = fkey_inv((uint32_t)(hi - 1)), scale = (float)kBins / (b_hi - b_lo);
+        // Intervals that no longer split take the keys below.
+        {
+          const float b_lo = fkey_inv((uint32_t)lo), b_hi = fkey_inv((uint32_t)(hi - 1)), scale = (float)kRowBins / (b_hi - b_lo);
           if (by_mass && pass > 0 && pass < 8 && lo > 0 && scale > 0.f && scale < 1e30f && b_lo - b_lo == 0.f) {
-            auto bin_of = [&](uint32_t q) { return min(kBins - 1, (int)((fkey_inv(q) - b_lo) * scale)); };
-            uint32_t (&hist)[3][kBins] = sh.hist[turn];
-            for (int e = tid; e < 3 * kBins; e += kVocThreads) (&hist[0][0])[e] = 0;
+            auto bin_of = [&](uint32_t q) { return min(kRowBins - 1, (int)((fkey_inv(q) - b_lo) * scale)); };
+            uint32_t (&hist)[3][kRowBins] = sh.hist[turn];
+            for (int e = tid; e < 3 * kRowBins; e += kVocThreads) (&hist[0][0])[e] = 0;
             __syncthreads();
             scan([&](uint32_t q, int) {
               if (q < (uint32_t)lo || (u64)q >= hi) return;
@@ -594,17 +1154,10 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
               atomicAdd(&hist[1][at], (uint32_t)w & 0xffffu);
               atomicAdd(&hist[2][at], (uint32_t)(w >> 16));
             });
-            voc_sync<NC>();
-            for (int e = tid; e < kBins; e += kVocThreads) {
-              u64 c = 0, m = 0;
-#pragma unroll
-              for (int r = 0; r < NC; ++r) {
-                uint32_t (&o)[3][kBins] = *cluster_ptr<NC>(&hist, r);
-                c += o[0][e];
-                m += o[1][e] + ((u64)o[2][e] << 16);
-              }
-              sh.tot_c[e] = c;
-              sh.tot_m[e] = m;
+            __syncthreads();
+            for (int e = tid; e < kRowBins; e += kVocThreads) {
+              sh.tot_c[e] = hist[0][e];
+              sh.tot_m[e] = hist[1][e] + ((u64)hist[2][e] << 16);
             }
             __syncthreads();
             turn ^= 1;  // (zeroed again two passes later, behind the barrier that follows every read of it)
@@ -641,7 +1194,7 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
                 }
                 return a;
               };
-              const u64 n_lo = best == 0 ? lo : first_in(best), n_hi = best == kBins - 1 ? hi : first_in(best + 1);
+              const u64 n_lo = best == 0 ? lo : first_in(best), n_hi = best == kRowBins - 1 ? hi : first_in(best + 1);
               if (n_lo > lo || n_hi < hi) {
                 lo = n_lo;
                 c_lo = c_in;
@@ -684,7 +1237,7 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
           v[0] = c1 | (u64)c2 << 32;
           v[1] = c3;
         }
-        cluster_sum(v);
+        block_sum5(v);
         const u64 c[3] = {v[0] & 0xffffffffull, v[0] >> 32, v[1]}, m[3] = {v[2], v[3], v[4]};
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
@@ -700,37 +1253,37 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
         }
       }
       if (hi - lo <= 1) return lo;
-      // few tokens left: block 0 decides
+      // few tokens left
       scan([&](uint32_t q, int) {
         if (q < lo || (u64)q >= hi || q == 0) return;
-        cluster_ptr<NC>(sh.list, 0)[atomicAdd(cluster_ptr<NC>(&sh.n_list, 0), 1u)] = q;
+        sh.list[atomicAdd(&sh.n_list, 1u)] = q;
       });
-      voc_sync<NC>();
-      if (rank == 0) {
-        const int nl = (int)sh.n_list;
-        for (int i = tid; i < nl; i += kVocThreads) sh.mass[i] = weight(sh.list[i]);
-        __syncthreads();
-        const int cand = tid >> 1;
-        const uint32_t key = cand < nl ? sh.list[cand] : 0u;
-        u64 c = 0, m = 0;
-        for (int j = tid & 1; j < nl; j += 2)
-          if (sh.list[j] >= key) {
-            c += 1;
-            m += sh.mass[j];
-          }
-        c += __shfl_xor_sync(0xffffffffu, c, 1);
-        m += __shfl_xor_sync(0xffffffffu, m, 1);
-        const bool ok = cand < nl && (by_mass ? m_hi + m : c_hi + c) >= goal;
-        const uint32_t wk = __reduce_max_sync(0xffffffffu, ok ? key : 0u);
-        if (lane == 0) sh.idx[warp] = (int)wk;
-        __syncthreads();
-        if (warp == 0) {
-          const uint32_t r = __reduce_max_sync(0xffffffffu, (uint32_t)sh.idx[lane & (kVocWarps - 1)]);
-          if (lane < NC) *cluster_ptr<NC>(&sh.result, lane) = r;
-          if (lane == 0) sh.n_list = 0;
+      __syncthreads();
+      const int nl = (int)sh.n_list;
+      for (int i = tid; i < nl; i += kVocThreads) sh.mass[i] = weight(sh.list[i]);
+      __syncthreads();
+      const int cand = tid >> 1;
+      const uint32_t key = cand < nl ? sh.list[cand] : 0u;
+      u64 c = 0, m = 0;
+      for (int j = tid & 1; j < nl; j += 2)
+        if (sh.list[j] >= key) {
+          c += 1;
+          m += sh.mass[j];
+        }
+      c += __shfl_xor_sync(0xffffffffu, c, 1);
+      m += __shfl_xor_sync(0xffffffffu, m, 1);
+      const bool ok = cand < nl && (by_mass ? m_hi + m : c_hi + c) >= goal;
+      const uint32_t wk = __reduce_max_sync(0xffffffffu, ok ? key : 0u);
+      if (lane == 0) sh.idx[warp] = (int)wk;
+      __syncthreads();
+      if (warp == 0) {
+        const uint32_t r = __reduce_max_sync(0xffffffffu, (uint32_t)sh.idx[lane & (kVocWarps - 1)]);
+        if (lane == 0) {
+          sh.result = r;
+          sh.n_list = 0;
         }
       }
-      voc_sync<NC>();
+      __syncthreads();
       return sh.result > lo ? sh.result : lo;
     };
     u64 lo = 0;
@@ -738,12 +1291,12 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
     if (use_p) {
       u64 v[5] = {0, 0, 0, 0, 0};  // tokens and mass of the top-k survivors (of the whole row without top-k)
       scan([&](uint32_t q, int i) {
-        if (i < n && q >= lo) {
+        if (i < V && q >= lo) {
           v[0] += 1;
           v[2] += weight(q);
         }
       });
-      cluster_sum(v);
+      block_sum5(v);
       u64 target = (u64)((double)p * (double)v[2]);
       if (target < 1) target = 1;
       lo = search(true, target, lo, v[0]);
@@ -755,14 +1308,13 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
   int bi = 0x7fffffff;
   const uint64_t sd = seed ? seed[b] : 0;
   scan([&](uint32_t q, int i) {
-    if (i >= n) return;
+    if (i >= V) return;
     if (q == 0) return;  // a NaN is never drawn
     const float raw = fkey_inv(q);
     if (raw < floor_logit) return;
-    const int v = start + i;
     float x = raw * inv_t;
-    if (!greedy) x += gumbel(sd, v);
-    argmax_merge(best, bi, x, v);
+    if (!greedy) x += gumbel(sd, i);
+    argmax_merge(best, bi, x, i);
   });
   // lowest index wins ties, in whatever order the blocks' winners are merged
 #pragma unroll
@@ -776,15 +1328,8 @@ sample_kernel(const float* __restrict__ logits, int ldl, const float* __restrict
   __syncthreads();
   if (tid == 0) {
     for (int w = 1; w < kVocWarps; ++w) argmax_merge(best, bi, sh.val[w], sh.idx[w]);
-    sh.best_val = best;
-    sh.best_idx = bi;
-  }
-  voc_sync<NC>();
-  if (rank == 0 && tid == 0) {
-    for (int c = 1; c < NC; ++c) argmax_merge(best, bi, *cluster_ptr<NC>(&sh.best_val, c), *cluster_ptr<NC>(&sh.best_idx, c));
     out[b] = bi < 0x7fffffff ? bi : 0;  // all-NaN row: emit a valid id, never an out-of-range one
   }
-  voc_sync<NC>();  // no block's shared memory goes away while block 0 reads it
 }
 
 // ---- OpenAI presence / frequency penalties: logits[b, tok] -= val for the (tok, val) entries of row b ----
@@ -1109,17 +1654,17 @@ cudaError_t launch_voc(K* kernel, int ctas, bool on_chip, cudaStream_t s, int B,
   return launch_k(kernel, dim3(B * ctas), dim3(kVocThreads), on_chip ? (size_t)voc_slice(V, ctas) * 4 : 0, s, true, args...);
 }
 // Blocks per row: one up to `whole` columns; else as many (at most `most`) as let the machine hold every row's blocks at once (33
-// clusters of eight), but enough that two blocks fit an SM (parts of 25000 columns).  Every shape gives the same tokens.  Us with 1 / 2 / 4 / 8 blocks per row:
-//   top_p 0.95   48 rows of 32768  57 / 49 / 42 / 65     128 of 16384  50 / 39 / 62 / 116    256 of 8192    34 / 57 / 97 / 200
+// clusters of eight), but enough that two blocks fit an SM (parts of `part` columns).  Every shape gives the same tokens.  Us with 1 / 2 / 4 / 8 blocks per row:
+//   top_p 0.95   48 rows of 32768  57 / 49 / 42 / 65     128 of 16384  50 / 39 / 62 / 116    256 of 8192    34 / 57 / 97 / 200   (before the bins)
 //   width 6      48 rows of 50000   - / 14 / 13 / 25     128 of 32768  12 / 13 / 24 / 47     256 of 8192   8.5 / 18 / 38 / 87
 //   top_p 0.95   32 rows of 128256  - /  - / 66 / 72      96 of 65536   - / 126 / 97 / 148   256 of 128256  - /  - / 510 / 512
 // (clusters of eight run 33 at a time whatever their size, which left 256 rows of 1000 to 8192 columns at 20 to 50 % of the speed
 // of the block per row that these kernels had replaced).
-int voc_ctas(int B, int V, int whole, int most) {
+int voc_ctas(int B, int V, int whole, int most, int part) {
   if (V <= whole) return 1;
   int ctas = most;
   while (ctas > 1 && (long)B * ctas > 264) ctas /= 2;
-  while (ctas < 8 && voc_slice(V, ctas) > 25000) ctas *= 2;
+  while (ctas < 8 && voc_slice(V, ctas) > part) ctas *= 2;
   return ctas;
 }
 #define HB_VOC(KERNEL, CTAS, ...)                                                             \
@@ -1152,7 +1697,9 @@ cudaError_t sample_tokens(cudaStream_t s, const float* logits, int ldl, const fl
     if (e != cudaSuccess) return e;
     return launch_k(sample_stage2_kernel, dim3(B), dim3(32), 0, s, true, (const float*)pv, (const int*)pi, out, chunks);
   }
-  HB_VOC(sample_kernel, filtered ? voc_ctas(B, V, 8192, 8) : 8, logits, ldl, temperature, seed, top_k, top_p, out, V);
+  if (filtered && V <= 8192)
+    return launch_k(sample_row_kernel, dim3(B), dim3(kVocThreads), (size_t)voc_slice(V, 1) * 4, s, true, logits, ldl, temperature, seed, top_k, top_p, out, V);
+  HB_VOC(sample_cluster_kernel, filtered ? voc_ctas(B, V, 0, 8, 22500) : 8, logits, ldl, temperature, seed, top_k, top_p, out, V);
 }
 cudaError_t apply_penalties(cudaStream_t s, float* logits, int ldl, const int32_t* pen_off, const void* pen, int B, int V) {
   if (B <= 0) return cudaSuccess;
@@ -1168,7 +1715,7 @@ cudaError_t logprob_topk(cudaStream_t s, const float* logits, int ldl, int V, co
   const bool few = part > kVocSmemFloats || B <= (part <= 25000 ? 33 : 16);
   if ((widest <= 2 && !(few && V > (widest <= 1 ? 32768 : 65536))) || (widest == 3 && B > 128))
     return launch_k(logprob_row_kernel, dim3(B), dim3(kLpThreads), 0, s, true, logits, ldl, V, sampled, width, out_ids, out_lp, max_width);
-  HB_VOC(logprob_topk_kernel, voc_ctas(B, V, 32768, V <= 65536 ? 4 : 8), logits, ldl, V, sampled, width, out_ids, out_lp, max_width);
+  HB_VOC(logprob_topk_kernel, voc_ctas(B, V, 32768, V <= 65536 ? 4 : 8, 25000), logits, ldl, V, sampled, width, out_ids, out_lp, max_width);
 }
 #undef HB_VOC
 cudaError_t cls_pool_l2(cudaStream_t s, const bf16* x, const int32_t* first_row, float* out, int B, int H) {
