@@ -29,29 +29,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// 2^x for two values on the FMA/ALU pipes only (no MUFU): round-to-nearest split x = n + f, f in [-0.5, 0.5], degree-3
-// minimax polynomial for 2^f (relative error 7.6e-5, far below the bf16 rounding P gets), n added into the exponent
-// field.  The SFU does 16 ex2/clk/SM: at 128x128 scores per kv tile that is exactly as long as the tile's two MMAs, so
-// part of every row's exponentials is computed here instead (the split FlashAttention-4 uses).
-__device__ __forceinline__ uint64_t exp2_poly2(uint64_t x2) {
-  float x0, x1;
-  f2_unpack(x2, x0, x1);
-  x2 = f2_pack(fmaxf(x0, -126.f), fmaxf(x1, -126.f));  // masked scores are -inf: clamp so the exponent add cannot wrap
-  const uint64_t magic = f2_pack(12582912.f, 12582912.f);  // 1.5 * 2^23: the sum's low mantissa bits hold round(x)
-  const uint64_t t2 = f2_add(x2, magic);
-  const uint64_t n2 = f2_add(t2, f2_pack(-12582912.f, -12582912.f));
-  const uint64_t f2 = f2_fma(n2, f2_pack(-1.f, -1.f), x2);
-  uint64_t p2 = f2_fma(f2_pack(0.05520550534f, 0.05520550534f), f2, f2_pack(0.24261397123f, 0.24261397123f));
-  p2 = f2_fma(p2, f2, f2_pack(0.69325476885f, 0.69325476885f));
-  p2 = f2_fma(p2, f2, f2_pack(0.99992769957f, 0.99992769957f));
-  float t0, t1, p0, p1;
-  f2_unpack(t2, t0, t1);
-  f2_unpack(p2, p0, p1);
-  const uint32_t r0 = __float_as_uint(p0) + (__float_as_uint(t0) << 23);
-  const uint32_t r1 = __float_as_uint(p1) + (__float_as_uint(t1) << 23);
-  return f2_pack(__uint_as_float(r0), __uint_as_float(r1));
-}
-
 // Optional event trace (tools/attn_test -DHB_ATTN_TRACE): CTA 0 stamps clock64() at the hand-off points of q tile 0.
 #ifdef HB_ATTN_TRACE
 __device__ unsigned long long g_attn_trace[8][4096];
@@ -114,7 +91,7 @@ struct ACfg {
 //                [row0, row0 + kv) of the expanded buffers).  A q / k row has DK / 64 sub-tiles: the head's unrotated part in
 //                all but the last, the rotated part (shared by all heads on the key side) in the last; parts that are no
 //                multiple of 64 wide are zero-filled by the tensor maps.
-template <int DK, int DV, int SRC, int POLY, bool SORTED>
+template <int DK, int DV, int SRC, bool SORTED>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
@@ -481,6 +458,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const int qt0 = it.q_off + it.q0 + t * BQ;  // absolute position of the tile's first q row
       const int qpos = qt0 + r;
       const int qrow = it.q0 + t * BQ + r;        // row within the sequence's q rows of this step
+      const int turns = min(it.n0, it.n1);  // tiles that both q tiles have
       float m_used = 0.f, l = 0.f;
       for (int j = 0; j < nt; ++j) {
         const int tile = jt + j;
@@ -553,9 +531,14 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
           }
         }
-        // ---- p = exp2(s*scale - m) (masked entries are -inf -> 0), row sum, P (bf16x2) written over the S buffer's head.
-        //      POLY of every 8 column pairs take the FMA-pipe exp2, the rest the SFU; scale/subtract and the sum are packed
+        // ---- p = exp2(s*scale - m) (masked entries are -inf -> 0), row sum, P (bf16x2) written over the S buffer's head;
+        //      scale/subtract and the sum are packed
         if (t == 0 && warp == 3 && lane == 0) HB_TRACE(4);  // loaded, max, rescale decision done
+        // The q tiles' warps of a quarter of the SM take turns with the exponentials (barriers 1 + qd: tile 0's turn, 5 + qd: tile 1's).  Left to
+        // themselves both worked on their exponentials at the same time and waited for scores, loads and barriers at the same time: a kv
+        // tile took 2000 cycles, 1620 now.  A turn is bound by the SFU (8 cycles per instruction of a warp, 504 of 680); some of the
+        // exponentials as polynomials on the FMA pipe (16 cycles per pair, as much as the SFU takes) paid before the turns, and not since.
+        if (j < turns && (t == 1 || j > 0)) bar_sync((t ? 5 : 1) + qd, 64);
         const uint64_t scale2 = f2_pack(sl2, sl2), negm2 = f2_pack(-m_used, -m_used);
         uint64_t sum2a = 0, sum2b = 0;
 #pragma unroll
@@ -565,17 +548,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           for (int i = 0; i < 8; ++i) {
             const uint64_t x2 = f2_fma(f2_pack(__uint_as_float(sv[c * 16 + 2 * i]), __uint_as_float(sv[c * 16 + 2 * i + 1])),
                                        scale2, negm2);
-            uint64_t p2;
-            if ((i * POLY) % 8 < POLY) {  // POLY of the 8 pairs, evenly interleaved with the SFU ones
-              p2 = exp2_poly2(x2);
-            } else {
-              float x0, x1;
-              f2_unpack(x2, x0, x1);
-              p2 = f2_pack(fast_exp2(x0), fast_exp2(x1));
-            }
+            float x0, x1;
+            f2_unpack(x2, x0, x1);
+            const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+            const uint64_t p2 = f2_pack(p0, p1);
             if (i & 1) sum2b = f2_add(sum2b, p2); else sum2a = f2_add(sum2a, p2);
-            float p0, p1;
-            f2_unpack(p2, p0, p1);
             pk[i] = pack_bf16x2(p0, p1);
           }
           tmem_st_32x32b_x8(tS + c * 8, pk);
@@ -590,6 +567,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_full[t * 2 + (tile & 1)]);
+        if (j + t < turns) bar_arrive((t ? 1 : 5) + qd, 64);  // the other tile's turn
         if (t == 0 && warp == 3 && lane == 0) HB_TRACE(6);  // P0(j) handed over
       }
       // ---- item epilogue: O / l -> global, then hand O_t back to the MMA issuer
@@ -704,8 +682,8 @@ bool sorts_items(const AttnPrefillArgs& a) {
   return (long long)max_q_pairs * a.B * a.Hq > (short_ones ? 2ll : 1ll) * effective_sms(device_sms()) &&
          a.T < (short_ones ? 0.8 : 0.9) * (double)a.B * a.max_seqlen;
 }
-template <int D, bool PAGED, int POLY, bool SORTED>
-cudaError_t launch_p(cudaStream_t stream, const AttnPrefillArgs& a) {
+template <int D, bool PAGED, bool SORTED>
+cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a) {
   constexpr int SRC = PAGED ? KV_PAGED : KV_PACKED;
   using C = ACfg<D, D, SRC>;
   CUtensorMap mq, mk, mv, mo;
@@ -720,7 +698,7 @@ cudaError_t launch_p(cudaStream_t stream, const AttnPrefillArgs& a) {
     if (!make_tmap_2d(&mk, a.k, TM_BF16, (uint64_t)a.Hkv * D, (uint64_t)a.T, (uint64_t)a.ldk * 2, 64, BKV)) return cudaErrorInvalidValue;
     if (!make_tmap_2d(&mv, a.v, TM_BF16, (uint64_t)a.Hkv * D, (uint64_t)a.T, (uint64_t)a.ldv * 2, 64, BKV)) return cudaErrorInvalidValue;
   }
-  auto kern = attn_prefill_kernel<D, D, SRC, POLY, SORTED>;
+  auto kern = attn_prefill_kernel<D, D, SRC, SORTED>;
   const int max_q_pairs = (a.max_seqlen + QPAIR - 1) / QPAIR;
   const long long items = (long long)max_q_pairs * a.B * a.Hq;
   const int grid = (int)std::min<long long>(items, effective_sms(device_sms()));  // hb_engine_cfg.sm_budget
@@ -744,7 +722,7 @@ cudaError_t launch_expanded(cudaStream_t stream, const AttnExpandedArgs& a) {
   if (!make_tmap_3d(&mk, a.k, TM_BF16, a.nope, H, rows, (uint64_t)a.nope * 2, (uint64_t)a.ldkv * 2, 64, 1, BKV)) return cudaErrorInvalidValue;
   if (!make_tmap_3d(&mv, a.v, TM_BF16, a.vdim, H, rows, (uint64_t)a.vdim * 2, (uint64_t)a.ldkv * 2, 64, 1, BKV)) return cudaErrorInvalidValue;
   if (!make_tmap_2d(&mkr, a.k_rot, TM_BF16, a.rot, rows, (uint64_t)a.ldkr * 2, 64, BKV)) return cudaErrorInvalidValue;
-  auto kern = attn_prefill_kernel<DK, DV, KV_EXPANDED, 2, false>;
+  auto kern = attn_prefill_kernel<DK, DV, KV_EXPANDED, false>;
   int longest = 0;
   for (int i = 0; i < a.runs.n; ++i) longest = std::max(longest, a.runs.len[i]);
   const int max_q_pairs = (longest + QPAIR - 1) / QPAIR;
@@ -789,39 +767,17 @@ __global__ void attn_naive_kernel(const bf16* q, int ldq, const bf16* k, int ldk
 
 }  // namespace
 
-// pairs (of every 8) whose exp2 runs on the FMA pipe; HB_ATTN_POLY overrides (tuning / A-B runs)
-int poly_pairs(int D) {
-  static int env = -2;
-  if (env == -2) {
-    const char* s = getenv("HB_ATTN_POLY");
-    env = s ? atoi(s) : -1;
-  }
-  if (env >= 0) return env;
-  (void)D;
-  return 2;  // measured on B200 (two issuers, 64-wide kv tiles), 0 / 2 / 4 of 8: D=128 1107 / 1171 / 1139, D=64 476 / 501 / 489 TFLOP/s
-}
-template <int D, bool PAGED, bool SORTED>
-cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a) {
-  switch (poly_pairs(D)) {
-    case 0: return launch_p<D, PAGED, 0, SORTED>(stream, a);
-    case 4: return launch_p<D, PAGED, 4, SORTED>(stream, a);
-    default: return launch_p<D, PAGED, 2, SORTED>(stream, a);
-  }
-}
-
 cudaError_t attn_prefill_init() {
   cudaError_t e;
-#define HB_ATTR1(D_, P_, Y_, S_)                                                                                     \
-  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<D_, D_, P_, Y_, S_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                S_ ? ACfg<D_, D_, P_>::SMEM_SORTED : ACfg<D_, D_, P_>::SMEM)) != cudaSuccess)         \
+#define HB_ATTR(D_, P_, S_)                                                                                      \
+  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<D_, D_, P_, S_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                S_ ? ACfg<D_, D_, P_>::SMEM_SORTED : ACfg<D_, D_, P_>::SMEM)) != cudaSuccess)     \
     return e;
-#define HB_ATTR(D_, P_, S_) HB_ATTR1(D_, P_, 0, S_) HB_ATTR1(D_, P_, 2, S_) HB_ATTR1(D_, P_, 4, S_)
   HB_ATTR(128, KV_PACKED, false) HB_ATTR(128, KV_PACKED, true) HB_ATTR(128, KV_PAGED, false)
   HB_ATTR(64, KV_PACKED, false) HB_ATTR(64, KV_PACKED, true) HB_ATTR(64, KV_PAGED, false)
 #undef HB_ATTR
-#undef HB_ATTR1
 #define HB_ATTRX(K_, V_)                                                                                                  \
-  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<K_, V_, KV_EXPANDED, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<K_, V_, KV_EXPANDED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                 ACfg<K_, V_, KV_EXPANDED>::SMEM)) != cudaSuccess)                                        \
     return e;
   HB_ATTRX(128, 64) HB_ATTRX(128, 128) HB_ATTRX(192, 64) HB_ATTRX(192, 128)
