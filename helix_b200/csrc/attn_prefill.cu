@@ -496,9 +496,15 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             sv[i + 1] = __float_as_uint(fmaf(rc, ea, cap_out));
           }
         }
-        if (need_mask) {  // diagonal / ragged tiles only: knock the invalid columns out once, the hot loops stay branch-free
+        if (need_mask) {  // diagonal / ragged tiles only: knock the invalid columns out once, the hot loops stay branch-free.  One comparison per
+          // column and, where a block or a window begins in the tile, another pass (both at once cost 700 cycles, half a tile)
+          const int upto = lim - kv0, from = lo - kv0;  // columns that the row sees
 #pragma unroll
-          for (int i = 0; i < BKV; ++i) sv[i] = (kv0 + i <= lim && kv0 + i >= lo) ? sv[i] : 0xff800000u;  // -inf
+          for (int i = 0; i < BKV; ++i) sv[i] = i <= upto ? sv[i] : 0xff800000u;  // -inf
+          if (from > 0) {
+#pragma unroll
+            for (int i = 0; i < BKV; ++i) sv[i] = i >= from ? sv[i] : 0xff800000u;
+          }
         }
         float mx8[8];  // eight independent chains instead of one long dependent max chain
 #pragma unroll
