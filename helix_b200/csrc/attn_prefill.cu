@@ -449,6 +449,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const uint32_t lane_sel = static_cast<uint32_t>(qd * 32) << 16;
     const uint32_t tO = tmem_base + lane_sel + 256 + t * 128;
     int jt = 0;  // kv tiles this warpgroup has processed so far (S buffer and barrier phases)
+    bool passed = false;  // this warp has passed on a turn (the very first one, of tile 0, is not waited for)
     for (int round = 0, idx = blockIdx.x; idx < num_items; idx = next_item(idx, ++round)) {
       const Item it = get_item(idx);
       if (!it.valid) continue;
@@ -544,7 +545,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // themselves both worked on their exponentials at the same time and waited for scores, loads and barriers at the same time: a kv
         // tile took 2000 cycles, 1620 now.  A turn is bound by the SFU (8 cycles per instruction of a warp, 504 of 680); some of the
         // exponentials as polynomials on the FMA pipe (16 cycles per pair, as much as the SFU takes) paid before the turns, and not since.
-        if (j < turns && (t == 1 || j > 0)) bar_sync((t ? 5 : 1) + qd, 64);
+        // Every turn is waited for, the first one of an item too: a warp that passed on its turn twice before the other had taken the first would
+        // complete the barrier by itself.
+        if (j < turns && (t == 1 || passed)) bar_sync((t ? 5 : 1) + qd, 64);
         const uint64_t scale2 = f2_pack(sl2, sl2), negm2 = f2_pack(-m_used, -m_used);
         uint64_t sum2a = 0, sum2b = 0;
 #pragma unroll
@@ -573,7 +576,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_full[t * 2 + (tile & 1)]);
-        if (j + t < turns) bar_arrive((t ? 1 : 5) + qd, 64);  // the other tile's turn
+        if (j < turns) {
+          bar_arrive((t ? 1 : 5) + qd, 64);  // the other tile's turn
+          passed = true;
+        }
         if (t == 0 && warp == 3 && lane == 0) HB_TRACE(6);  // P0(j) handed over
       }
       // ---- item epilogue: O / l -> global, then hand O_t back to the MMA issuer
