@@ -101,7 +101,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     int max_pages, int Hkv, int chunk, int sink, const float* __restrict__ head_gate, int ldg,
                     int window, float cap_in, float cap_out, const bf16* __restrict__ sink_w,
                     const __grid_constant__ CUtensorMap map_qr, const __grid_constant__ CUtensorMap map_kr,
-                    const __grid_constant__ AttnRuns runs, int vdim) {
+                    const __grid_constant__ AttnRuns runs, int vdim, int pack) {
   using C = ACfg<DK, DV, SRC>;
   constexpr bool PAGED = SRC == KV_PAGED, EXPANDED = SRC == KV_EXPANDED;
   constexpr int KST = C::STAGES;
@@ -133,6 +133,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     int j_lo;  // first kv tile of the item (block mask: the tile that holds the block start of the pair's first row)
     bool valid, act1;
   };
+  // A q row is a (token, head) pair: with pack > 0 the 1 << pack neighbouring query heads of an item, which share a kv head, sit side by side
+  // in the rows of a tile (row = token << pack | head), so a tile covers 128 >> pack tokens; `it.h` counts such groups of heads.
   // sequence b: its first row in the packed activation, its q rows in this step, its kv positions
   auto set_seq = [&](Item& it, int b) {
     it.b = b;
@@ -146,6 +148,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       it.kv_len = PAGED ? kv_lens[b] : it.len;
     }
     it.q_off = it.kv_len - it.len;  // position of the first q row (0 unless this is a later chunk of a long prompt)
+    if constexpr (!EXPANDED) it.len <<= pack;
   };
   auto set_pair = [&](Item& it, int qp) {
     it.q0 = qp * QPAIR;
@@ -157,10 +160,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // itself; tiles before the block of the pair's first row are skipped, n0 / n1 / n count tiles from j_lo
     // sliding window (window > 0, paged only): a row sees the `window` positions that end with itself; tiles before the
     // window of the pair's first row are skipped
-    it.j_lo = (PAGED && chunk > 0) ? ((it.q_off + it.q0) / chunk * chunk) / BKV
-              : (SRC != KV_PACKED && window > 0) ? max(0, it.q_off + it.q0 - window + 1) / BKV : 0;
-    it.n0 = (causal ? min(kv_tiles, (it.q_off + it.q0 + BQ - 1) / BKV + 1) : kv_tiles) - it.j_lo;
-    it.n1 = it.act1 ? (causal ? min(kv_tiles, (it.q_off + it.q0 + 2 * BQ - 1) / BKV + 1) : kv_tiles) - it.j_lo : 0;
+    it.j_lo = (PAGED && chunk > 0) ? ((it.q_off + (it.q0 >> pack)) / chunk * chunk) / BKV
+              : (SRC != KV_PACKED && window > 0) ? max(0, it.q_off + (it.q0 >> pack) - window + 1) / BKV : 0;
+    it.n0 = (causal ? min(kv_tiles, (it.q_off + ((it.q0 + BQ - 1) >> pack)) / BKV + 1) : kv_tiles) - it.j_lo;
+    it.n1 = it.act1 ? (causal ? min(kv_tiles, (it.q_off + ((it.q0 + 2 * BQ - 1) >> pack)) / BKV + 1) : kv_tiles) - it.j_lo : 0;
     it.n = max(it.n0, it.n1);
   };
   if (threadIdx.x == 0) {
@@ -246,7 +249,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);  // warp-uniform for the compiler too
   const int rows = SORTED ? s_rows[0] : -1;
-  const int num_items = (SORTED && rows >= 0 ? rows : max_q_pairs * B) * Hq;
+  const int groups = Hq >> pack;  // of heads that an item takes together
+  const int num_items = (SORTED && rows >= 0 ? rows : max_q_pairs * B) * groups;
   auto next_item = [&](int idx, int round) {
     if constexpr (SORTED) {
       if (rows >= 0) return round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
@@ -257,20 +261,20 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     Item it;
     if constexpr (SORTED) {
       if (rows >= 0) {
-        const int row = idx / Hq;
-        it.h = idx - row * Hq;
-        it.kvh = it.h / group;
+        const int row = idx / groups;
+        it.h = idx - row * groups;
+        it.kvh = (it.h << pack) / group;
         set_seq(it, s_order[row] & 255);
         set_pair(it, s_order[row] >> 8);
         return it;
       }
     }
-    const int per_qp = B * Hq;
+    const int per_qp = B * groups;
     const int qp = max_q_pairs - 1 - idx / per_qp;  // latest q rows first, one "round" per q pair index
     const int rem = idx % per_qp;
-    const int b = rem / Hq;
-    it.h = rem % Hq;
-    it.kvh = it.h / group;
+    const int b = rem / groups;
+    it.h = rem % groups;
+    it.kvh = (it.h << pack) / group;
     set_seq(it, b);
     set_pair(it, qp);
     return it;
@@ -293,11 +297,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
             for (int c = 0; c < C::SUBK; ++c) {
               uint8_t* dst = sQ + t * C::Q_BYTES + c * (BQ * 128);
-              const int row = it.seq0 + it.q0 + t * BQ;
+              const int row = it.seq0 + ((it.q0 + t * BQ) >> pack);
               if constexpr (EXPANDED)
                 tma_load_3d(dst, c < C::SUBK - 1 ? &map_q : &map_qr, q_full, c < C::SUBK - 1 ? c * 64 : 0, it.h, row, kEvictFirst);
               else
-                tma_load_2d(dst, &map_q, q_full, it.h * DK + c * 64, row, kEvictFirst);
+                tma_load_3d(dst, &map_q, q_full, c * 64, it.h << pack, row, kEvictFirst);
             }
         }
         ++qi;
@@ -456,9 +460,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const int nt = t == 0 ? it.n0 : it.n1;
       if (nt == 0) continue;
       const int len = it.kv_len;                  // kv positions of the sequence
-      const int qt0 = it.q_off + it.q0 + t * BQ;  // absolute position of the tile's first q row
-      const int qpos = qt0 + r;
-      const int qrow = it.q0 + t * BQ + r;        // row within the sequence's q rows of this step
+      const int qt0 = it.q_off + ((it.q0 + t * BQ) >> pack), qt1 = qt0 + ((BQ - 1) >> pack);  // absolute positions of the tile's first and last q row
+      const int qpos = qt0 + (r >> pack);
+      const bool live = it.q0 + t * BQ + r < it.len;  // the row exists
+      const int token = it.seq0 + ((it.q0 + t * BQ + r) >> pack), head = (it.h << pack) + (r & ((1 << pack) - 1));
       const int turns = min(it.n0, it.n1);  // tiles that both q tiles have
       float m_used = 0.f, l = 0.f;
       for (int j = 0; j < nt; ++j) {
@@ -471,7 +476,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const int kv0 = (it.j_lo + j) * BKV;
         const int lo = chunk > 0 ? qpos / chunk * chunk : (window > 0 ? qpos - window + 1 : 0);  // first kv position this row sees
         const bool need_mask = (kv0 + BKV > len) || (causal && (kv0 + BKV - 1 > qt0)) ||
-                               (chunk > 0 && kv0 < (qt0 + BQ - 1) / chunk * chunk) || (window > 0 && kv0 < qt0 + BQ - window);
+                               (chunk > 0 && kv0 < qt1 / chunk * chunk) || (window > 0 && kv0 <= qt1 - window);
         const int lim = causal ? min(len - 1, qpos) : len - 1;  // last valid kv position for this row
         // ---- the S row: back-to-back TMEM loads, ONE wait, then max / exp2 / pack entirely in registers
         uint32_t sv[BKV];
@@ -586,10 +591,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       mbar_wait(&pv_done[t * 2 + ((jt + nt - 1) & 1)], ((jt + nt - 1) >> 1) & 1);
       tc_fence_after();
       if (sink) l += fast_exp2(-m_used);  // one more unit in the denominator: a key of score 0 that carries no value
-      if (sink_w != nullptr) l += fast_exp2(__bfloat162float(sink_w[it.h]) * 1.4426950408889634f - m_used);  // a learned one per head
+      if (sink_w != nullptr) l += fast_exp2(__bfloat162float(sink_w[head]) * 1.4426950408889634f - m_used);  // a learned one per head
       float inv_l = l > 0.f ? 1.0f / l : 0.f;
       // optional output gate: the head's rows are scaled by sigmoid(head_gate[token][head]) on their way out
-      if (head_gate != nullptr && qrow < it.len) inv_l *= 1.f / (1.f + __expf(-head_gate[(size_t)(it.seq0 + qrow) * ldg + it.h]));
+      if (head_gate != nullptr && live) inv_l *= 1.f / (1.f + __expf(-head_gate[(size_t)token * ldg + head]));
       bool staged = false;
       if constexpr (C::STAGE_O) {
         // Every thread writing its own 128-byte row straight to global is 32 distinct lines per store instruction: ncu
@@ -623,7 +628,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           if (lane == 0) {
 #pragma unroll
             for (int c = 0; c < C::SUBV; ++c)
-              tma_store_2d(&map_o, stage + c * (32 * 128), it.h * DV + c * 64, it.seq0 + it.q0 + t * BQ + qd * 32);
+              tma_store_3d(&map_o, stage + c * (32 * 128), c * 64, it.h << pack, it.seq0 + ((it.q0 + t * BQ + qd * 32) >> pack));
             tma_store_commit();
             mbar_arrive(&o_free[t]);
           }
@@ -631,13 +636,13 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       }
       if (!staged) {
         const int dv = EXPANDED ? vdim : DV;
-        bf16* orow = out + (size_t)(it.seq0 + qrow) * ldo + it.h * dv;
+        bf16* orow = out + (size_t)token * ldo + head * dv;
 #pragma unroll
         for (int c = 0; c < DV / 32; ++c) {
           uint32_t o[32];
           tmem_ld_32x32b_x32(tO + c * 32, o);
           tmem_ld_wait();
-          if (qrow < it.len) {
+          if (live) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               if (EXPANDED && c * 32 + i * 8 >= dv) break;  // vdim is a multiple of 8
@@ -687,20 +692,22 @@ int device_sms() {
 //     62 / 66, of 1125 to 1500 129 / 122);
 //   - more items than SMs, twice as many there (3 sequences of 37 to 300 12.4 / 14.5, of 75 to 600 20.3 / 20.5, of 187 to 1500 53 / 31).
 // Gains are 20 % on average over such launches.  The indices have to fit the order's entries.
-bool sorts_items(const AttnPrefillArgs& a) {
-  const int max_q_pairs = (a.max_seqlen + QPAIR - 1) / QPAIR;
-  if (a.B <= 1 || a.B > 256 || max_q_pairs < 2 || max_q_pairs > 255 || a.T < (long long)BKV * a.B) return false;
+bool sorts_items(const AttnPrefillArgs& a, int pack) {
+  const int max_q_pairs = ((a.max_seqlen << pack) + QPAIR - 1) / QPAIR;
+  if (a.B <= 1 || a.B > 256 || max_q_pairs < 2 || max_q_pairs > 255 || ((long long)a.T << pack) < (long long)BKV * a.B) return false;
   const bool short_ones = max_q_pairs <= 3;
-  return (long long)max_q_pairs * a.B * a.Hq > (short_ones ? 2ll : 1ll) * effective_sms(device_sms()) &&
+  return (long long)max_q_pairs * a.B * (a.Hq >> pack) > (short_ones ? 2ll : 1ll) * effective_sms(device_sms()) &&
          a.T < (short_ones ? 0.8 : 0.9) * (double)a.B * a.max_seqlen;
 }
 template <int D, bool PAGED, bool SORTED>
-cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a) {
+cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a, int pack) {
   constexpr int SRC = PAGED ? KV_PAGED : KV_PACKED;
   using C = ACfg<D, D, SRC>;
   CUtensorMap mq, mk, mv, mo;
-  if (!make_tmap_2d(&mo, a.out, TM_BF16, (uint64_t)a.Hq * D, (uint64_t)a.T, (uint64_t)a.ldo * 2, 64, 32)) return cudaErrorInvalidValue;
-  if (!make_tmap_2d(&mq, a.q, TM_BF16, (uint64_t)a.Hq * D, (uint64_t)a.T, (uint64_t)a.ldq * 2, 64, BQ)) return cudaErrorInvalidValue;
+  const uint64_t hd = (uint64_t)D * 2;
+  const uint32_t heads = 1u << pack;
+  if (!make_tmap_3d(&mo, a.out, TM_BF16, D, a.Hq, a.T, hd, (uint64_t)a.ldo * 2, 64, heads, 32 >> pack)) return cudaErrorInvalidValue;
+  if (!make_tmap_3d(&mq, a.q, TM_BF16, D, a.Hq, a.T, hd, (uint64_t)a.ldq * 2, 64, heads, BQ >> pack)) return cudaErrorInvalidValue;
   if (PAGED) {
     // pool plane = [page][kv head][64 positions][D]: one 3-D block per (page, kv head), as in the decode kernel
     const uint64_t blocks = (uint64_t)a.num_pages * a.Hkv;
@@ -711,15 +718,15 @@ cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a) {
     if (!make_tmap_2d(&mv, a.v, TM_BF16, (uint64_t)a.Hkv * D, (uint64_t)a.T, (uint64_t)a.ldv * 2, 64, BKV)) return cudaErrorInvalidValue;
   }
   auto kern = attn_prefill_kernel<D, D, SRC, SORTED>;
-  const int max_q_pairs = (a.max_seqlen + QPAIR - 1) / QPAIR;
-  const long long items = (long long)max_q_pairs * a.B * a.Hq;
+  const int max_q_pairs = (int)((((long long)a.max_seqlen << pack) + QPAIR - 1) / QPAIR);
+  const long long items = (long long)max_q_pairs * a.B * (a.Hq >> pack);
   const int grid = (int)std::min<long long>(items, effective_sms(device_sms()));  // hb_engine_cfg.sm_budget
   const float scale_log2 = a.scale * 1.4426950408889634f;
   kern<<<grid, kThreads, SORTED ? C::SMEM_SORTED : C::SMEM, stream>>>(mq, mk, mv, mo, a.out, a.ldo, a.cu_seqlens, a.B, a.Hq, a.Hq / a.Hkv, a.causal,
                                             scale_log2, max_q_pairs, a.kv_lens, a.page_table, a.max_pages, a.Hkv,
                                             paged_only(a.block_mask, PAGED), a.unit_sink, a.head_gate, a.ldg,
                                             paged_only(a.window, PAGED), a.softcap > 0.f ? a.scale / a.softcap : 0.f,
-                                            a.softcap > 0.f ? a.softcap * 1.4426950408889634f : 0.f, a.sink, mq, mk, AttnRuns{}, D);
+                                            a.softcap > 0.f ? a.softcap * 1.4426950408889634f : 0.f, a.sink, mq, mk, AttnRuns{}, D, pack);
   return cudaGetLastError();
 }
 
@@ -745,7 +752,7 @@ cudaError_t launch_expanded(cudaStream_t stream, const AttnExpandedArgs& a) {
   const int grid = (int)std::min<long long>(items, effective_sms(num_sms));
   kern<<<grid, kThreads, C::SMEM, stream>>>(mq, mk, mv, mq, a.out, a.ldo, nullptr, a.runs.n, a.H, 1, 1, a.scale * 1.4426950408889634f,
                                             max_q_pairs, nullptr, nullptr, 0, a.H, 0, 0, a.head_gate, a.ldg, a.window, 0.f, 0.f, a.sink,
-                                            mqr, mkr, a.runs, a.vdim);
+                                            mqr, mkr, a.runs, a.vdim, 0);
   return cudaGetLastError();
 }
 
@@ -797,6 +804,25 @@ cudaError_t attn_prefill_init() {
   return cudaSuccess;
 }
 
+// Query heads (a power of two, given as its logarithm) that share a kv head and the rows of a tile.  Packed tiles span fewer tokens, so less
+// of their diagonal is masked and less of a last tile is empty: 6 prompts of 300 to 3000 tokens, 32 heads over 8: 173 kv tiles per SM -> 148, 223 ->
+// 193 us; 8 of about 1000 97 -> 87.  They are also fewer: the packing that leaves the SMs the least to do one after the other is taken (a lone q
+// tile takes about 4/5 of a pair's time; 100 rows over 4000 keys 53 us unpacked, 61 by four).
+int packed_heads(const AttnPrefillArgs& a) {
+  const int group = a.Hq / a.Hkv, sms = effective_sms(device_sms());
+  int best = 0;
+  long long least = 0;
+  for (int p = 0; p <= 5 && group % (1 << p) == 0; ++p) {
+    const long long rows = (long long)a.max_seqlen << p, items = (rows + QPAIR - 1) / QPAIR * a.B * (a.Hq >> p);
+    const long long cost = (items + sms - 1) / sms * (rows <= BQ ? 4 : 5);
+    if (p == 0 || cost <= least) {
+      best = p;
+      least = cost;
+    }
+  }
+  return best;
+}
+
 cudaError_t attn_prefill(cudaStream_t stream, const AttnPrefillArgs& a) {
   if (a.B <= 0 || a.T <= 0) return cudaSuccess;
   if (a.Hq % a.Hkv) return cudaErrorInvalidValue;
@@ -806,13 +832,15 @@ cudaError_t attn_prefill(cudaStream_t stream, const AttnPrefillArgs& a) {
   if (a.window < 0 || (a.window > 0 && (!paged || !a.causal || a.block_mask > 0))) return cudaErrorInvalidValue;
   if (paged) {
     if (!a.v_cache || !a.page_table || !a.kv_lens || a.max_pages <= 0 || a.num_pages <= 0 || a.page_size != 64) return cudaErrorInvalidValue;
-    if (a.D == 128) return launch<128, true, false>(stream, a);
-    if (a.D == 64) return launch<64, true, false>(stream, a);
+    const int pack = packed_heads(a);
+    if (a.D == 128) return launch<128, true, false>(stream, a, pack);
+    if (a.D == 64) return launch<64, true, false>(stream, a, pack);
     return cudaErrorInvalidValue;
   }
-  const bool sorted = sorts_items(a);
-  if (a.D == 128) return sorted ? launch<128, false, true>(stream, a) : launch<128, false, false>(stream, a);
-  if (a.D == 64) return sorted ? launch<64, false, true>(stream, a) : launch<64, false, false>(stream, a);
+  const int pack = packed_heads(a);
+  const bool sorted = sorts_items(a, pack);
+  if (a.D == 128) return sorted ? launch<128, false, true>(stream, a, pack) : launch<128, false, false>(stream, a, pack);
+  if (a.D == 64) return sorted ? launch<64, false, true>(stream, a, pack) : launch<64, false, false>(stream, a, pack);
   return cudaErrorInvalidValue;
 }
 

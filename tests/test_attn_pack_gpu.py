@@ -1,0 +1,70 @@
+"""Prefill attention with the query heads of a kv head packed into a tile's rows: groups of every size (powers of two, others, single heads),
+lengths around a tile's tokens for each packing, packed and paged keys, heads with gates and sinks of their own."""
+import math
+
+import pytest
+import torch
+
+import helix_b200 as hb
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+def want(q, k, v, first, scale):
+    """q [n, H, D], k / v [m, G, D] in fp32; query i sees the keys up to position first + i."""
+    g = q.shape[1] // k.shape[1]
+    s = torch.einsum("nhd,mhd->hnm", q, k.repeat_interleave(g, 1)) * scale
+    at = torch.arange(k.shape[0], device=q.device)[None] > first + torch.arange(q.shape[0], device=q.device)[:, None]
+    return torch.einsum("hnm,mhd->nhd", torch.softmax(s.masked_fill(at, -math.inf), -1), v.repeat_interleave(g, 1))
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(2, 2), (4, 2), (12, 2), (32, 8), (16, 2), (16, 1), (32, 1), (40, 1), (64, 1)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("lens", [[1], [31, 32, 33], [64, 63, 65, 5], [127, 129, 257], [300, 700, 1, 513], [1100] * 4])
+def test_packed_keys(Hq, Hkv, D, lens):
+    L = hb.lib()
+    assert L.hbk_init() == 0
+    T, ld = sum(lens), (Hq + 2 * Hkv) * D
+    g = torch.Generator(device="cuda").manual_seed(T + Hq)
+    qkv = torch.randn(T, ld, generator=g, device="cuda").to(BF)
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), device="cuda", dtype=torch.int32)
+    out = torch.full((T, Hq * D), float("nan"), device="cuda", dtype=BF)
+    q = qkv.data_ptr()
+    assert L.hbk_attn_prefill(q, ld, q + 2 * Hq * D, ld, q + 2 * (Hq + Hkv) * D, ld, out.data_ptr(), Hq * D, cu.data_ptr(), len(lens), T, max(lens),
+                              Hq, Hkv, D, 1, D ** -0.5) == 0
+    torch.cuda.synchronize()
+    at = 0
+    for n in lens:
+        x = qkv[at:at + n].float().view(n, Hq + 2 * Hkv, D)
+        w = want(x[:, :Hq], x[:, Hq:Hq + Hkv], x[:, Hq + Hkv:], 0, D ** -0.5).reshape(n, -1)
+        # averages of unit normals: bf16 probabilities (2^-9 of a value below 5) and one bf16 rounding of the result
+        assert (out[at:at + n].float() - w).abs().max() < 2 * 5 * 2.0 ** -9
+        at += n
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(4, 4), (12, 2), (32, 8), (16, 1)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("rows,ctx", [(1, [1, 64, 300]), (33, [33, 97, 1000]), (64, [64, 2100]), (200, [300, 200, 4000]), (777, [6000])])
+def test_pages(Hq, Hkv, D, rows, ctx):
+    L = hb.lib()
+    assert L.hbk_init() == 0
+    B, g = len(ctx), torch.Generator(device="cuda").manual_seed(rows + Hq + D)
+    pages = [(c + 63) // 64 for c in ctx]
+    table = torch.zeros((B, max(pages)), device="cuda", dtype=torch.int32)
+    perm, at = torch.randperm(sum(pages), generator=g, device="cuda").to(torch.int32), 0
+    for i, n in enumerate(pages):
+        table[i, :n] = perm[at:at + n]
+        at += n
+    k, v = (torch.randn((sum(pages), Hkv, 64, D), generator=g, device="cuda").to(BF) for _ in range(2))
+    q = torch.randn((B * rows, Hq * D), generator=g, device="cuda").to(BF)
+    out = torch.full((B * rows, Hq * D), float("nan"), device="cuda", dtype=BF)
+    lens, cu = torch.tensor(ctx, device="cuda", dtype=torch.int32), torch.arange(B + 1, device="cuda", dtype=torch.int32) * rows
+    assert L.hbk_attn_prefill_paged(q.data_ptr(), Hq * D, k.data_ptr(), v.data_ptr(), table.data_ptr(), table.shape[1], lens.data_ptr(), out.data_ptr(), Hq * D,
+                                    cu.data_ptr(), B, B * rows, rows, Hq, Hkv, D, 1, D ** -0.5, sum(pages)) == 0
+    torch.cuda.synchronize()
+    for b in range(B):
+        n = pages[b]
+        kk, vv = (t[table[b, :n].long()].permute(0, 2, 1, 3).reshape(-1, Hkv, D)[:ctx[b]].float() for t in (k, v))
+        w = want(q[b * rows:(b + 1) * rows].float().view(rows, Hq, D), kk, vv, ctx[b] - rows, D ** -0.5).reshape(rows, -1)
+        assert (out[b * rows:(b + 1) * rows].float() - w).abs().max() < 2 * 5 * 2.0 ** -9
