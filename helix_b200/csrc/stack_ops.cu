@@ -64,16 +64,17 @@ __global__ void __launch_bounds__(256) gemm_rt_kernel(const float* __restrict__ 
 }
 
 // The same product for fp32 operands whose rows along k are 16-byte pieces (every product of the exact mode at sizes that are multiples
-// of four and of more than 64 terms): for prompts bound by the FMA pipe and, at one block per SM, by the latency of its shared-memory reads
-// (30 of 72 TFLOP/s; which of the two is not settled), for single tokens by the weights' bytes, where the kernel
+// of four and of more than 64 terms): for prompts bound by the FMA pipe (a packed FMA with three different operands takes 2.3 cycles of a quarter of
+// an SM, 62 TFLOP/s) and by what else the warps issue: half of all instructions made addresses for the copies (30 TFLOP/s) until each
+// thread kept to one 16-byte column of the stage and walked the rows by a stride, 42 since; for single tokens by the weights' bytes, where the kernel
 // above was bound by scalar loads with no copies in flight and one thread per sum of K terms.
 // K is cut into kRtParts equal parts; a group of threads per part keeps its own stages of cp.async copies and the groups' sums
 // are added in order of k at the end; inside a part even and odd k have a sum each (packed FMAs on register pairs as they are
 // loaded).  The parts depend on K alone, so a row's bits do not depend on M or on the tile.
 // Thread (ty, tx) of a group holds rows ty + i TM / RM and columns tx + j TN / RN; operands lie k-contiguous with a pitch of BK + 4
 // floats, which spreads the 16-byte reads of neighbouring threads over all banks.
-// Measured against the kernel above: 600 x 4096 x 1024 340 -> 168 us (30 TFLOP/s), 600 x 1024 x 4096 436 -> 195, 2 x 4096 x 1024 64 -> 8;
-// relative error against 64 bits 5.7e-7 -> 2.9e-7 (1024 terms).
+// Measured (the kernel above, then 64 x 64 and 16 x 64 tiles, now): 600 x 4096 x 1024 340 -> 168 -> 129 us, 600 x 1024 x 4096 436 -> 195 -> 144,
+// 2000 x 1024 x 4096 531 -> 367, 40 x 1024 x 4096 53 -> 31, 2 x 4096 x 1024 64 -> 8; relative error against 64 bits 5.7e-7 -> 2.9e-7 (1024 terms).
 constexpr int kRtParts = 4;
 __device__ __forceinline__ void cp16_or_zero(float* dst, const float* src, bool live) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -87,7 +88,7 @@ struct RtTile {
   static constexpr int FLOATS = kRtParts * ST * STAGE > kRtParts * TM * TN ? kRtParts * ST * STAGE : kRtParts * TM * TN;
 };
 template <int TM, int TN, int RM, int RN, int BK, int ST>
-__global__ void __launch_bounds__(RtTile<TM, TN, RM, RN, BK, ST>::NT * kRtParts, TM == 16 ? 3 : 1)
+__global__ void __launch_bounds__(RtTile<TM, TN, RM, RN, BK, ST>::NT * kRtParts, TM == 16 ? 3 : TM == 32 ? 2 : 1)
 gemm_rt_tile_kernel(const float* __restrict__ A, long lda, long a_bs, const float* __restrict__ W, long w_sn, long w_bs,
                     float* __restrict__ C, long ldc, long c_bs, const float* __restrict__ bias, int M, int N, int K) {
   using T = RtTile<TM, TN, RM, RN, BK, ST>;
@@ -104,18 +105,35 @@ gemm_rt_tile_kernel(const float* __restrict__ A, long lda, long a_bs, const floa
   const int k_lo = grp * part, k_hi = min(K, k_lo + part);
   const int steps = k_hi > k_lo ? (k_hi - k_lo + BK - 1) / BK : 0;
   float* const mine = sm + grp * ST * T::STAGE;
-  auto load = [&](int step) {
-    if (step < steps) {
-      float* const d = mine + step % ST * T::STAGE;
-      const int k0 = k_lo + step * BK;
-      for (int e = t; e < (TM + TN) * (BK / 4); e += NT) {
-        const int r = e / (BK / 4), k = k0 + e % (BK / 4) * 4;
-        const bool is_a = r < TM;
-        const int row = is_a ? m0 + r : n0 + r - TM;
-        const bool live = k < k_hi && row < (is_a ? M : N);
-        const float* src = !live ? A : is_a ? A + (size_t)row * lda + k : W + (size_t)row * w_sn + k;
-        cp16_or_zero(d + r * P + e % (BK / 4) * 4, src, live);
+  // A thread copies the same 16 bytes of every row RPP apart (rows beyond M or N and terms beyond the part arrive as zeros)
+  constexpr int CPR = BK / 4, RPP = NT / CPR, AP = (TM + RPP - 1) / RPP, WP = TN / RPP;
+  static_assert(NT % CPR == 0 && TN % RPP == 0 && (TM % RPP == 0 || TM < RPP), "whole passes over a tile's rows");
+  const int r0 = t / CPR, ck = t % CPR * 4;
+  const float* pa = A + (size_t)(m0 + r0) * lda + k_lo + ck;
+  const float* pw = W + (size_t)(n0 + r0) * w_sn + k_lo + ck;
+  const long da = RPP * lda, dw = RPP * w_sn;
+  int put = 0, left = steps, k_left = k_hi - k_lo - ck;  // stage to fill, steps to load, terms from this thread's first on
+  auto load = [&] {
+    if (left > 0) {
+      float* const d = mine + put * T::STAGE + r0 * P + ck;
+      const bool in = k_left > 0;
+      const float* src = pa;
+#pragma unroll
+      for (int i = 0; i < AP; ++i, src += da) {
+        const bool live = in && m0 + r0 + i * RPP < M;
+        if (TM % RPP == 0 || r0 < TM) cp16_or_zero(d + i * RPP * P, live ? src : A, live);
       }
+      src = pw;
+#pragma unroll
+      for (int i = 0; i < WP; ++i, src += dw) {
+        const bool live = in && n0 + r0 + i * RPP < N;
+        cp16_or_zero(d + (TM + i * RPP) * P, live ? src : A, live);
+      }
+      pa += BK;
+      pw += BK;
+      k_left -= BK;
+      --left;
+      put = put + 1 == ST ? 0 : put + 1;
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -129,13 +147,15 @@ gemm_rt_tile_kernel(const float* __restrict__ A, long lda, long a_bs, const floa
 #pragma unroll
     for (int j = 0; j < RN; ++j) acc[i][j] = make_float2(0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < ST - 1; ++i) load(i);
+  for (int i = 0; i < ST - 1; ++i) load();
+  int get = 0;
   for (int step = 0; step < steps; ++step) {
     asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
     group_sync();
-    load(step + ST - 1);  // into the stage that every thread of the group left before this barrier
-    const float* as = mine + step % ST * T::STAGE + ty * P;
-    const float* ws = mine + step % ST * T::STAGE + (TM + tx) * P;
+    load();  // into the stage that every thread of the group left before this barrier
+    const float* as = mine + get * T::STAGE + ty * P;
+    const float* ws = mine + get * T::STAGE + (TM + tx) * P;
+    get = get + 1 == ST ? 0 : get + 1;
 #pragma unroll
     for (int k = 0; k < BK; k += 4) {
       float4 a[RM], w[RN];
@@ -1023,8 +1043,8 @@ cudaError_t stack_ops_init() {
   HB_SMEM((latent_attn_kernel<bf16, bf16>), big);
   HB_SMEM((gemm_rt_tile_kernel<2, 32, 2, 1, 32, 4>), (RtTile<2, 32, 2, 1, 32, 4>::FLOATS * 4));
   HB_SMEM((gemm_rt_tile_kernel<8, 32, 8, 1, 32, 4>), (RtTile<8, 32, 8, 1, 32, 4>::FLOATS * 4));
-  HB_SMEM((gemm_rt_tile_kernel<16, 64, 8, 4, 16, 3>), (RtTile<16, 64, 8, 4, 16, 3>::FLOATS * 4));
-  HB_SMEM((gemm_rt_tile_kernel<64, 64, 8, 4, 16, 3>), (RtTile<64, 64, 8, 4, 16, 3>::FLOATS * 4));
+  HB_SMEM((gemm_rt_tile_kernel<16, 32, 4, 4, 32, 2>), (RtTile<16, 32, 4, 4, 32, 2>::FLOATS * 4));
+  HB_SMEM((gemm_rt_tile_kernel<32, 64, 8, 8, 32, 2>), (RtTile<32, 64, 8, 8, 32, 2>::FLOATS * 4));
   HB_SMEM(gla_recurrence_kernel<16>, 80 * 1024);
   HB_SMEM(gla_recurrence_kernel<32>, 80 * 1024);
   HB_SMEM(gla_recurrence_kernel<64>, 80 * 1024);
@@ -1042,10 +1062,11 @@ cudaError_t gemm_rt(cudaStream_t s, const GemmRtArgs& a) {
   if (a.f32 && pieces && (a.M + 15) / 16 <= 65535) {
     if (a.M <= 2) return launch_rt_tile<2, 32, 2, 1, 32, 4>(s, a);
     if (a.M <= 8) return launch_rt_tile<8, 32, 8, 1, 32, 4>(s, a);
-    // 64-row tiles read operands less often, 16-row ones (three blocks per SM) fill the machine sooner: 2000 x 4096 x 1024 469 / 522 us,
-    // 600 x 4096 x 1024 (640 blocks of 64 rows) 168 / 166, 600 x 1024 x 4096 (160 blocks) 250 / 195, 100 x 1024 x 2048 68 / 29
-    const long blocks = (long)((a.N + 63) / 64) * ((a.M + 63) / 64) * a.batch;
-    return blocks >= 4 * effective_sms(148) ? launch_rt_tile<64, 64, 8, 4, 16, 3>(s, a) : launch_rt_tile<16, 64, 8, 4, 16, 3>(s, a);
+    // 32 x 64 tiles (8 x 8 sums a thread) read shared memory least, 16 x 32 ones (three blocks per SM) fill the machine sooner: from four wide
+    // tiles per SM on the wide ones (us wide / narrow: 600 x 6208 x 1024 182 / 209, 2000 x 1024 x 4096 367 / 418, 600 x 1024 x 4096, 304 tiles, 162 / 144,
+    // 100 x 6208 x 1024, 388 tiles, 51 / 49, 40 x 1024 x 4096 68 / 31)
+    const long blocks = (long)((a.N + 63) / 64) * ((a.M + 31) / 32) * a.batch;
+    return blocks >= 4 * effective_sms(148) ? launch_rt_tile<32, 64, 8, 8, 32, 2>(s, a) : launch_rt_tile<16, 32, 4, 4, 32, 2>(s, a);
   }
   dim3 grid((a.N + GT - 1) / GT, (a.M + GT - 1) / GT, a.batch);
   if (a.f32)
