@@ -465,7 +465,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const bool live = it.q0 + t * BQ + r < it.len;  // the row exists
       const int token = it.seq0 + ((it.q0 + t * BQ + r) >> pack), head = (it.h << pack) + (r & ((1 << pack) - 1));
       const int turns = min(it.n0, it.n1);  // tiles that both q tiles have
-      float m_used = 0.f, l = 0.f;
+      float m_used = -1e30f, l = 0.f;  // (rows that see nothing yet: far below every score, and finite)
       for (int j = 0; j < nt; ++j) {
         const int tile = jt + j;
         const uint32_t tS = tmem_base + lane_sel + t * 128 + (tile & 1) * BKV;
@@ -527,7 +527,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           if (__any_sync(0xffffffffu, need)) {
             mbar_wait(&pv_done[t * 2 + ((tile - 1) & 1)], ((tile - 1) >> 1) & 1);  // PV(j-1), hence every PV so far, is in O_t
             tc_fence_after();
-            m_new = fmaxf(m_new, m_used);
+            // (where heads can be packed, which depends on the whole launch, only the rows that need it: a row's bits do not depend on the
+            // rows beside it.  Expanded rows always stand beside the same ones, and follow them)
+            m_new = EXPANDED ? fmaxf(m_new, m_used) : need ? m_new : m_used;
             const float f = fast_exp2(m_used - m_new);
             m_used = m_new;
             l *= f;

@@ -71,19 +71,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {  // never waits
-  uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return;
   long long t0 = clock64();
@@ -94,22 +81,6 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
       __trap();
     }
   }
-}
-
-// Every lane of a converged warp waits for a barrier of its own (or a shared one).
-__device__ __forceinline__ void mbar_wait_all(uint64_t* bar, uint32_t parity) {
-  bool ok = mbar_try_wait(bar, parity);
-  if (!__all_sync(0xffffffffu, ok)) {
-    const long long t0 = clock64();
-    do {
-      if (!ok) ok = mbar_try_wait(bar, parity);
-      if (!ok && clock64() - t0 > HB_WAIT_TIMEOUT_CYCLES) {
-        printf("hb: mbarrier wait timeout block %d thread %d bar %u parity %u\n", blockIdx.x, threadIdx.x, smem_u32(bar), parity);
-        __trap();
-      }
-    } while (!__all_sync(0xffffffffu, ok));
-  }
-  __syncwarp();
 }
 
 // ---------------------------------------------------------------- cluster
@@ -244,16 +215,6 @@ __device__ __forceinline__ void tma_store_wait_all() {
 __device__ __forceinline__ void bar_sync(uint32_t id, uint32_t nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
-// ... and whether any of the threads brought `v`
-__device__ __forceinline__ bool bar_any(uint32_t id, uint32_t nthreads, bool v) {
-  uint32_t r;
-  asm volatile(
-      "{\n.reg .pred p, q;\nsetp.ne.u32 p, %3, 0;\nbarrier.cta.red.or.pred q, %1, %2, p;\nselp.u32 %0, 1, 0, q;\n}"
-      : "=r"(r)
-      : "r"(id), "r"(nthreads), "r"((uint32_t)v)
-      : "memory");
-  return r != 0;
-}
 __device__ __forceinline__ void bar_arrive(uint32_t id, uint32_t nthreads) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
@@ -353,15 +314,6 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
-}
-__device__ __forceinline__ float tmem_ld_32x32b_x1(uint32_t taddr) {
-  uint32_t r;
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-  return __uint_as_float(r);
-}
-__device__ __forceinline__ void tmem_st_32x32b_x1(uint32_t taddr, float v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(__float_as_uint(v)) : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // 32 lanes x 32b, 16 consecutive columns from registers into TMEM.

@@ -68,3 +68,23 @@ def test_pages(Hq, Hkv, D, rows, ctx):
         kk, vv = (t[table[b, :n].long()].permute(0, 2, 1, 3).reshape(-1, Hkv, D)[:ctx[b]].float() for t in (k, v))
         w = want(q[b * rows:(b + 1) * rows].float().view(rows, Hq, D), kk, vv, ctx[b] - rows, D ** -0.5).reshape(rows, -1)
         assert (out[b * rows:(b + 1) * rows].float() - w).abs().max() < 2 * 5 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(32, 8), (16, 1), (12, 2)])
+def test_a_prompt_does_not_depend_on_its_launch(Hq, Hkv):
+    """Alone (few items: heads apart) and among others (packed, sorted): the same bits, also where large scores rescale the sums."""
+    L, D = hb.lib(), 128
+    assert L.hbk_init() == 0
+    lens, ld = [90, 300, 1800, 700, 33], (Hq + 2 * Hkv) * D
+    g = torch.Generator(device="cuda").manual_seed(Hq)
+    qkv = (torch.randn(sum(lens), ld, generator=g, device="cuda") * 3).to(BF)
+    run = []
+    for at, ns in [(0, lens)] + [(sum(lens[:i]), [n]) for i, n in enumerate(lens)]:
+        cu = torch.tensor([0] + list(torch.tensor(ns).cumsum(0)), device="cuda", dtype=torch.int32)
+        out = torch.empty((sum(ns), Hq * D), device="cuda", dtype=BF)
+        q = qkv[at:].data_ptr()
+        assert L.hbk_attn_prefill(q, ld, q + 2 * Hq * D, ld, q + 2 * (Hq + Hkv) * D, ld, out.data_ptr(), Hq * D, cu.data_ptr(), len(ns), sum(ns), max(ns),
+                                  Hq, Hkv, D, 1, D ** -0.5) == 0
+        run.append(out)
+    torch.cuda.synchronize()
+    assert torch.equal(run[0], torch.cat(run[1:]))
