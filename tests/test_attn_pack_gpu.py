@@ -45,7 +45,10 @@ def test_packed_keys(Hq, Hkv, D, lens):
 
 @pytest.mark.parametrize("Hq,Hkv", [(4, 4), (12, 2), (32, 8), (16, 1)])
 @pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("rows,ctx", [(1, [1, 64, 300]), (33, [33, 97, 1000]), (64, [64, 2100]), (200, [300, 200, 4000]), (777, [6000])])
+@pytest.mark.parametrize("rows,ctx", [(1, [1, 64, 300]), (33, [33, 97, 1000]), (64, [64, 2100]), (200, [300, 200, 4000]), (777, [6000]),
+                                      # kv tiles shared out to a cluster: 2, 4 and 8 shares, lone q tiles, sequences too short for a share each, a last
+                                      # share (tile 16 of 17) that begins behind the keys of the lower q tile
+                                      (1, [4000]), (150, [1030]), (200, [1088, 2100]), (256, [8000]), (300, [600, 520, 5000])])
 def test_pages(Hq, Hkv, D, rows, ctx):
     L = hb.lib()
     assert L.hbk_init() == 0
