@@ -119,6 +119,7 @@ __device__ __noinline__ void exchange_split(const SplitRows x, float m_used, flo
   if (!some) return;
   float m = m_used;
   for (int q = 0; q < parts - 1; ++q) m = fmaxf(m, came[q * QPAIR].x);
+  const bool seen = l != 0.f;  // (a share in which the row sees nothing is left out: its products hold 0 x what later tokens may have made infinite)
   const float f_own = fast_exp2(m_used - m);
   l *= f_own;
   for (int q = 0; q < parts - 1; ++q) l = fmaf(came[q * QPAIR].y, fast_exp2(came[q * QPAIR].x - m), l);
@@ -133,8 +134,9 @@ __device__ __noinline__ void exchange_split(const SplitRows x, float m_used, flo
     if constexpr (G == 32) tmem_ld_32x32b_x32(x.tO + (rank * blocks + c) * G, o); else tmem_ld_32x32b_x16(x.tO + (rank * blocks + c) * G, o);
     tmem_ld_wait();
 #pragma unroll
-    for (int i = 0; i < G; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f_own);
+    for (int i = 0; i < G; ++i) o[i] = seen ? __float_as_uint(__uint_as_float(o[i]) * f_own) : 0u;
     for (int q = 0; q < parts - 1; ++q) {
+      if (came[q * QPAIR].y == 0.f) continue;
       const float f = fast_exp2(came[q * QPAIR].x - m);
       const uint8_t* src = x.smem + block_at(q, c) + lane * (G * 4);
 #pragma unroll
@@ -977,6 +979,7 @@ cudaError_t attn_prefill_init() {
 // Measured, whole / by 2 / by 4, 32 heads over 8: 100 rows over 4000 keys 53 / 37 / 25 us, 512 over 2500 43 / 33 / 45, 512 over 1000 22.6 / 22.6 / 35,
 // 2 x 777 over 6000 170 / 165 / 229 (D = 64 160 / 138 / 203), 3 x 400 over 2500 70 / 83 / 118; 12 heads of their own, 2 x 333 over 4500
 // 72 / 48 / 55.  Eighths never won (15 clusters of 8 run at a time, 120 SMs).
+// A split portion's sums are added in another order, so its last bits depend on the cut, as a decoded token's do on decode_splits; packing alone changes none.
 struct Cut {
   int pack, split;
 };
@@ -995,7 +998,7 @@ Cut cut_of(const AttnPrefillArgs& a, bool paged) {
     for (int s = 1; s <= (paged ? kMaxSplit : 1); s *= 2) {
       if (s > 1 && (tiles < s * kLeastShare || !whole)) break;
       const long long at_once = s == 1 ? sms : max_clusters[s];
-      if (at_once <= 0) break;
+      if (s > 1 && items > at_once) continue;  // (several rounds of clusters gain little, 2 x 777 over 6000 above, and change a portion's last bits)
       const double cost = (double)((items + at_once - 1) / at_once) * (each * (double)((tiles + s - 1) / s) + (s > 1 ? kSplitCost : 0));
       if ((p == 0 && s == 1) || (s == 1 ? cost <= least : cost < 0.95 * least)) {
         best = {p, s};
