@@ -21,6 +21,7 @@ constexpr int QPAIR = 256;  // q rows per CTA: two q tiles ping-pong on the tens
 constexpr int BKV = 64;     // kv positions per tile (= one KV page)
 constexpr int kThreads = 352;  // producer warp, one MMA issuer warp per q tile, two softmax warpgroups
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
+constexpr int kPolyPairs = 2;  // of eight pairs of exponentials, on the FMA pipe
 constexpr int kMaxSplit = 4;   // CTAs that share the kv tiles of an item
 constexpr int kLeastShare = 8;  // kv tiles of the smallest share
 constexpr int kMaxRows = 512;  // (q pair, sequence) rows of a launch whose order is sorted
@@ -29,6 +30,33 @@ __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// 2^x for two values on the FMA and ALU pipes only: x = n + f with n the nearest whole number, f in [-0.5, 0.5], a degree-3 minimax
+// polynomial for 2^f (relative error 7.6e-5, far below the bf16 rounding that P gets), n added into the exponent field: the share of the
+// exponentials that FlashAttention-4 takes off the SFU.  Masked scores are -inf: the clamp keeps the exponent from wrapping.  It lets a NaN through
+// (fmaxf would make it a weight of 2^-126), which leaves as the largest finite number and makes the row's result infinite or NaN.
+__device__ __forceinline__ float clamp_exponent(float x) {
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(-126.f));
+  return x;
+}
+__device__ __forceinline__ uint64_t exp2_poly2(uint64_t x2) {
+  float x0, x1;
+  f2_unpack(x2, x0, x1);
+  x2 = f2_pack(clamp_exponent(x0), clamp_exponent(x1));
+  const uint64_t magic = f2_pack(12582912.f, 12582912.f);  // 1.5 * 2^23: the sum's low mantissa bits hold round(x)
+  const uint64_t t2 = f2_add(x2, magic);
+  const uint64_t n2 = f2_add(t2, f2_pack(-12582912.f, -12582912.f));
+  const uint64_t f2 = f2_fma(n2, f2_pack(-1.f, -1.f), x2);
+  uint64_t p2 = f2_fma(f2_pack(0.05520550534f, 0.05520550534f), f2, f2_pack(0.24261397123f, 0.24261397123f));
+  p2 = f2_fma(p2, f2, f2_pack(0.69325476885f, 0.69325476885f));
+  p2 = f2_fma(p2, f2, f2_pack(0.99992769957f, 0.99992769957f));
+  float t0, t1, p0, p1;
+  f2_unpack(t2, t0, t1);
+  f2_unpack(p2, p0, p1);
+  const uint32_t r0 = __float_as_uint(p0) + (__float_as_uint(t0) << 23);
+  const uint32_t r1 = __float_as_uint(p1) + (__float_as_uint(t1) << 23);
+  return f2_pack(__uint_as_float(r0), __uint_as_float(r1));
 }
 
 // Optional event trace (tools/attn_test -DHB_ATTN_TRACE): CTA 0 stamps clock64() at the hand-off points of q tile 0.
@@ -677,8 +705,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (t == 0 && warp == 3 && lane == 0) HB_TRACE(4);  // loaded, max, rescale decision done
         // The q tiles' warps of a quarter of the SM take turns with the exponentials (barriers 1 + qd: tile 0's turn, 5 + qd: tile 1's).  Left to
         // themselves both worked on their exponentials at the same time and waited for scores, loads and barriers at the same time: a kv
-        // tile took 2000 cycles, 1620 now.  A turn is bound by the SFU (8 cycles per instruction of a warp, 504 of 680); some of the
-        // exponentials as polynomials on the FMA pipe (16 cycles per pair, as much as the SFU takes) paid before the turns, and not since.
+        // tile took 2000 cycles, 1620 with the SFU alone (8 cycles per instruction of a warp, 504 of a turn of 680).  Two of eight pairs as
+        // polynomials (kPolyPairs) cost a little more than they save now that there are turns: all on the SFU | so, 6 prompts of 300 to 3000 tokens with 32
+        // heads over 8 184 | 187 us (64 columns 154 | 162), 64 chunks of 64 to 512 tokens 62 | 64, 100 rows over 4000 keys, whose q tiles have no partner, 57 | 55.
+        // They stay for the results: the logits of a 16-layer decoder, 5 prompts x 32 steps, have the same rms error (0.02061 | 0.02057), but other single
+        // errors, and with the SFU alone the largest ones pass what the full-size tests allow.
         // Every turn is waited for, the first one of an item too: a warp that passed on its turn twice before the other had taken the first would
         // complete the barrier by itself.
         if (j < turns && (t == 1 || passed)) bar_sync((t ? 5 : 1) + qd, 64);
@@ -691,10 +722,16 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           for (int i = 0; i < 8; ++i) {
             const uint64_t x2 = f2_fma(f2_pack(__uint_as_float(sv[c * 16 + 2 * i]), __uint_as_float(sv[c * 16 + 2 * i + 1])),
                                        scale2, negm2);
-            float x0, x1;
-            f2_unpack(x2, x0, x1);
-            const float p0 = fast_exp2(x0), p1 = fast_exp2(x1);
-            const uint64_t p2 = f2_pack(p0, p1);
+            uint64_t p2;
+            if (i % (8 / kPolyPairs) == 0) {  // evenly between the SFU's
+              p2 = exp2_poly2(x2);
+            } else {
+              float x0, x1;
+              f2_unpack(x2, x0, x1);
+              p2 = f2_pack(fast_exp2(x0), fast_exp2(x1));
+            }
+            float p0, p1;
+            f2_unpack(p2, p0, p1);
             if (i & 1) sum2b = f2_add(sum2b, p2); else sum2a = f2_add(sum2a, p2);
             pk[i] = pack_bf16x2(p0, p1);
           }

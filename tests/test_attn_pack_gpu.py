@@ -91,3 +91,27 @@ def test_a_prompt_does_not_depend_on_its_launch(Hq, Hkv):
         run.append(out)
     torch.cuda.synchronize()
     assert torch.equal(run[0], torch.cat(run[1:]))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Hq,Hkv", [(4, 4), (8, 2)])
+def test_a_key_that_is_not_a_number_shows(Hq, Hkv, D):
+    """Prompts with one NaN key at every column of two 8-column groups (each exponential has its own way): rows that see it are not finite, the others are right."""
+    L, n = hb.lib(), 150
+    assert L.hbk_init() == 0
+    ld, at = (Hq + 2 * Hkv) * D, list(range(16)) + [63, 64, 72, 149]
+    g = torch.Generator(device="cuda").manual_seed(D)
+    qkv = torch.randn(len(at), n, ld, generator=g, device="cuda").to(BF)
+    clean = qkv.clone()
+    for b, c in enumerate(at):
+        qkv[b, c, Hq * D:(Hq + Hkv) * D] = float("nan")
+    cu, out = torch.arange(len(at) + 1, device="cuda", dtype=torch.int32) * n, torch.zeros((len(at), n, Hq * D), device="cuda", dtype=BF)
+    q = qkv.data_ptr()
+    assert L.hbk_attn_prefill(q, ld, q + 2 * Hq * D, ld, q + 2 * (Hq + Hkv) * D, ld, out.data_ptr(), Hq * D, cu.data_ptr(), len(at), len(at) * n, n, Hq, Hkv, D, 1,
+                              D ** -0.5) == 0
+    torch.cuda.synchronize()
+    for b, c in enumerate(at):
+        assert not torch.isfinite(out[b, c:].float()).any(), c
+        x = clean[b].float().view(n, Hq + 2 * Hkv, D)
+        w = want(x[:, :Hq], x[:, Hq:Hq + Hkv], x[:, Hq + Hkv:], 0, D ** -0.5).reshape(n, -1)
+        assert (out[b, :c].float() - w[:c]).abs().max() < 2 * 5 * 2.0 ** -9 if c else True
