@@ -34,10 +34,12 @@ __device__ __forceinline__ float fast_exp2(float x) {
 
 // 2^x for two values on the FMA and ALU pipes only: x = n + f with n the nearest whole number, f in [-0.5, 0.5], a degree-3 minimax
 // polynomial for 2^f (relative error 7.6e-5, far below the bf16 rounding that P gets), n added into the exponent field: the share of the
-// exponentials that FlashAttention-4 takes off the SFU.  Masked scores are -inf: the clamp keeps the exponent from wrapping.  It lets a NaN through
-// (fmaxf would make it a weight of 2^-126), which leaves as the largest finite number and makes the row's result infinite or NaN.
+// exponentials that FlashAttention-4 takes off the SFU.  Masked scores are -inf, and the clamp keeps the exponent from wrapping: at -127 + 2^-13 the
+// polynomial is just above one, so what is left is 0x67 * 2^-149, a bf16 zero (a weight of 2^-126 let large values behind the mask
+// through, and its products changed the last bits of sums in the tensor cores).  A NaN passes the clamp (fmaxf would make it a weight of zero); it leaves as
+// the largest finite number and makes the row's result infinite or NaN.
 __device__ __forceinline__ float clamp_exponent(float x) {
-  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(-126.f));
+  asm("max.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(-127.f + 1.f / 8192.f));
   return x;
 }
 __device__ __forceinline__ uint64_t exp2_poly2(uint64_t x2) {

@@ -115,3 +115,22 @@ def test_a_key_that_is_not_a_number_shows(Hq, Hkv, D):
         x = clean[b].float().view(n, Hq + 2 * Hkv, D)
         w = want(x[:, :Hq], x[:, Hq:Hq + Hkv], x[:, Hq + Hkv:], 0, D ** -0.5).reshape(n, -1)
         assert (out[b, :c].float() - w[:c]).abs().max() < 2 * 5 * 2.0 ** -9 if c else True
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Hq,Hkv", [(4, 4), (8, 2)])
+def test_values_behind_the_mask_have_no_weight(Hq, Hkv, D):
+    """Prompts whose value rows from one position on are the largest there are: the rows before it are what they are without them."""
+    L, n = hb.lib(), 150
+    assert L.hbk_init() == 0
+    ld, at = (Hq + 2 * Hkv) * D, list(range(1, 17)) + [63, 64, 72, 149]
+    g = torch.Generator(device="cuda").manual_seed(D)
+    qkv = torch.randn(n, ld, generator=g, device="cuda").to(BF).repeat(1 + len(at), 1, 1)
+    for b, c in enumerate(at):
+        qkv[1 + b, c:, (Hq + Hkv) * D:] = torch.finfo(BF).max
+    B, out = 1 + len(at), torch.zeros((1 + len(at), n, Hq * D), device="cuda", dtype=BF)
+    cu, q = torch.arange(B + 1, device="cuda", dtype=torch.int32) * n, qkv.data_ptr()
+    assert L.hbk_attn_prefill(q, ld, q + 2 * Hq * D, ld, q + 2 * (Hq + Hkv) * D, ld, out.data_ptr(), Hq * D, cu.data_ptr(), B, B * n, n, Hq, Hkv, D, 1, D ** -0.5) == 0
+    torch.cuda.synchronize()
+    for b, c in enumerate(at):
+        assert torch.equal(out[1 + b, :c], out[0, :c]), c
