@@ -22,8 +22,6 @@ constexpr int BKV = 64;     // kv positions per tile (= one KV page)
 constexpr int kThreads = 352;  // producer warp, one MMA issuer warp per q tile, two softmax warpgroups
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 constexpr int kPolyPairs = 2;  // of eight pairs of exponentials, on the FMA pipe
-constexpr int kMaxSplit = 4;   // CTAs that share the kv tiles of an item
-constexpr int kLeastShare = 8;  // kv tiles of the smallest share
 constexpr int kMaxRows = 512;  // (q pair, sequence) rows of a launch whose order is sorted
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -96,111 +94,7 @@ struct ACfg {
   static_assert(SRC != KV_PACKED || SMEM_SORTED <= 227 * 1024, "shared memory");
   static constexpr int SUBK = DK / 64, SUBV = DV / 64;  // 64-column swizzle sub-tiles per row
   static_assert(SMEM <= 227 * 1024, "shared memory");
-  // (what a split item's other shares send stands where Q, K and V were)
-  static_assert(SRC != KV_PAGED || kMaxSplit * QPAIR * 8 + (kMaxSplit - 1) * QPAIR * DV * 4 / kMaxSplit <= 2 * Q_BYTES + STAGES * (K_BYTES + V_BYTES), "shared memory");
 };
-
-// The end of a split item, for a softmax warp: every CTA of the cluster ends up with some of the columns.  The warp sends the others' columns of
-// its 32 rows there, relative to the rows' own maxima, with m and l, and adds what comes to its own columns, in the order of the shares.
-// (A function of its own, not inlined: the kv loop's registers are at their limit, and inlined, or with the CTA's rank kept over it, it cost 12 % of the
-// whole at D = 64.)  2.3 + 1.4 us per item with 2 x 256 rows of 128 columns: 1.2 the two barriers, the rest copies of 64 KB each way; pulled a row at a
-// time by plain reads it took 6, sent 16 bytes of each row at a time 8.
-struct SplitRows {
-  uint8_t *smem, *stage;
-  uint32_t tO;
-  int chunk, rank, parts, q0, len, seq0, head0, pack, sink, ldg, ldo;
-  const float* head_gate;
-  const bf16* sink_w;
-  bf16* out;
-};
-template <int DV>
-__device__ __noinline__ void exchange_split(const SplitRows x, float m_used, float l) {
-  constexpr int G = DV / 4, PIECES = G / 4;  // columns of a block, 16-byte pieces of its rows: block = [32 rows][G fp32], pieces swizzled
-  const int lane = threadIdx.x & 31, parts = x.parts, rank = x.rank;
-  const int blocks = 4 / parts;  // of a CTA's columns
-  const auto block_at = [&](int q, int c) { return kMaxSplit * QPAIR * 8 + ((q * 8 + x.chunk) * blocks + c) * (32 * G * 4); };  // that comes from share q
-  const auto swizzled = [&](int k) { return (k ^ (PIECES == 8 ? lane & 7 : (lane >> 1) & 3)) << 4; };
-  float2* came = reinterpret_cast<float2*>(x.smem) + x.chunk * 32 + lane;  // m and l, [share][row]
-  cluster_sync_all();  // every product of every share is done: nothing reads the Q, K and V slots any more
-  const bool some = x.q0 + x.chunk * 32 < x.len;
-  if (some) {
-    for (int i = 1; i < parts; ++i) {
-      const int to = (rank + i) & (parts - 1), q = rank - (rank > to);
-      st_cluster_f32x2(cluster_addr(smem_u32(came + q * QPAIR), to), m_used, l);
-      for (int c = 0; c < blocks; ++c) {
-        uint32_t o[G];
-        if constexpr (G == 32) tmem_ld_32x32b_x32(x.tO + (to * blocks + c) * G, o); else tmem_ld_32x32b_x16(x.tO + (to * blocks + c) * G, o);
-        tmem_ld_wait();
-        uint8_t* st = x.stage + (c & 1) * (32 * G * 4);
-        __syncwarp();  // (the stage has been read)
-#pragma unroll
-        for (int k = 0; k < PIECES; ++k) *reinterpret_cast<uint4*>(st + lane * (G * 4) + swizzled(k)) = make_uint4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
-        __syncwarp();
-        const uint32_t dst = cluster_addr(smem_u32(x.smem) + block_at(q, c) + lane * 16, to);
-#pragma unroll
-        for (int k = 0; k < PIECES; ++k) {  // (512 bytes in a row; 16 from each thread's own row took longer)
-          const uint4 v = *reinterpret_cast<const uint4*>(st + k * 512 + lane * 16);
-          st_cluster_b32x4(dst + k * 512, v.x, v.y, v.z, v.w);
-        }
-      }
-    }
-  }
-  cluster_sync_all();  // all has come
-  if (!some) return;
-  float m = m_used;
-  for (int q = 0; q < parts - 1; ++q) m = fmaxf(m, came[q * QPAIR].x);
-  const bool seen = l != 0.f;  // (a share in which the row sees nothing is left out: its products hold 0 x what later tokens may have made infinite)
-  const float f_own = fast_exp2(m_used - m);
-  l *= f_own;
-  for (int q = 0; q < parts - 1; ++q) l = fmaf(came[q * QPAIR].y, fast_exp2(came[q * QPAIR].x - m), l);
-  const int mine = x.q0 + x.chunk * 32 + lane, heads = (1 << x.pack) - 1;
-  const int token = x.seq0 + (mine >> x.pack), head = x.head0 + (mine & heads);
-  if (x.sink) l += fast_exp2(-m);
-  if (x.sink_w != nullptr) l += fast_exp2(__bfloat162float(x.sink_w[head]) * 1.4426950408889634f - m);
-  float inv_l = l > 0.f ? 1.0f / l : 0.f;
-  if (x.head_gate != nullptr && mine < x.len) inv_l *= 1.f / (1.f + __expf(-x.head_gate[(size_t)token * x.ldg + head]));
-  for (int c = 0; c < blocks; ++c) {
-    uint32_t o[G];
-    if constexpr (G == 32) tmem_ld_32x32b_x32(x.tO + (rank * blocks + c) * G, o); else tmem_ld_32x32b_x16(x.tO + (rank * blocks + c) * G, o);
-    tmem_ld_wait();
-#pragma unroll
-    for (int i = 0; i < G; ++i) o[i] = seen ? __float_as_uint(__uint_as_float(o[i]) * f_own) : 0u;
-    for (int q = 0; q < parts - 1; ++q) {
-      if (came[q * QPAIR].y == 0.f) continue;
-      const float f = fast_exp2(came[q * QPAIR].x - m);
-      const uint8_t* src = x.smem + block_at(q, c) + lane * (G * 4);
-#pragma unroll
-      for (int k = 0; k < PIECES; ++k) {
-        const float4 v = *reinterpret_cast<const float4*>(src + swizzled(k));
-        o[4 * k] = __float_as_uint(fmaf(v.x, f, __uint_as_float(o[4 * k])));
-        o[4 * k + 1] = __float_as_uint(fmaf(v.y, f, __uint_as_float(o[4 * k + 1])));
-        o[4 * k + 2] = __float_as_uint(fmaf(v.z, f, __uint_as_float(o[4 * k + 2])));
-        o[4 * k + 3] = __float_as_uint(fmaf(v.w, f, __uint_as_float(o[4 * k + 3])));
-      }
-    }
-    // G bf16 of each row through the stage, so that a store takes whole segments of 8 or 16 rows
-    constexpr int OUT = G / 8;  // 16-byte pieces
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < OUT; ++k) {
-      uint4 w;
-      w.x = pack_bf16x2(__uint_as_float(o[8 * k + 0]) * inv_l, __uint_as_float(o[8 * k + 1]) * inv_l);
-      w.y = pack_bf16x2(__uint_as_float(o[8 * k + 2]) * inv_l, __uint_as_float(o[8 * k + 3]) * inv_l);
-      w.z = pack_bf16x2(__uint_as_float(o[8 * k + 4]) * inv_l, __uint_as_float(o[8 * k + 5]) * inv_l);
-      w.w = pack_bf16x2(__uint_as_float(o[8 * k + 6]) * inv_l, __uint_as_float(o[8 * k + 7]) * inv_l);
-      *reinterpret_cast<uint4*>(x.stage + lane * (G * 2) + ((k ^ (OUT == 4 ? (lane >> 1) & 3 : (lane >> 2) & 1)) << 4)) = w;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < OUT; ++k) {
-      const int row = (k * 32 + lane) / OUT, piece = lane % OUT, at = x.q0 + x.chunk * 32 + row;
-      if (at < x.len)
-        *reinterpret_cast<uint4*>(x.out + (size_t)(x.seq0 + (at >> x.pack)) * x.ldo + (x.head0 + (at & heads)) * DV +
-                                  (rank * blocks + c) * G + piece * 8) =
-            *reinterpret_cast<const uint4*>(x.stage + row * (G * 2) + ((piece ^ (OUT == 4 ? (row >> 1) & 3 : (row >> 2) & 1)) << 4));
-    }
-  }
-}
 
 // PERSISTENT kernel: one CTA per SM walks a static list of (256-row q pair, sequence, q-head) items, heaviest
 // (most kv tiles) first and dealt forth and back, so the TMEM allocation, barrier setup and the latency of an
@@ -223,13 +117,11 @@ __device__ __noinline__ void exchange_split(const SplitRows x, float m_used, flo
 // KV_PAGED: the q rows are the LAST q_len positions of a kv_len-long sequence whose K/V (including the chunk's own,
 //                written by the RoPE/KV-write kernel just before) live in the paged pool (chunked prefill, prefix-cache
 //                hits): tile j is page_table[b][j].
-//                SPLIT: not persistent: a cluster of 2 or 4 CTAs takes one item, each CTA a share of its kv tiles (cut_of), and their rows are
-//                put together at the end (exchange_split).
 // KV_EXPANDED: batch entry b is run b of `runs` (q rows [t0, t0 + len) of the packed activation, the last rows of the kv rows
 //                [row0, row0 + kv) of the expanded buffers).  A q / k row has DK / 64 sub-tiles: the head's unrotated part in
 //                all but the last, the rotated part (shared by all heads on the key side) in the last; parts that are no
 //                multiple of 64 wide are zero-filled by the tensor maps.
-template <int DK, int DV, int SRC, bool SORTED, bool SPLIT>
+template <int DK, int DV, int SRC, bool SORTED>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
@@ -270,7 +162,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     int b, h, kvh, q0, seq0, len, kv_len, q_off, n0, n1, n;
     int j_lo;  // first kv tile of the item (block mask: the tile that holds the block start of the pair's first row)
     bool valid, act1;
-    int parts;  // SPLIT: CTAs of the cluster that have a share of the kv tiles
   };
   // A q row is a (token, head) pair: with pack > 0 the 1 << pack neighbouring query heads of an item, which share a kv head, sit side by side
   // in the rows of a tile (row = token << pack | head), so a tile covers 128 >> pack tokens; `it.h` counts such groups of heads.
@@ -303,21 +194,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
               : (SRC != KV_PACKED && window > 0) ? max(0, it.q_off + (it.q0 >> pack) - window + 1) / BKV : 0;
     it.n0 = (causal ? min(kv_tiles, (it.q_off + ((it.q0 + BQ - 1) >> pack)) / BKV + 1) : kv_tiles) - it.j_lo;
     it.n1 = it.act1 ? (causal ? min(kv_tiles, (it.q_off + ((it.q0 + 2 * BQ - 1) >> pack)) / BKV + 1) : kv_tiles) - it.j_lo : 0;
-    it.n = max(it.n0, it.n1);
-  };
-  // SPLIT: this CTA's share of the item's kv tiles: a half or a quarter, none below kLeastShare tiles (as many, and no fewer than the
-  // number of shares, leave none of them empty).  A lower q tile whose keys end before the share begins takes one tile of it, which its mask empties.
-  auto take_share = [&](Item& it) {
-    const int rank = (int)cluster_ctarank(), ranks = (int)cluster_nctarank();
-    it.parts = 1;
-    if (!it.valid) return;
-    it.parts = ranks;
-    while (it.parts > 1 && it.n < it.parts * kLeastShare) it.parts >>= 1;
-    const int per = (it.n + it.parts - 1) / it.parts, lo = rank * per;
-    it.valid = rank < it.parts;
-    it.j_lo += lo;
-    it.n0 = max(1, min(it.n0 - lo, per));
-    it.n1 = it.act1 ? min(it.n1 - lo, per) : 0;
     it.n = max(it.n0, it.n1);
   };
   if (threadIdx.x == 0) {
@@ -405,9 +281,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const int rows = SORTED ? s_rows[0] : -1;
   const int groups = Hq >> pack;  // of heads that an item takes together
   const int num_items = (SORTED && rows >= 0 ? rows : max_q_pairs * B) * groups;
-  const int first_item = SPLIT ? (int)(blockIdx.x / cluster_nctarank()) : (int)blockIdx.x;
   auto next_item = [&](int idx, int round) {
-    if constexpr (SPLIT) return num_items;  // one item per cluster
     if constexpr (SORTED) {
       if (rows >= 0) return round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
     }
@@ -433,7 +307,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     it.kvh = (it.h << pack) / group;
     set_seq(it, b);
     set_pair(it, qp);
-    if constexpr (SPLIT) take_share(it);
     return it;
   };
 
@@ -444,7 +317,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const bool leader = elect_one_sync();
     {
       int kt = 0, qi = 0;  // running kv-tile / item counters: barrier phases continue across items
-      for (int round = 0, idx = first_item; idx < num_items; idx = next_item(idx, ++round)) {
+      for (int round = 0, idx = blockIdx.x; idx < num_items; idx = next_item(idx, ++round)) {
         const Item it = get_item(idx);
         if (!it.valid) continue;
         mbar_wait(q_empty, (qi & 1) ^ 1);  // every S MMA of the previous item has retired: the Q pair buffer is free
@@ -576,7 +449,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       v_advance();
       if (FAST || has_k) k_advance();
     };
-    for (int round = 0, idx = first_item; idx < num_items; idx = next_item(idx, ++round)) {
+    for (int round = 0, idx = blockIdx.x; idx < num_items; idx = next_item(idx, ++round)) {
       const Item it = get_item(idx);
       if (!it.valid) continue;
       const int nt = t == 0 ? it.n0 : it.n1, n = it.n;
@@ -611,7 +484,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const uint32_t tO = tmem_base + lane_sel + 256 + t * 128;
     int jt = 0;  // kv tiles this warpgroup has processed so far (S buffer and barrier phases)
     bool passed = false;  // this warp has passed on a turn (the very first one, of tile 0, is not waited for)
-    for (int round = 0, idx = first_item; idx < num_items; idx = next_item(idx, ++round)) {
+    for (int round = 0, idx = blockIdx.x; idx < num_items; idx = next_item(idx, ++round)) {
       const Item it = get_item(idx);
       if (!it.valid) continue;
       const int nt = t == 0 ? it.n0 : it.n1;
@@ -758,13 +631,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       // ---- item epilogue: O / l -> global, then hand O_t back to the MMA issuer
       mbar_wait(&pv_done[t * 2 + ((jt + nt - 1) & 1)], ((jt + nt - 1) >> 1) & 1);
       tc_fence_after();
-      if constexpr (SPLIT) {
-        if (it.parts > 1) {
-          exchange_split<DV>({smem, sO + (warp - 3) * C::O_STAGE_BYTES, tO, t * 4 + qd, (int)cluster_ctarank(), it.parts, it.q0, it.len, it.seq0, it.h << pack, pack, sink, ldg,
-                              ldo, head_gate, sink_w, out}, m_used, l);
-          continue;
-        }
-      }
       if (sink) l += fast_exp2(-m_used);  // one more unit in the denominator: a key of score 0 that carries no value
       if (sink_w != nullptr) l += fast_exp2(__bfloat162float(sink_w[head]) * 1.4426950408889634f - m_used);  // a learned one per head
       float inv_l = l > 0.f ? 1.0f / l : 0.f;
@@ -841,14 +707,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
   }
 
-  if constexpr (SPLIT) {  // the exchange's two barriers, for the warps that have no rows
-    const Item it = get_item(first_item);
-    if (it.parts > 1 && !(it.valid && warp >= 3 && (warp < 7 || it.act1))) {
-      __syncwarp();
-      cluster_sync_all();
-      cluster_sync_all();
-    }
-  }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -857,8 +715,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   }
 }
 
-constexpr double kSplitCost = 45;  // of a split item beyond its kv tiles (about 8 us), in the units of cut_of (a lone q tile and a kv tile are 4)
-int max_clusters[kMaxSplit + 1];  // clusters of so many CTAs that run at a time (attn_prefill_init)
 inline int paged_only(int v, bool paged) { return paged ? v : 0; }
 int device_sms() {
   static int num_sms = 0;
@@ -884,8 +740,8 @@ bool sorts_items(const AttnPrefillArgs& a, int pack) {
   return (long long)max_q_pairs * a.B * (a.Hq >> pack) > (short_ones ? 2ll : 1ll) * effective_sms(device_sms()) &&
          a.T < (short_ones ? 0.8 : 0.9) * (double)a.B * a.max_seqlen;
 }
-template <int D, bool PAGED, bool SORTED, bool SPLIT = false>
-cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a, int pack, int split = 1) {
+template <int D, bool PAGED, bool SORTED>
+cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a, int pack) {
   constexpr int SRC = PAGED ? KV_PAGED : KV_PACKED;
   using C = ACfg<D, D, SRC>;
   CUtensorMap mq, mk, mv, mo;
@@ -902,26 +758,17 @@ cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a, int pack, int 
     if (!make_tmap_2d(&mk, a.k, TM_BF16, (uint64_t)a.Hkv * D, (uint64_t)a.T, (uint64_t)a.ldk * 2, 64, BKV)) return cudaErrorInvalidValue;
     if (!make_tmap_2d(&mv, a.v, TM_BF16, (uint64_t)a.Hkv * D, (uint64_t)a.T, (uint64_t)a.ldv * 2, 64, BKV)) return cudaErrorInvalidValue;
   }
-  auto kern = attn_prefill_kernel<D, D, SRC, SORTED, SPLIT>;
+  auto kern = attn_prefill_kernel<D, D, SRC, SORTED>;
   const int max_q_pairs = (int)((((long long)a.max_seqlen << pack) + QPAIR - 1) / QPAIR);
   const long long items = (long long)max_q_pairs * a.B * (a.Hq >> pack);
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute cluster;
-  cfg.gridDim = dim3((unsigned)(SPLIT ? items * split : std::min<long long>(items, effective_sms(device_sms()))));  // hb_engine_cfg.sm_budget
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = SORTED ? C::SMEM_SORTED : C::SMEM;
-  cfg.stream = stream;
-  if (SPLIT) {
-    cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim = {(unsigned)split, 1, 1};
-    cfg.attrs = &cluster;
-    cfg.numAttrs = 1;
-  }
+  const int grid = (int)std::min<long long>(items, effective_sms(device_sms()));  // hb_engine_cfg.sm_budget
   const float scale_log2 = a.scale * 1.4426950408889634f;
-  return cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, mo, a.out, a.ldo, a.cu_seqlens, a.B, a.Hq, a.Hq / a.Hkv, a.causal, scale_log2, max_q_pairs, a.kv_lens,
-                            a.page_table, a.max_pages, a.Hkv, paged_only(a.block_mask, PAGED), a.unit_sink, a.head_gate, a.ldg,
-                            paged_only(a.window, PAGED), a.softcap > 0.f ? a.scale / a.softcap : 0.f,
-                            a.softcap > 0.f ? a.softcap * 1.4426950408889634f : 0.f, a.sink, mq, mk, AttnRuns{}, D, pack);
+  kern<<<grid, kThreads, SORTED ? C::SMEM_SORTED : C::SMEM, stream>>>(mq, mk, mv, mo, a.out, a.ldo, a.cu_seqlens, a.B, a.Hq, a.Hq / a.Hkv, a.causal,
+                                            scale_log2, max_q_pairs, a.kv_lens, a.page_table, a.max_pages, a.Hkv,
+                                            paged_only(a.block_mask, PAGED), a.unit_sink, a.head_gate, a.ldg,
+                                            paged_only(a.window, PAGED), a.softcap > 0.f ? a.scale / a.softcap : 0.f,
+                                            a.softcap > 0.f ? a.softcap * 1.4426950408889634f : 0.f, a.sink, mq, mk, AttnRuns{}, D, pack);
+  return cudaGetLastError();
 }
 
 // latent attention over expanded rows
@@ -935,7 +782,7 @@ cudaError_t launch_expanded(cudaStream_t stream, const AttnExpandedArgs& a) {
   if (!make_tmap_3d(&mk, a.k, TM_BF16, a.nope, H, rows, (uint64_t)a.nope * 2, (uint64_t)a.ldkv * 2, 64, 1, BKV)) return cudaErrorInvalidValue;
   if (!make_tmap_3d(&mv, a.v, TM_BF16, a.vdim, H, rows, (uint64_t)a.vdim * 2, (uint64_t)a.ldkv * 2, 64, 1, BKV)) return cudaErrorInvalidValue;
   if (!make_tmap_2d(&mkr, a.k_rot, TM_BF16, a.rot, rows, (uint64_t)a.ldkr * 2, 64, BKV)) return cudaErrorInvalidValue;
-  auto kern = attn_prefill_kernel<DK, DV, KV_EXPANDED, false, false>;
+  auto kern = attn_prefill_kernel<DK, DV, KV_EXPANDED, false>;
   int longest = 0;
   for (int i = 0; i < a.runs.n; ++i) longest = std::max(longest, a.runs.len[i]);
   const int max_q_pairs = (longest + QPAIR - 1) / QPAIR;
@@ -982,67 +829,36 @@ __global__ void attn_naive_kernel(const bf16* q, int ldq, const bf16* k, int ldk
 
 cudaError_t attn_prefill_init() {
   cudaError_t e;
-#define HB_ATTR(D_, P_, S_, X_)                                                                                      \
-  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<D_, D_, P_, S_, X_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                S_ ? ACfg<D_, D_, P_>::SMEM_SORTED : ACfg<D_, D_, P_>::SMEM)) != cudaSuccess)         \
+#define HB_ATTR(D_, P_, S_)                                                                                      \
+  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<D_, D_, P_, S_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                S_ ? ACfg<D_, D_, P_>::SMEM_SORTED : ACfg<D_, D_, P_>::SMEM)) != cudaSuccess)     \
     return e;
-  HB_ATTR(128, KV_PACKED, false, false) HB_ATTR(128, KV_PACKED, true, false) HB_ATTR(128, KV_PAGED, false, false) HB_ATTR(128, KV_PAGED, false, true)
-  HB_ATTR(64, KV_PACKED, false, false) HB_ATTR(64, KV_PACKED, true, false) HB_ATTR(64, KV_PAGED, false, false) HB_ATTR(64, KV_PAGED, false, true)
+  HB_ATTR(128, KV_PACKED, false) HB_ATTR(128, KV_PACKED, true) HB_ATTR(128, KV_PAGED, false)
+  HB_ATTR(64, KV_PACKED, false) HB_ATTR(64, KV_PACKED, true) HB_ATTR(64, KV_PAGED, false)
 #undef HB_ATTR
 #define HB_ATTRX(K_, V_)                                                                                                  \
-  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<K_, V_, KV_EXPANDED, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<K_, V_, KV_EXPANDED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                 ACfg<K_, V_, KV_EXPANDED>::SMEM)) != cudaSuccess)                                        \
     return e;
   HB_ATTRX(128, 64) HB_ATTRX(128, 128) HB_ATTRX(192, 64) HB_ATTRX(192, 128)
 #undef HB_ATTRX
-  for (int split = 2; split <= kMaxSplit; split *= 2) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute cluster;
-    cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim = {(unsigned)split, 1, 1};
-    cfg.gridDim = dim3(device_sms() / split * split);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = ACfg<128, 128, KV_PAGED>::SMEM;
-    cfg.attrs = &cluster;
-    cfg.numAttrs = 1;
-    if ((e = cudaOccupancyMaxActiveClusters(&max_clusters[split], attn_prefill_kernel<128, 128, KV_PAGED, false, true>, &cfg)) != cudaSuccess) return e;
-  }
   return cudaSuccess;
 }
 
-// How a launch is cut.  pack: query heads (a power of two, given as its logarithm) that share a kv head and the rows of a tile.  Packed tiles
-// span fewer tokens, so less of their diagonal is masked and less of a last tile is empty: 6 prompts of 300 to 3000 tokens, 32 heads over 8: 173 kv
-// tiles per SM -> 148, 223 -> 193 us; 8 of about 1000 97 -> 87.  split (paged): CTAs of a cluster that share the kv tiles of an item, where the
-// items leave SMs idle.  Taken is what leaves the SMs the least to do one after the other: a lone q tile takes 4/5 of a pair's time per kv tile (0.69
-// and 0.86 us); a split item 8 us more than its kv tiles (its CTA is not a persistent one's next item: first loads 3, the exchange 5).
-// Measured, whole / by 2 / by 4, 32 heads over 8: 100 rows over 4000 keys 53 / 37 / 25 us, 512 over 2500 43 / 33 / 45, 512 over 1000 22.6 / 22.6 / 35,
-// 2 x 777 over 6000 170 / 165 / 229 (D = 64 160 / 138 / 203), 3 x 400 over 2500 70 / 83 / 118; 12 heads of their own, 2 x 333 over 4500
-// 72 / 48 / 55.  Eighths never won (15 clusters of 8 run at a time, 120 SMs).
-// A split portion's sums are added in another order, so its last bits depend on the cut, as a decoded token's do on decode_splits; packing alone changes none.
-struct Cut {
-  int pack, split;
-};
-Cut cut_of(const AttnPrefillArgs& a, bool paged) {
+// Query heads (a power of two, given as its logarithm) that share a kv head and the rows of a tile.  Packed tiles span fewer tokens, so less
+// of their diagonal is masked and less of a last tile is empty: 6 prompts of 300 to 3000 tokens, 32 heads over 8: 173 kv tiles per SM -> 148, 223 ->
+// 193 us; 8 of about 1000 97 -> 87.  They are also fewer: the packing that leaves the SMs the least to do one after the other is taken (a lone q
+// tile takes about 4/5 of a pair's time; 100 rows over 4000 keys 53 us unpacked, 61 by four).
+int packed_heads(const AttnPrefillArgs& a) {
   const int group = a.Hq / a.Hkv, sms = effective_sms(device_sms());
-  const bool whole = sms == device_sms();  // (a partition of the SMs may have no room for a cluster)
-  // kv tiles of an item at most
-  long long tiles = a.longest_kv > 0 ? std::min((a.longest_kv + BKV - 1) / BKV, a.max_pages) : a.max_pages;
-  if (a.window > 0) tiles = std::min<long long>(tiles, (a.window + a.max_seqlen) / BKV + 2);
-  if (a.block_mask > 0) tiles = std::min<long long>(tiles, (a.block_mask + a.max_seqlen) / BKV + 2);
-  Cut best = {0, 1};
-  double least = 0;
+  int best = 0;
+  long long least = 0;
   for (int p = 0; p <= 5 && group % (1 << p) == 0; ++p) {
     const long long rows = (long long)a.max_seqlen << p, items = (rows + QPAIR - 1) / QPAIR * a.B * (a.Hq >> p);
-    const double each = rows <= BQ ? 4 : 5;
-    for (int s = 1; s <= (paged ? kMaxSplit : 1); s *= 2) {
-      if (s > 1 && (tiles < s * kLeastShare || !whole)) break;
-      const long long at_once = s == 1 ? sms : max_clusters[s];
-      if (s > 1 && items > at_once) continue;  // (several rounds of clusters gain little, 2 x 777 over 6000 above, and change a portion's last bits)
-      const double cost = (double)((items + at_once - 1) / at_once) * (each * (double)((tiles + s - 1) / s) + (s > 1 ? kSplitCost : 0));
-      if ((p == 0 && s == 1) || (s == 1 ? cost <= least : cost < 0.95 * least)) {
-        best = {p, s};
-        least = cost;
-      }
+    const long long cost = (items + sms - 1) / sms * (rows <= BQ ? 4 : 5);
+    if (p == 0 || cost <= least) {
+      best = p;
+      least = cost;
     }
   }
   return best;
@@ -1057,12 +873,12 @@ cudaError_t attn_prefill(cudaStream_t stream, const AttnPrefillArgs& a) {
   if (a.window < 0 || (a.window > 0 && (!paged || !a.causal || a.block_mask > 0))) return cudaErrorInvalidValue;
   if (paged) {
     if (!a.v_cache || !a.page_table || !a.kv_lens || a.max_pages <= 0 || a.num_pages <= 0 || a.page_size != 64) return cudaErrorInvalidValue;
-    const Cut c = cut_of(a, true);
-    if (a.D == 128) return c.split > 1 ? launch<128, true, false, true>(stream, a, c.pack, c.split) : launch<128, true, false>(stream, a, c.pack);
-    if (a.D == 64) return c.split > 1 ? launch<64, true, false, true>(stream, a, c.pack, c.split) : launch<64, true, false>(stream, a, c.pack);
+    const int pack = packed_heads(a);
+    if (a.D == 128) return launch<128, true, false>(stream, a, pack);
+    if (a.D == 64) return launch<64, true, false>(stream, a, pack);
     return cudaErrorInvalidValue;
   }
-  const int pack = cut_of(a, false).pack;
+  const int pack = packed_heads(a);
   const bool sorted = sorts_items(a, pack);
   if (a.D == 128) return sorted ? launch<128, false, true>(stream, a, pack) : launch<128, false, false>(stream, a, pack);
   if (a.D == 64) return sorted ? launch<64, false, true>(stream, a, pack) : launch<64, false, false>(stream, a, pack);

@@ -671,7 +671,7 @@ int Engine::forward_llama(int T, int B, bool prefill, int max_seqlen, const Step
       if (paged) {  // some sequence continues a partly prefilled prompt: K/V (this chunk's were just written) from the pool
         a.k_cache = kc; a.v_cache = vc;
         a.page_table = pt; a.max_pages = max_pages_per_seq_;
-        a.kv_lens = ctx; a.longest_kv = step_longest_;
+        a.kv_lens = ctx;
         a.num_pages = num_pages_; a.page_size = page_;
       }
       SPAN(1, attn_flops_, attn_prefill(stream_, a));
@@ -1335,7 +1335,6 @@ int Engine::run_prefill(std::vector<Request*>& batch) {
   int32_t* pt = (int32_t*)(h_step_ + L.pt);
   L.total = al16(L.pen + 8 * fill_sampling(batch.data(), B, L, T));
   int t = 0;
-  step_longest_ = 0;
   for (int i = 0; i < B; ++i) {
     Request* r = batch[i];
     cu[i] = t;
@@ -1354,7 +1353,6 @@ int Engine::run_prefill(std::vector<Request*>& batch) {
     }
     last[i] = t - 1;
     ctx[i] = end;
-    if (i < Bp || is_stack()) step_longest_ = std::max(step_longest_, end);
     if (paged || i >= Bp || is_stack()) {
       const int np = (end + page_ - 1) / page_;
       for (int j = 0; j < np; ++j) pt[(size_t)i * max_pages_per_seq_ + j] = r->pages[j];

@@ -144,7 +144,6 @@ class Engine {
   int drain_spans();
   bool profile_ = false;
   bool step_is_prefill_ = true;
-  int step_longest_ = 0;  // kv positions of the current prefill step's longest sequence
   double attn_flops_ = 0, attn_bytes_ = 0;  // per-layer attention work of the current step
   std::vector<cudaEvent_t> ev_pool_;
   size_t ev_next_ = 0;

@@ -1215,7 +1215,7 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
         fa.cu_seqlens = cu; fa.B = B; fa.T = T; fa.max_seqlen = longest;
         fa.Hq = H; fa.Hkv = G; fa.D = Dk; fa.causal = 1; fa.scale = l.scale;
         fa.k_cache = (const bf16*)kplane; fa.v_cache = (const bf16*)vplane;
-        fa.page_table = pt; fa.kv_lens = (const int32_t*)(d_step_ + L.ctx); fa.longest_kv = step_longest_;
+        fa.page_table = pt; fa.kv_lens = (const int32_t*)(d_step_ + L.ctx);
         fa.max_pages = max_pages_per_seq_; fa.num_pages = num_pages_; fa.page_size = page_;
         fa.block_mask = l.mask == HB_MASK_CHUNK ? l.window : 0;
         fa.window = (l.mask == HB_MASK_WINDOW && l.window < cfg_.max_ctx) ? l.window : 0;

@@ -130,7 +130,6 @@ struct AttnPrefillArgs {
   const int32_t* page_table = nullptr;  // [B, max_pages]
   const int32_t* kv_lens = nullptr;     // [B] kv length including this step's q rows
   int max_pages = 0, num_pages = 0, page_size = 64;
-  int longest_kv = 0;  // of kv_lens, where the host knows it: it says how a launch is cut (0: max_pages pages)
   // paged + causal only.  block_mask > 0: a position sees only the keys of its own block of block_mask positions (blocks
   // counted from position 0 of the sequence).  unit_sink: one unit added to the softmax denominator (a key of score 0 that
   // carries no value)

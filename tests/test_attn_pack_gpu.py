@@ -46,8 +46,7 @@ def test_packed_keys(Hq, Hkv, D, lens):
 @pytest.mark.parametrize("Hq,Hkv", [(4, 4), (12, 2), (32, 8), (16, 1)])
 @pytest.mark.parametrize("D", [64, 128])
 @pytest.mark.parametrize("rows,ctx", [(1, [1, 64, 300]), (33, [33, 97, 1000]), (64, [64, 2100]), (200, [300, 200, 4000]), (777, [6000]),
-                                      # kv tiles shared out to a cluster: 2, 4 and 8 shares, lone q tiles, sequences too short for a share each, a last
-                                      # share (tile 16 of 17) that begins behind the keys of the lower q tile
+                                      # few rows over many keys, lone q tiles, a last kv tile that only some rows of the lower q tile see
                                       (1, [4000]), (150, [1030]), (200, [1088, 2100]), (256, [8000]), (300, [600, 520, 5000])])
 def test_pages(Hq, Hkv, D, rows, ctx):
     L = hb.lib()
@@ -91,6 +90,32 @@ def test_a_prompt_does_not_depend_on_its_launch(Hq, Hkv):
         run.append(out)
     torch.cuda.synchronize()
     assert torch.equal(run[0], torch.cat(run[1:]))
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(32, 8), (16, 1), (12, 2), (4, 4)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_a_portion_has_the_bits_of_its_prompt(Hq, Hkv, D):
+    """The last rows of a prompt over its pages: alone, with a wider page table, beside other sequences, and as part of the whole prompt, the same bits."""
+    L, n, ld = hb.lib(), 3000, (Hq + 2 * Hkv) * D
+    assert L.hbk_init() == 0
+    g = torch.Generator(device="cuda").manual_seed(Hq + D)
+    qkv = (torch.randn(n, ld, generator=g, device="cuda") * 2).to(BF)
+    cu, whole, p = torch.tensor([0, n], device="cuda", dtype=torch.int32), torch.empty((n, Hq * D), device="cuda", dtype=BF), qkv.data_ptr()
+    assert L.hbk_attn_prefill(p, ld, p + 2 * Hq * D, ld, p + 2 * (Hq + Hkv) * D, ld, whole.data_ptr(), Hq * D, cu.data_ptr(), 1, n, n, Hq, Hkv, D, 1, D ** -0.5) == 0
+    pages = (n + 63) // 64
+    pool = torch.zeros((2, pages * 64, Hkv, D), device="cuda", dtype=BF)
+    pool[0, :n], pool[1, :n] = (qkv[:, a:a + Hkv * D].view(n, Hkv, D) for a in (Hq * D, (Hq + Hkv) * D))
+    k, v = pool.view(2, pages, 64, Hkv, D).transpose(2, 3).contiguous()
+    for rows in (90, 128, 517):
+        for others, width in ((0, pages), (0, 400), (2, pages), (40, pages)):
+            B = 1 + others
+            table = torch.arange(width, device="cuda", dtype=torch.int32).clamp(max=pages - 1).repeat(B, 1).contiguous()
+            at, kv = torch.arange(B + 1, device="cuda", dtype=torch.int32) * rows, torch.full((B,), n, device="cuda", dtype=torch.int32)
+            q = qkv[n - rows:, :Hq * D].repeat(B, 1).contiguous()
+            out = torch.empty_like(q)
+            assert L.hbk_attn_prefill_paged(q.data_ptr(), Hq * D, k.data_ptr(), v.data_ptr(), table.data_ptr(), width, kv.data_ptr(), out.data_ptr(), Hq * D, at.data_ptr(),
+                                            B, B * rows, rows, Hq, Hkv, D, 1, D ** -0.5, pages) == 0
+            assert torch.equal(out, whole[n - rows:].repeat(B, 1)), (rows, others, width)
 
 
 @pytest.mark.parametrize("D", [64, 128])
