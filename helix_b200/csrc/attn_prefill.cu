@@ -483,6 +483,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const uint32_t lane_sel = static_cast<uint32_t>(qd * 32) << 16;
     const uint32_t tO = tmem_base + lane_sel + 256 + t * 128;
     int jt = 0;  // kv tiles this warpgroup has processed so far (S buffer and barrier phases)
+    const bool follow = !causal && (group & 1);  // rows are rescaled with their warp
     bool passed = false;  // this warp has passed on a turn (the very first one, of tile 0, is not waited for)
     for (int round = 0, idx = blockIdx.x; idx < num_items; idx = next_item(idx, ++round)) {
       const Item it = get_item(idx);
@@ -557,9 +558,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           if (__any_sync(0xffffffffu, need)) {
             mbar_wait(&pv_done[t * 2 + ((tile - 1) & 1)], ((tile - 1) >> 1) & 1);  // PV(j-1), hence every PV so far, is in O_t
             tc_fence_after();
-            // (where heads can be packed, which depends on the whole launch, only the rows that need it: a row's bits do not depend on the
-            // rows beside it.  Expanded rows always stand beside the same ones, and follow them)
-            m_new = EXPANDED ? fmaxf(m_new, m_used) : need ? m_new : m_used;
+            // (A row that follows its warp has the weight one, without a rounding, at its new maximum.  Where heads can be packed, which depends on the
+            // whole launch, and in causal prompts, which may come in portions, only the rows that need it do: a row's bits do not depend on the rows
+            // beside it.  The rows of an encoder and expanded rows always stand beside the same ones.  Error against 64 bits with scores of deviation 4,
+            // following / not: 1.95e-3 / 2.00e-3; of deviation 1, where hardly any row is rescaled, 1.98e-3 both)
+            m_new = EXPANDED || follow ? fmaxf(m_new, m_used) : need ? m_new : m_used;
             const float f = fast_exp2(m_used - m_new);
             m_used = m_new;
             l *= f;

@@ -159,3 +159,22 @@ def test_values_behind_the_mask_have_no_weight(Hq, Hkv, D):
     torch.cuda.synchronize()
     for b, c in enumerate(at):
         assert torch.equal(out[1 + b, :c], out[0, :c]), c
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_encoder_rows_are_rescaled_with_their_warp(D):
+    """Rows whose largest score comes in the second kv tile, up to 2^7.8 above the first's, beside one row per warp that has to be rescaled: their weight there
+    is one, so the result has no rounding but its own (half a unit of 2^-7; the polynomial's 7.6e-5 in the sum of the other weights)."""
+    L, n = hb.lib(), 128
+    assert L.hbk_init() == 0
+    qkv = torch.zeros((n, 3 * D), device="cuda", dtype=BF)
+    a = torch.linspace(0.2, 5.4, n, device="cuda").to(BF)
+    qkv[:, 0] = a * 8
+    qkv[::32, 0], qkv[::32, 1] = 0, 16 * 8
+    qkv[100, D] = qkv[101, D + 1] = 1
+    qkv[100, 2 * D:] = 1
+    cu, out, q = torch.tensor([0, n], device="cuda", dtype=torch.int32), torch.empty((n, D), device="cuda", dtype=BF), qkv.data_ptr()
+    assert L.hbk_attn_prefill(q, 3 * D, q + 2 * D, 3 * D, q + 4 * D, 3 * D, out.data_ptr(), D, cu.data_ptr(), 1, n, n, 1, 1, D, 0, 0.125) == 0
+    e = a.double().exp()
+    w, rows = e / (e + n - 1), torch.arange(n, device="cuda") % 32 != 0
+    assert ((out.double() - w[:, None]).abs() <= (2.0 ** (torch.floor(torch.log2(w)) - 8) + 1e-4 * w)[:, None])[rows].all()
