@@ -230,7 +230,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   // (ranks by counting, about a microsecond).  With sequences of unequal length the plain order, q pair by q pair with a slot
   // for every sequence whether it has that pair or not, left the longest-loaded CTA 24 to 30 % above the mean (6 prompts of 300
   // to 3000 tokens: 231 tile times of a mean of 187, now 191; 64 chunks of 64 to 512: 74 of 57, now 60).  Measured: 250 -> 233 us and 70.8 -> 62.6 us.
-  // Everything else runs the kernel with the plain walk: launches whose sequences are short or of about equal lengths (sorts_items below), and
+  // Everything else runs the kernel with the plain walk: launches whose sequences are short or of about equal lengths (wants_order below), and
   // keys from a page pool or an expanded run (portions of a long context are level already).  The plain order also stands in where a
   // launch turns out to have more rows than kMaxRows.
   if constexpr (SORTED) {
@@ -735,14 +735,16 @@ int device_sms() {
 //   - empty (sequence, position) slots: a tenth of all, a fifth where the longest has only two or three pairs (16 sequences of 375 to 500
 //     62 / 66, of 1125 to 1500 129 / 122);
 //   - more items than SMs, twice as many there (3 sequences of 37 to 300 12.4 / 14.5, of 75 to 600 20.3 / 20.5, of 187 to 1500 53 / 31).
-// Gains are 20 % on average over such launches.  The indices have to fit the order's entries.
-bool sorts_items(const AttnPrefillArgs& a, int pack) {
-  const int max_q_pairs = ((a.max_seqlen << pack) + QPAIR - 1) / QPAIR;
-  if (a.B <= 1 || a.B > 256 || max_q_pairs < 2 || max_q_pairs > 255 || ((long long)a.T << pack) < (long long)BKV * a.B) return false;
-  const bool short_ones = max_q_pairs <= 3;
-  return (long long)max_q_pairs * a.B * (a.Hq >> pack) > (short_ones ? 2ll : 1ll) * effective_sms(device_sms()) &&
-         a.T < (short_ones ? 0.8 : 0.9) * (double)a.B * a.max_seqlen;
+// Gains are 20 % on average over such launches.  The indices have to fit the order's entries (order_fits).
+int q_pairs(const AttnPrefillArgs& a, int pack) { return (int)((((long long)a.max_seqlen << pack) + QPAIR - 1) / QPAIR); }
+bool wants_order(const AttnPrefillArgs& a, int pack, int sms) {
+  const int pairs = q_pairs(a, pack);
+  if (a.B <= 1 || a.B > 256 || pairs < 2 || ((long long)a.T << pack) < (long long)BKV * a.B) return false;
+  const bool short_ones = pairs <= 3;
+  return (long long)pairs * a.B * (a.Hq >> pack) > (short_ones ? 2ll : 1ll) * sms && a.T < (short_ones ? 0.8 : 0.9) * (double)a.B * a.max_seqlen;
 }
+// (for sure: the host knows no more of the rows than that a sequence's last pair may be cut short)
+bool order_fits(const AttnPrefillArgs& a, int pack) { return q_pairs(a, pack) <= 255 && ((long long)a.T << pack) / QPAIR + a.B <= kMaxRows; }
 template <int D, bool PAGED, bool SORTED>
 cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a, int pack) {
   constexpr int SRC = PAGED ? KV_PAGED : KV_PACKED;
@@ -762,7 +764,7 @@ cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a, int pack) {
     if (!make_tmap_2d(&mv, a.v, TM_BF16, (uint64_t)a.Hkv * D, (uint64_t)a.T, (uint64_t)a.ldv * 2, 64, BKV)) return cudaErrorInvalidValue;
   }
   auto kern = attn_prefill_kernel<D, D, SRC, SORTED>;
-  const int max_q_pairs = (int)((((long long)a.max_seqlen << pack) + QPAIR - 1) / QPAIR);
+  const int max_q_pairs = q_pairs(a, pack);
   const long long items = (long long)max_q_pairs * a.B * (a.Hq >> pack);
   const int grid = (int)std::min<long long>(items, effective_sms(device_sms()));  // hb_engine_cfg.sm_budget
   const float scale_log2 = a.scale * 1.4426950408889634f;
@@ -851,12 +853,18 @@ cudaError_t attn_prefill_init() {
 // Query heads (a power of two, given as its logarithm) that share a kv head and the rows of a tile.  Packed tiles span fewer tokens, so less
 // of their diagonal is masked and less of a last tile is empty: 6 prompts of 300 to 3000 tokens, 32 heads over 8: 173 kv tiles per SM -> 148, 223 ->
 // 193 us; 8 of about 1000 97 -> 87.  They are also fewer: the packing that leaves the SMs the least to do one after the other is taken (a lone q
-// tile takes about 4/5 of a pair's time; 100 rows over 4000 keys 53 us unpacked, 61 by four).
-int packed_heads(const AttnPrefillArgs& a) {
-  const int group = a.Hq / a.Hkv, sms = effective_sms(device_sms());
+// tile takes about 4/5 of a pair's time; 100 rows over 4000 keys 53 us unpacked, 61 by four; one prompt of 128 tokens, 128 columns 8.7 | 10.4).
+// A wide packing has more q pairs, and where they are more than the order holds, the order is worth more than the packing.  us with 1 | 2 | 4 | .. heads
+// per tile, [ ] in plain order: 32 heads over 8, 16 prompts of 500 to 4500 tokens 1037 | 978 | [1045], 6 of 2000 to 11300 2732 | 2669 | [3165], 30 of 500
+// to 6200 3844 | [3827] | [4048], 20 of 500 to 5000 1971 | 1875 | [1840]; 32 over 1, 8 of 200 to 1800 157 | 134 | 128 | 126 | 122 | [165], 10 of
+// 500 to 3500 476 | 433 | 394 | [417] | [480] | [431].
+AttnPrefillPlan attn_prefill_plan(const AttnPrefillArgs& a, int sms) {
+  const int group = a.Hq / a.Hkv;
+  const bool paged = a.k_cache != nullptr;
   int best = 0;
   long long least = 0;
   for (int p = 0; p <= 5 && group % (1 << p) == 0; ++p) {
+    if (!paged && p > 0 && wants_order(a, p, sms) && !order_fits(a, p) && order_fits(a, 0)) break;
     const long long rows = (long long)a.max_seqlen << p, items = (rows + QPAIR - 1) / QPAIR * a.B * (a.Hq >> p);
     const long long cost = (items + sms - 1) / sms * (rows <= BQ ? 4 : 5);
     if (p == 0 || cost <= least) {
@@ -864,7 +872,8 @@ int packed_heads(const AttnPrefillArgs& a) {
       least = cost;
     }
   }
-  return best;
+  // (launches that may or may not fit: the kernel counts)
+  return {best, !paged && wants_order(a, best, sms) && q_pairs(a, best) <= 255};
 }
 
 cudaError_t attn_prefill(cudaStream_t stream, const AttnPrefillArgs& a) {
@@ -876,13 +885,12 @@ cudaError_t attn_prefill(cudaStream_t stream, const AttnPrefillArgs& a) {
   if (a.window < 0 || (a.window > 0 && (!paged || !a.causal || a.block_mask > 0))) return cudaErrorInvalidValue;
   if (paged) {
     if (!a.v_cache || !a.page_table || !a.kv_lens || a.max_pages <= 0 || a.num_pages <= 0 || a.page_size != 64) return cudaErrorInvalidValue;
-    const int pack = packed_heads(a);
+    const int pack = attn_prefill_plan(a, effective_sms(device_sms())).pack;
     if (a.D == 128) return launch<128, true, false>(stream, a, pack);
     if (a.D == 64) return launch<64, true, false>(stream, a, pack);
     return cudaErrorInvalidValue;
   }
-  const int pack = packed_heads(a);
-  const bool sorted = sorts_items(a, pack);
+  const auto [pack, sorted] = attn_prefill_plan(a, effective_sms(device_sms()));
   if (a.D == 128) return sorted ? launch<128, false, true>(stream, a, pack) : launch<128, false, false>(stream, a, pack);
   if (a.D == 64) return sorted ? launch<64, false, true>(stream, a, pack) : launch<64, false, false>(stream, a, pack);
   return cudaErrorInvalidValue;

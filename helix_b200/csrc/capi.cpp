@@ -300,6 +300,13 @@ int hbk_attn_prefill_paged(const void* q, int ldq, const void* k_cache, const vo
   a.page_table = page_table; a.max_pages = max_pages; a.kv_lens = kv_lens; a.num_pages = num_pages;
   return kret(hb::attn_prefill(0, a));
 }
+int hbk_attn_prefill_plan(int B, int T, int max_seqlen, int Hq, int Hkv, int paged, int sms) {
+  if (B <= 0 || T <= 0 || max_seqlen <= 0 || Hkv <= 0 || Hq <= 0 || Hq % Hkv || sms <= 0) return -1;
+  hb::AttnPrefillArgs a = mk_prefill(nullptr, 0, nullptr, 0, nullptr, 0, nullptr, 0, nullptr, B, T, max_seqlen, Hq, Hkv, 64, 1, 1.f);
+  if (paged) a.k_cache = reinterpret_cast<const hb::bf16*>(&a);  // (any: only whether there is one matters)
+  const hb::AttnPrefillPlan p = hb::attn_prefill_plan(a, sms);
+  return 1 << p.pack | (int)p.sorted << 8;
+}
 int hbk_attn_naive(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, float* out, int ldo,
                    const int32_t* cu, int B, int T, int max_seqlen, int Hq, int Hkv, int D, int causal, float scale) {
   return kret(hb::attn_naive_check(0, mk_prefill(q, ldq, k, ldk, v, ldv, nullptr, ldo, cu, B, T, max_seqlen, Hq, Hkv, D, causal, scale), out));

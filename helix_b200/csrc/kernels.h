@@ -141,6 +141,12 @@ struct AttnPrefillArgs {
   float softcap = 0.f;
   const bf16* sink = nullptr;
 };
+// How a launch is cut on `sms` SMs: query heads (their logarithm) that share the rows of a tile, and whether its items are sorted
+struct AttnPrefillPlan {
+  int pack;
+  bool sorted;
+};
+AttnPrefillPlan attn_prefill_plan(const AttnPrefillArgs& a, int sms);
 cudaError_t attn_prefill(cudaStream_t stream, const AttnPrefillArgs& a);
 // The same kernel for latent attention over EXPANDED rows (long prompt portions): per cached position a row [k_0 .. k_(H-1) |
 // v_0 .. v_(H-1)] made from its latent, and one rotated key part shared by all heads.  Run b: q rows [t0, t0 + len) of the packed

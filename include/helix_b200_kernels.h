@@ -60,6 +60,9 @@ int hbk_attn_prefill(const void* q, int ldq, const void* k, int ldk, const void*
 int hbk_attn_prefill_paged(const void* q, int ldq, const void* k_cache, const void* v_cache, const int32_t* page_table,
                            int max_pages, const int32_t* kv_lens, void* out, int ldo, const int32_t* cu_seqlens, int B,
                            int T, int max_q_len, int Hq, int Hkv, int D, int causal, float scale, int num_pages);
+/* how hbk_attn_prefill (paged 0) or hbk_attn_prefill_paged (1) cuts a launch of these sizes on `sms` SMs: query heads of a kv head that
+ * share the rows of a tile, + 256 where the items are sorted by length.  Host arithmetic only; -1 for sizes that are refused. */
+int hbk_attn_prefill_plan(int B, int T, int max_seqlen, int Hq, int Hkv, int paged, int sms);
 int hbk_attn_naive(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, float* out_f32, int ldo,
                    const int32_t* cu_seqlens, int B, int T, int max_seqlen, int Hq, int Hkv, int D, int causal,
                    float scale);

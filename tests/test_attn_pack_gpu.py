@@ -74,12 +74,15 @@ def test_pages(Hq, Hkv, D, rows, ctx):
 
 @pytest.mark.parametrize("Hq,Hkv", [(32, 8), (16, 1), (12, 2)])
 def test_a_prompt_does_not_depend_on_its_launch(Hq, Hkv):
-    """Alone (few items: heads apart) and among others (packed, sorted): the same bits, also where large scores rescale the sums."""
+    """Alone (few items: the short ones with heads apart) and among others (packed, sorted): the same bits, also where large scores rescale the sums."""
     L, D = hb.lib(), 128
     assert L.hbk_init() == 0
     lens, ld = [90, 300, 1800, 700, 33], (Hq + 2 * Hkv) * D
     g = torch.Generator(device="cuda").manual_seed(Hq)
     qkv = (torch.randn(sum(lens), ld, generator=g, device="cuda") * 3).to(BF)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    plans = [L.hbk_attn_prefill_plan(len(ns), sum(ns), max(ns), Hq, Hkv, 0, sms) for ns in [lens] + [[n] for n in lens]]
+    assert plans[0] == 256 + (Hq // Hkv & -(Hq // Hkv)) and 1 in plans
     run = []
     for at, ns in [(0, lens)] + [(sum(lens[:i]), [n]) for i, n in enumerate(lens)]:
         cu = torch.tensor([0] + list(torch.tensor(ns).cumsum(0)), device="cuda", dtype=torch.int32)
