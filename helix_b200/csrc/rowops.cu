@@ -910,7 +910,9 @@ sample_cluster_kernel(const float* __restrict__ logits, int ldl, const float* __
       __syncthreads();
       const int b_lo = sh.bin[0], b_hi = sh.bin[1];
       const uint32_t c_hi = sh.upto[1];
-      if (sh.upto[0] - c_hi > (uint32_t)kFin) return 0;
+      const bool many = sh.upto[0] - c_hi > (uint32_t)kFin;
+      __syncthreads();  // (the caller may ask again, which writes these four anew)
+      if (many) return 0;
       u64 m_hi = 0;
       if (by_mass) {
         scan([&](float x) {

@@ -49,3 +49,23 @@ def test_bins_draw_what_keys_draw(kind, V):
         torch.cuda.synchronize()
         assert torch.equal(out[0], out[1]), (s, [filters[i] for i in (out[0] != out[1]).nonzero().flatten().tolist()])
         assert (out[0] >= 0).all()
+
+
+@pytest.mark.parametrize("B", [4, 60, 130, 250])  # eight, four, two blocks and one per row
+def test_more_survivors_than_a_list_holds(B):
+    """top_k beyond a list's 1024 tokens together with top_p: the bins are asked twice, first for both thresholds and, since that is too many tokens, for
+    the k-th alone.  The second question must not reach threads that still read the answer to the first."""
+    L, V = hb.lib(), 16384
+    f = lambda v, t: torch.tensor(v, device="cuda", dtype=t)  # noqa: E731
+    filters = [(t, k, p) for k in (1025, 1500, 3000, 8000) for t in (0.7, 4.0) for p in (0.3, 0.8, 0.99)]
+    x = rows("bulk", B, B)
+    wide = torch.full((B, V), -float("inf"), device="cuda")
+    wide[:, :8192] = x
+    temp, tk, tp = (f([filters[b % len(filters)][i] for b in range(B)], t) for i, t in ((0, torch.float32), (1, torch.int32), (2, torch.float32)))
+    out = [torch.full((B,), -1, device="cuda", dtype=torch.int32) for _ in range(2)]
+    for s in range(30):
+        seed = torch.arange(B, device="cuda", dtype=torch.int64) * 7877 + s
+        for o, r in zip(out, (x, wide)):
+            assert L.hbk_sample_filtered(r.data_ptr(), r.shape[1], temp.data_ptr(), seed.data_ptr(), tk.data_ptr(), tp.data_ptr(), o.data_ptr(), B, r.shape[1]) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(out[0], out[1]), s
