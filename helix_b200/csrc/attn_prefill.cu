@@ -506,8 +506,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (t == 0 && warp == 3 && lane == 0) HB_TRACE(3);  // got S0(j)
         const int kv0 = (it.j_lo + j) * BKV;
         const int lo = chunk > 0 ? qpos / chunk * chunk : (window > 0 ? qpos - window + 1 : 0);  // first kv position this row sees
-        const bool need_mask = (kv0 + BKV > len) || (causal && (kv0 + BKV - 1 > qt0)) ||
-                               (chunk > 0 && kv0 < qt1 / chunk * chunk) || (window > 0 && kv0 <= qt1 - window);
+        const bool begins = (chunk > 0 && kv0 < qt1 / chunk * chunk) || (window > 0 && kv0 <= qt1 - window);  // some row's block or window, in this tile
+        const bool need_mask = (kv0 + BKV > len) || (causal && (kv0 + BKV - 1 > qt0)) || begins;
         const int lim = causal ? min(len - 1, qpos) : len - 1;  // last valid kv position for this row
         // ---- the S row: back-to-back TMEM loads, ONE wait, then max / exp2 / pack entirely in registers
         uint32_t sv[BKV];
@@ -538,7 +538,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           const int upto = lim - kv0, from = lo - kv0;  // columns that the row sees
 #pragma unroll
           for (int i = 0; i < BKV; ++i) sv[i] = i <= upto ? sv[i] : 0xff800000u;  // -inf
-          if (from > 0) {
+          if (begins) {  // (of the whole q tile: a branch on a row's own `from` would part the warp before the aligned operations below)
 #pragma unroll
             for (int i = 0; i < BKV; ++i) sv[i] = i >= from ? sv[i] : 0xff800000u;
           }
@@ -624,11 +624,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&p_full[t * 2 + (tile & 1)]);
-        if (j < turns) {
+        if (j < turns) {  // (before lane 0 goes its own way: bar.arrive wants the whole warp)
           bar_arrive((t ? 1 : 5) + qd, 64);  // the other tile's turn
           passed = true;
         }
+        if (lane == 0) mbar_arrive(&p_full[t * 2 + (tile & 1)]);
         if (t == 0 && warp == 3 && lane == 0) HB_TRACE(6);  // P0(j) handed over
       }
       // ---- item epilogue: O / l -> global, then hand O_t back to the MMA issuer

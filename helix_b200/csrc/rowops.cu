@@ -526,6 +526,7 @@ sample_cluster_kernel(const float* __restrict__ logits, int ldl, const float* __
   auto share_bar = [&] { bar = fkey_inv(__reduce_max_sync(__activemask(), fkey(bar))); };
 
   if (tid == 0) sh.n_list = 0;
+  __syncwarp();  // (the aligned barrier wants converged warps)
   if constexpr (NC > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // (this block runs: others may write to it)
   float mx = -INFINITY;
   if constexpr (SM) {  // (entries behind the slice's end read as NaN)
