@@ -456,7 +456,7 @@ __device__ __forceinline__ void load_slice(const float* __restrict__ src, int n,
 // passes and the draw over 32 tokens a thread each, and seven cluster barriers.
 // Measured (us, with passes of three keys or 128 bins of masses | now): 32 rows of 128256, kinds of filters mixed 60 | 32, top_p 0.95 68 | 35, top_k 40 25 | 21;
 // 1 row 38 | 23; 64 rows of 32768 35 | 23.  The bins cost two barriers before anything is known, so rows whose first pass of keys had left next to
-// nothing are a little slower (temperature 0.1, top_p 0.8, 64 rows of 32768 18 | 21; of 128256 53 | 50).
+// nothing gain nothing (cold ones, below).
 constexpr int kFin = 1024, kBins = 4096, kHeavy = 512;
 constexpr float kReach = 80.f;  // tokens on either side of the estimate
 struct alignas(16) SampleShared {
@@ -776,11 +776,16 @@ sample_cluster_kernel(const float* __restrict__ logits, int ldl, const float* __
       return max((u64)decide(by_mass, goal, c_hi, m_hi, false), lo);
     };
     // ---- bins
-    const float width = fmaxf(16.f, 22.5f * temp);  // tokens further below the maximum than 22.2 T weigh nothing
+    // Tokens further below the maximum than 22.2 T weigh nothing and, without a top_k that counts them too, need no bins.  Cold rows' nucleus ends far above that, so
+    // they have bins for 10 T only, which spares most of the counting (where it does end below, the keys are searched).  us before the bins | bins for 16
+    // at least | now, top_p 0.8 at temperature 0.1: 64 rows of 32768 18.3 | 21.1 | 17.4, 128 of 16384 16.8 | 20.4 | 16.6, 64 of 12000 15.2 | 18.6 | 15.7, 32 of
+    // 128256 28 | 26 | 21; top_p 0.9 at 0.3: 18.6 | 21.1 | 19.4, 17.8 | 20.4 | 19.1, 15.4 | 18.6 | 16.7, 28 | 26 | 25.  (At 0.5, 32 of 128256 39 | 27; with 10 T 36.)
+    const bool cold = !use_k && temp < 0.45f;
+    const float width = use_k ? fmaxf(16.f, 22.5f * temp) : cold ? 10.f * temp : 22.5f * temp;
     const float scale = (float)kBins / width, shift = (width - mx) * scale;
     auto bin_of = [&](float x) { return (int)min(__float2uint_rz(fmaf(x, scale, shift)), (unsigned)kBins - 1); };  // (0, not counted: NaN and what weighs nothing)
     // (the second bound keeps a bin's edge within 1.1 bins of where it should be; below it lies -inf too, and no maximum is a NaN)
-    const bool binned = V > kFin && fabsf(mx) * scale < 8388608.f;
+    const bool binned = fabsf(mx) * scale < 8388608.f;
     u64 total = 0;
     uint32_t tokens = 0, above[8], c_next = 0;  // tokens in the bins; those in this thread's eight bins and everything above each; above all eight
     float above_m[8], m_next = 0.f;  // and an estimate of their mass
@@ -790,7 +795,18 @@ sample_cluster_kernel(const float* __restrict__ logits, int ldl, const float* __
       __syncthreads();
       u64 m = 0;
       const bool weigh = use_p && !use_k;
-      if (weigh) {
+      if (cold) {  // (all that weighs something counts in the total)
+        const float lowest = mx - 22.5f * temp;
+        scan([&](float x) {
+          if (!(x >= lowest)) return;
+          const u64 w = weight_at(x);
+          m += w;
+          const int at = bin_of(x);
+          if (at == 0) return;
+          atomicAdd(&sh.hist[at], 1u);
+          if (at >= kBins - kHeavy) atomicAdd(&sh.heavy[at - (kBins - kHeavy)], (uint32_t)(w >> 12));
+        });
+      } else if (weigh) {
         scan([&](float x) {
           const int at = bin_of(x);
           if (at == 0) return;

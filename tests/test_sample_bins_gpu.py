@@ -69,3 +69,25 @@ def test_more_survivors_than_a_list_holds(B):
             assert L.hbk_sample_filtered(r.data_ptr(), r.shape[1], temp.data_ptr(), seed.data_ptr(), tk.data_ptr(), tp.data_ptr(), o.data_ptr(), B, r.shape[1]) == 0
         torch.cuda.synchronize()
         assert torch.equal(out[0], out[1]), s
+
+
+@pytest.mark.parametrize("kind", ["bulk", "grid", "equal", "far", "nan", "inf"])
+@pytest.mark.parametrize("V", [8200, 32768])
+def test_cold_rows(kind, V):
+    """Nuclei of cold rows (bins for ten temperatures only, below 0.45): inside the bins, at their end, far below them."""
+    L = hb.lib()
+    f = lambda v, t: torch.tensor(v, device="cuda", dtype=t)  # noqa: E731
+    filters = [(t, p) for t in (0.02, 0.1, 0.3, 0.449, 0.45) for p in (0.3, 0.9, 0.9999, 0.99999, 0.9999999)]
+    B = len(filters)
+    x = rows(kind, B, V)
+    x[1::2, :40] -= 5  # (every other row without tokens that stand out)
+    wide = torch.full((B, V), -float("inf"), device="cuda")
+    wide[:, :8192] = x
+    temp, tp = (f([q[i] for q in filters], torch.float32) for i in (0, 1))
+    out = [torch.full((B,), -1, device="cuda", dtype=torch.int32) for _ in range(2)]
+    for s in range(10):
+        seed = torch.arange(B, device="cuda", dtype=torch.int64) * 7877 + s
+        for o, r in zip(out, (x, wide)):
+            assert L.hbk_sample_filtered(r.data_ptr(), r.shape[1], temp.data_ptr(), seed.data_ptr(), None, tp.data_ptr(), o.data_ptr(), B, r.shape[1]) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(out[0], out[1]), (s, [filters[i] for i in (out[0] != out[1]).nonzero().flatten().tolist()])
