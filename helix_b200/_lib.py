@@ -149,6 +149,7 @@ SIGNATURES = {
     "hbk_cls_pool_l2": (I, [P, P, P, I, I]),
     "hbk_attn_prefill": (I, [P, I, P, I, P, I, P, I, P, I, I, I, I, I, I, I, C.c_float]),
     "hbk_attn_prefill_paged": (I, [P, I, P, P, P, I, P, P, I, P, I, I, I, I, I, I, I, C.c_float, I]),
+    "hbk_attn_prefill_paged_with": (I, [P, I, P, P, P, I, P, P, I, P, I, I, I, I, I, I, C.c_float, I, I, I, C.c_float, I, P, P, I]),
     "hbk_attn_prefill_plan": (I, [I, I, I, I, I, I, I]),
     "hbk_attn_naive": (I, [P, I, P, I, P, I, P, I, P, I, I, I, I, I, I, I, C.c_float]),
     "hbk_attn_decode": (I, [P, I, P, P, P, I, P, P, I, P, I, I, I, I, I, I, C.c_float, I]),

@@ -300,6 +300,17 @@ int hbk_attn_prefill_paged(const void* q, int ldq, const void* k_cache, const vo
   a.page_table = page_table; a.max_pages = max_pages; a.kv_lens = kv_lens; a.num_pages = num_pages;
   return kret(hb::attn_prefill(0, a));
 }
+int hbk_attn_prefill_paged_with(const void* q, int ldq, const void* k_cache, const void* v_cache, const int32_t* page_table,
+                                int max_pages, const int32_t* kv_lens, void* out, int ldo, const int32_t* cu, int B, int T,
+                                int max_q_len, int Hq, int Hkv, int D, float scale, int num_pages, int window, int block_mask,
+                                float softcap, int unit_sink, const void* sink, const float* head_gate, int ldg) {
+  hb::AttnPrefillArgs a = mk_prefill(q, ldq, nullptr, 0, nullptr, 0, out, ldo, cu, B, T, max_q_len, Hq, Hkv, D, 1, scale);
+  a.k_cache = (const hb::bf16*)k_cache; a.v_cache = (const hb::bf16*)v_cache;
+  a.page_table = page_table; a.max_pages = max_pages; a.kv_lens = kv_lens; a.num_pages = num_pages;
+  a.window = window; a.block_mask = block_mask; a.softcap = softcap; a.unit_sink = unit_sink;
+  a.sink = (const hb::bf16*)sink; a.head_gate = head_gate; a.ldg = ldg;
+  return kret(hb::attn_prefill(0, a));
+}
 int hbk_attn_prefill_plan(int B, int T, int max_seqlen, int Hq, int Hkv, int paged, int sms) {
   if (B <= 0 || T <= 0 || max_seqlen <= 0 || Hkv <= 0 || Hq <= 0 || Hq % Hkv || sms <= 0) return -1;
   hb::AttnPrefillArgs a = mk_prefill(nullptr, 0, nullptr, 0, nullptr, 0, nullptr, 0, nullptr, B, T, max_seqlen, Hq, Hkv, 64, 1, 1.f);

@@ -60,6 +60,13 @@ int hbk_attn_prefill(const void* q, int ldq, const void* k, int ldk, const void*
 int hbk_attn_prefill_paged(const void* q, int ldq, const void* k_cache, const void* v_cache, const int32_t* page_table,
                            int max_pages, const int32_t* kv_lens, void* out, int ldo, const int32_t* cu_seqlens, int B,
                            int T, int max_q_len, int Hq, int Hkv, int D, int causal, float scale, int num_pages);
+/* the same, causal, with what layers add to it: window > 0: a position sees that many, itself included; block_mask > 0: those of its own
+ * block of so many positions; softcap > 0: scores pass softcap * tanh(s / softcap); unit_sink: one unit more in the denominator;
+ * sink [Hq] bf16 (or NULL): exp(sink[h]) more; head_gate fp32 [T, ldg] (or NULL): head h's result times sigmoid(head_gate[t][h]). */
+int hbk_attn_prefill_paged_with(const void* q, int ldq, const void* k_cache, const void* v_cache, const int32_t* page_table,
+                                int max_pages, const int32_t* kv_lens, void* out, int ldo, const int32_t* cu_seqlens, int B,
+                                int T, int max_q_len, int Hq, int Hkv, int D, float scale, int num_pages, int window,
+                                int block_mask, float softcap, int unit_sink, const void* sink, const float* head_gate, int ldg);
 /* how hbk_attn_prefill (paged 0) or hbk_attn_prefill_paged (1) cuts a launch of these sizes on `sms` SMs: query heads of a kv head that
  * share the rows of a tile, + 256 where the items are sorted by length.  Host arithmetic only; -1 for sizes that are refused. */
 int hbk_attn_prefill_plan(int B, int T, int max_seqlen, int Hq, int Hkv, int paged, int sms);

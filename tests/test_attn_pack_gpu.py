@@ -1,5 +1,5 @@
 """Prefill attention with the query heads of a kv head packed into a tile's rows: groups of every size (powers of two, others, single heads),
-lengths around a tile's tokens for each packing, packed and paged keys, heads with gates and sinks of their own."""
+lengths around a tile's tokens for each packing, packed and paged keys, heads with gates and sinks of their own, windows, blocks and capped scores."""
 import math
 
 import pytest
@@ -70,6 +70,48 @@ def test_pages(Hq, Hkv, D, rows, ctx):
         kk, vv = (t[table[b, :n].long()].permute(0, 2, 1, 3).reshape(-1, Hkv, D)[:ctx[b]].float() for t in (k, v))
         w = want(q[b * rows:(b + 1) * rows].float().view(rows, Hq, D), kk, vv, ctx[b] - rows, D ** -0.5).reshape(rows, -1)
         assert (out[b * rows:(b + 1) * rows].float() - w).abs().max() < 2 * 5 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(3, 3), (12, 2), (32, 8), (16, 1)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("rows,ctx", [(33, [33, 97, 400]), (129, [129, 700, 1000]), (300, [300, 2100])])
+@pytest.mark.parametrize("opts", [dict(window=1), dict(window=64, sink=1), dict(window=150, softcap=5.0), dict(block=50, unit=1, gate=1), dict(block=64, sink=1),
+                                  dict(softcap=2.0, gate=1), dict(unit=1, sink=1, gate=1)], ids=str)
+def test_what_layers_add(opts, rows, ctx, D, Hq, Hkv):
+    """Windows, blocks, capped scores, sinks and gates over pages; each query head has its own sink and gates."""
+    L, B = hb.lib(), len(ctx)
+    assert L.hbk_init() == 0
+    window, block, cap, unit = (opts.get(k, 0) for k in ("window", "block", "softcap", "unit"))
+    g = torch.Generator(device="cuda").manual_seed(rows + Hq + D)
+    pages = [(c + 63) // 64 for c in ctx]
+    table = torch.zeros((B, max(pages)), device="cuda", dtype=torch.int32)
+    perm, at = torch.randperm(sum(pages), generator=g, device="cuda").to(torch.int32), 0
+    for i, n in enumerate(pages):
+        table[i, :n] = perm[at:at + n]
+        at += n
+    k, v = (torch.randn((sum(pages), Hkv, 64, D), generator=g, device="cuda").to(BF) for _ in range(2))
+    q = torch.randn((B * rows, Hq * D), generator=g, device="cuda").to(BF)
+    sink = torch.randn(Hq, generator=g, device="cuda").mul(2).to(BF) if opts.get("sink") else None
+    gate = torch.randn((B * rows, Hq + 5), generator=g, device="cuda") if opts.get("gate") else None
+    out, p = torch.full((B * rows, Hq * D), float("nan"), device="cuda", dtype=BF), lambda t: None if t is None else t.data_ptr()
+    lens, cu = torch.tensor(ctx, device="cuda", dtype=torch.int32), torch.arange(B + 1, device="cuda", dtype=torch.int32) * rows
+    assert L.hbk_attn_prefill_paged_with(p(q), Hq * D, p(k), p(v), p(table), table.shape[1], p(lens), p(out), Hq * D, p(cu), B, B * rows, rows, Hq, Hkv, D, D ** -0.5,
+                                         sum(pages), window, block, cap, unit, p(sink), p(gate), Hq + 5) == 0
+    torch.cuda.synchronize()
+    for b in range(B):
+        kk, vv = (t[table[b, :pages[b]].long()].permute(0, 2, 1, 3).reshape(-1, Hkv, D)[:ctx[b]].float().repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+        s = torch.einsum("nhd,mhd->hnm", q[b * rows:(b + 1) * rows].float().view(rows, Hq, D), kk) * D ** -0.5
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        i, j = torch.arange(ctx[b] - rows, ctx[b], device="cuda")[:, None], torch.arange(ctx[b], device="cuda")[None]
+        seen = (j <= i) & (j > i - window if window else True) & (j >= i // block * block if block else True)
+        e = torch.exp(s.masked_fill(~seen, -math.inf))
+        extra = unit + (torch.exp(sink.float())[:, None, None] if sink is not None else 0)
+        w = torch.einsum("hnm,mhd->nhd", e / (e.sum(-1, keepdim=True) + extra), vv)
+        if gate is not None:
+            w = w * torch.sigmoid(gate[b * rows:(b + 1) * rows, :Hq, None])
+        # averages of unit normals: bf16 probabilities (2^-9 of a value below 5) and one bf16 rounding of the result
+        assert (out[b * rows:(b + 1) * rows].float() - w.reshape(rows, -1)).abs().max() < 2 * 5 * 2.0 ** -9
 
 
 @pytest.mark.parametrize("Hq,Hkv", [(32, 8), (16, 1), (12, 2)])
