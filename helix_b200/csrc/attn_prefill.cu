@@ -495,7 +495,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const int qpos = qt0 + (r >> pack);
       const bool live = it.q0 + t * BQ + r < it.len;  // the row exists
       const int token = it.seq0 + ((it.q0 + t * BQ + r) >> pack), head = (it.h << pack) + (r & ((1 << pack) - 1));
-      const int turns = min(it.n0, it.n1);  // tiles that both q tiles have
+      const int turns = DK <= 128 ? min(it.n0, it.n1) : 0;  // tiles that both q tiles have
       float m_used = -1e30f, l = 0.f;  // (rows that see nothing yet: far below every score, and finite)
       for (int j = 0; j < nt; ++j) {
         const int tile = jt + j;
@@ -589,7 +589,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // They stay for the results: the logits of a 16-layer decoder, 5 prompts x 32 steps, have the same rms error (0.02061 | 0.02057), but other single
         // errors, and with the SFU alone the largest ones pass what the full-size tests allow.
         // Every turn is waited for, the first one of an item too: a warp that passed on its turn twice before the other had taken the first would
-        // complete the barrier by itself.
+        // complete the barrier by itself.  Keys of 192 columns take no turns (with | without: 16 heads, 512 rows over 6000 expanded keys 119 | 99 us, 2048 rows of
+        // their own keys 50 | 46); of 128 they do (2 x 1500 rows with a window of 512, before the turns 45.5, with them 43.7).
         if (j < turns && (t == 1 || passed)) bar_sync((t ? 5 : 1) + qd, 64);
         const uint64_t scale2 = f2_pack(sl2, sl2), negm2 = f2_pack(-m_used, -m_used);
         uint64_t sum2a = 0, sum2b = 0;
