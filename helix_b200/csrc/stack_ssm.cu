@@ -772,6 +772,7 @@ __device__ __forceinline__ void st_pair(float* f, bf16* b, float4 v) {
     *reinterpret_cast<uint2*>(b) = pk;
   }
 }
+__device__ __forceinline__ float sum_of_squares(float4 v) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x))); }
 // one block per (part, token)
 template <typename WT>
 __global__ void __launch_bounds__(256) gated_group_norm_kernel(const float* __restrict__ y, long ldy, const float* __restrict__ z, long ldz,
@@ -818,7 +819,8 @@ __global__ void __launch_bounds__(256) gated_group_norm_kernel(const float* __re
   }
 }
 
-// Parts of up to 1024 entries: a warp each, no barrier, and no idle half of a block (a block per part of 512 entries: 11k tokens x 8 parts 185 -> 83 us)
+// Many parts of up to 512 entries: a warp each, no barrier, and no idle half of a block (a block per part of 512 entries: 11k tokens x 8 parts 185 -> 83
+// us).  The sum is the block's below, where warp c has 128 entries: a sum for each 128, added in the order of block_sum, so the two give the same bits.
 template <typename WT, int CH>
 __global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const float* __restrict__ y, long ldy, const float* __restrict__ z, const bf16* __restrict__ zb, long ldz,
                                                                     const WT* __restrict__ w, float eps, int parts, float* __restrict__ out,
@@ -831,8 +833,9 @@ __global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const float*
   const float* ys = y + (size_t)t * ldy + c0;
   const float* zs = z ? z + (size_t)t * ldz + c0 : nullptr;
   const bf16* zbs = zb ? zb + (size_t)t * ldz + c0 : nullptr;
+  static_assert(CH <= 4, "the order of four sums");
   float4 u[CH], g[CH];
-  float ss = 0.f;
+  float ss[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     const int i = (lane + c * 32) * 4;
@@ -846,9 +849,9 @@ __global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const float*
     const float4 s = make_float4(sigmoidf_(g[c].x), sigmoidf_(g[c].y), sigmoidf_(g[c].z), sigmoidf_(g[c].w));
     if (!gate_last) u[c] = make_float4(u[c].x * (g[c].x * s.x), u[c].y * (g[c].y * s.y), u[c].z * (g[c].z * s.z), u[c].w * (g[c].w * s.w));
     g[c] = gate_last ? s : make_float4(1.f, 1.f, 1.f, 1.f);
-    ss += u[c].x * u[c].x + u[c].y * u[c].y + u[c].z * u[c].z + u[c].w * u[c].w;
+    ss[c] = warp_sum(sum_of_squares(u[c]));
   }
-  const float rs = 1.f / sqrtf(warp_sum(ss) / (float)len + eps);
+  const float rs = 1.f / sqrtf(((ss[0] + ss[2]) + (ss[1] + ss[3])) / (float)len + eps);
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     const int i = (lane + c * 32) * 4;
@@ -868,7 +871,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
   __shared__ float red[32];
   pdl_launch_dependents();
   pdl_wait();
-  const int t = blockIdx.y, part = blockIdx.x, len = n / parts, c0 = part * len;
+  const int t = blockIdx.x, part = blockIdx.y, len = n / parts, c0 = part * len;
   const float* ys = y + (size_t)t * ldy + c0;
   const float* zs = z ? z + (size_t)t * ldz + c0 : nullptr;
   const bf16* zbs = zb ? zb + (size_t)t * ldz + c0 : nullptr;
@@ -887,7 +890,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
     const float4 s = make_float4(sigmoidf_(g[c].x), sigmoidf_(g[c].y), sigmoidf_(g[c].z), sigmoidf_(g[c].w));
     if (!gate_last) u[c] = make_float4(u[c].x * (g[c].x * s.x), u[c].y * (g[c].y * s.y), u[c].z * (g[c].z * s.z), u[c].w * (g[c].w * s.w));
     g[c] = gate_last ? s : make_float4(1.f, 1.f, 1.f, 1.f);
-    ss += u[c].x * u[c].x + u[c].y * u[c].y + u[c].z * u[c].z + u[c].w * u[c].w;
+    ss += sum_of_squares(u[c]);
   }
   const float rs = 1.f / sqrtf(block_sum(ss, red) / (float)len + eps);
 #pragma unroll
@@ -1167,10 +1170,12 @@ cudaError_t gated_group_norm(cudaStream_t s, const float* y, long ldy, const flo
   const int len = n / parts;
   if (len % 4 == 0 && len <= 8192 && ((ldy | ldz) & 3) == 0 && (((uintptr_t)y | (uintptr_t)z | (uintptr_t)out) & 15) == 0 && (((uintptr_t)outb | (uintptr_t)zb) & 7) == 0) {
 #define HB_GGN(WT, CH) \
-  return launch_k(gated_group_norm_vec_kernel<WT, CH>, grid, dim3(256), 0, s, true, y, ldy, z, zb, ldz, (const WT*)w, eps, parts, out, outb, n, (int)gate_last)
+  return launch_k(gated_group_norm_vec_kernel<WT, CH>, dim3(T, parts), dim3(256), 0, s, true, y, ldy, z, zb, ldz, (const WT*)w, eps, parts, out, outb, n, (int)gate_last)
 #define HB_GGN_T(CH) do { if (f32) HB_GGN(float, CH); else HB_GGN(bf16, CH); } while (0)
-    if (len <= 1024) {
-      if ((long)T * parts > INT_MAX) return cudaErrorInvalidValue;
+    // Fewer parts than the blocks that fit the machine are through sooner with a block each (us block | warp: 16 tokens x 8 parts of 512 entries 2.4 | 4.2, of
+    // 256 2.4 | 3.0, 64 tokens 3.3 | 4.3 and 3.0 | 3.1, 300 tokens 6.6 | 6.0 and 6.2 | 4.3; of 128 2.7 | 2.4 at 16 tokens), wide parts always (2000 tokens x 4
+    // parts of 1024 21 | 24)
+    if (len <= 512 && (len <= 128 || (long)T * parts > 8 * effective_sms(148)) && (long)T * parts <= INT_MAX) {
       const int items = T * parts;
 #define HB_GGW(WT, CH)                                                                                                                                        \
   return launch_k(gated_group_norm_warp_kernel<WT, CH>, dim3((items + 7) / 8), dim3(256), 0, s, true, y, ldy, z, zb, ldz, (const WT*)w, eps, parts, out, outb, \
@@ -1178,12 +1183,12 @@ cudaError_t gated_group_norm(cudaStream_t s, const float* y, long ldy, const flo
 #define HB_GGW_T(CH) do { if (f32) HB_GGW(float, CH); else HB_GGW(bf16, CH); } while (0)
       if (len <= 128) HB_GGW_T(1);
       if (len <= 256) HB_GGW_T(2);
-      if (len <= 512) HB_GGW_T(4);
-      HB_GGW_T(8);
+      HB_GGW_T(4);
 #undef HB_GGW_T
 #undef HB_GGW
     }
-    if (len <= 2048) HB_GGN_T(2);
+    if (len <= 1024) HB_GGN_T(1);
+    else if (len <= 2048) HB_GGN_T(2);
     else if (len <= 4096) HB_GGN_T(4);
     else HB_GGN_T(8);
 #undef HB_GGN_T

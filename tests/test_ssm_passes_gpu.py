@@ -42,3 +42,17 @@ def test_group_norm_parts(heads, vdim, groups):
         got = e.seq_step([(e.seq_open(), toks, list(range(21)))])
     # the exact mode's bound of the design's tests
     assert (np.sqrt(((got - want) ** 2).mean(-1)) / np.sqrt((want ** 2).mean(-1))).max() < 2e-4
+
+
+@pytest.mark.parametrize("heads,vdim,groups", [(8, 64, 8), (9, 96, 8), (8, 132, 8), (16, 128, 8), (16, 256, 8), (16, 260, 8)])
+def test_group_norm_parts_by_warps_and_blocks(heads, vdim, groups):
+    """400 tokens in one step (a warp per part of up to 512 entries) against portions of 40 (a block per part): the same bits (exact mode)."""
+    l = E.LayerDesc(mixer=E.MIXER_MAMBA2, heads=heads, vdim=vdim, dim=8, kv_heads=1, norm_groups=groups, conv_taps=2)
+    d = E.StackDesc(width=64, vocab=128, layers=[l], compute_f32=1, norm_eps=1e-5, norm_place=E.NORM_PARALLEL, embed_norm=1, plain_gains=1, tie_head=1)
+    toks = np.random.default_rng(vdim).integers(0, 128, 400).tolist()
+    with hb.Engine(hb.EngineConfig(max_seqs=2, max_ctx=448, max_batched_tokens=448, kv_pool_tokens=896)) as e:
+        e.load_random(d, 19)
+        want = e.seq_step([(e.seq_open(), toks, list(range(400)))])
+        s = e.seq_open()
+        got = np.concatenate([e.seq_step([(s, toks[i:i + 40], list(range(40)))]) for i in range(0, 400, 40)])
+    assert np.isfinite(want).all() and np.array_equal(got, want)
