@@ -613,10 +613,14 @@ __global__ void __launch_bounds__(32 * W, MB) lin_portion_kernel(LinRecArgs a) {
       *reinterpret_cast<float4*>(st + (size_t)(2 * i + 1) * a.Dv + e) = make_float4(S[e][i].y, S[e + 1][i].y, S[e + 2][i].y, S[e + 3][i].y);
     }
 }
-// (portions of up to eight tokens on average are bound by the state's bytes, which the smaller pieces above have more of in flight: 32 sequences of 5 to
-// 10 tokens x 32 heads of 128 x 64 states 31 us there, 33 here)
+// Narrower blocks where the wide ones are no more than the SMs (us wide / narrow: one sequence of 2048 tokens x 64 heads of 128 x 64 states
+// 492 / 383, four of 500 to 1000 316 / 361; 32 heads of 256 x 40 125 / 92)
+bool lin_portion_narrow(const LinRecArgs& a) { return a.Dk <= 64 || (long)a.B * a.H * ((a.Dv + 63) / 64) <= effective_sms(148); }
+// Short portions are bound by the state's bytes, which the smaller pieces above have more of in flight: from more than eight tokens on average on narrow blocks, 24 on
+// wide ones (us there | here, 32 sequences x 32 heads of 128 x 64 states: of 5 to 10 tokens 31 | 33, of 9 27 | 30, of 12 31 | 33, of 40 70 | 67; 8 sequences of 20
+// 19.4 | 20.2; 32 of 9 with 4 heads of 256 x 256 31 | 34; narrow, 8 of 9 with 4 heads of 256 x 256 15.6 | 12.5, 32 heads of 64 x 64 9.5 | 9.6)
 bool lin_portion_ok(const LinRecArgs& a) {
-  return !a.nq && a.T > 8 * a.B && a.Dk > 32 && a.Dv > 32 && ((a.Dk | a.Dv | (int)a.ldq | (int)a.ldk | (int)a.ldv | a.q_off | a.k_off | a.v_off) & 3) == 0 &&
+  return !a.nq && a.T > (lin_portion_narrow(a) ? 8 : 24) * a.B && a.Dk > 32 && a.Dv > 32 && ((a.Dk | a.Dv | (int)a.ldq | (int)a.ldk | (int)a.ldv | a.q_off | a.k_off | a.v_off) & 3) == 0 &&
          ((a.slot_stride | (long)a.s_off) & 3) == 0 && (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.state) & 15) == 0;
 }
 template <int DKP, int CH, int W>
@@ -1126,15 +1130,13 @@ cudaError_t lin_recurrence(cudaStream_t s, const LinRecArgs& a) {
   if (a.G <= 0 || a.H % a.G || a.Dk > 256 || a.Dk <= 0) return cudaErrorInvalidValue;
   if (lin_step_ok(a)) return launch_k(lin_step_kernel, dim3(a.B, a.H, (a.Dv + 63) / 64), dim3((a.Dk + 15) / 16 * 32), 0, s, true, a);
   if (lin_portion_ok(a)) {
-    // narrower blocks where the wide ones are no more than the SMs (us wide / narrow: one sequence of 2048 tokens x 64 heads of 128 x 64 states
-    // 492 / 383, four of 500 to 1000 316 / 361; 32 heads of 256 x 40 125 / 92)
-    const bool few = (long)a.B * a.H * ((a.Dv + 63) / 64) <= effective_sms(148);
+    const bool few = lin_portion_narrow(a);
     if (a.Dk <= 64) return launch_portion<64, 8, 4, 5>(s, a);
     if (a.Dk <= 128) return few ? launch_portion<128, 8, 4, 5>(s, a) : launch_portion<128, 16, 4, 4>(s, a);
     return few ? launch_portion<256, 16, 4, 4>(s, a) : launch_portion<256, 16, 8, 2>(s, a);
   }
   // two columns per lane (blocks of 64 columns) halve the shared-memory reads per product; heads of up to 32 value columns
-  // keep one.  HB_REC_COLS=1 forces the narrow blocks (A/B measurements)
+  // keep one.  HB_REC_COLS=1 forces the narrow blocks of this kernel (A/B measurements)
   // (the arithmetic per column is the same either way, so the choice never shows in a result; narrow blocks for small grids
   // measured no faster)
   static const bool narrow = [] { const char* e = getenv("HB_REC_COLS"); return e && atoi(e) == 1; }();
