@@ -583,11 +583,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (t == 0 && warp == 3 && lane == 0) HB_TRACE(4);  // loaded, max, rescale decision done
         // The q tiles' warps of a quarter of the SM take turns with the exponentials (barriers 1 + qd: tile 0's turn, 5 + qd: tile 1's).  Left to
         // themselves both worked on their exponentials at the same time and waited for scores, loads and barriers at the same time: a kv
-        // tile took 2000 cycles, 1620 with the SFU alone (8 cycles per instruction of a warp, 504 of a turn of 680).  Two of eight pairs as
-        // polynomials (kPolyPairs) cost a little more than they save now that there are turns: all on the SFU | so, 6 prompts of 300 to 3000 tokens with 32
-        // heads over 8 184 | 187 us (64 columns 154 | 162), 64 chunks of 64 to 512 tokens 62 | 64, 100 rows over 4000 keys, whose q tiles have no partner, 57 | 55.
-        // They stay for the results: the logits of a 16-layer decoder, 5 prompts x 32 steps, have the same rms error (0.02061 | 0.02057), but other single
-        // errors, and with the SFU alone the largest ones pass what the full-size tests allow.
+        // tile took 2000 cycles, 1580 now, of which the SFU has 2 x 48 exponentials of 8 cycles.  Two of eight pairs are polynomials (kPolyPairs), which costs a
+        // little more than it saves now that there are turns: all on the SFU | so, 6 prompts of 300 to 3000 tokens with 32 heads over 8 184 | 187 us (64
+        // columns 154 | 162), 64 chunks of 64 to 512 tokens 62 | 64, 100 rows over 4000 keys, whose q tiles have no partner, 57 | 55.  They stay for the results:
+        // the logits of a 16-layer decoder, 5 prompts x 32 steps, have the same rms error (0.02061 | 0.02057), but other single errors, and with the SFU alone
+        // the largest ones exceed what the full-size tests allow.
         // Every turn is waited for, the first one of an item too: a warp that passed on its turn twice before the other had taken the first would
         // complete the barrier by itself.  Keys of 192 columns take no turns (with | without: 16 heads, 512 rows over 6000 expanded keys 119 | 99 us, 2048 rows of
         // their own keys 50 | 46); of 128 they do (2 x 1500 rows with a window of 512, before the turns 45.5, with them 43.7).

@@ -1674,9 +1674,9 @@ cudaError_t launch_voc(K* kernel, int ctas, bool on_chip, cudaStream_t s, int B,
 }
 // Blocks per row: one up to `whole` columns; else as many (at most `most`) as let the machine hold every row's blocks at once (33
 // clusters of eight), but enough that two blocks fit an SM (parts of `part` columns).  Every shape gives the same tokens.  Us with 1 / 2 / 4 / 8 blocks per row:
-//   top_p 0.95   48 rows of 32768  57 / 49 / 42 / 65     128 of 16384  50 / 39 / 62 / 116    256 of 8192    34 / 57 / 97 / 200   (before the bins)
+//   top_p 0.95   48 rows of 32768  33 / 28 / 25 / 38     128 of 16384  27 / 24 / 39 / 71     16 of 12000     17 / 18 / 18 / 18
+//                32 rows of 128256  - /  - / 38 / 35      96 of 65536   - / 66 / 55 / 71      256 of 128256  - /  - / 281 / 242
 //   width 6      48 rows of 50000   - / 14 / 13 / 25     128 of 32768  12 / 13 / 24 / 47     256 of 8192   8.5 / 18 / 38 / 87
-//   top_p 0.95   32 rows of 128256  - /  - / 66 / 72      96 of 65536   - / 126 / 97 / 148   256 of 128256  - /  - / 510 / 512
 // (clusters of eight run 33 at a time whatever their size, which left 256 rows of 1000 to 8192 columns at 20 to 50 % of the speed
 // of the block per row that these kernels had replaced).
 int voc_ctas(int B, int V, int whole, int most, int part) {

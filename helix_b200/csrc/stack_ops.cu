@@ -64,9 +64,9 @@ __global__ void __launch_bounds__(256) gemm_rt_kernel(const float* __restrict__ 
 }
 
 // The same product for fp32 operands whose rows along k are 16-byte pieces (every product of the exact mode at sizes that are multiples
-// of four and of more than 64 terms): for prompts bound by the FMA pipe (a packed FMA with three different operands takes 2.3 cycles of a quarter of
-// an SM, 62 TFLOP/s) and by what else the warps issue: half of all instructions made addresses for the copies (30 TFLOP/s) until each
-// thread kept to one 16-byte column of the stage and walked the rows by a stride, 42 since; for single tokens by the weights' bytes, where the kernel
+// of four and of more than 64 terms): for prompts bound by the FMA pipe (active 62 % of the cycles) and by what else the warps issue: half of all
+// instructions made addresses for the copies (30 TFLOP/s) until each thread kept to one 16-byte column of the stage and walked the rows by a
+// stride, 39 to 45 since; for single tokens by the weights' bytes, where the kernel
 // above was bound by scalar loads with no copies in flight and one thread per sum of K terms.
 // K is cut into kRtParts equal parts; a group of threads per part keeps its own stages of cp.async copies and the groups' sums
 // are added in order of k at the end; inside a part even and odd k have a sum each (packed FMAs on register pairs as they are

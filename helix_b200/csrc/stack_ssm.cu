@@ -430,12 +430,12 @@ __global__ void __launch_bounds__(DKP * 2, 512 / DKP) lin_recurrence_kernel(LinR
 
 // Portions without a normaliser: the same arithmetic (state elements, channel sums of eight, their sums pair by pair: the same bits as the
 // kernel above and the single-token one) in larger pieces.  A lane keeps CH channels of kPortionCols neighbouring columns, LS = DKP / CH lanes
-// share the columns.  What bounds it is the rate of packed products with three different operands (2.3 cycles each on a quarter of an SM, so
-// 220 per token for a block of 128 x 64 states), and close behind shared memory: a read hands a lane 16 bytes, 512 a warp, at 128 bytes a cycle
+// share the columns.  What bounds it is the FMA pipe (active 68 % of the cycles, and what warps wait for first), and close behind shared memory: a read
+// hands a lane 16 bytes, 512 a warp, at 128 bytes a cycle
 // whoever shares the address, so q and k have to serve four columns each (two columns per lane, as above, take 84 cycles per warp and token,
 // four 45).  Tokens go in pairs, so that the 8 sums of a lane fold over the LS lanes with all of them useful and one
 // token's products cover the other's shuffles; one barrier per 16 tokens, no partial sums in shared memory.  Entries are taken longest first.
-// Prompts of 700 to 2048 tokens, 8 sequences x 64 heads of 128 x 64 states: 1670 -> 1030 us (320 cycles per token and head on a full SM, 430 before);
+// Prompts of 700 to 2048 tokens, 8 sequences x 64 heads of 128 x 64 states: 1670 -> 1030 us (327 active cycles of an SM per token and head);
 // one sequence of 2048 723 -> 383; 32 heads of 64 x 64, 8 sequences 237 -> 125.
 constexpr int kPortionCols = 4;
 // Sums of r[0 .. CNT) over LS lanes, neighbours first: while a lane has several it gives half of them away, so that lane s ends up with the sum `at`.
