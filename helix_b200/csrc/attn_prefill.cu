@@ -884,14 +884,16 @@ cudaError_t attn_prefill(cudaStream_t stream, const AttnPrefillArgs& a) {
   if ((a.ldq % 8) || (a.ldo % 8) || (!paged && ((a.ldk % 8) || (a.ldv % 8)))) return cudaErrorInvalidValue;
   if (a.block_mask < 0 || (a.block_mask > 0 && (!paged || !a.causal))) return cudaErrorInvalidValue;
   if (a.window < 0 || (a.window > 0 && (!paged || !a.causal || a.block_mask > 0))) return cudaErrorInvalidValue;
+  const int sms = effective_sms(device_sms());
+  if (sms <= 0) return cudaErrorNoDevice;
   if (paged) {
     if (!a.v_cache || !a.page_table || !a.kv_lens || a.max_pages <= 0 || a.num_pages <= 0 || a.page_size != 64) return cudaErrorInvalidValue;
-    const int pack = attn_prefill_plan(a, effective_sms(device_sms())).pack;
+    const int pack = attn_prefill_plan(a, sms).pack;
     if (a.D == 128) return launch<128, true, false>(stream, a, pack);
     if (a.D == 64) return launch<64, true, false>(stream, a, pack);
     return cudaErrorInvalidValue;
   }
-  const auto [pack, sorted] = attn_prefill_plan(a, effective_sms(device_sms()));
+  const auto [pack, sorted] = attn_prefill_plan(a, sms);
   if (a.D == 128) return sorted ? launch<128, false, true>(stream, a, pack) : launch<128, false, false>(stream, a, pack);
   if (a.D == 64) return sorted ? launch<64, false, true>(stream, a, pack) : launch<64, false, false>(stream, a, pack);
   return cudaErrorInvalidValue;

@@ -1,5 +1,8 @@
 """How prefill attention cuts a launch (host arithmetic): heads that share a tile's rows, and the order of the items."""
+import os
 import random
+import subprocess
+import sys
 
 import pytest
 
@@ -49,3 +52,12 @@ def test_launches_sorted_with_heads_apart_are_sorted_packed():
         assert (hq // hkv) % heads == 0 and ordered and longest * heads <= 65280 and sum(lens) * heads // 256 + len(lens) <= 512, (lens, hq, hkv)
         seen += 1
     assert seen > 500
+
+
+def test_no_device_is_an_error():
+    """The entries answer with an error where there is no device.  (The output's address, off by 8 bytes, is refused on the host where there is one.)"""
+    code = ("import helix_b200 as hb; L = hb.load_library(); "
+            "a = L.hbk_attn_prefill(16, 256, 16, 256, 16, 256, 8, 256, 16, 1, 10, 10, 2, 2, 64, 1, 0.1); "
+            "b = L.hbk_attn_prefill_paged(16, 256, 16, 16, 16, 1, 16, 8, 256, 16, 1, 10, 10, 2, 2, 64, 1, 0.1, 1); print(a, b)")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0 and all(int(x) != 0 for x in r.stdout.split()), (r.returncode, r.stdout)
