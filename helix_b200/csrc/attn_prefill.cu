@@ -227,15 +227,16 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   }
   // Order of the items (SORTED): rows (q pair, sequence) by falling number of kv tiles, a row's heads side by side (they share keys), dealt
   // to the CTAs forth and back (round r of CTA c is item r G + c, or r G + G - 1 - c in odd rounds).  Every CTA sorts the rows itself
-  // (ranks by counting, about a microsecond).  With sequences of unequal length the plain order, q pair by q pair with a slot
+  // (a thread per row, ranks by counting four keys a read; a thread per sequence that walked its rows, and one key a read, cost 2 us more: 6 prompts of 300 to 3000
+  // tokens, 64 columns 158.7 -> 156.6).  With sequences of unequal length the plain order, q pair by q pair with a slot
   // for every sequence whether it has that pair or not, left the longest-loaded CTA 24 to 30 % above the mean (6 prompts of 300
   // to 3000 tokens: 231 tile times of a mean of 187, now 191; 64 chunks of 64 to 512: 74 of 57, now 60).  Measured: 250 -> 233 us and 70.8 -> 62.6 us.
   // Everything else runs the kernel with the plain walk: launches whose sequences are short or of about equal lengths (wants_order below), and
   // keys from a page pool or an expanded run (portions of a long context are level already).  The plain order also stands in where a
   // launch turns out to have more rows than kMaxRows.
   if constexpr (SORTED) {
-    uint32_t* keys = reinterpret_cast<uint32_t*>(sK);            // scratch over the K ring (nothing has been loaded yet)
-    uint16_t* ids = reinterpret_cast<uint16_t*>(keys + kMaxRows);
+    uint32_t* keys = reinterpret_cast<uint32_t*>(sK);  // scratch over the K ring (nothing has been loaded yet): [kMaxRows] keys, first row of each sequence
+    int* starts = reinterpret_cast<int*>(keys + kMaxRows);
     const int b = threadIdx.x;
     Item it;
     int pairs = 0;
@@ -252,23 +253,39 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     if (lane == 31) s_rows[1 + warp] = upto;
     __syncthreads();
     int before = 0, rows = 0;
+#pragma unroll
     for (int w = 0; w < kThreads / 32; ++w) {
-      if (w < warp) before += s_rows[1 + w];
-      rows += s_rows[1 + w];
+      const int v = s_rows[1 + w];
+      if (w < warp) before += v;
+      rows += v;
     }
     if (rows <= kMaxRows) {
-      for (int qp = 0; qp < pairs; ++qp) {
-        const int r = before + upto - pairs + qp;
-        set_pair(it, qp);
-        keys[r] = (uint32_t)(3 * it.n + min(it.n0, it.n1) + 6) * kMaxRows + (kMaxRows - 1 - r);  // (a lone q tile takes about 3/4 of a pair's time)
-        ids[r] = (uint16_t)(qp << 8 | b);
+      if (b < B) starts[b] = before + upto - pairs;
+      __syncthreads();
+      for (int r = threadIdx.x; r < (rows + 3) / 4 * 4; r += kThreads) {
+        uint32_t key = 0;  // (no row: nothing is behind it)
+        if (r < rows) {
+          int q = 0;  // the last sequence that starts at or before row r
+          for (int step = 128; step > 0; step >>= 1)
+            if (q + step < B && starts[q + step] <= r) q += step;
+          set_seq(it, q);
+          set_pair(it, r - starts[q]);
+          key = (uint32_t)(3 * it.n + min(it.n0, it.n1) + 6) * kMaxRows + (kMaxRows - 1 - r);  // (a lone q tile takes about 3/4 of a pair's time)
+        }
+        keys[r] = key;
       }
       __syncthreads();
       for (int r = threadIdx.x; r < rows; r += kThreads) {
         const uint32_t key = keys[r];
-        int rank = 0;
-        for (int i = 0; i < rows; ++i) rank += keys[i] > key;
-        s_order[rank] = ids[r];
+        int rank = 0, q = 0;
+#pragma unroll 8
+        for (int i = 0; i < (rows + 3) / 4; ++i) {
+          const uint4 k4 = reinterpret_cast<const uint4*>(keys)[i];
+          rank += (k4.x > key) + (k4.y > key) + (k4.z > key) + (k4.w > key);
+        }
+        for (int step = 128; step > 0; step >>= 1)
+          if (q + step < B && starts[q + step] <= r) q += step;
+        s_order[rank] = (uint16_t)((r - starts[q]) << 8 | q);
       }
       fence_proxy_async_smem();  // the scratch becomes a target of asynchronous copies
     }
