@@ -1,6 +1,7 @@
 // K5: varlen flash attention for prefill (causal, GQA) and for the BERT encoder
 // (bidirectional), on tcgen05 tensor cores with S, P and the output accumulator O all resident in TMEM.
 // See the kernel comment for the warp roles and the two-q-tile ping-pong schedule.
+#include <limits.h>
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -74,6 +75,18 @@ __device__ int g_attn_trace_n[8];
 #define HB_TRACE(ev) do {} while (0)
 #endif
 
+// The walk of a launch's items: q pair by q pair, the same with its last round as lone q tiles, or sorted by kv tiles (below)
+enum Order : int { ORDER_PLAIN = 0, ORDER_SPLIT = 1, ORDER_SORTED = 2 };
+// Split walk: the pairs from this one on, those of the last round, are taken as two lone q tiles each, where twice as many of them are no more than
+// there are CTAs (elsewhere the answer is `pairs`): a lone q tile takes about 3/4 of a pair's time, and the SMs that would have had nothing take the other
+// ones.  us, 32 heads over 8 of 128 columns: 777 x 2 rows over 6000 keys 173 -> 163 (64 columns 163 -> 150), 512 over 2500 46 -> 40; 12 heads of their own,
+// 333 x 2 over 4500 71 -> 62
+// An instance of its own: the walk's few registers in the plain one cost every other launch 2 % (2048 rows over 7000 191.5 -> 196.5).
+__host__ __device__ inline int first_split(int pairs, int ctas) {
+  const int full = (pairs - 1) / ctas * ctas;
+  return 2 * (pairs - full) <= ctas ? full : pairs;
+}
+
 // Where K and V rows come from: the packed activation, the paged planes, or (latent attention) expanded rows — per-head key and
 // value parts made from cached latents plus one rotated key part that all heads share.
 enum KvSource : int { KV_PACKED = 0, KV_PAGED = 1, KV_EXPANDED = 2 };
@@ -121,7 +134,7 @@ struct ACfg {
 //                [row0, row0 + kv) of the expanded buffers).  A q / k row has DK / 64 sub-tiles: the head's unrotated part in
 //                all but the last, the rotated part (shared by all heads on the key side) in the last; parts that are no
 //                multiple of 64 wide are zero-filled by the tensor maps.
-template <int DK, int DV, int SRC, bool SORTED>
+template <int DK, int DV, int SRC, int ORDER>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o,
@@ -133,7 +146,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const __grid_constant__ CUtensorMap map_qr, const __grid_constant__ CUtensorMap map_kr,
                     const __grid_constant__ AttnRuns runs, int vdim, int pack) {
   using C = ACfg<DK, DV, SRC>;
-  constexpr bool PAGED = SRC == KV_PAGED, EXPANDED = SRC == KV_EXPANDED;
+  constexpr bool PAGED = SRC == KV_PAGED, EXPANDED = SRC == KV_EXPANDED, SORTED = ORDER == ORDER_SORTED;
   constexpr int KST = C::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -180,11 +193,11 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     it.q_off = it.kv_len - it.len;  // position of the first q row (0 unless this is a later chunk of a long prompt)
     if constexpr (!EXPANDED) it.len <<= pack;
   };
-  auto set_pair = [&](Item& it, int qp) {
-    it.q0 = qp * QPAIR;
+  auto set_rows = [&](Item& it, int q0, bool both) {
+    it.q0 = q0;
     it.valid = it.q0 < it.len;
     const int kv_tiles = (it.kv_len + BKV - 1) / BKV;
-    it.act1 = it.q0 + BQ < it.len;
+    it.act1 = both && it.q0 + BQ < it.len;
     // causal: q tile t needs kv tiles up to the one holding its last row's own position
     // block mask (chunk > 0, paged only): a row sees its own block of `chunk` positions, counted from position 0, up to
     // itself; tiles before the block of the pair's first row are skipped, n0 / n1 / n count tiles from j_lo
@@ -269,7 +282,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
           for (int step = 128; step > 0; step >>= 1)
             if (q + step < B && starts[q + step] <= r) q += step;
           set_seq(it, q);
-          set_pair(it, r - starts[q]);
+          set_rows(it, (r - starts[q]) * QPAIR, true);
           key = (uint32_t)(3 * it.n + min(it.n0, it.n1) + 6) * kMaxRows + (kMaxRows - 1 - r);  // (a lone q tile takes about 3/4 of a pair's time)
         }
         keys[r] = key;
@@ -297,7 +310,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);  // warp-uniform for the compiler too
   const int rows = SORTED ? s_rows[0] : -1;
   const int groups = Hq >> pack;  // of heads that an item takes together
-  const int num_items = (SORTED && rows >= 0 ? rows : max_q_pairs * B) * groups;
+  const int num_pairs = (SORTED && rows >= 0 ? rows : max_q_pairs * B) * groups;
+  const int split_from = ORDER == ORDER_SPLIT ? first_split(num_pairs, gridDim.x) : num_pairs;
+  const int num_items = 2 * num_pairs - split_from;
   auto next_item = [&](int idx, int round) {
     if constexpr (SORTED) {
       if (rows >= 0) return round * (int)gridDim.x + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
@@ -312,10 +327,13 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         it.h = idx - row * groups;
         it.kvh = (it.h << pack) / group;
         set_seq(it, s_order[row] & 255);
-        set_pair(it, s_order[row] >> 8);
+        set_rows(it, (s_order[row] >> 8) * QPAIR, true);
         return it;
       }
     }
+    const bool lone = ORDER == ORDER_SPLIT && idx >= split_from;
+    const int second = lone ? (idx - split_from) & 1 : 0;
+    if (lone) idx = split_from + ((idx - split_from) >> 1);
     const int per_qp = B * groups;
     const int qp = max_q_pairs - 1 - idx / per_qp;  // latest q rows first, one "round" per q pair index
     const int rem = idx % per_qp;
@@ -323,7 +341,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     it.h = rem % groups;
     it.kvh = (it.h << pack) / group;
     set_seq(it, b);
-    set_pair(it, qp);
+    set_rows(it, qp * QPAIR + second * BQ, !lone);
     return it;
   };
 
@@ -763,7 +781,7 @@ bool wants_order(const AttnPrefillArgs& a, int pack, int sms) {
 }
 // (for sure: the host knows no more of the rows than that a sequence's last pair may be cut short)
 bool order_fits(const AttnPrefillArgs& a, int pack) { return q_pairs(a, pack) <= 255 && ((long long)a.T << pack) / QPAIR + a.B <= kMaxRows; }
-template <int D, bool PAGED, bool SORTED>
+template <int D, bool PAGED, int ORDER>
 cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a, int pack) {
   constexpr int SRC = PAGED ? KV_PAGED : KV_PACKED;
   using C = ACfg<D, D, SRC>;
@@ -781,12 +799,13 @@ cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a, int pack) {
     if (!make_tmap_2d(&mk, a.k, TM_BF16, (uint64_t)a.Hkv * D, (uint64_t)a.T, (uint64_t)a.ldk * 2, 64, BKV)) return cudaErrorInvalidValue;
     if (!make_tmap_2d(&mv, a.v, TM_BF16, (uint64_t)a.Hkv * D, (uint64_t)a.T, (uint64_t)a.ldv * 2, 64, BKV)) return cudaErrorInvalidValue;
   }
-  auto kern = attn_prefill_kernel<D, D, SRC, SORTED>;
+  auto kern = attn_prefill_kernel<D, D, SRC, ORDER>;
   const int max_q_pairs = q_pairs(a, pack);
   const long long items = (long long)max_q_pairs * a.B * (a.Hq >> pack);
-  const int grid = (int)std::min<long long>(items, effective_sms(device_sms()));  // hb_engine_cfg.sm_budget
+  const int sms = effective_sms(device_sms());  // hb_engine_cfg.sm_budget
+  const int grid = (int)std::min<long long>(ORDER == ORDER_SPLIT && 2 * items <= sms ? 2 * items : items, sms);
   const float scale_log2 = a.scale * 1.4426950408889634f;
-  kern<<<grid, kThreads, SORTED ? C::SMEM_SORTED : C::SMEM, stream>>>(mq, mk, mv, mo, a.out, a.ldo, a.cu_seqlens, a.B, a.Hq, a.Hq / a.Hkv, a.causal,
+  kern<<<grid, kThreads, ORDER == ORDER_SORTED ? C::SMEM_SORTED : C::SMEM, stream>>>(mq, mk, mv, mo, a.out, a.ldo, a.cu_seqlens, a.B, a.Hq, a.Hq / a.Hkv, a.causal,
                                             scale_log2, max_q_pairs, a.kv_lens, a.page_table, a.max_pages, a.Hkv,
                                             paged_only(a.block_mask, PAGED), a.unit_sink, a.head_gate, a.ldg,
                                             paged_only(a.window, PAGED), a.softcap > 0.f ? a.scale / a.softcap : 0.f,
@@ -805,7 +824,7 @@ cudaError_t launch_expanded(cudaStream_t stream, const AttnExpandedArgs& a) {
   if (!make_tmap_3d(&mk, a.k, TM_BF16, a.nope, H, rows, (uint64_t)a.nope * 2, (uint64_t)a.ldkv * 2, 64, 1, BKV)) return cudaErrorInvalidValue;
   if (!make_tmap_3d(&mv, a.v, TM_BF16, a.vdim, H, rows, (uint64_t)a.vdim * 2, (uint64_t)a.ldkv * 2, 64, 1, BKV)) return cudaErrorInvalidValue;
   if (!make_tmap_2d(&mkr, a.k_rot, TM_BF16, a.rot, rows, (uint64_t)a.ldkr * 2, 64, BKV)) return cudaErrorInvalidValue;
-  auto kern = attn_prefill_kernel<DK, DV, KV_EXPANDED, false>;
+  auto kern = attn_prefill_kernel<DK, DV, KV_EXPANDED, ORDER_PLAIN>;
   int longest = 0;
   for (int i = 0; i < a.runs.n; ++i) longest = std::max(longest, a.runs.len[i]);
   const int max_q_pairs = (longest + QPAIR - 1) / QPAIR;
@@ -854,13 +873,16 @@ cudaError_t attn_prefill_init() {
   cudaError_t e;
 #define HB_ATTR(D_, P_, S_)                                                                                      \
   if ((e = cudaFuncSetAttribute(attn_prefill_kernel<D_, D_, P_, S_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                S_ ? ACfg<D_, D_, P_>::SMEM_SORTED : ACfg<D_, D_, P_>::SMEM)) != cudaSuccess)     \
+                                S_ == ORDER_SORTED ? ACfg<D_, D_, P_>::SMEM_SORTED : ACfg<D_, D_, P_>::SMEM)) != cudaSuccess)     \
     return e;
-  HB_ATTR(128, KV_PACKED, false) HB_ATTR(128, KV_PACKED, true) HB_ATTR(128, KV_PAGED, false)
-  HB_ATTR(64, KV_PACKED, false) HB_ATTR(64, KV_PACKED, true) HB_ATTR(64, KV_PAGED, false)
+#define HB_ATTRD(D_)                                                                                                        \
+  HB_ATTR(D_, KV_PACKED, ORDER_PLAIN) HB_ATTR(D_, KV_PACKED, ORDER_SPLIT) HB_ATTR(D_, KV_PACKED, ORDER_SORTED)               \
+  HB_ATTR(D_, KV_PAGED, ORDER_PLAIN) HB_ATTR(D_, KV_PAGED, ORDER_SPLIT)
+  HB_ATTRD(128) HB_ATTRD(64)
+#undef HB_ATTRD
 #undef HB_ATTR
 #define HB_ATTRX(K_, V_)                                                                                                  \
-  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<K_, V_, KV_EXPANDED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+  if ((e = cudaFuncSetAttribute(attn_prefill_kernel<K_, V_, KV_EXPANDED, ORDER_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                 ACfg<K_, V_, KV_EXPANDED>::SMEM)) != cudaSuccess)                                        \
     return e;
   HB_ATTRX(128, 64) HB_ATTRX(128, 128) HB_ATTRX(192, 64) HB_ATTRX(192, 128)
@@ -876,6 +898,7 @@ cudaError_t attn_prefill_init() {
 // per tile, [ ] in plain order: 32 heads over 8, 16 prompts of 500 to 4500 tokens 1037 | 978 | [1045], 6 of 2000 to 11300 2732 | 2669 | [3165], 30 of 500
 // to 6200 3844 | [3827] | [4048], 20 of 500 to 5000 1971 | 1875 | [1840]; 32 over 1, 8 of 200 to 1800 157 | 134 | 128 | 126 | 122 | [165], 10 of
 // 500 to 3500 476 | 433 | 394 | [417] | [480] | [431].
+static bool splits(long long pairs, int sms) { return pairs <= INT_MAX / 2 && first_split((int)pairs, (int)std::min<long long>(2 * pairs, sms)) < pairs; }
 AttnPrefillPlan attn_prefill_plan(const AttnPrefillArgs& a, int sms) {
   const int group = a.Hq / a.Hkv;
   const bool paged = a.k_cache != nullptr;
@@ -884,7 +907,8 @@ AttnPrefillPlan attn_prefill_plan(const AttnPrefillArgs& a, int sms) {
   for (int p = 0; p <= 5 && group % (1 << p) == 0; ++p) {
     if (!paged && p > 0 && wants_order(a, p, sms) && !order_fits(a, p) && order_fits(a, 0)) break;
     const long long rows = (long long)a.max_seqlen << p, items = (rows + QPAIR - 1) / QPAIR * a.B * (a.Hq >> p);
-    const long long cost = (items + sms - 1) / sms * (rows <= BQ ? 4 : 5);
+    const bool halves = rows > BQ && (paged || !wants_order(a, p, sms)) && splits(items, sms);
+    const long long cost = (items + sms - 1) / sms * (rows <= BQ ? 40 : 50) - (halves ? 9 : 0);  // (a last round of lone q tiles, after those that are lone anyway)
     if (p == 0 || cost <= least) {
       best = p;
       least = cost;
@@ -905,14 +929,17 @@ cudaError_t attn_prefill(cudaStream_t stream, const AttnPrefillArgs& a) {
   if (sms <= 0) return cudaErrorNoDevice;
   if (paged) {
     if (!a.v_cache || !a.page_table || !a.kv_lens || a.max_pages <= 0 || a.num_pages <= 0 || a.page_size != 64) return cudaErrorInvalidValue;
-    const int pack = attn_prefill_plan(a, sms).pack;
-    if (a.D == 128) return launch<128, true, false>(stream, a, pack);
-    if (a.D == 64) return launch<64, true, false>(stream, a, pack);
-    return cudaErrorInvalidValue;
   }
   const auto [pack, sorted] = attn_prefill_plan(a, sms);
-  if (a.D == 128) return sorted ? launch<128, false, true>(stream, a, pack) : launch<128, false, false>(stream, a, pack);
-  if (a.D == 64) return sorted ? launch<64, false, true>(stream, a, pack) : launch<64, false, false>(stream, a, pack);
+  // (sequences of one lone q tile have nothing to split)
+  const bool split = ((long long)a.max_seqlen << pack) > BQ && splits((long long)q_pairs(a, pack) * a.B * (a.Hq >> pack), sms);
+#define HB_LAUNCH(D_)                                                                                                                              \
+  if (paged) return split ? launch<D_, true, ORDER_SPLIT>(stream, a, pack) : launch<D_, true, ORDER_PLAIN>(stream, a, pack);                       \
+  return sorted ? launch<D_, false, ORDER_SORTED>(stream, a, pack)                                                                                 \
+         : split ? launch<D_, false, ORDER_SPLIT>(stream, a, pack) : launch<D_, false, ORDER_PLAIN>(stream, a, pack)
+  if (a.D == 128) { HB_LAUNCH(128); }
+  if (a.D == 64) { HB_LAUNCH(64); }
+#undef HB_LAUNCH
   return cudaErrorInvalidValue;
 }
 
