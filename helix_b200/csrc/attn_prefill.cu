@@ -209,6 +209,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     it.n1 = it.act1 ? (causal ? min(kv_tiles, (it.q_off + ((it.q0 + 2 * BQ - 1) >> pack)) / BKV + 1) : kv_tiles) - it.j_lo : 0;
     it.n = max(it.n0, it.n1);
   };
+  pdl_launch_dependents();
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_k);
@@ -238,6 +239,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     tmem_alloc(tmem_ptr, 512);
     tmem_relinquish();
   }
+  pdl_wait();  // nothing above touches memory that a kernel before this one may write
   // Order of the items (SORTED): rows (q pair, sequence) by falling number of kv tiles, a row's heads side by side (they share keys), dealt
   // to the CTAs forth and back (round r of CTA c is item r G + c, or r G + G - 1 - c in odd rounds).  Every CTA sorts the rows itself
   // (a thread per row, ranks by counting four keys a read; a thread per sequence that walked its rows, and one key a read, cost 2 us more: 6 prompts of 300 to 3000
@@ -805,12 +807,11 @@ cudaError_t launch(cudaStream_t stream, const AttnPrefillArgs& a, int pack) {
   const int sms = effective_sms(device_sms());  // hb_engine_cfg.sm_budget
   const int grid = (int)std::min<long long>(ORDER == ORDER_SPLIT && 2 * items <= sms ? 2 * items : items, sms);
   const float scale_log2 = a.scale * 1.4426950408889634f;
-  kern<<<grid, kThreads, ORDER == ORDER_SORTED ? C::SMEM_SORTED : C::SMEM, stream>>>(mq, mk, mv, mo, a.out, a.ldo, a.cu_seqlens, a.B, a.Hq, a.Hq / a.Hkv, a.causal,
-                                            scale_log2, max_q_pairs, a.kv_lens, a.page_table, a.max_pages, a.Hkv,
+  return launch_k(kern, dim3(grid), dim3(kThreads), ORDER == ORDER_SORTED ? C::SMEM_SORTED : C::SMEM, stream, true, mq, mk, mv, mo, a.out, a.ldo, a.cu_seqlens, a.B, a.Hq,
+                  a.Hq / a.Hkv, a.causal, scale_log2, max_q_pairs, a.kv_lens, a.page_table, a.max_pages, a.Hkv,
                                             paged_only(a.block_mask, PAGED), a.unit_sink, a.head_gate, a.ldg,
                                             paged_only(a.window, PAGED), a.softcap > 0.f ? a.scale / a.softcap : 0.f,
                                             a.softcap > 0.f ? a.softcap * 1.4426950408889634f : 0.f, a.sink, mq, mk, AttnRuns{}, D, pack);
-  return cudaGetLastError();
 }
 
 // latent attention over expanded rows
@@ -833,10 +834,9 @@ cudaError_t launch_expanded(cudaStream_t stream, const AttnExpandedArgs& a) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   const int grid = (int)std::min<long long>(items, effective_sms(num_sms));
-  kern<<<grid, kThreads, C::SMEM, stream>>>(mq, mk, mv, mq, a.out, a.ldo, nullptr, a.runs.n, a.H, 1, 1, a.scale * 1.4426950408889634f,
-                                            max_q_pairs, nullptr, nullptr, 0, a.H, 0, 0, a.head_gate, a.ldg, a.window, 0.f, 0.f, a.sink,
-                                            mqr, mkr, a.runs, a.vdim, 0);
-  return cudaGetLastError();
+  return launch_k(kern, dim3(grid), dim3(kThreads), C::SMEM, stream, true, mq, mk, mv, mq, a.out, a.ldo, nullptr, a.runs.n, a.H, 1, 1,
+                  a.scale * 1.4426950408889634f, max_q_pairs, nullptr, nullptr, 0, a.H, 0, 0, a.head_gate, a.ldg, a.window, 0.f, 0.f, a.sink, mqr, mkr,
+                  a.runs, a.vdim, 0);
 }
 
 // ---------------------------------------------------------------- test-only on-device checker

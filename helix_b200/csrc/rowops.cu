@@ -175,8 +175,10 @@ layernorm_warp_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gamma
                       bf16* __restrict__ out, int rows, int H, float eps, const int32_t* __restrict__ tokens,
                       const int32_t* __restrict__ positions, const bf16* __restrict__ word, const bf16* __restrict__ pos,
                       const bf16* __restrict__ type0) {
+  pdl_launch_dependents();
   const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
+  pdl_wait();
   if (r >= rows) return;
   const int nvec = H / 8;
   float vals[4][8];
@@ -1628,8 +1630,8 @@ cudaError_t layernorm(cudaStream_t s, const bf16* x, const bf16* gamma, const bf
   if (rows <= 0) return cudaSuccess;
   if (H % 8 || H > kMaxVec * kRowThreads * 8) return cudaErrorInvalidValue;
   if (H <= 1024)
-    layernorm_warp_kernel<false><<<(rows + 3) / 4, 128, 0, s>>>(x, gamma, beta, out, rows, H, eps, nullptr, nullptr, nullptr,
-                                                                nullptr, nullptr);
+    return launch_k(layernorm_warp_kernel<false>, dim3((rows + 3) / 4), dim3(128), 0, s, true, x, gamma, beta, out, rows, H, eps, nullptr, nullptr, nullptr, nullptr,
+                    nullptr);
   else
     layernorm_kernel<false><<<rows, kRowThreads, 0, s>>>(x, gamma, beta, out, H, eps, nullptr, nullptr, nullptr, nullptr, nullptr);
   return cudaGetLastError();
@@ -1640,7 +1642,7 @@ cudaError_t bert_embed_ln(cudaStream_t s, const int32_t* tokens, const int32_t* 
   if (T <= 0) return cudaSuccess;
   if (H % 8 || H > kMaxVec * kRowThreads * 8) return cudaErrorInvalidValue;
   if (H <= 1024)
-    layernorm_warp_kernel<true><<<(T + 3) / 4, 128, 0, s>>>(nullptr, gamma, beta, x, T, H, eps, tokens, positions, word, pos, type0);
+    return launch_k(layernorm_warp_kernel<true>, dim3((T + 3) / 4), dim3(128), 0, s, true, nullptr, gamma, beta, x, T, H, eps, tokens, positions, word, pos, type0);
   else
     layernorm_kernel<true><<<T, kRowThreads, 0, s>>>(nullptr, gamma, beta, x, H, eps, tokens, positions, word, pos, type0);
   return cudaGetLastError();

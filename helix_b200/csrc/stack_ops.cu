@@ -94,6 +94,7 @@ gemm_rt_tile_kernel(const float* __restrict__ A, long lda, long a_bs, const floa
   using T = RtTile<TM, TN, RM, RN, BK, ST>;
   constexpr int NT = T::NT, P = T::P, MT = TM / RM, NTX = TN / RN;
   extern __shared__ __align__(16) float sm[];
+  pdl_launch_dependents();
   const int grp = threadIdx.x / NT, t = threadIdx.x % NT;
   const int tx = t % NTX, ty = t / NTX;
   const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
@@ -146,6 +147,7 @@ gemm_rt_tile_kernel(const float* __restrict__ A, long lda, long a_bs, const floa
   for (int i = 0; i < RM; ++i)
 #pragma unroll
     for (int j = 0; j < RN; ++j) acc[i][j] = make_float2(0.f, 0.f);
+  pdl_wait();
 #pragma unroll
   for (int i = 0; i < ST - 1; ++i) load();
   int get = 0;
@@ -193,9 +195,8 @@ template <int TM, int TN, int RM, int RN, int BK, int ST>
 cudaError_t launch_rt_tile(cudaStream_t s, const GemmRtArgs& a) {
   using T = RtTile<TM, TN, RM, RN, BK, ST>;
   dim3 grid((a.N + TN - 1) / TN, (a.M + TM - 1) / TM, a.batch);
-  gemm_rt_tile_kernel<TM, TN, RM, RN, BK, ST><<<grid, T::NT * kRtParts, T::FLOATS * 4, s>>>(
-      a.A, a.lda, a.a_bs, (const float*)a.W, a.w_sn, a.w_bs, a.C, a.ldc, a.c_bs, (const float*)a.bias, a.M, a.N, a.K);
-  return cudaGetLastError();
+  return launch_k(gemm_rt_tile_kernel<TM, TN, RM, RN, BK, ST>, grid, dim3(T::NT * kRtParts), T::FLOATS * 4, s, true, a.A, a.lda, a.a_bs, (const float*)a.W,
+                  a.w_sn, a.w_bs, a.C, a.ldc, a.c_bs, (const float*)a.bias, a.M, a.N, a.K);
 }
 
 // ------------------------------------------------------------------ row kernels
