@@ -584,19 +584,22 @@ cudaError_t launch_epi(cudaStream_t stream, const GemmArgs& g, int num_sms) {
   if (bn == 0) {
     // The tile shape whose waves end first.  Per shape: us per 64-deep k block of one tile, the least a wave takes (its epilogue, when K
     // is short) and the part of a launch that does not depend on K, fitted to runs on random operands:
-    //                          256 x 256 pair  256 x 128 pair  128 x 256  128 x 128  128 x 64
-    //   512 x 4096 x 14336 (R)       73.6            59.1         88.1       71.8     112.9 us
-    //  1100 x 4096 x 14336 (R)      178.4           186.1        106.3      130.6     250.5
-    //  1280 x 4096 x  4096 (R)       71.0            45.1         62.9       54.2      76.0
-    //  6000 x 10304 x 2048          199.6           228.4        202.5      263.9     415.8
-    //   600 x  768 x   768 (R)       12.3            10.2         12.3        9.1       8.2
-    // 13400 x 3072 x   768 (gelu)    63.6            79.3         72.6       83.2     124.9
-    // (R: residual epilogue.)  Narrow tiles read more operand bytes from L2 per product (24 KB per SM and block for 128 x 64, 32 KB for
-    // four times the products in a pair's 256 x 256), wide ones leave SMs without a tile.  The rule before, "halve the width until there
-    // are two waves", took 128 x 64 for the first, second and fifth line.  Every shape walks K in order: a row's result does not
-    // depend on the choice.
+    //                          256 x 256 pair  256 x 192 pair  256 x 128 pair  128 x 256  128 x 128  128 x 64
+    //   512 x 4096 x 14336 (R)       73.6            72.6            59.1         88.1       71.8     112.9 us
+    //  1100 x 4096 x 14336 (R)      178.4           127.9           186.1        106.3      130.6     250.5
+    //  1280 x 4096 x  4096 (R)       71.0            47.1            45.1         62.9       54.2      76.0
+    //  5000 x 2048 x  8192 (R)      136.2           113.7           141.4        152.5      164.7
+    // 13800 x  768 x  3072 (R)       61.5            56.2            62.5         68.6       70.6
+    //  6000 x 10304 x 2048          199.6                           228.4        202.5      263.9     415.8
+    //   600 x  768 x   768 (R)       12.3                            10.2         12.3        9.1       8.2
+    // 13400 x 3072 x   768 (gelu)    63.6            65.6            79.3         72.6       83.2     124.9
+    // (R: residual epilogue; the second column, the fourth and the fifth line are of another run than the rest.)  Narrow tiles read more
+    // operand bytes from L2 per product (24 KB per SM and block for 128 x 64, 32 KB for
+    // four times the products in a pair's 256 x 256, 28 KB for three times in 256 x 192), wide ones leave SMs without a tile.  The rule before,
+    // "halve the width until there are two waves", took 128 x 64 for the first, third and seventh line.  Every shape walks K in order: a row's
+    // result does not depend on the choice.
     struct Shape { int bn, cg; double kb, floor, fixed; };
-    static constexpr Shape shapes[] = {{256, 2, 0.36, 5.6, 8.5}, {128, 2, 0.235, 3.4, 8.0}, {256, 1, 0.42, 6.0, 7.0}, {128, 1, 0.28, 3.9, 6.5}, {64, 1, 0.235, 3.1, 6.0}};
+    static constexpr Shape shapes[] = {{256, 2, 0.36, 5.6, 8.5}, {192, 2, 0.29, 4.8, 8.3}, {128, 2, 0.235, 3.4, 8.0}, {256, 1, 0.42, 6.0, 7.0}, {128, 1, 0.28, 3.9, 6.5}, {64, 1, 0.235, 3.1, 6.0}};
     const int num_kb = (g.K + BLOCK_K - 1) / BLOCK_K;
     double best = 1e30;
     for (const Shape& t : shapes) {
@@ -612,6 +615,9 @@ cudaError_t launch_epi(cudaStream_t stream, const GemmArgs& g, int num_sms) {
   switch (bn * 10 + cg) {
     case 2562: return launch_cfg<256, EPI, 2>(stream, g, num_sms);
     case 2561: return launch_cfg<256, EPI, 1>(stream, g, num_sms);
+    case 1922:
+      if constexpr (!kWideOnly) return launch_cfg<192, EPI, 2>(stream, g, num_sms);
+      return cudaErrorInvalidValue;
     case 1282:
       if constexpr (!kWideOnly) return launch_cfg<128, EPI, 2>(stream, g, num_sms);
       return cudaErrorInvalidValue;
@@ -638,6 +644,7 @@ cudaError_t set_attr_epi() {
   if ((e = set_attr<256, EPI, 2>()) != cudaSuccess) return e;
   if ((e = set_attr<256, EPI, 1>()) != cudaSuccess) return e;
   if constexpr (EPI != EPI_SWIGLU && EPI != EPI_GEGLU && EPI != EPI_CLAMPGLU && EPI != EPI_ROPE) {
+    if ((e = set_attr<192, EPI, 2>()) != cudaSuccess) return e;
     if ((e = set_attr<128, EPI, 2>()) != cudaSuccess) return e;
     if ((e = set_attr<128, EPI, 1>()) != cudaSuccess) return e;
     return set_attr<64, EPI, 1>();
