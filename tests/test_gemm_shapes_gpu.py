@@ -94,3 +94,24 @@ def test_silu_on_columns_gives_the_same_rows_on_every_tile():
     assert np.isfinite(got[0]).all()
     for g in got[1:]:
         assert np.array_equal(got[0], g)
+
+
+@pytest.mark.parametrize("M,N,K", [(1280, 2048, 1032), (2305, 2056, 72), (2305, 4104, 72), (1537, 1544, 1032), (2561, 2048, 64), (2305, 3976, 328)])
+@pytest.mark.parametrize("epi", [0, 2, 3, 6])  # bf16, bias + gelu, bf16 + residual, fp32
+def test_tiles_of_192_columns(M, N, K, epi):
+    """Sizes whose waves end first in 256 x 192: whole and ragged rows and columns, a last tile of a few columns, one k block."""
+    l = hb.lib()
+    assert l.hbk_init() == 0
+    A, W, R, b = rnd(M, K, seed=6), rnd(N, K, scale=K ** -0.5, seed=7), rnd(M, N, seed=8), rnd(N, seed=9)
+    outs = []
+    for bn in (0, 64):
+        out = torch.full((M, N), float("nan"), device="cuda", dtype=torch.float32 if epi == 6 else BF)
+        assert l.hbk_gemm(A.data_ptr(), K, W.data_ptr(), K, out.data_ptr(), N, R.data_ptr(), N, b.data_ptr(), M, N, K, epi, bn) == 0
+        torch.cuda.synchronize()
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    want = A.double() @ W.double().T
+    want = want + R.double() if epi == 3 else torch.nn.functional.gelu(want + b.double()) if epi == 2 else want
+    # fp32 sums of K products of unit variance / K (2^-24 sqrt(K) at most), then one bf16 rounding of values below 8 (below 16 with a bias; the gelu's polynomial 6.5e-4)
+    bound = 2.0 ** -24 * math.sqrt(K) * 8 if epi == 6 else 16 * 2.0 ** -9 + 1e-3
+    assert (outs[0].double() - want).abs().max() < bound
