@@ -245,6 +245,7 @@ class Engine {
   float* rope_cs_ = nullptr;  // [t_cap][head_dim] cos | sin of the current step's positions (EPI_ROPE)
   float* logits_ = nullptr;
   float* dec_ws_ = nullptr;
+  size_t skinny_floats_ = 0;    // of skinny_ws_, layer-list decoders
   float* skinny_ws_ = nullptr;  // fp32 partial slabs of the decode-step GEMMs
   SkinnyPlan plan_qkv_{}, plan_o_{}, plan_gu_{}, plan_down_{}, plan_head_{};
   int skinny_max_b_ = 0;

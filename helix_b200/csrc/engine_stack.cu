@@ -174,6 +174,19 @@ int Engine::load_random_stack(const hb_stack_desc& sd, const hb_layer_desc* laye
 }
 
 // ------------------------------------------------------------------ sizing
+// State-space layers with a squared-relu unit beside them (both read the same stream): in steps of up to 256 tokens the two products
+// that read the stream are one launch, and so are the two whose outputs join it.  Where every entry is one token their readers (convolution, gated norm,
+// residual step) sum the slabs themselves: six launches of a layer instead of thirteen, each a link of 4 to 7 us in a chain that nothing else
+// fills (a turn of 16 sequences, 2 layers of width 1024, 12 tokens each: 3070 -> 2560 us, of it about 25 us a step on the host: sizes
+// of the slabs worked out for every product).  The same products in every step of up to 256 tokens, so a row's sums do not
+// depend on whether a portion is among the entries
+static bool paired_ok(const Model& m, int i) {
+  const hb_layer_desc& l = m.sl[i];
+  const int W = m.sd.width, n_in = m.sw[i].n_in, inner = l.heads * l.vdim, ocols = m.sw[i].o_cols ? m.sw[i].o_cols : inner;
+  auto fits = [](int N, int K) { return K % 8 == 0 && K >= 64 && N >= 64 && N % 4 == 0; };
+  return !m.sd.compute_f32 && m.sd.norm_place == HB_NORM_PARALLEL && l.mixer == HB_MIXER_MAMBA2 && l.ff > 0 && l.ff_kind == HB_FF_RELU2 &&
+         fits(n_in, W) && fits(l.ff, W) && fits(W, ocols) && fits(W, l.ff) && W <= 8192 && inner / l.norm_groups % 4 == 0 && inner / l.norm_groups <= 8192;
+}
 // fp32 partial slabs of the weight-streaming GEMM that serves steps of <= 256 tokens (every projection it may be given)
 static size_t stack_skinny_floats(const Model& m) {
   size_t f = 0;
@@ -184,6 +197,11 @@ static size_t stack_skinny_floats(const Model& m) {
     shape(m.sw[i].n_in, W);
     shape(W, m.sw[i].o_cols ? (size_t)m.sw[i].o_cols : (size_t)l.heads * l.vdim);
     if (l.ff > 0 && l.ff_kind == HB_FF_RELU2) shape(l.ff, W);
+    if (paired_ok(m, i)) {
+      const int oc = m.sw[i].o_cols ? m.sw[i].o_cols : l.heads * l.vdim;
+      f = std::max(f, gemm_skinny_pair_floats(m.sw[i].n_in, (int)W, l.ff, (int)W, 256, 148));
+      f = std::max(f, gemm_skinny_pair_floats((int)W, oc, (int)W, l.ff, 256, 148));
+    }
     if (l.mixer == HB_MIXER_LATENT && l.q_rank > 0) shape((size_t)l.heads * (l.dim + l.rot_dim), l.q_rank);
     if (l.ff > 0) {
       shape(2 * (size_t)l.ff, W);
@@ -418,6 +436,10 @@ int Engine::alloc_runtime_stack() {
       CU(gemm_skinny_plan(model_.sw[i].n_in, sd.width, &pl));
       CU(gemm_skinny_plan(sd.width, model_.sw[i].o_cols ? model_.sw[i].o_cols : l.heads * l.vdim, &pl));
       if (l.ff > 0 && l.ff_kind == HB_FF_RELU2) CU(gemm_skinny_plan(l.ff, sd.width, &pl));
+      if (paired_ok(model_, i)) {
+        CU(gemm_skinny_pair_plan(model_.sw[i].n_in, sd.width, l.ff, sd.width, &pl));
+        CU(gemm_skinny_pair_plan(sd.width, model_.sw[i].o_cols ? model_.sw[i].o_cols : l.heads * l.vdim, sd.width, l.ff, &pl));
+      }
       if (l.mixer == HB_MIXER_LATENT && l.q_rank > 0) CU(gemm_skinny_plan(l.heads * (l.dim + l.rot_dim), l.q_rank, &pl));
       if (l.ff > 0) {
         CU(gemm_skinny_plan(2 * l.ff, sd.width, &pl));
@@ -551,7 +573,8 @@ int Engine::alloc_runtime_stack() {
   sample_ws_ = take(sample_scratch_bytes(cfg_.max_seqs, sd.vocab));
   lp_ids_ = (int32_t*)take((size_t)cfg_.max_seqs * HB_MAX_LOGPROBS * 4);
   lp_vals_ = (float*)take((size_t)cfg_.max_seqs * HB_MAX_LOGPROBS * 4);
-  skinny_ws_ = sd.compute_f32 ? nullptr : (float*)take(stack_skinny_floats(model_) * 4);
+  skinny_floats_ = sd.compute_f32 ? 0 : stack_skinny_floats(model_);
+  skinny_ws_ = sd.compute_f32 ? nullptr : (float*)take(skinny_floats_ * 4);
   if (!sd.compute_f32) {
     sk_.q16 = (bf16*)take(T * (size_t)sk_.ld2 * 2);
     sk_.ctx16 = (bf16*)take(T * (size_t)sk_.ldctx * 2);
@@ -636,6 +659,10 @@ void Engine::drop_slot(Request* r) {
 }
 
 // ------------------------------------------------------------------ forward
+static bool few_token_gemm() {  // HB_STACK_SKINNY=0: the tiled GEMM for few tokens too (A/B and bring-up)
+  static const bool off = [] { const char* e = getenv("HB_STACK_SKINNY"); return e && atoi(e) == 0; }();
+  return !off;
+}
 bool Engine::stack_tc(int N, int K, int lda, int ldc) const {
   static const bool simt_only = [] { const char* e = getenv("HB_STACK_SIMT"); return e && atoi(e) != 0; }();
   return !model_.sd.compute_f32 && !simt_only && K % 8 == 0 && lda % 8 == 0 && K >= 64 && N >= 64 && ldc % 4 == 0;
@@ -647,13 +674,12 @@ int Engine::stack_gemm(const float* A, const bf16* A16, int lda, const void* Wt,
   static const bool simt_only = [] { const char* e = getenv("HB_STACK_SIMT"); return e && atoi(e) != 0; }();  // A/B and bring-up
   const double flops = 2.0 * M * N * K;
   const bool tc = !f32 && !simt_only && A16 && !bias && K % 8 == 0 && lda % 8 == 0 && K >= 64 && N >= 64;
-  static const bool no_skinny = [] { const char* e = getenv("HB_STACK_SKINNY"); return e && atoi(e) == 0; }();
-  if (tc && M <= 256 && skinny_ws_ && !no_skinny) {
+  if (tc && M <= 256 && skinny_ws_ && few_token_gemm()) {
     // steps of a few tokens (decoding): the weights are the MMA's M operand and stream through every SM once (stream-K over
     // (tile, k-block) units, fp32 slabs summed in slab order: the result does not depend on who finishes first)
     SkinnyPlan plan{};
     CU(gemm_skinny_plan(N, K, &plan));
-    if (gemm_skinny_ws_floats(plan, M, N) <= stack_skinny_floats(model_)) {
+    if (gemm_skinny_ws_floats(plan, M, N) <= skinny_floats_) {
       SPAN(4, 2.0 * N * K + 2.0 * M * K + 4.0 * M * N, gemm_skinny(stream_, plan, A16, lda, (const bf16*)Wt, K, skinny_ws_, M, N, K));
       SPAN(3, 8.0 * M * N, dec_sum_slabs(stream_, skinny_ws_, plan, C, ldc, M, N, relu2));
       if (relu2) *relu2_done = true;
@@ -804,7 +830,8 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
   // a mixture's router product on the tensor cores (its rows padded with zero rows to one MMA tile)
   auto router_tc = [&](const hb_layer_desc& l) { return T > 256 && l.experts + l.identity_experts <= 64 && stack_tc(64, W, W, k.ldz) && k.ldz >= 64; };
   // parallel sublayers: x += mixer + feed-forward (+ bias), and the two normed inputs of the layer `next` (none behind the last)
-  auto par_step = [&](const float* y, const float* y2, const void* bias, float bias_scale, int next, const ParScale* scale) -> cudaError_t {
+  struct ParNext { const void *w1, *w2; float *h1, *h2; };
+  auto par_next = [&](int next) {
     const void* w1 = next < sd.n_layers ? model_.sw[next].norm1 : nullptr;
     const void* w2 = two_norms && next < sd.n_layers && model_.sl[next].ff > 0 ? model_.sw[next].norm2 : nullptr;
     // the fp32 copies are written only where a product of the next layer reads them (shapes the tensor-core GEMMs do not take)
@@ -817,8 +844,12 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       else h2_f32 = !stack_tc(nl.ff_kind == HB_FF_RELU2 ? nl.ff : 2 * nl.ff, W, W, k.ld1);
       if (!two_norms && nl.ff > 0) h1_f32 |= h2_f32;
     }
-    return parallel_step(stream_, k.x, nullptr, y, y2, bias, bias_scale, w1, w2, f32, sd.norm_eps, y ? k.x : nullptr, h1_f32 ? k.hn : nullptr, x16,
-                         h2_f32 ? k.hn2 : nullptr, f32 ? nullptr : k.x16b, T, W, scale);
+    return ParNext{w1, w2, h1_f32 ? k.hn : nullptr, h2_f32 ? k.hn2 : nullptr};
+  };
+  auto par_step = [&](const float* y, const float* y2, const void* bias, float bias_scale, int next, const ParScale* scale) -> cudaError_t {
+    const ParNext n = par_next(next);
+    return parallel_step(stream_, k.x, nullptr, y, y2, bias, bias_scale, n.w1, n.w2, f32, sd.norm_eps, y || (scale && scale->y_slabs.ws) ? k.x : nullptr, n.h1,
+                         x16, n.h2, f32 ? nullptr : k.x16b, T, W, scale);
   };
   // pre-normed stacks: the output y of a sublayer (or its expert rows) joins the stream copies, and the input of what follows —
   // sublayer `sub` (0 mixer, 1 feed-forward) of layer `next`, or behind the last layer the sum of the copies — is read and normed
@@ -1010,10 +1041,10 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
     bigram.table = model_.s_bigram; bigram.prev = (const int32_t*)(d_step_ + L.prev);
     bigram.buckets = sd.bigram_buckets; bigram.mul_prev = sd.bigram_mul_prev; bigram.mul_cur = sd.bigram_mul_cur;
   }
+  const double preb = (2.0 * std::max(sd.streams, 1) + 2.0) * rowb;
   float* x_emb = pre ? k.y : k.x;  // (pre-normed stacks: the first step below makes the copies)
   SPAN(3, rowb, embed_rows_f32(stream_, tokens, model_.s_embed, f32, x_emb, pre ? nullptr : x16, T, W, sd.embed_scale != 0.f ? sd.embed_scale : 1.f, bigram));
   if (sd.embed_norm) SPAN(3, 2 * rowb, norm_rows(x_emb, nullptr, model_.s_embed_norm, x_emb, both || pre ? nullptr : x16, T));
-  const double preb = (2.0 * std::max(sd.streams, 1) + 2.0) * rowb;
   if (pre) SPAN(3, preb, pre_step(k.y, nullptr, nullptr, nullptr, 0, 0, nullptr));
   if (both) SPAN(3, 2 * rowb, norm_rows(k.x, nullptr, model_.sw[0].norm1, k.hn, x16, T));
   if (par) SPAN(3, 3 * rowb, par_step(nullptr, nullptr, nullptr, 0.f, 0, nullptr));
@@ -1029,12 +1060,13 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
     int rc = HB_OK, longest_entry = 0;
     for (const StepEntry& en : step_entries_) longest_entry = std::max(longest_entry, en.n);
     // linear attention over a long portion: bf16 rows, the activations of q | k | v on the accumulators' way out
+    const bool paired = T <= 256 && skinny_ws_ && k.gu16 && paired_ok(model_, i) && stack_tc(w.n_in, W, W, k.ld1) && few_token_gemm();
     const bool chunked = light_chunk_ok(model_, l) && T > 256 && longest_entry >= kAttDenseMin && k.gu16 && stack_tc(w.n_in, W, W, w.n_in);
     if (chunked) {
       GemmArgs g{x16, W, (const bf16*)w.w_in, W, k.gu16, w.n_in, nullptr, 0, nullptr, T, w.n_in, W, EPI_SILU_COLS, 0};
       g.silu_cols = w.off_g;
       SPAN(0, 2.0 * T * w.n_in * W, gemm_bf16_tn(stream_, g));
-    } else {
+    } else if (!paired) {
       rc = stack_gemm(xin, x16, W, w.w_in, w.n_in, W, k.p1, ldin, T);
       if (rc != HB_OK) return rc;
     }
@@ -1055,6 +1087,27 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
         ca.single = T == B;  // (no entry is empty)
         ca.off_dt = w.off_a; ca.H = H; ca.a_dt = w.a_dt; ca.ab = k.ab; ca.ldab = k.ldab;
       }
+      Slabs in_slabs;
+      if (paired) {
+        SkinnyPlan plan{};
+        CU(gemm_skinny_pair_plan(w.n_in, W, l.ff, W, &plan));
+        float* up_ws = skinny_ws_ + (size_t)plan.max_segs * T * w.n_in;
+        const SkinnyProduct in{x16, W, (const bf16*)w.w_in, W, skinny_ws_, w.n_in, W}, up{ff_in16, W, (const bf16*)w.w_gu, W, up_ws, l.ff, W};
+        SPAN(4, 2.0 * (T + w.n_in + l.ff) * W + 4.0 * T * (w.n_in + l.ff), gemm_skinny_pair(stream_, plan, in, up, T));
+        in_slabs = Slabs{skinny_ws_, plan.seg_count, T, w.n_in};
+        const Slabs up_slabs{up_ws, plan.seg_count + plan.n_tiles, T, l.ff};
+        if (ca.single && (w.off_a & 3) == 0 && (w.off_g & 3) == 0) {  // its readers take the slabs
+          ca.slabs = in_slabs;
+          ca.up = up_slabs;
+          ca.up_out = k.gu16;
+        } else {
+          SkinnyPlan second = plan;
+          second.seg_count += plan.n_tiles;
+          SPAN(3, 8.0 * T * w.n_in, dec_sum_slabs(stream_, skinny_ws_, plan, k.p1, k.ld1, T, w.n_in));
+          SPAN(3, 6.0 * T * l.ff, dec_sum_slabs(stream_, up_ws, second, nullptr, 0, T, l.ff, k.gu16));
+          in_slabs.ws = nullptr;
+        }
+      }
       SPAN(3, 4.0 * T * C * (l.conv_taps + 1) + 12.0 * T * H, short_conv(stream_, ca));
       if (!ca.single) SPAN(3, 8.0 * B * C * l.conv_taps, conv_tails(stream_, ca));
       if (!fused) SPAN(3, 12.0 * T * H, ssm_steps(stream_, k.p1, k.ld1, w.off_a, w.a_dt, f32, k.ab, k.ldab, T, H));
@@ -1070,9 +1123,23 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       ra.cu = cu; ra.first_pos = first; ra.slots = sslot;
       ra.T = T; ra.B = B; ra.H = H; ra.G = G; ra.Dk = N; ra.Dv = Dv;
       ra.single = T == B;
+      ra.settled = true;  // (a layer's states are written once per step, and every step is waited for)
       SPAN(6, 4.0 * T * H * N * Dv, lin_recurrence(stream_, ra));
-      SPAN(3, 16.0 * T * inner, gated_group_norm(stream_, k.ctx, k.ldctx, k.p1 + w.off_g, k.ld1, w.hnorm, f32, sd.norm_eps, l.norm_groups, mo_f32,
-                                                 mo16, T, inner));
+      SPAN(3, 16.0 * T * inner, gated_group_norm(stream_, k.ctx, k.ldctx, in_slabs.ws ? nullptr : k.p1 + w.off_g, k.ld1, w.hnorm, f32, sd.norm_eps,
+                                                 l.norm_groups, mo_f32, mo16, T, inner, false, nullptr, in_slabs.ws ? &in_slabs : nullptr, w.off_g));
+      if (paired) {
+        SkinnyPlan plan{};
+        CU(gemm_skinny_pair_plan(W, ocols, W, l.ff, &plan));
+        float* down_ws = skinny_ws_ + (size_t)plan.max_segs * T * W;
+        const SkinnyProduct o{mo16, ocols, (const bf16*)w.wo, ocols, skinny_ws_, W, ocols}, down{k.gu16, l.ff, (const bf16*)w.w_down, l.ff, down_ws, W, l.ff};
+        SPAN(4, 2.0 * (T + W) * (ocols + l.ff) + 8.0 * T * W, gemm_skinny_pair(stream_, plan, o, down, T));
+        ParScale scale;
+        scale.s1 = w.ls1; scale.s2 = w.ls2; scale.m = sd.resid_mult != 0.f ? sd.resid_mult : 1.f;
+        scale.y_slabs = Slabs{skinny_ws_, plan.seg_count, T, W};
+        scale.y2_slabs = Slabs{down_ws, plan.seg_count + plan.n_tiles, T, W};
+        SPAN(3, 5 * rowb, par_step(nullptr, nullptr, w.o_bias, l.mix_scale != 0.f ? l.mix_scale : 1.f, i + 1, &scale));
+        continue;
+      }
     } else if (l.mixer == HB_MIXER_MLSTM) {
       rc = run_memory(w, k.ld1, 0, ocols, 1.f, mo_f32);
       if (rc != HB_OK) return rc;

@@ -15,6 +15,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "kernels.h"
@@ -179,13 +180,22 @@ __device__ __noinline__ void finish_tile(const SkinnyEpi& epi, const uint8_t* __
   }
 }
 
-template <int MPAD>
+// A second product behind the first (PAIR): its units follow the first one's in the stream-K line, so two products that wait for
+// nothing of one another (a layer's input and feed-forward projections, its two output projections) cost one launch
+struct SecondProduct {
+  CUtensorMap map_w, map_x;
+  float* ws;
+  int N, K;
+};
+struct NoSecond {};
+
+template <int MPAD, bool PAIR>
 __global__ void __launch_bounds__(kThreads, (MPAD <= 64 ? 2 : 1))
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                    float* __restrict__ ws, int M, int N, int K, const int* sig_wait, int sig_wait_count, int* sig_done,
                    int bank_units, const bf16* __restrict__ Wp, int ldw, unsigned long long* trace,
                    const __grid_constant__ SkinnyEpi epi, const uint8_t* __restrict__ segs, const int* dep_wait, int dep_count,
-                   int* dep_done) {
+                   int* dep_done, const __grid_constant__ std::conditional_t<PAIR, SecondProduct, NoSecond> second) {
   using C = SCfg<MPAD>;
   constexpr int STAGES = C::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -205,8 +215,35 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int KB = (K + BLOCK_K - 1) / BLOCK_K;
   const int n_tiles = (N + BLOCK_N - 1) / BLOCK_N;
-  const long long U = (long long)n_tiles * KB;
+  const long long U1 = (long long)n_tiles * KB;
+  long long U = U1;
+  int KB2 = 0;
+  if constexpr (PAIR) {
+    KB2 = (second.K + BLOCK_K - 1) / BLOCK_K;
+    U += (long long)((second.N + BLOCK_N - 1) / BLOCK_N) * KB2;
+  }
   const int G = gridDim.x;
+  // unit u of the line: (second product?, tile, k block)
+  struct Unit { bool two; int tile, kb; };
+  auto unit = [&](long long u) {
+    if (PAIR && u >= U1) return Unit{true, (int)((u - U1) / KB2), (int)((u - U1) % KB2)};
+    return Unit{false, (int)(u / KB), (int)(u % KB)};
+  };
+  auto tile_end = [&](const Unit& x) { return PAIR && x.two ? U1 + (long long)(x.tile + 1) * KB2 : (long long)(x.tile + 1) * KB; };  // behind its tile's last unit
+  auto load_w = [&](uint8_t* dst, uint64_t* bar, long long u) {
+    const Unit x = unit(u);
+    if constexpr (PAIR) {
+      if (x.two) return tma_load_2d(dst, &second.map_w, bar, x.kb * BLOCK_K, x.tile * BLOCK_N, kEvictFirst);
+    }
+    tma_load_2d(dst, &map_w, bar, x.kb * BLOCK_K, x.tile * BLOCK_N, kEvictFirst);
+  };
+  auto load_x = [&](uint8_t* dst, uint64_t* bar, long long u) {
+    const Unit x = unit(u);
+    if constexpr (PAIR) {
+      if (x.two) return tma_load_2d(dst, &second.map_x, bar, x.kb * BLOCK_K, 0, kEvictLast);
+    }
+    tma_load_2d(dst, &map_x, bar, x.kb * BLOCK_K, 0, kEvictLast);
+  };
   const long long u0 = range_start(blockIdx.x, U, G), u1 = range_start(blockIdx.x + 1, U, G);
 
   pdl_launch_dependents();
@@ -215,6 +252,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     trace_ev(trace, 0);
     tma_prefetch_desc(&map_w);
     tma_prefetch_desc(&map_x);
+    if constexpr (PAIR) {
+      tma_prefetch_desc(&second.map_w);
+      tma_prefetch_desc(&second.map_x);
+    }
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&full_bar[i], 1);
       mbar_init(&empty_bar[i], 1);
@@ -246,7 +287,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int s = (int)(u - u0);
         if (elected) {
           mbar_arrive_expect_tx(&full_bar[s], C::STAGE_BYTES);
-          tma_load_2d(smem_w + s * C::W_BYTES, &map_w, &full_bar[s], (int)(u % KB) * BLOCK_K, (int)(u / KB) * BLOCK_N, kEvictFirst);
+          load_w(smem_w + s * C::W_BYTES, &full_bar[s], u);
         }
       }
       if (pre_end >= u1 && elected) sig_add(sig_done);  // the whole range fitted into the ring
@@ -261,18 +302,17 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       if (elected) trace_ev(trace, 3);
       for (long long u = u0; u < pre_end; ++u) {
         const int s = (int)(u - u0);
-        if (elected) tma_load_2d(smem_x + s * C::X_BYTES, &map_x, &full_bar[s], (int)(u % KB) * BLOCK_K, 0, kEvictLast);
+        if (elected) load_x(smem_x + s * C::X_BYTES, &full_bar[s], u);
       }
       int s = 0;
       uint32_t phase = 1;  // the ring has been filled once
       if (pre_end - u0 < STAGES) { s = (int)(pre_end - u0); phase = 0; }
       for (long long u = pre_end; u < u1; ++u) {
-        const int tile = (int)(u / KB), kb = (int)(u % KB);
         mbar_wait(&empty_bar[s], phase ^ 1);
         if (elected) {
           mbar_arrive_expect_tx(&full_bar[s], C::STAGE_BYTES);
-          tma_load_2d(smem_w + s * C::W_BYTES, &map_w, &full_bar[s], kb * BLOCK_K, tile * BLOCK_N, kEvictFirst);
-          tma_load_2d(smem_x + s * C::X_BYTES, &map_x, &full_bar[s], kb * BLOCK_K, 0, kEvictLast);
+          load_w(smem_w + s * C::W_BYTES, &full_bar[s], u);
+          load_x(smem_x + s * C::X_BYTES, &full_bar[s], u);
           if (u + 1 == u1) { sig_add(sig_done); trace_ev(trace, 5); }  // this CTA's HBM demand ends here
         }
         if (++s == STAGES) { s = 0; phase ^= 1; }
@@ -287,8 +327,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       int it = 0;
       long long u = u0;
       while (u < u1) {
-        const int tile = (int)(u / KB);
-        const long long seg_end = min(u1, (long long)(tile + 1) * KB);
+        const long long seg_end = min(u1, tile_end(unit(u)));
         const int as = it & 1;
         mbar_wait(&tmem_empty[as], ((it >> 1) & 1) ^ 1);
         tc_fence_after();
@@ -360,33 +399,39 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       bar_sync(2, 128);
     }
     while (u < u1) {
-      const int tile = (int)(u / KB);
-      const long long seg_end = min(u1, (long long)(tile + 1) * KB);
-      const int seg = blockIdx.x - owner_of((long long)tile * KB, U, G);  // slab index: fixed by the partition
+      const Unit at = unit(u);
+      const int tile = at.tile;
+      const long long end = tile_end(at), seg_end = min(u1, end);
+      const int seg = blockIdx.x - owner_of(end - (PAIR && at.two ? KB2 : KB), U, G);  // slab index: fixed by the partition
       const int as = it & 1;
       mbar_wait(&tmem_full[as], (it >> 1) & 1);
       tc_fence_after();
       const uint32_t t_tile = tmem_base + as * MPAD + (static_cast<uint32_t>(q * 32) << 16);
       const int n = tile * BLOCK_N + row;
-      float* dst = ws + (size_t)seg * M * N + n;
+      int ld = N;
+      float* slabs = ws;
+      if constexpr (PAIR) {
+        if (at.two) { ld = second.N; slabs = second.ws; }
+      }
+      float* dst = slabs + (size_t)seg * M * ld + n;
 #pragma unroll 1
       for (int c = 0; c < MPAD / 32; ++c) {
         if (c * 32 >= M) break;  // warp-uniform
         uint32_t v[32];
         tmem_ld_32x32b_x32(t_tile + c * 32, v);
         tmem_ld_wait();
-        if (n < N) {
+        if (n < ld) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int m = c * 32 + j;
-            if (m < M) dst[(size_t)m * N] = __uint_as_float(v[j]);  // 32 lanes -> 128 contiguous bytes per m
+            if (m < M) dst[(size_t)m * ld] = __uint_as_float(v[j]);  // 32 lanes -> 128 contiguous bytes per m
           }
         }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[as]);
-      if (epi.mode != SK_SLABS) {
+      if (!PAIR && epi.mode != SK_SLABS) {
         // arrival: the last CTA to deliver a slab of this tile (pair of tiles for SwiGLU) finishes it
         const int et = threadIdx.x - 64;  // 0..127 over the four epilogue warps
         const int group = epi.mode == SK_SWIGLU ? (tile >> 1) : tile;
@@ -424,8 +469,24 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 }
 
 struct PlanKey {
-  int dev, N, K, sms;
-  bool operator<(const PlanKey& o) const { return std::tie(dev, N, K, sms) < std::tie(o.dev, o.N, o.K, o.sms); }
+  int dev, N, K, N2, K2, sms;
+  bool operator<(const PlanKey& o) const { return std::tie(dev, N, K, N2, K2, sms) < std::tie(o.dev, o.N, o.K, o.N2, o.K2, o.sms); }
+};
+// the stream-K line of one product or of two behind one another: slabs of every 128-column tile
+struct Line {
+  int grid = 0;
+  std::vector<uint8_t> segs;
+  Line(int N, int K, int N2, int K2, int sms) {
+    const int kb[2] = {(K + BLOCK_K - 1) / BLOCK_K, (K2 + BLOCK_K - 1) / BLOCK_K}, tiles[2] = {(N + BLOCK_N - 1) / BLOCK_N, (N2 + BLOCK_N - 1) / BLOCK_N};
+    const long long U1 = (long long)tiles[0] * kb[0], U = U1 + (long long)tiles[1] * kb[1];
+    grid = (int)std::min<long long>(sms, std::max<long long>(1, U / 4));
+    for (int p = 0; p < 2; ++p)
+      for (int t = 0; t < tiles[p]; ++t) {
+        const long long first = (p ? U1 : 0) + (long long)t * kb[p];
+        segs.push_back((uint8_t)(owner_of(first + kb[p] - 1, U, grid) - owner_of(first, U, grid) + 1));
+      }
+  }
+  int most(int from, int to) const { return *std::max_element(segs.begin() + from, segs.begin() + to); }
 };
 std::mutex g_plan_mu;
 std::map<PlanKey, SkinnyPlan> g_plans;
@@ -450,14 +511,31 @@ cudaError_t launch(cudaStream_t stream, const SkinnyPlan& plan, const bf16* X, i
   CUtensorMap mw, mx;
   if (!make_tmap_2d(&mw, W, TM_BF16, (uint64_t)K, (uint64_t)N, (uint64_t)ldw * 2, BLOCK_K, BLOCK_N)) return cudaErrorInvalidValue;
   if (!make_tmap_2d(&mx, X, TM_BF16, (uint64_t)K, (uint64_t)M, (uint64_t)ldx * 2, BLOCK_K, MPAD)) return cudaErrorInvalidValue;
-  return launch_k(gemm_skinny_kernel<MPAD>, dim3(plan.grid), dim3(kThreads), C::SMEM, stream, true, mw, mx, ws, M, N, K,
+  return launch_k(gemm_skinny_kernel<MPAD, false>, dim3(plan.grid), dim3(kThreads), C::SMEM, stream, true, mw, mx, ws, M, N, K,
                   sig->wait, sig->wait_count, sig->done, bank_units, W, ldw, sig->trace, *epi, plan.seg_count, sig->dep.wait,
-                  sig->dep.wait_count, sig->dep.done);
+                  sig->dep.wait_count, sig->dep.done, NoSecond{});
+}
+
+template <int MPAD>
+cudaError_t launch_pair(cudaStream_t stream, const SkinnyPlan& plan, const SkinnyProduct& a, const SkinnyProduct& b, int M) {
+  using C = SCfg<MPAD>;
+  CUtensorMap mw, mx;
+  SecondProduct second;
+  if (!make_tmap_2d(&mw, a.W, TM_BF16, (uint64_t)a.K, (uint64_t)a.N, (uint64_t)a.ldw * 2, BLOCK_K, BLOCK_N)) return cudaErrorInvalidValue;
+  if (!make_tmap_2d(&mx, a.X, TM_BF16, (uint64_t)a.K, (uint64_t)M, (uint64_t)a.ldx * 2, BLOCK_K, MPAD)) return cudaErrorInvalidValue;
+  if (!make_tmap_2d(&second.map_w, b.W, TM_BF16, (uint64_t)b.K, (uint64_t)b.N, (uint64_t)b.ldw * 2, BLOCK_K, BLOCK_N)) return cudaErrorInvalidValue;
+  if (!make_tmap_2d(&second.map_x, b.X, TM_BF16, (uint64_t)b.K, (uint64_t)M, (uint64_t)b.ldx * 2, BLOCK_K, MPAD)) return cudaErrorInvalidValue;
+  second.ws = b.ws;
+  second.N = b.N;
+  second.K = b.K;
+  return launch_k(gemm_skinny_kernel<MPAD, true>, dim3(plan.grid), dim3(kThreads), C::SMEM, stream, true, mw, mx, a.ws, M, a.N, a.K, (const int*)nullptr, 0,
+                  (int*)nullptr, 0, a.W, a.ldw, (unsigned long long*)nullptr, SkinnyEpi{}, plan.seg_count, (const int*)nullptr, 0, (int*)nullptr, second);
 }
 
 template <int MPAD>
 cudaError_t set_attr() {
-  return cudaFuncSetAttribute(gemm_skinny_kernel<MPAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCfg<MPAD>::SMEM);
+  cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<MPAD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCfg<MPAD>::SMEM);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(gemm_skinny_kernel<MPAD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCfg<MPAD>::SMEM);
 }
 
 }  // namespace
@@ -470,7 +548,9 @@ cudaError_t gemm_skinny_init() {
   return set_attr<256>();
 }
 
-cudaError_t gemm_skinny_plan(int N, int K, SkinnyPlan* out) {
+cudaError_t gemm_skinny_plan(int N, int K, SkinnyPlan* out) { return gemm_skinny_pair_plan(N, K, 0, 0, out); }
+
+cudaError_t gemm_skinny_pair_plan(int N, int K, int N2, int K2, SkinnyPlan* out) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -478,41 +558,35 @@ cudaError_t gemm_skinny_plan(int N, int K, SkinnyPlan* out) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   sms = effective_sms(sms);  // hb_engine_cfg.sm_budget of the calling engine
   std::lock_guard<std::mutex> g(g_plan_mu);
-  auto it = g_plans.find(PlanKey{dev, N, K, sms});
+  const PlanKey key{dev, N, K, N2, K2, sms};
+  auto it = g_plans.find(key);
   if (it != g_plans.end()) {
     *out = it->second;
     return cudaSuccess;
   }
-  const int KB = (K + BLOCK_K - 1) / BLOCK_K, n_tiles = (N + BLOCK_N - 1) / BLOCK_N;
-  const long long U = (long long)n_tiles * KB;
+  const Line line(N, K, N2, K2, sms);
   SkinnyPlan p{};
-  p.n_tiles = n_tiles;
-  p.grid = (int)std::min<long long>(sms, std::max<long long>(1, U / 4));
-  std::vector<uint8_t> segs(n_tiles);
-  int smax = 1;
-  for (int t = 0; t < n_tiles; ++t) {
-    const int first = owner_of((long long)t * KB, U, p.grid), last = owner_of((long long)t * KB + KB - 1, U, p.grid);
-    segs[t] = (uint8_t)(last - first + 1);
-    smax = std::max(smax, last - first + 1);
-  }
-  p.max_segs = smax;
+  p.n_tiles = (N + BLOCK_N - 1) / BLOCK_N;
+  p.grid = line.grid;
+  p.max_segs = line.most(0, p.n_tiles);
+  if (N2 > 0) p.max_segs2 = line.most(p.n_tiles, (int)line.segs.size());
   uint8_t* d = nullptr;
-  if ((e = cudaMalloc(&d, n_tiles)) != cudaSuccess) return e;
-  if ((e = cudaMemcpy(d, segs.data(), n_tiles, cudaMemcpyHostToDevice)) != cudaSuccess) return e;
+  if ((e = cudaMalloc(&d, line.segs.size())) != cudaSuccess) return e;
+  if ((e = cudaMemcpy(d, line.segs.data(), line.segs.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
   p.seg_count = d;
-  g_plans[PlanKey{dev, N, K, sms}] = p;
+  g_plans[key] = p;
   *out = p;
   return cudaSuccess;
 }
 
 int gemm_skinny_max_segs(int N, int K, int sms) {
-  const int KB = (K + BLOCK_K - 1) / BLOCK_K, n_tiles = (N + BLOCK_N - 1) / BLOCK_N;
-  const long long U = (long long)n_tiles * KB;
-  const int G = (int)std::min<long long>(sms, std::max<long long>(1, U / 4));
-  int smax = 1;
-  for (int t = 0; t < n_tiles; ++t)
-    smax = std::max(smax, owner_of((long long)t * KB + KB - 1, U, G) - owner_of((long long)t * KB, U, G) + 1);
-  return smax;
+  const Line line(N, K, 0, 0, sms);
+  return line.most(0, (int)line.segs.size());
+}
+size_t gemm_skinny_pair_floats(int N, int K, int N2, int K2, int M, int sms) {
+  const Line line(N, K, N2, K2, sms);
+  const int n1 = (N + BLOCK_N - 1) / BLOCK_N;
+  return (size_t)M * ((size_t)line.most(0, n1) * N + (size_t)line.most(n1, (int)line.segs.size()) * N2);
 }
 
 size_t gemm_skinny_ws_floats(const SkinnyPlan& p, int M, int N) { return (size_t)p.max_segs * M * N; }
@@ -524,6 +598,16 @@ cudaError_t gemm_skinny(cudaStream_t stream, const SkinnyPlan& plan, const bf16*
   if (M <= 64) return launch<64>(stream, plan, X, ldx, W, ldw, ws, M, N, K, sig, epi);
   if (M <= 128) return launch<128>(stream, plan, X, ldx, W, ldw, ws, M, N, K, sig, epi);
   return launch<256>(stream, plan, X, ldx, W, ldw, ws, M, N, K, sig, epi);
+}
+
+cudaError_t gemm_skinny_pair(cudaStream_t stream, const SkinnyPlan& plan, const SkinnyProduct& a, const SkinnyProduct& b, int M) {
+  if (M <= 0 || M > 256 || a.N <= 0 || b.N <= 0) return cudaErrorInvalidValue;
+  for (const SkinnyProduct* p : {&a, &b})
+    if ((p->K % 8) || (p->ldx % 8) || (p->ldw % 8)) return cudaErrorInvalidValue;
+  if (M <= 32) return launch_pair<32>(stream, plan, a, b, M);
+  if (M <= 64) return launch_pair<64>(stream, plan, a, b, M);
+  if (M <= 128) return launch_pair<128>(stream, plan, a, b, M);
+  return launch_pair<256>(stream, plan, a, b, M);
 }
 
 }  // namespace hb

@@ -243,7 +243,8 @@ struct SkinnyPlan {
   int grid;                  // CTAs (== SMs unless the problem is tiny)
   int n_tiles;               // ceil(N/128)
   int max_segs;              // max #slabs any tile is split into
-  const uint8_t* seg_count;  // device [n_tiles]: slabs of each 128-column tile
+  const uint8_t* seg_count;  // device [n_tiles]: slabs of each 128-column tile (of two products: the second one's tiles behind the first one's)
+  int max_segs2 = 0;         // the same of a second product
 };
 // Tile finisher of the decode GEMM: the LAST CTA that contributes a slab to an output tile (one counter per tile) sums
 // the tile's slabs in slab order — bit-deterministic whoever finishes — and applies the op that follows the projection
@@ -281,6 +282,13 @@ int gemm_skinny_max_segs(int N, int K, int sms);  // pure host arithmetic (memor
 // ws[seg][m][n] (seg < seg_count[n/128]) = partial sums of X[M,K] . W[N,K]^T
 cudaError_t gemm_skinny(cudaStream_t stream, const SkinnyPlan& plan, const bf16* X, int ldx, const bf16* W, int ldw,
                         float* ws, int M, int N, int K, const StreamSig* sig = nullptr, const SkinnyEpi* epi = nullptr);
+// Two products of the same M rows in one launch, the units of both in one stream-K line; a plan of its own (slabs only)
+struct SkinnyProduct { const bf16* X; int ldx; const bf16* W; int ldw; float* ws; int N, K; };
+cudaError_t gemm_skinny_pair_plan(int N, int K, int N2, int K2, SkinnyPlan* out);
+size_t gemm_skinny_pair_floats(int N, int K, int N2, int K2, int M, int sms);  // of both products' slabs, pure host arithmetic
+cudaError_t gemm_skinny_pair(cudaStream_t stream, const SkinnyPlan& plan, const SkinnyProduct& a, const SkinnyProduct& b, int M);
+// A product's slabs where a kernel takes them instead of the summed rows (it sums a value's slabs in slab order, as dec_sum_slabs does)
+struct Slabs { const float* ws = nullptr; const uint8_t* segs = nullptr; int M = 0, N = 0; };  // N a multiple of four
 // consumers of the slabs (each sums the slabs in fixed order, then applies its fused epilogue)
 // relu2 given: relu(sum)^2 as dense bf16 rows there instead of the sums in out
 cudaError_t dec_sum_slabs(cudaStream_t s, const float* ws, const SkinnyPlan& p, float* out, int ldo, int M, int N, bf16* relu2 = nullptr);
@@ -567,6 +575,8 @@ struct ConvArgs {
   bool single = false;  // what conv_tails does, when every entry is exactly one token;
   // ab given: what ssm_steps does for the same rows (on `in` with these arguments)
   int off_dt = 0, H = 0; const void* a_dt = nullptr; float* ab = nullptr; long ldab = 0;
+  // slabs given (single only): `in` is not read, its rows are these slabs' sums; and relu(sum)^2 of the slabs `up` goes to up_out [T, up.N]
+  Slabs slabs, up; bf16* up_out = nullptr;
 };
 cudaError_t short_conv(cudaStream_t s, const ConvArgs& a);
 bool short_conv_fused(const ConvArgs& a);
@@ -608,6 +618,9 @@ struct LinRecArgs {
   int silu = 0;
   bool single = false;  // every entry is exactly one token
   int T = 0;            // tokens of all entries
+  // Nothing that may still run when this launch begins writes the slots' states (a step of an engine that waits for its steps): single tokens
+  // may read theirs before the kernels ahead of them are done
+  bool settled = false;
 };
 cudaError_t lin_recurrence(cudaStream_t s, const LinRecArgs& a);
 // S_t = decay_h S_(t-1) + k_t v_t^T, out_t = S_t^T q_t on the tensor cores, chunk by chunk (stack_lightning.cu): q, k [T, H * Dk] and
@@ -632,9 +645,11 @@ cudaError_t memory_readout(cudaStream_t s, const float* num, long ldnum, const f
                            long ldout, int col0, int T, int H, int Dv);
 // State-space read-out: u = y[t, :] * silu(z[t, :]) over n entries, divided by its root mean square in `parts` equal parts,
 // times w; out [T, n] (+ bf16 copy).  gate_last: u = y[t, :], and the normed row is multiplied by sigmoid(z[t, :]) instead
-// (linear attention with constant decays).  z_b16: z as bf16 instead (then n / parts is a multiple of 4, at most 8192)
+// (linear attention with constant decays).  z_b16: z as bf16 instead, or z_slabs: its columns from z_col on are
+// z (with either, n / parts is a multiple of 4, at most 8192)
 cudaError_t gated_group_norm(cudaStream_t s, const float* y, long ldy, const float* z, long ldz, const void* w, bool f32, float eps,
-                             int parts, float* out, bf16* out_b16, int T, int n, bool gate_last = false, const bf16* z_b16 = nullptr);
+                             int parts, float* out, bf16* out_b16, int T, int n, bool gate_last = false, const bf16* z_b16 = nullptr,
+                             const Slabs* z_slabs = nullptr, int z_col = 0);
 // out[t, col0 + e] = in[t, e] * sigmoid(g[t, e]) * scale, e < n (in: fp32, or bf16 when in_b16 is given instead)
 cudaError_t gate_scale_rows(cudaStream_t s, const float* in, const bf16* in_b16, long ldi, const float* g, long ldg, float scale,
                             float* out, bf16* out_b16, long ldout, int col0, int T, int n);
@@ -647,6 +662,7 @@ struct ParScale {
   const void* s1 = nullptr; const void* s2 = nullptr;
   float m = 1.f;
   const bf16* rows = nullptr; const int32_t* row_of = nullptr; const float* wts = nullptr; int top_k = 0;
+  Slabs y_slabs, y2_slabs;  // given: y and y2 are their sums (both or neither; rows of W, a multiple of 4 up to 8192)
 };
 cudaError_t parallel_step(cudaStream_t s, const float* x, const int32_t* row_index, const float* y, const float* y2, const void* bias,
                           float bias_scale, const void* w1, const void* w2, bool f32, float eps, float* x_out, float* h1, bf16* h1_b16,

@@ -36,6 +36,34 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
   float t = (l < nw) ? red[l] : 0.f;
   return warp_sum(t);
 }
+// sums of a product's slabs, in slab order: four columns from n (a multiple of four) of row m, or column n
+__device__ __forceinline__ float4 slab_sum4(const Slabs& s, size_t m, int n) {
+  const int ns = s.segs[n >> 7];
+  const size_t step = (size_t)s.M * s.N;
+  const float* p = s.ws + m * s.N + n;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  int i = 0;
+  for (; i + 4 <= ns; i += 4) {  // four loads in flight
+    float4 v[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = *reinterpret_cast<const float4*>(p + (i + e) * step);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc = make_float4(acc.x + v[e].x, acc.y + v[e].y, acc.z + v[e].z, acc.w + v[e].w);
+  }
+  for (; i < ns; ++i) {
+    const float4 v = *reinterpret_cast<const float4*>(p + i * step);
+    acc = make_float4(acc.x + v.x, acc.y + v.y, acc.z + v.z, acc.w + v.w);
+  }
+  return acc;
+}
+__device__ __forceinline__ float slab_sum1(const Slabs& s, size_t m, int n) {
+  const int ns = s.segs[n >> 7];
+  const size_t step = (size_t)s.M * s.N;
+  const float* p = s.ws + m * s.N + n;
+  float acc = 0.f;
+  for (int i = 0; i < ns; ++i) acc += p[i * step];
+  return acc;
+}
 __device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + expf(-z)); }
 
 }  // namespace

@@ -29,11 +29,21 @@ namespace {
 __device__ __forceinline__ float softplus_(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 
 template <typename WT>
-__device__ __forceinline__ void ssm_step(const float* __restrict__ p, long ldp, int off_dt, const WT* __restrict__ a_dt, float* __restrict__ ab, long ldab,
-                                         int t, int H, int h) {
-  const float dt = softplus_(p[(size_t)t * ldp + off_dt + h] + ldf<WT>(a_dt, H + h));
+__device__ __forceinline__ void ssm_step(float raw, const WT* __restrict__ a_dt, float* __restrict__ ab, long ldab, int t, int H, int h) {
+  const float dt = softplus_(raw + ldf<WT>(a_dt, H + h));
   ab[(size_t)t * ldab + h] = expf(-expf(ldf<WT>(a_dt, h)) * dt);
   ab[(size_t)t * ldab + H + h] = dt;
+}
+
+__device__ __forceinline__ void st_pair(float* f, bf16* b, float4 v) {
+  if (f) *reinterpret_cast<float4*>(f) = v;
+  if (b) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+    uint2 pk;
+    pk.x = *reinterpret_cast<unsigned*>(&lo);
+    pk.y = *reinterpret_cast<unsigned*>(&hi);
+    *reinterpret_cast<uint2*>(b) = pk;
+  }
 }
 
 // ------------------------------------------------------------------ short convolutions
@@ -73,8 +83,20 @@ __global__ void __launch_bounds__(128) short_conv_run_kernel(ConvArgs a) {
   const int tb = blockIdx.y * RUN;
   if (a.ab && blockIdx.x == gridDim.x - 1) {  // the last column of blocks makes the run's step sizes
     for (int e = threadIdx.x; e < RUN * a.H; e += blockDim.x)
-      if (tb + e / a.H < a.T) ssm_step<WT>(a.in, a.ldi, a.off_dt, (const WT*)a.a_dt, a.ab, a.ldab, tb + e / a.H, a.H, e % a.H);
+      if (const int t = tb + e / a.H, col = a.off_dt + e % a.H; t < a.T)
+        ssm_step<WT>(RUN == 1 && a.slabs.ws ? slab_sum1(a.slabs, t, col) : a.in[(size_t)t * a.ldi + col], (const WT*)a.a_dt, a.ab, a.ldab, t, a.H, e % a.H);
     return;
+  }
+  if constexpr (RUN == 1) {
+    const int across = (a.C / 4 + 127) / 128;
+    if (a.up_out && blockIdx.x >= across) {  // the feed-forward's inner row, which waits for the same launch
+      const int e = ((blockIdx.x - across) * 128 + threadIdx.x) * 4;
+      if (e >= a.up.N) return;
+      const float4 u = slab_sum4(a.up, tb, e);
+      const float4 r = make_float4(fmaxf(u.x, 0.f), fmaxf(u.y, 0.f), fmaxf(u.z, 0.f), fmaxf(u.w, 0.f));
+      st_pair(nullptr, a.up_out + (size_t)tb * a.up.N + e, make_float4(r.x * r.x, r.y * r.y, r.z * r.z, r.w * r.w));
+      return;
+    }
   }
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (c >= a.C) return;
@@ -146,7 +168,7 @@ __global__ void __launch_bounds__(128) short_conv_run_kernel(ConvArgs a) {
         else win[j] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
-    const float4 x = f4add(*reinterpret_cast<const float4*>(a.in + (size_t)t * a.ldi + a.off + c), ib);
+    const float4 x = f4add(RUN == 1 && a.slabs.ws ? slab_sum4(a.slabs, t, a.off + c) : *reinterpret_cast<const float4*>(a.in + (size_t)t * a.ldi + a.off + c), ib);
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < TAPS - 1; ++j) {  // oldest tap first, as the per-channel kernel
@@ -175,6 +197,8 @@ __global__ void __launch_bounds__(128) short_conv_run_kernel(ConvArgs a) {
 constexpr int kMaxConvTail = 15;
 template <typename WT>
 __global__ void __launch_bounds__(256) conv_tails_kernel(ConvArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int b = blockIdx.y, nt = a.taps - 1;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= a.C || nt <= 0) return;
@@ -202,7 +226,7 @@ __global__ void ssm_steps_kernel(const float* __restrict__ p, long ldp, int off_
                                  long ldab, int T, int H) {
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long)T * H) return;
-  ssm_step<WT>(p, ldp, off_dt, a_dt, ab, ldab, (int)(idx / H), H, (int)(idx % H));
+  ssm_step<WT>(p[(size_t)(idx / H) * ldp + off_dt + idx % H], a_dt, ab, ldab, (int)(idx / H), H, (int)(idx % H));
 }
 
 // One warp per (entry, head).  The step m -> max(m + f, i) is the pair (f, i); two steps compose to
@@ -642,7 +666,7 @@ cudaError_t launch_portion(cudaStream_t s, const LinRecArgs& a) {
 __global__ void lin_step_kernel(LinRecArgs a) {
   __shared__ __align__(8) float obuf[16][64];
   pdl_launch_dependents();
-  pdl_wait();
+  if (!a.settled) pdl_wait();
   const int b = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * 64, kvh = h / (a.H / a.G);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i0 = w * 16, j0 = c0 + lane * 2;
   const int t = a.cu[b];
@@ -655,6 +679,7 @@ __global__ void lin_step_kernel(LinRecArgs a) {
   float4 q4[4], k4[4];
 #pragma unroll
   for (int i = 0; i < 16; ++i) S[i] = !fresh && cols && i0 + i < a.Dk ? *reinterpret_cast<const float2*>(st + (size_t)i * a.Dv) : make_float2(0.f, 0.f);
+  if (a.settled) pdl_wait();  // (the step's descriptors, read above, were there before its first kernel began)
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const bool in = i0 + 4 * i < a.Dk;  // (Dk is a multiple of four)
@@ -766,16 +791,6 @@ __device__ __forceinline__ float4 ldf4(const WT* p) {
   const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
   return make_float4(a.x, a.y, b.x, b.y);
 }
-__device__ __forceinline__ void st_pair(float* f, bf16* b, float4 v) {
-  if (f) *reinterpret_cast<float4*>(f) = v;
-  if (b) {
-    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-    uint2 pk;
-    pk.x = *reinterpret_cast<unsigned*>(&lo);
-    pk.y = *reinterpret_cast<unsigned*>(&hi);
-    *reinterpret_cast<uint2*>(b) = pk;
-  }
-}
 __device__ __forceinline__ float sum_of_squares(float4 v) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x))); }
 // one block per (part, token)
 template <typename WT>
@@ -828,7 +843,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_kernel(const float* __re
 template <typename WT, int CH>
 __global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const float* __restrict__ y, long ldy, const float* __restrict__ z, const bf16* __restrict__ zb, long ldz,
                                                                     const WT* __restrict__ w, float eps, int parts, float* __restrict__ out,
-                                                                    bf16* __restrict__ outb, int n, int gate_last, int items) {
+                                                                    bf16* __restrict__ outb, int n, int gate_last, int items, const Slabs zsl, int z_col) {
   pdl_launch_dependents();
   pdl_wait();
   const int item = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -846,7 +861,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const float*
     u[c] = g[c] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i >= len) continue;
     u[c] = *reinterpret_cast<const float4*>(ys + i);
-    g[c] = zs ? *reinterpret_cast<const float4*>(zs + i) : ldf4<bf16>(zbs + i);
+    g[c] = zsl.ws ? slab_sum4(zsl, t, z_col + c0 + i) : zs ? *reinterpret_cast<const float4*>(zs + i) : ldf4<bf16>(zbs + i);
   }
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
@@ -871,7 +886,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const float*
 template <typename WT, int CH>
 __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* __restrict__ y, long ldy, const float* __restrict__ z, const bf16* __restrict__ zb, long ldz,
                                                                    const WT* __restrict__ w, float eps, int parts, float* __restrict__ out,
-                                                                   bf16* __restrict__ outb, int n, int gate_last) {
+                                                                   bf16* __restrict__ outb, int n, int gate_last, const Slabs zsl, int z_col) {
   __shared__ float red[32];
   pdl_launch_dependents();
   pdl_wait();
@@ -887,7 +902,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
     u[c] = g[c] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i >= len) continue;
     u[c] = *reinterpret_cast<const float4*>(ys + i);
-    g[c] = zs ? *reinterpret_cast<const float4*>(zs + i) : ldf4<bf16>(zbs + i);
+    g[c] = zsl.ws ? slab_sum4(zsl, t, z_col + c0 + i) : zs ? *reinterpret_cast<const float4*>(zs + i) : ldf4<bf16>(zbs + i);
   }
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
@@ -1005,9 +1020,9 @@ __global__ void __launch_bounds__(256) parallel_step_vec_kernel(const float* x, 
     const int i = (threadIdx.x + c * 256) * 4;
     if (i >= W) continue;
     float4 a = *reinterpret_cast<const float4*>(xs + i);
-    if (y) {
-      float4 u = *reinterpret_cast<const float4*>(y + r * W + i);
-      float4 u2 = y2 ? *reinterpret_cast<const float4*>(y2 + r * W + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (y || sc.y_slabs.ws) {
+      float4 u = y ? *reinterpret_cast<const float4*>(y + r * W + i) : slab_sum4(sc.y_slabs, r, i);
+      float4 u2 = !y ? slab_sum4(sc.y2_slabs, r, i) : y2 ? *reinterpret_cast<const float4*>(y2 + r * W + i) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int k = 0; k < kParTop; ++k)
         if (k < sc.top_k) u2 = fma4(wk[k], ldf4<bf16>(sc.rows + rk[k] + i), u2);
@@ -1034,6 +1049,8 @@ __global__ void __launch_bounds__(256) parallel_step_vec_kernel(const float* x, 
 }
 
 __global__ void relu2_kernel(const float* __restrict__ in, long ldi, float* __restrict__ out, bf16* __restrict__ outb, int n) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.y, e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
   const float r = fmaxf(in[(size_t)t * ldi + e], 0.f), v = r * r;
@@ -1084,7 +1101,8 @@ cudaError_t short_conv(cudaStream_t s, const ConvArgs& a) {
     const int across = (a.C / 4 + 127) / 128;
     // runs of one token until runs of eight give every SM two blocks (or where the tails ride along)
     const bool one = a.single || (long)across * ((a.T + kConvRun - 1) / kConvRun) < 2 * effective_sms(148);
-    const dim3 g(across + (a.ab ? 1 : 0), one ? a.T : (a.T + kConvRun - 1) / kConvRun);
+    if (a.slabs.ws && (!a.single || !a.ab || !a.up_out || (a.up.N & 3) || (a.off_dt & 3))) return cudaErrorInvalidValue;
+    const dim3 g(across + (a.up_out ? (a.up.N / 4 + 127) / 128 : 0) + (a.ab ? 1 : 0), one ? a.T : (a.T + kConvRun - 1) / kConvRun);
 #define HB_CONV_T(WT, TP) return one ? launch_k(short_conv_run_kernel<WT, TP, 1>, g, dim3(128), 0, s, true, a) : launch_k(short_conv_run_kernel<WT, TP, kConvRun>, g, dim3(128), 0, s, true, a)
 #define HB_CONV(TP) do { if (a.f32) HB_CONV_T(float, TP); else HB_CONV_T(bf16, TP); } while (0)
     if (a.taps == 1) HB_CONV(1);
@@ -1094,7 +1112,7 @@ cudaError_t short_conv(cudaStream_t s, const ConvArgs& a) {
 #undef HB_CONV
 #undef HB_CONV_T
   }
-  if (a.single || a.ab) return cudaErrorInvalidValue;
+  if (a.single || a.ab || a.slabs.ws) return cudaErrorInvalidValue;
   dim3 grid((a.C + 255) / 256, a.T);
   if (a.f32) short_conv_kernel<float><<<grid, 256, 0, s>>>(a);
   else short_conv_kernel<bf16><<<grid, 256, 0, s>>>(a);
@@ -1104,9 +1122,8 @@ cudaError_t short_conv(cudaStream_t s, const ConvArgs& a) {
 cudaError_t conv_tails(cudaStream_t s, const ConvArgs& a) {
   if (a.B <= 0 || a.taps <= 1 || a.C <= 0) return cudaSuccess;
   dim3 grid((a.C + 255) / 256, a.B);
-  if (a.f32) conv_tails_kernel<float><<<grid, 256, 0, s>>>(a);
-  else conv_tails_kernel<bf16><<<grid, 256, 0, s>>>(a);
-  return cudaGetLastError();
+  if (a.f32) return launch_k(conv_tails_kernel<float>, grid, dim3(256), 0, s, true, a);
+  return launch_k(conv_tails_kernel<bf16>, grid, dim3(256), 0, s, true, a);
 }
 
 cudaError_t ssm_steps(cudaStream_t s, const float* p, long ldp, int off_dt, const void* a_dt, bool f32, float* ab, long ldab, int T, int H) {
@@ -1165,14 +1182,17 @@ cudaError_t memory_readout(cudaStream_t s, const float* num, long ldnum, const f
 }
 
 cudaError_t gated_group_norm(cudaStream_t s, const float* y, long ldy, const float* z, long ldz, const void* w, bool f32, float eps, int parts,
-                             float* out, bf16* outb, int T, int n, bool gate_last, const bf16* zb) {
+                             float* out, bf16* outb, int T, int n, bool gate_last, const bf16* zb,
+                             const Slabs* z_slabs, int z_col) {
   if (T <= 0) return cudaSuccess;
   if (parts < 1 || n % parts) return cudaErrorInvalidValue;
   dim3 grid(parts, T);
   const int len = n / parts;
+  const Slabs zsl = z_slabs ? *z_slabs : Slabs();
+  if (z_slabs && ((z_slabs->N | z_col) & 3)) return cudaErrorInvalidValue;
   if (len % 4 == 0 && len <= 8192 && ((ldy | ldz) & 3) == 0 && (((uintptr_t)y | (uintptr_t)z | (uintptr_t)out) & 15) == 0 && (((uintptr_t)outb | (uintptr_t)zb) & 7) == 0) {
 #define HB_GGN(WT, CH) \
-  return launch_k(gated_group_norm_vec_kernel<WT, CH>, dim3(T, parts), dim3(256), 0, s, true, y, ldy, z, zb, ldz, (const WT*)w, eps, parts, out, outb, n, (int)gate_last)
+  return launch_k(gated_group_norm_vec_kernel<WT, CH>, dim3(T, parts), dim3(256), 0, s, true, y, ldy, z, zb, ldz, (const WT*)w, eps, parts, out, outb, n, (int)gate_last, zsl, z_col)
 #define HB_GGN_T(CH) do { if (f32) HB_GGN(float, CH); else HB_GGN(bf16, CH); } while (0)
     // Fewer parts than the blocks that fit the machine are through sooner with a block each (us block | warp: 16 tokens x 8 parts of 512 entries 2.4 | 4.2, of
     // 256 2.4 | 3.0, 64 tokens 3.3 | 4.3 and 3.0 | 3.1, 300 tokens 6.6 | 6.0 and 6.2 | 4.3; of 128 2.7 | 2.4 at 16 tokens), wide parts always (2000 tokens x 4
@@ -1181,7 +1201,7 @@ cudaError_t gated_group_norm(cudaStream_t s, const float* y, long ldy, const flo
       const int items = T * parts;
 #define HB_GGW(WT, CH)                                                                                                                                        \
   return launch_k(gated_group_norm_warp_kernel<WT, CH>, dim3((items + 7) / 8), dim3(256), 0, s, true, y, ldy, z, zb, ldz, (const WT*)w, eps, parts, out, outb, \
-                  n, (int)gate_last, items)
+                  n, (int)gate_last, items, zsl, z_col)
 #define HB_GGW_T(CH) do { if (f32) HB_GGW(float, CH); else HB_GGW(bf16, CH); } while (0)
       if (len <= 128) HB_GGW_T(1);
       if (len <= 256) HB_GGW_T(2);
@@ -1196,7 +1216,7 @@ cudaError_t gated_group_norm(cudaStream_t s, const float* y, long ldy, const flo
 #undef HB_GGN_T
 #undef HB_GGN
   }
-  if (zb) return cudaErrorInvalidValue;
+  if (zb || z_slabs) return cudaErrorInvalidValue;
   if (f32) gated_group_norm_kernel<float><<<grid, 256, 0, s>>>(y, ldy, z, ldz, (const float*)w, eps, parts, out, outb, n, gate_last);
   else gated_group_norm_kernel<bf16><<<grid, 256, 0, s>>>(y, ldy, z, ldz, (const bf16*)w, eps, parts, out, outb, n, gate_last);
   return cudaGetLastError();
@@ -1215,6 +1235,7 @@ cudaError_t parallel_step(cudaStream_t s, const float* x, const int32_t* row_ind
                           bf16* h2b, int rows, int W, const ParScale* scale) {
   if (rows <= 0) return cudaSuccess;
   const ParScale sc = scale ? *scale : ParScale();
+  if ((sc.y_slabs.ws != nullptr) != (sc.y2_slabs.ws != nullptr) || (sc.y_slabs.ws && (y || y2 || sc.top_k > 0))) return cudaErrorInvalidValue;
   if (((y2 || sc.top_k > 0) && !y) || (sc.top_k > 0 && (y2 || !sc.rows || !sc.row_of || !sc.wts))) return cudaErrorInvalidValue;
   const uintptr_t al = (uintptr_t)x | (uintptr_t)y | (uintptr_t)y2 | (uintptr_t)bias | (uintptr_t)w1 | (uintptr_t)w2 | (uintptr_t)x_out | (uintptr_t)h1 |
                        (uintptr_t)h1b | (uintptr_t)h2 | (uintptr_t)h2b | (uintptr_t)sc.s1 | (uintptr_t)sc.s2 | (uintptr_t)sc.rows;
@@ -1228,7 +1249,7 @@ cudaError_t parallel_step(cudaStream_t s, const float* x, const int32_t* row_ind
     else { if (f32) HB_PAR(float, 8); else HB_PAR(bf16, 8); }
 #undef HB_PAR
   }
-  if ((size_t)W * 4 > 200 * 1024) return cudaErrorInvalidValue;
+  if ((size_t)W * 4 > 200 * 1024 || sc.y_slabs.ws) return cudaErrorInvalidValue;
   const size_t smem = (size_t)W * 4;
   if (f32)
     parallel_step_kernel<float><<<rows, 256, smem, s>>>(x, row_index, y, y2, (const float*)bias, bias_scale, (const float*)w1, (const float*)w2,
@@ -1241,8 +1262,7 @@ cudaError_t parallel_step(cudaStream_t s, const float* x, const int32_t* row_ind
 
 cudaError_t relu2_rows(cudaStream_t s, const float* in, long ldi, float* out, bf16* outb, int T, int n) {
   if (T <= 0 || n <= 0) return cudaSuccess;
-  relu2_kernel<<<dim3((n + 255) / 256, T), 256, 0, s>>>(in, ldi, out, outb, n);
-  return cudaGetLastError();
+  return launch_k(relu2_kernel, dim3((n + 255) / 256, T), dim3(256), 0, s, true, in, ldi, out, outb, n);
 }
 cudaError_t relu2_rows_b16(cudaStream_t s, const bf16* in, long ldi, bf16* out, int T, int n) {
   if (T <= 0 || n <= 0) return cudaSuccess;
