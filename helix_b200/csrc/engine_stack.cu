@@ -1043,11 +1043,17 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
   }
   const double preb = (2.0 * std::max(sd.streams, 1) + 2.0) * rowb;
   float* x_emb = pre ? k.y : k.x;  // (pre-normed stacks: the first step below makes the copies)
+  const ParNext start = par && sd.n_layers > 0 ? par_next(0) : ParNext{};
+  if (par && sd.embed_norm && !tnorm && embed_step_ok(model_.s_embed, model_.s_embed_norm, start.w1, start.w2, bigram, W)) {
+    SPAN(3, 3 * rowb, embed_step(stream_, tokens, model_.s_embed, sd.embed_scale != 0.f ? sd.embed_scale : 1.f, bigram, model_.s_embed_norm, goff, start.w1,
+                                 start.w2, f32, sd.norm_eps, k.x, start.h1, x16, start.h2, f32 ? nullptr : k.x16b, T, W));
+  } else {
   SPAN(3, rowb, embed_rows_f32(stream_, tokens, model_.s_embed, f32, x_emb, pre ? nullptr : x16, T, W, sd.embed_scale != 0.f ? sd.embed_scale : 1.f, bigram));
   if (sd.embed_norm) SPAN(3, 2 * rowb, norm_rows(x_emb, nullptr, model_.s_embed_norm, x_emb, both || pre ? nullptr : x16, T));
   if (pre) SPAN(3, preb, pre_step(k.y, nullptr, nullptr, nullptr, 0, 0, nullptr));
   if (both) SPAN(3, 2 * rowb, norm_rows(k.x, nullptr, model_.sw[0].norm1, k.hn, x16, T));
   if (par) SPAN(3, 3 * rowb, par_step(nullptr, nullptr, nullptr, 0.f, 0, nullptr));
+  }
   for (size_t si = 0; si < k.freq_sets.size(); ++si)  // cos / sin of the step's positions, once per distinct rotation
     SPAN(3, 8.0 * T * k.freq_half[si], stack_rope_table(stream_, positions, k.freq_sets[si], k.freq_half[si], k.rope_cs[si], T, k.freq_mult[si]));
   for (int i = 0; i < sd.n_layers; ++i) {

@@ -667,6 +667,11 @@ struct ParScale {
 cudaError_t parallel_step(cudaStream_t s, const float* x, const int32_t* row_index, const float* y, const float* y2, const void* bias,
                           float bias_scale, const void* w1, const void* w2, bool f32, float eps, float* x_out, float* h1, bf16* h1_b16,
                           float* h2, bf16* h2_b16, int rows, int W, const ParScale* sc = nullptr);
+// The start of such a stack: x[r] = v / rms(v) * (off + w0) of the embedding row v = scale table[token] (+ its bigram row), and the two normed
+// inputs of the first layer, h1 and h2, as parallel_step makes them.  embed_step_ok: the rows' sizes and addresses it takes
+bool embed_step_ok(const void* table, const void* w0, const void* w1, const void* w2, const BigramArgs& bg, int W);
+cudaError_t embed_step(cudaStream_t s, const int32_t* tokens, const void* table, float scale, const BigramArgs& bg, const void* w0, float off, const void* w1,
+                       const void* w2, bool f32, float eps, float* x, float* h1, bf16* h1_b16, float* h2, bf16* h2_b16, int T, int W);
 // out = relu(in)^2 (fp32 in, row stride ldi; fp32 and / or bf16 out, dense rows of n)
 cudaError_t relu2_rows(cudaStream_t s, const float* in, long ldi, float* out, bf16* out_b16, int T, int n);
 // the same on bf16 rows (tensor-core path)
