@@ -656,7 +656,9 @@ cudaError_t launch_portion(cudaStream_t s, const LinRecArgs& a) {
   constexpr int BC = portion_cols<DKP, CH, W>();
   const long blocks = (long)a.B * a.H * ((a.Dv + BC - 1) / BC);
   if (blocks > INT_MAX) return cudaErrorInvalidValue;
-  return launch_k(lin_portion_kernel<DKP, CH, W, MB>, dim3((unsigned)blocks), dim3(32 * W), portion_smem<DKP, CH, W>(), s, true, a);
+  // Not while the kernel before it drains, as others are: few long blocks, dealt out while that one still fills most SMs, sat three to five to an SM beside
+  // empty ones (3 sequences x 32 heads, a step 640 -> 752 us)
+  return launch_k(lin_portion_kernel<DKP, CH, W, MB>, dim3((unsigned)blocks), dim3(32 * W), portion_smem<DKP, CH, W>(), s, false, a);
 }
 
 // The same for entries of one token (decoding): bound by the state's bytes, 32 KB in and out per block of a 128 x 64 state.  Everything a
@@ -753,7 +755,7 @@ cudaError_t launch_rec(cudaStream_t s, const LinRecArgs& a) {
   constexpr int KS = DKP / 16, BC = 32 * NC, kRecTch = 16 / NC;
   const size_t smem = (size_t)(2 * kRecTch * (2 * DKP + BC + 4) + kRecTch * KS * BC + kRecTch * KS) * 4;
   dim3 grid(a.B, a.H, (a.Dv + BC - 1) / BC);
-  return launch_k(lin_recurrence_kernel<DKP, NC>, grid, dim3(DKP * 2), smem, s, true, a);
+  return launch_k(lin_recurrence_kernel<DKP, NC>, grid, dim3(DKP * 2), smem, s, false, a);  // (as launch_portion)
 }
 
 // ------------------------------------------------------------------ read-outs
@@ -838,9 +840,10 @@ __global__ void __launch_bounds__(256) gated_group_norm_kernel(const float* __re
   }
 }
 
+// (z from slabs is an instance of its own: the branch in the loop kept the rows' loads from being issued together, 114 -> 136 us)
 // Many parts of up to 512 entries: a warp each, no barrier, and no idle half of a block (a block per part of 512 entries: 11k tokens x 8 parts 185 -> 83
 // us).  The sum is the block's below, where warp c has 128 entries: a sum for each 128, added in the order of block_sum, so the two give the same bits.
-template <typename WT, int CH>
+template <typename WT, int CH, bool SLABS>
 __global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const float* __restrict__ y, long ldy, const float* __restrict__ z, const bf16* __restrict__ zb, long ldz,
                                                                     const WT* __restrict__ w, float eps, int parts, float* __restrict__ out,
                                                                     bf16* __restrict__ outb, int n, int gate_last, int items, const Slabs zsl, int z_col) {
@@ -861,7 +864,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const float*
     u[c] = g[c] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i >= len) continue;
     u[c] = *reinterpret_cast<const float4*>(ys + i);
-    g[c] = zsl.ws ? slab_sum4(zsl, t, z_col + c0 + i) : zs ? *reinterpret_cast<const float4*>(zs + i) : ldf4<bf16>(zbs + i);
+    g[c] = SLABS ? slab_sum4(zsl, t, z_col + c0 + i) : zs ? *reinterpret_cast<const float4*>(zs + i) : ldf4<bf16>(zbs + i);
   }
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
@@ -883,7 +886,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const float*
 }
 
 // The same with a part in registers as float4 (parts of a multiple of 4 entries, up to 4 * 256 * CH)
-template <typename WT, int CH>
+template <typename WT, int CH, bool SLABS>
 __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* __restrict__ y, long ldy, const float* __restrict__ z, const bf16* __restrict__ zb, long ldz,
                                                                    const WT* __restrict__ w, float eps, int parts, float* __restrict__ out,
                                                                    bf16* __restrict__ outb, int n, int gate_last, const Slabs zsl, int z_col) {
@@ -902,7 +905,7 @@ __global__ void __launch_bounds__(256) gated_group_norm_vec_kernel(const float* 
     u[c] = g[c] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i >= len) continue;
     u[c] = *reinterpret_cast<const float4*>(ys + i);
-    g[c] = zsl.ws ? slab_sum4(zsl, t, z_col + c0 + i) : zs ? *reinterpret_cast<const float4*>(zs + i) : ldf4<bf16>(zbs + i);
+    g[c] = SLABS ? slab_sum4(zsl, t, z_col + c0 + i) : zs ? *reinterpret_cast<const float4*>(zs + i) : ldf4<bf16>(zbs + i);
   }
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
@@ -1245,20 +1248,20 @@ cudaError_t gated_group_norm(cudaStream_t s, const float* y, long ldy, const flo
   dim3 grid(parts, T);
   const int len = n / parts;
   const Slabs zsl = z_slabs ? *z_slabs : Slabs();
-  if (z_slabs && ((z_slabs->N | z_col) & 3)) return cudaErrorInvalidValue;
+  if (z_slabs && (f32 || ((z_slabs->N | z_col) & 3))) return cudaErrorInvalidValue;
   if (len % 4 == 0 && len <= 8192 && ((ldy | ldz) & 3) == 0 && (((uintptr_t)y | (uintptr_t)z | (uintptr_t)out) & 15) == 0 && (((uintptr_t)outb | (uintptr_t)zb) & 7) == 0) {
-#define HB_GGN(WT, CH) \
-  return launch_k(gated_group_norm_vec_kernel<WT, CH>, dim3(T, parts), dim3(256), 0, s, true, y, ldy, z, zb, ldz, (const WT*)w, eps, parts, out, outb, n, (int)gate_last, zsl, z_col)
-#define HB_GGN_T(CH) do { if (f32) HB_GGN(float, CH); else HB_GGN(bf16, CH); } while (0)
+#define HB_GGN(WT, CH, SLABS) \
+  return launch_k(gated_group_norm_vec_kernel<WT, CH, SLABS>, dim3(T, parts), dim3(256), 0, s, true, y, ldy, z, zb, ldz, (const WT*)w, eps, parts, out, outb, n, (int)gate_last, zsl, z_col)
+#define HB_GGN_T(CH) do { if (f32) HB_GGN(float, CH, false); else if (z_slabs) HB_GGN(bf16, CH, true); else HB_GGN(bf16, CH, false); } while (0)
     // Fewer parts than the blocks that fit the machine are through sooner with a block each (us block | warp: 16 tokens x 8 parts of 512 entries 2.4 | 4.2, of
     // 256 2.4 | 3.0, 64 tokens 3.3 | 4.3 and 3.0 | 3.1, 300 tokens 6.6 | 6.0 and 6.2 | 4.3; of 128 2.7 | 2.4 at 16 tokens), wide parts always (2000 tokens x 4
     // parts of 1024 21 | 24)
     if (len <= 512 && (len <= 128 || (long)T * parts > 8 * effective_sms(148)) && (long)T * parts <= INT_MAX) {
       const int items = T * parts;
-#define HB_GGW(WT, CH)                                                                                                                                        \
-  return launch_k(gated_group_norm_warp_kernel<WT, CH>, dim3((items + 7) / 8), dim3(256), 0, s, true, y, ldy, z, zb, ldz, (const WT*)w, eps, parts, out, outb, \
-                  n, (int)gate_last, items, zsl, z_col)
-#define HB_GGW_T(CH) do { if (f32) HB_GGW(float, CH); else HB_GGW(bf16, CH); } while (0)
+#define HB_GGW(WT, CH, SLABS)                                                                                                                                 \
+  return launch_k(gated_group_norm_warp_kernel<WT, CH, SLABS>, dim3((items + 7) / 8), dim3(256), 0, s, true, y, ldy, z, zb, ldz, (const WT*)w, eps, parts,    \
+                  out, outb, n, (int)gate_last, items, zsl, z_col)
+#define HB_GGW_T(CH) do { if (f32) HB_GGW(float, CH, false); else if (z_slabs) HB_GGW(bf16, CH, true); else HB_GGW(bf16, CH, false); } while (0)
       if (len <= 128) HB_GGW_T(1);
       if (len <= 256) HB_GGW_T(2);
       HB_GGW_T(4);
