@@ -453,15 +453,15 @@ __global__ void __launch_bounds__(DKP * 2, 512 / DKP) lin_recurrence_kernel(LinR
 }
 
 // Portions without a normaliser: the same arithmetic (state elements, channel sums of eight, their sums pair by pair: the same bits as the
-// kernel above and the single-token one) in larger pieces.  A lane keeps CH channels of kPortionCols neighbouring columns, LS = DKP / CH lanes
-// share the columns.  What bounds it is the FMA pipe (active 68 % of the cycles, and what warps wait for first), and close behind shared memory: a read
-// hands a lane 16 bytes, 512 a warp, at 128 bytes a cycle
-// whoever shares the address, so q and k have to serve four columns each (two columns per lane, as above, take 84 cycles per warp and token,
-// four 45).  Tokens go in pairs, so that the 8 sums of a lane fold over the LS lanes with all of them useful and one
-// token's products cover the other's shuffles; one barrier per 16 tokens, no partial sums in shared memory.  Entries are taken longest first.
-// Prompts of 700 to 2048 tokens, 8 sequences x 64 heads of 128 x 64 states: 1670 -> 1030 us (327 active cycles of an SM per token and head);
-// one sequence of 2048 723 -> 383; 32 heads of 64 x 64, 8 sequences 237 -> 125.
-constexpr int kPortionCols = 4;
+// kernel above and the single-token one) in larger pieces.  A lane keeps CH channels of NC neighbouring columns, LS = DKP / CH lanes
+// share the columns.  What bounds it is the FMA pipe (active 68 % of the cycles with four columns, and what warps wait for first), and close behind shared
+// memory: a read hands a lane 16 bytes, 512 a warp, at 128 bytes a cycle whoever shares the address, so q and k have to serve many columns each.  Per warp and
+// token that is 84 cycles with two columns per lane, as above, 45 with four (16 channels of a 128-channel state), 36 with eight (8 channels: half the
+// reads of q and k for twice the sums over lanes), where three blocks fit an SM instead of four.  Tokens go in pairs, so that the sums of a lane fold over the
+// LS lanes with all of them useful and one token's products cover the other's shuffles; one barrier per 16 tokens, no partial sums in shared memory.
+// Entries are taken longest first.
+// Prompts of 700 to 2048 tokens, 8 sequences x 64 heads of 128 x 64 states: two columns 1670, four 1030, eight 1000 us (lin_portion_many);
+// one sequence of 2048 723 -> 383 (four columns); 32 heads of 64 x 64, 8 sequences 237 -> 125.
 // Sums of r[0 .. CNT) over LS lanes, neighbours first: while a lane has several it gives half of them away, so that lane s ends up with the sum `at`.
 template <int CNT, int X, int LS, int M>
 __device__ __forceinline__ void fold_lanes(float (&r)[M], int s, int& at) {
@@ -482,9 +482,8 @@ __device__ __forceinline__ void fold_lanes(float (&r)[M], int s, int& at) {
     }
   }
 }
-template <int DKP, int CH, int W, int MB>
+template <int DKP, int CH, int NC, int W, int MB>
 __global__ void __launch_bounds__(32 * W, MB) lin_portion_kernel(LinRecArgs a) {
-  constexpr int NC = kPortionCols;
   constexpr int LS = DKP / CH, CW = 32 / LS * NC, BC = W * CW, kTok = 16, NB = CH / 8, NT = 32 * W;
   constexpr int PS = LS + (CH == 8 ? 4 : 2), QS = CH * PS;  // float4 between pieces, floats of a row
   constexpr int per_tok = 2 * QS + BC + 4, stage_floats = kTok * per_tok;
@@ -640,6 +639,10 @@ __global__ void __launch_bounds__(32 * W, MB) lin_portion_kernel(LinRecArgs a) {
 // Narrower blocks where the wide ones are no more than the SMs (us wide / narrow: one sequence of 2048 tokens x 64 heads of 128 x 64 states
 // 492 / 383, four of 500 to 1000 316 / 361; 32 heads of 256 x 40 125 / 92)
 bool lin_portion_narrow(const LinRecArgs& a) { return a.Dk <= 64 || (long)a.B * a.H * ((a.Dv + 63) / 64) <= effective_sms(148); }
+// Eight columns per lane where there are more blocks than three per SM; fewer are bound by a token's chain, which the sums over twice the lanes lengthen (a step,
+// us, four columns | eight: 3 prompts of 1000 to 2048 tokens x 64 heads 1201 | 1217, 8 of 700 to 1500 x 32 heads 1022 | 1045; 8 of 200 to 400 x 64 heads
+// 697 | 679, of 700 to 2048 2578 | 2540, 32 of 50 to 100 x 32 heads with two tokens each 912 | 901)
+bool lin_portion_many(const LinRecArgs& a) { return (long)a.B * a.H * ((a.Dv + 63) / 64) > 3 * effective_sms(148); }
 // Short portions are bound by the state's bytes, which the smaller pieces above have more of in flight: from more than eight tokens on average on narrow blocks, 24 on
 // wide ones (us there | here, 32 sequences x 32 heads of 128 x 64 states: of 5 to 10 tokens 31 | 33, of 9 27 | 30, of 12 31 | 33, of 40 70 | 67; 8 sequences of 20
 // 19.4 | 20.2; 32 of 9 with 4 heads of 256 x 256 31 | 34; narrow, 8 of 9 with 4 heads of 256 x 256 15.6 | 12.5, 32 heads of 64 x 64 9.5 | 9.6)
@@ -647,18 +650,18 @@ bool lin_portion_ok(const LinRecArgs& a) {
   return !a.nq && a.T > (lin_portion_narrow(a) ? 8 : 24) * a.B && a.Dk > 32 && a.Dv > 32 && ((a.Dk | a.Dv | (int)a.ldq | (int)a.ldk | (int)a.ldv | a.q_off | a.k_off | a.v_off) & 3) == 0 &&
          ((a.slot_stride | (long)a.s_off) & 3) == 0 && (((uintptr_t)a.q | (uintptr_t)a.k | (uintptr_t)a.v | (uintptr_t)a.state) & 15) == 0;
 }
-template <int DKP, int CH, int W>
-constexpr int portion_cols() { return W * (32 / (DKP / CH)) * kPortionCols; }
-template <int DKP, int CH, int W>
-constexpr int portion_smem() { return 2 * 16 * (2 * CH * (DKP / CH + (CH == 8 ? 4 : 2)) + portion_cols<DKP, CH, W>() + 4) * 4; }
-template <int DKP, int CH, int W, int MB>
+template <int DKP, int CH, int NC, int W>
+constexpr int portion_cols() { return W * (32 / (DKP / CH)) * NC; }
+template <int DKP, int CH, int NC, int W>
+constexpr int portion_smem() { return 2 * 16 * (2 * CH * (DKP / CH + (CH == 8 ? 4 : 2)) + portion_cols<DKP, CH, NC, W>() + 4) * 4; }
+template <int DKP, int CH, int NC, int W, int MB>
 cudaError_t launch_portion(cudaStream_t s, const LinRecArgs& a) {
-  constexpr int BC = portion_cols<DKP, CH, W>();
+  constexpr int BC = portion_cols<DKP, CH, NC, W>();
   const long blocks = (long)a.B * a.H * ((a.Dv + BC - 1) / BC);
   if (blocks > INT_MAX) return cudaErrorInvalidValue;
   // Not while the kernel before it drains, as others are: few long blocks, dealt out while that one still fills most SMs, sat three to five to an SM beside
   // empty ones (3 sequences x 32 heads, a step 640 -> 752 us)
-  return launch_k(lin_portion_kernel<DKP, CH, W, MB>, dim3((unsigned)blocks), dim3(32 * W), portion_smem<DKP, CH, W>(), s, false, a);
+  return launch_k(lin_portion_kernel<DKP, CH, NC, W, MB>, dim3((unsigned)blocks), dim3(32 * W), portion_smem<DKP, CH, NC, W>(), s, false, a);
 }
 
 // The same for entries of one token (decoding): bound by the state's bytes, 32 KB in and out per block of a 128 x 64 state.  Everything a
@@ -1138,11 +1141,12 @@ cudaError_t stack_ssm_init() {
   HB_SMEM((lin_recurrence_kernel<64, 2>), 96 * 1024);
   HB_SMEM((lin_recurrence_kernel<128, 2>), 128 * 1024);
   HB_SMEM((lin_recurrence_kernel<256, 2>), 200 * 1024);
-  HB_SMEM((lin_portion_kernel<64, 8, 4, 5>), (portion_smem<64, 8, 4>()));
-  HB_SMEM((lin_portion_kernel<128, 8, 4, 5>), (portion_smem<128, 8, 4>()));
-  HB_SMEM((lin_portion_kernel<128, 16, 4, 4>), (portion_smem<128, 16, 4>()));
-  HB_SMEM((lin_portion_kernel<256, 16, 4, 4>), (portion_smem<256, 16, 4>()));
-  HB_SMEM((lin_portion_kernel<256, 16, 8, 2>), (portion_smem<256, 16, 8>()));
+  HB_SMEM((lin_portion_kernel<64, 8, 4, 4, 5>), (portion_smem<64, 8, 4, 4>()));
+  HB_SMEM((lin_portion_kernel<128, 8, 4, 4, 5>), (portion_smem<128, 8, 4, 4>()));
+  HB_SMEM((lin_portion_kernel<128, 16, 4, 4, 4>), (portion_smem<128, 16, 4, 4>()));
+  HB_SMEM((lin_portion_kernel<128, 8, 8, 4, 3>), (portion_smem<128, 8, 8, 4>()));
+  HB_SMEM((lin_portion_kernel<256, 16, 4, 4, 4>), (portion_smem<256, 16, 4, 4>()));
+  HB_SMEM((lin_portion_kernel<256, 16, 4, 8, 2>), (portion_smem<256, 16, 4, 8>()));
   HB_SMEM(parallel_step_kernel<float>, 200 * 1024);
   HB_SMEM(parallel_step_kernel<bf16>, 200 * 1024);
 #undef HB_SMEM
@@ -1207,9 +1211,9 @@ cudaError_t lin_recurrence(cudaStream_t s, const LinRecArgs& a) {
   if (lin_step_ok(a)) return launch_k(lin_step_kernel, dim3(a.B, a.H, (a.Dv + 63) / 64), dim3((a.Dk + 15) / 16 * 32), 0, s, true, a);
   if (lin_portion_ok(a)) {
     const bool few = lin_portion_narrow(a);
-    if (a.Dk <= 64) return launch_portion<64, 8, 4, 5>(s, a);
-    if (a.Dk <= 128) return few ? launch_portion<128, 8, 4, 5>(s, a) : launch_portion<128, 16, 4, 4>(s, a);
-    return few ? launch_portion<256, 16, 4, 4>(s, a) : launch_portion<256, 16, 8, 2>(s, a);
+    if (a.Dk <= 64) return launch_portion<64, 8, 4, 4, 5>(s, a);
+    if (a.Dk <= 128) return few ? launch_portion<128, 8, 4, 4, 5>(s, a) : lin_portion_many(a) ? launch_portion<128, 8, 8, 4, 3>(s, a) : launch_portion<128, 16, 4, 4, 4>(s, a);
+    return few ? launch_portion<256, 16, 4, 4, 4>(s, a) : launch_portion<256, 16, 4, 8, 2>(s, a);
   }
   // two columns per lane (blocks of 64 columns) halve the shared-memory reads per product; heads of up to 32 value columns
   // keep one.  HB_REC_COLS=1 forces the narrow blocks of this kernel (A/B measurements)
