@@ -1114,9 +1114,6 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
           in_slabs.ws = nullptr;
         }
       }
-      SPAN(3, 4.0 * T * C * (l.conv_taps + 1) + 12.0 * T * H, short_conv(stream_, ca));
-      if (!ca.single) SPAN(3, 8.0 * B * C * l.conv_taps, conv_tails(stream_, ca));
-      if (!fused) SPAN(3, 12.0 * T * H, ssm_steps(stream_, k.p1, k.ld1, w.off_a, w.a_dt, f32, k.ab, k.ldab, T, H));
       LinRecArgs ra{};
       ra.q = k.cv; ra.ldq = k.ldcv; ra.q_off = inner + G * N;
       ra.k = k.cv; ra.ldk = k.ldcv; ra.k_off = inner;
@@ -1130,9 +1127,17 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       ra.T = T; ra.B = B; ra.H = H; ra.G = G; ra.Dk = N; ra.Dv = Dv;
       ra.single = T == B;
       ra.settled = true;  // (a layer's states are written once per step, and every step is waited for)
-      SPAN(6, 4.0 * T * H * N * Dv, lin_recurrence(stream_, ra));
-      SPAN(3, 16.0 * T * inner, gated_group_norm(stream_, k.ctx, k.ldctx, in_slabs.ws ? nullptr : k.p1 + w.off_g, k.ld1, w.hnorm, f32, sd.norm_eps,
-                                                 l.norm_groups, mo_f32, mo16, T, inner, false, nullptr, in_slabs.ws ? &in_slabs : nullptr, w.off_g));
+      SsmTokenArgs ta{ca, ra, w.hnorm, sd.norm_eps, w.off_g, mo16};
+      if (in_slabs.ws && ssm_token_ok(ta, l.norm_groups)) {
+        SPAN(6, 4.0 * T * H * N * Dv, ssm_token(stream_, ta));
+      } else {
+        SPAN(3, 4.0 * T * C * (l.conv_taps + 1) + 12.0 * T * H, short_conv(stream_, ca));
+        if (!ca.single) SPAN(3, 8.0 * B * C * l.conv_taps, conv_tails(stream_, ca));
+        if (!fused) SPAN(3, 12.0 * T * H, ssm_steps(stream_, k.p1, k.ld1, w.off_a, w.a_dt, f32, k.ab, k.ldab, T, H));
+        SPAN(6, 4.0 * T * H * N * Dv, lin_recurrence(stream_, ra));
+        SPAN(3, 16.0 * T * inner, gated_group_norm(stream_, k.ctx, k.ldctx, in_slabs.ws ? nullptr : k.p1 + w.off_g, k.ld1, w.hnorm, f32, sd.norm_eps,
+                                                   l.norm_groups, mo_f32, mo16, T, inner, false, nullptr, in_slabs.ws ? &in_slabs : nullptr, w.off_g));
+      }
       if (paired) {
         SkinnyPlan plan{};
         CU(gemm_skinny_pair_plan(W, ocols, W, l.ff, &plan));

@@ -623,6 +623,15 @@ struct LinRecArgs {
   bool settled = false;
 };
 cudaError_t lin_recurrence(cudaStream_t s, const LinRecArgs& a);
+// A single-token step of a state-space layer between its two pairs of products, in one launch: what short_conv (with its tails, step sizes and squared
+// relu), lin_recurrence and gated_group_norm make of the slabs, the same bits.  c: as for short_conv with slabs; r: as for lin_recurrence
+// (q, k, v, ab and out are not used); the norm over the heads of a kv head, z in the columns from z_col on.  ssm_token_ok: the shapes it takes
+struct SsmTokenArgs {
+  ConvArgs c; LinRecArgs r;
+  const void* norm_w; float eps; int z_col; bf16* out;  // [T, H Dv]
+};
+bool ssm_token_ok(const SsmTokenArgs& a, int norm_groups);
+cudaError_t ssm_token(cudaStream_t s, const SsmTokenArgs& a);
 // S_t = decay_h S_(t-1) + k_t v_t^T, out_t = S_t^T q_t on the tensor cores, chunk by chunk (stack_lightning.cu): q, k [T, H * Dk] and
 // v [T, H * Dv] are bf16 columns (behind their activations) of rows of stride ld, out fp32, the state as for lin_recurrence.
 // error: a word that the host can read; set to 1 when a wait inside the kernel ran out (results are then void).

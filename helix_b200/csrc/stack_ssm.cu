@@ -21,6 +21,7 @@
 
 #include "kernels.h"
 #include "launch.h"
+#include "ptx.cuh"
 #include "stack_common.cuh"
 
 namespace hb {
@@ -664,6 +665,46 @@ cudaError_t launch_portion(cudaStream_t s, const LinRecArgs& a) {
   return launch_k(lin_portion_kernel<DKP, CH, NC, W, MB>, dim3((unsigned)blocks), dim3(32 * W), portion_smem<DKP, CH, NC, W>(), s, false, a);
 }
 
+// One token on 16 channels of two neighbouring columns (x, y of S): the states move on, o: their products with q; even and odd channels of eight
+// have a sum each.  k and q: four channels at a time
+template <typename K, typename Q>
+__device__ __forceinline__ void step_channels(float2 (&S)[16], float da, float bx, float by, K&& k, Q&& q, float2& o) {
+  float2 ox[2], oy[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 k4 = k(i), q4 = q(i);
+    const float kk[4] = {k4.x, k4.y, k4.z, k4.w}, qq[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float2& s = S[4 * i + e];
+      s.x = __fmaf_rn(da, s.x, __fmul_rn(kk[e], bx));
+      s.y = __fmaf_rn(da, s.y, __fmul_rn(kk[e], by));
+      float& sx = e & 1 ? ox[i / 2].y : ox[i / 2].x;
+      float& sy = e & 1 ? oy[i / 2].y : oy[i / 2].x;
+      sx = i % 2 == 0 && e < 2 ? __fmul_rn(s.x, qq[e]) : __fmaf_rn(s.x, qq[e], sx);
+      sy = i % 2 == 0 && e < 2 ? __fmul_rn(s.y, qq[e]) : __fmaf_rn(s.y, qq[e], sy);
+    }
+  }
+  o = make_float2((ox[0].x + ox[0].y) + (ox[1].x + ox[1].y), (oy[0].x + oy[0].y) + (oy[1].x + oy[1].y));
+}
+// the warps' shares of a lane's two columns, pair by pair
+template <int MAX>
+__device__ __forceinline__ float2 step_total(const float (&obuf)[MAX][64], int lane, int warps) {
+  float2 part[MAX];
+#pragma unroll
+  for (int ww = 0; ww < MAX; ++ww) part[ww] = ww < warps ? *reinterpret_cast<const float2*>(&obuf[ww][lane * 2]) : make_float2(0.f, 0.f);
+#pragma unroll
+  for (int st = 1; st < MAX; st *= 2) {
+    if (st >= warps) break;
+#pragma unroll
+    for (int ww = 0; ww < MAX; ww += 2 * st) {
+      part[ww].x += part[ww + st].x;
+      part[ww].y += part[ww + st].y;
+    }
+  }
+  return part[0];
+}
+
 // The same for entries of one token (decoding): bound by the state's bytes, 32 KB in and out per block of a 128 x 64 state.  Everything a
 // block needs is loaded at once (the staging above spent a round trip on the state, one on the token and three barriers): 16
 // sequences x 32 heads 12.2 -> 9.1 us.  Warp w has key channels 16 w .. 16 w + 15, a lane two neighbouring columns; the
@@ -703,45 +744,17 @@ __global__ void lin_step_kernel(LinRecArgs a) {
     act(vv.x);
     act(vv.y);
   }
-  // columns j0 (x) and j0 + 1 (y); even and odd channels of eight have a sum each
-  const float bx = db * vv.x, by = db * vv.y;
-  float2 ox[2], oy[2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float kk[4] = {k4[i].x, k4[i].y, k4[i].z, k4[i].w}, qq[4] = {q4[i].x, q4[i].y, q4[i].z, q4[i].w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float2& s = S[4 * i + e];
-      s.x = __fmaf_rn(da, s.x, __fmul_rn(kk[e], bx));
-      s.y = __fmaf_rn(da, s.y, __fmul_rn(kk[e], by));
-      float& sx = e & 1 ? ox[i / 2].y : ox[i / 2].x;
-      float& sy = e & 1 ? oy[i / 2].y : oy[i / 2].x;
-      sx = i % 2 == 0 && e < 2 ? __fmul_rn(s.x, qq[e]) : __fmaf_rn(s.x, qq[e], sx);
-      sy = i % 2 == 0 && e < 2 ? __fmul_rn(s.y, qq[e]) : __fmaf_rn(s.y, qq[e], sy);
-    }
-  }
+  float2 o2;
+  step_channels(S, da, db * vv.x, db * vv.y, [&](int i) { return k4[i]; }, [&](int i) { return q4[i]; }, o2);
 #pragma unroll
   for (int i = 0; i < 16; ++i)
     if (cols && i0 + i < a.Dk) *reinterpret_cast<float2*>(st + (size_t)i * a.Dv) = S[i];
-  obuf[w][lane * 2] = (ox[0].x + ox[0].y) + (ox[1].x + ox[1].y);
-  obuf[w][lane * 2 + 1] = (oy[0].x + oy[0].y) + (oy[1].x + oy[1].y);
+  *reinterpret_cast<float2*>(&obuf[w][lane * 2]) = o2;
   __syncthreads();
   const int warps = blockDim.x >> 5;
   if (w == 0 && cols) {
     const float skip = a.skip ? (a.f32 ? ((const float*)a.skip)[h] : __bfloat162float(((const bf16*)a.skip)[h])) : 0.f;
-    float2 part[16];
-#pragma unroll
-    for (int ww = 0; ww < 16; ++ww) part[ww] = ww < warps ? *reinterpret_cast<const float2*>(&obuf[ww][lane * 2]) : make_float2(0.f, 0.f);
-#pragma unroll
-    for (int st = 1; st < 16; st *= 2) {
-      if (st >= warps) break;
-#pragma unroll
-      for (int ww = 0; ww < 16; ww += 2 * st) {
-        part[ww].x += part[ww + st].x;
-        part[ww].y += part[ww + st].y;
-      }
-    }
-    const float2 o = part[0];
+    const float2 o = step_total<16>(obuf, lane, warps);
     *reinterpret_cast<float2*>(a.out + (size_t)t * a.ldo + (size_t)h * a.Dv + j0) = make_float2(fmaf(skip, vv.x, o.x * a.q_scale), fmaf(skip, vv.y, o.y * a.q_scale));
   }
 }
@@ -946,6 +959,154 @@ __global__ void gate_scale_kernel(const float* __restrict__ in, const bf16* __re
   const size_t d = (size_t)t * ldout + col0 + e;
   if (out) out[d] = v;
   if (outb) outb[d] = __float2bfloat16(v);
+}
+
+// ------------------------------------------------------------------ a single-token step between the products
+// Block = one head of one token, cluster = the HG heads that share a kv head (and a part of the gated norm).  A block convolves its head's
+// value channels and its share of the group's k and q channels, which meet in every block's shared memory; then the recurrence as in
+// lin_step_kernel, and the norm's sums of squares meet the same way, added in the order of gated_group_norm_vec_kernel.  The blocks behind the
+// tokens' make the feed-forward's inner rows.  What bounds it: the state's bytes (read before the products' launch is over) and a chain of
+// two round trips to L2, two cluster barriers and the recurrence; as three launches the same was 15 us of
+// a layer's 33 (16 sequences x 32 heads), 8 now; a turn of 2 such layers and 12 tokens 2520 -> 2450.
+template <typename T>
+__device__ __forceinline__ T* block_of_cluster(T* p, uint32_t cta) {  // the same shared-memory object in another block of the cluster
+  uint64_t r;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t>(p)), "r"(cta));
+  return reinterpret_cast<T*>(r);
+}
+constexpr int kTokDk = 128, kTokDv = 64, kTokTaps = 4;
+template <int HG>
+__global__ void __cluster_dims__(HG, 1, 1) __launch_bounds__(256, 4) ssm_token_kernel(const __grid_constant__ SsmTokenArgs a) {
+  __shared__ __align__(16) float kq[2 * kTokDk], vs[kTokDv], zs[kTokDv], quads[HG][16];
+  __shared__ __align__(16) float obuf[8][64];
+  __shared__ float ab[2];
+  pdl_launch_dependents();
+  const LinRecArgs& r = a.r;
+  const ConvArgs& c = a.c;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, heads = r.B * r.H;
+  if ((int)blockIdx.x >= heads) {  // (whole clusters of them)
+    const int per = (c.up.N / 4 + 255) / 256, at = blockIdx.x - heads, t = at / per, e = (at % per * 256 + tid) * 4;
+    pdl_wait();
+    if (t >= c.T || e >= c.up.N) return;
+    const float4 u = slab_sum4(c.up, t, e);
+    const float4 f = make_float4(fmaxf(u.x, 0.f), fmaxf(u.y, 0.f), fmaxf(u.z, 0.f), fmaxf(u.w, 0.f));
+    st_pair(nullptr, c.up_out + (size_t)t * c.up.N + e, make_float4(f.x * f.x, f.y * f.y, f.z * f.z, f.w * f.w));
+    return;
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // (this block runs: the others may write to it)
+  const uint32_t rank = cluster_ctarank();
+  const int b = blockIdx.x / r.H, h = blockIdx.x % r.H, kvh = h / HG, inner = r.H * kTokDv;
+  // what earlier steps and the loading of the model left, before the products are done
+  const int t = r.cu[b];
+  const bool fresh = r.first_pos[b] == 0;
+  float* const slot = r.state + (size_t)r.slots[b] * r.slot_stride;
+  const int i0 = w * 16, j0 = lane * 2;
+  float* const st = slot + r.s_off + (size_t)h * kTokDk * kTokDv + (size_t)i0 * kTokDv + j0;
+  float2 S[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) S[i] = fresh ? make_float2(0.f, 0.f) : *reinterpret_cast<const float2*>(st + (size_t)i * kTokDv);
+  // conv threads: four channels each, first the head's values, then this block's share of k | q
+  constexpr int kShare = 2 * kTokDk / HG, kConvThreads = (kTokDv + kShare) / 4;
+  const int ch = tid * 4 < kTokDv ? h * kTokDv + tid * 4 : 0, shared_at = tid * 4 - kTokDv + (int)rank * kShare;  // place in k | q
+  const bool conv = tid < kConvThreads, value = tid * 4 < kTokDv;
+  const int cc = value ? ch : inner + (shared_at < kTokDk ? kvh * kTokDk + shared_at : r.G * kTokDk + kvh * kTokDk + shared_at - kTokDk);
+  float4 win[kTokTaps - 1];
+  uint4 cw[2];  // four taps of the four channels
+  uint2 cb = make_uint2(0u, 0u);
+  float* const tail = slot + c.tail_off + cc;
+  if (conv) {
+#pragma unroll
+    for (int j = 0; j < kTokTaps - 1; ++j) win[j] = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(tail + (size_t)j * c.C);
+    cw[0] = reinterpret_cast<const uint4*>((const bf16*)c.w + (size_t)cc * kTokTaps)[0];
+    cw[1] = reinterpret_cast<const uint4*>((const bf16*)c.w + (size_t)cc * kTokTaps)[1];
+    if (c.bias) cb = *reinterpret_cast<const uint2*>((const bf16*)c.bias + cc);
+  }
+  pdl_wait();
+  if (tid >= 128 && tid < 144) {
+    *reinterpret_cast<float4*>(&zs[(tid - 128) * 4]) = slab_sum4(c.slabs, t, a.z_col + h * kTokDv + (tid - 128) * 4);
+  } else if (tid == 160) {
+    const bf16* p = (const bf16*)c.a_dt;
+    const float dt = softplus_(slab_sum1(c.slabs, t, c.off_dt + h) + ldf<bf16>(p, r.H + h));
+    ab[0] = expf(-expf(ldf<bf16>(p, h)) * dt);
+    ab[1] = dt;
+  }
+  float4 made = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (conv) {
+    const float4 x = slab_sum4(c.slabs, t, c.off + cc);
+    const uint32_t wp[8] = {cw[0].x, cw[0].y, cw[0].z, cw[0].w, cw[1].x, cw[1].y, cw[1].z, cw[1].w}, bp[2] = {cb.x, cb.y};
+    auto half = [](uint32_t u, int hi) { return __uint_as_float(hi ? u & 0xffff0000u : u << 16); };
+    float acc[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      auto of = [&](const float4& v) { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; };
+      acc[e] = 0.f;
+#pragma unroll
+      for (int j = 0; j < kTokTaps; ++j) acc[e] = fmaf(half(wp[2 * e + j / 2], j & 1), of(j < kTokTaps - 1 ? win[j] : x), acc[e]);
+      if (c.bias) acc[e] += half(bp[e / 2], e & 1);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] = acc[e] * sigmoidf_(acc[e]);
+    made = make_float4(acc[0], acc[1], acc[2], acc[3]);
+#pragma unroll
+    for (int j = 0; j + 1 < kTokTaps - 1; ++j) *reinterpret_cast<float4*>(tail + (size_t)j * c.C) = win[j + 1];
+    *reinterpret_cast<float4*>(tail + (size_t)(kTokTaps - 2) * c.C) = x;
+    if (value) *reinterpret_cast<float4*>(&vs[tid * 4]) = made;
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (conv && !value) {
+#pragma unroll
+    for (int o = 0; o < HG; ++o) *block_of_cluster(reinterpret_cast<float4*>(&kq[shared_at]), o) = made;
+  }
+  __syncwarp();
+  cluster_sync_all();
+  const float da = ab[0], db = ab[1];
+  const float2 vv = *reinterpret_cast<const float2*>(&vs[j0]);
+  float2 o2;
+  step_channels(S, da, db * vv.x, db * vv.y, [&](int i) { return *reinterpret_cast<const float4*>(&kq[i0 + 4 * i]); },
+                [&](int i) { return *reinterpret_cast<const float4*>(&kq[kTokDk + i0 + 4 * i]); }, o2);
+  *reinterpret_cast<float2*>(&obuf[w][j0]) = o2;
+  __syncthreads();
+  float4 u = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (w == 0) {
+    const float skip = r.skip ? __bfloat162float(((const bf16*)r.skip)[h]) : 0.f;
+    const float2 o = step_total<8>(obuf, lane, 8);
+    *reinterpret_cast<float2*>(&vs[j0]) = make_float2(fmaf(skip, vv.x, o.x * r.q_scale), fmaf(skip, vv.y, o.y * r.q_scale));  // (a lane's own columns)
+    __syncwarp();
+    if (lane < 16) {
+      const float4 y = *reinterpret_cast<const float4*>(&vs[lane * 4]), z = *reinterpret_cast<const float4*>(&zs[lane * 4]);
+      const float4 s = make_float4(sigmoidf_(z.x), sigmoidf_(z.y), sigmoidf_(z.z), sigmoidf_(z.w));
+      u = make_float4(y.x * (z.x * s.x), y.y * (z.y * s.y), y.z * (z.z * s.z), y.w * (z.w * s.w));
+      const float ss = sum_of_squares(u);
+#pragma unroll
+      for (int o2 = 0; o2 < HG; ++o2) *block_of_cluster(&quads[rank][lane], o2) = ss;
+    }
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) *reinterpret_cast<float2*>(st + (size_t)i * kTokDv) = S[i];
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (w == 0) {
+    float part[HG / 2];  // a warp of the block kernel has 128 entries, two heads: one's below lane 16, the other's above
+#pragma unroll
+    for (int p = 0; p < HG / 2; ++p) {
+      float s = quads[2 * p][lane & 15] + quads[2 * p + 1][lane & 15];
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      part[p] = s;
+    }
+#pragma unroll
+    for (int o = HG / 4; o > 0; o >>= 1)
+#pragma unroll
+      for (int p = 0; p < o; ++p) part[p] += part[p + o];
+    const float rs = 1.f / sqrtf(part[0] / (float)(HG * kTokDv) + a.eps);
+    if (lane < 16) {
+      const int col = h * kTokDv + lane * 4;
+      const bf16* nw = (const bf16*)a.norm_w + col;
+      st_pair(nullptr, a.out + (size_t)t * inner + col, make_float4(u.x * rs * ldf<bf16>(nw, 0), u.y * rs * ldf<bf16>(nw, 1), u.z * rs * ldf<bf16>(nw, 2), u.w * rs * ldf<bf16>(nw, 3)));
+    }
+  }
 }
 
 // ------------------------------------------------------------------ residual step of parallel sublayers
@@ -1220,6 +1381,25 @@ cudaError_t exp_gate_scan(cudaStream_t s, const GateScanArgs& a) {
   if (a.f32) exp_gate_scan_kernel<float><<<dim3(a.B, a.H), 32, 0, s>>>(a);
   else exp_gate_scan_kernel<bf16><<<dim3(a.B, a.H), 32, 0, s>>>(a);
   return cudaGetLastError();
+}
+
+bool ssm_token_ok(const SsmTokenArgs& a, int norm_groups) {
+  const ConvArgs& c = a.c;
+  const LinRecArgs& r = a.r;
+  const int hg = r.G > 0 && r.H % r.G == 0 ? r.H / r.G : 0;
+  return (hg == 2 || hg == 4 || hg == 8) && norm_groups == r.G && r.Dk == kTokDk && r.Dv == kTokDv && c.taps == kTokTaps && c.act == 1 && !c.f32 && !c.in_bias &&
+         r.settled && r.single && c.single && !r.head_decay && !r.silu && !r.nq && c.slabs.ws && c.up_out && c.a_dt &&
+         c.C == (r.H * kTokDv + 2 * r.G * kTokDk) && c.T == r.B && r.state == c.state && r.slot_stride == c.slot_stride &&
+         (((long)c.off | c.off_dt | a.z_col | c.slot_stride | (long)c.tail_off | (long)r.s_off | c.slabs.N | c.up.N) & 3) == 0 && ((uintptr_t)c.state & 15) == 0 &&
+         (((uintptr_t)a.out | (uintptr_t)c.up_out | (uintptr_t)c.bias) & 7) == 0 && ((uintptr_t)c.w & 15) == 0;
+}
+cudaError_t ssm_token(cudaStream_t s, const SsmTokenArgs& a) {
+  if (a.r.B <= 0) return cudaSuccess;
+  const int hg = a.r.H / a.r.G, up = a.c.T * ((a.c.up.N / 4 + 255) / 256);
+  const dim3 grid(a.r.B * a.r.H + (up + hg - 1) / hg * hg);
+  if (hg == 8) return launch_k(ssm_token_kernel<8>, grid, dim3(256), 0, s, true, a);
+  if (hg == 4) return launch_k(ssm_token_kernel<4>, grid, dim3(256), 0, s, true, a);
+  return hg == 2 ? launch_k(ssm_token_kernel<2>, grid, dim3(256), 0, s, true, a) : cudaErrorInvalidValue;
 }
 
 cudaError_t lin_recurrence(cudaStream_t s, const LinRecArgs& a) {

@@ -1,0 +1,40 @@
+"""Single-token steps of state-space layers in one launch between the products (heads of 128 x 64 states, four taps, a norm part per kv head): the bits
+of the same tokens beside a portion, where every entry takes the kernels for portions, for 2, 4 and 8 heads per kv head, sequences that start beside
+running ones, inner rows that are no whole number of blocks."""
+import numpy as np
+import pytest
+
+import helix_b200 as hb
+from helix_b200 import engine as E
+
+pytestmark = pytest.mark.gpu
+VOCAB = 192
+
+
+@pytest.mark.parametrize("heads,groups,ff", [(2, 1, 256), (4, 1, 1032), (8, 1, 512), (8, 2, 2056), (16, 2, 320), (4, 2, 64)])
+@pytest.mark.parametrize("seqs", [1, 3, 33])
+def test_single_tokens_have_the_bits_of_portions(heads, groups, ff, seqs):
+    layers = [E.LayerDesc(mixer=E.MIXER_MAMBA2, heads=heads, vdim=64, dim=128, kv_heads=groups, norm_groups=groups, conv_taps=4, ff_kind=E.FF_RELU2, ff=ff)
+              for _ in range(2)]
+    d = E.StackDesc(width=128, vocab=VOCAB, layers=layers, norm_eps=1e-5, norm_place=E.NORM_PARALLEL, embed_norm=1, plain_gains=1, tie_head=1)
+    rng = np.random.default_rng(heads * 100 + seqs)
+    toks = rng.integers(0, VOCAB, (seqs, 9)).astype(np.int32)
+    steps, got, launches = 9, [], []
+    with hb.Engine(hb.EngineConfig(max_seqs=seqs + 1, max_ctx=64, max_batched_tokens=256, kv_pool_tokens=64 * (seqs + 1))) as e:
+        e.load_random(d, 5)
+        for beside in (False, True):
+            ids, rows = [e.seq_open() for _ in range(seqs)], []
+            for t in range(steps):
+                live = [i for i in range(seqs) if i % 3 <= t]  # sequences begin at three different steps
+                feed = [(ids[i], toks[i, t - i % 3:t - i % 3 + 1], [0]) for i in live]
+                other = [e.seq_open()] if beside else []
+                n0 = e.stats()["kernel_launches"]
+                rows.append(e.seq_step(feed + [(s, [1, 2], []) for s in other]))
+                launches.append(e.stats()["kernel_launches"] - n0)
+                for s in other:
+                    e.seq_close(s)
+            for s in ids:
+                e.seq_close(s)
+            got.append(np.concatenate(rows))
+    assert launches[0] < launches[-1]  # (another path)
+    assert np.isfinite(got[0]).all() and np.array_equal(got[0], got[1])
