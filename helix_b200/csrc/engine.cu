@@ -166,6 +166,7 @@ void Engine::free_all() {
     p = nullptr;
   };
   frh(h_step_);
+  frh(h_rows_);
   frh(h_sampled_);
   frh(kernel_error_);
   frh(h_lp_ids_);
@@ -1372,6 +1373,8 @@ int Engine::run_prefill(std::vector<Request*>& batch) {
   if (rc != HB_OK) return rc;
   CU(cudaEventRecord(fwd_b_, stream_));
   if (!step_driven_) CU(cudaMemcpyAsync(h_sampled_, sampled_, (size_t)B * 4, cudaMemcpyDeviceToHost, stream_));
+  else if (n_extra > 0 && (size_t)n_extra * d.vocab <= h_rows_floats_)
+    CU(cudaMemcpyAsync(h_rows_, all_logits_, (size_t)n_extra * d.vocab * 4, cudaMemcpyDeviceToHost, stream_));
   CU(cudaStreamSynchronize(stream_));
   if (kernel_error_ && *kernel_error_) {
     *kernel_error_ = 0;

@@ -245,6 +245,8 @@ class Engine {
   float* rope_cs_ = nullptr;  // [t_cap][head_dim] cos | sin of the current step's positions (EPI_ROPE)
   float* logits_ = nullptr;
   float* dec_ws_ = nullptr;
+  float* h_rows_ = nullptr;     // pinned: a driven step's logits on their way out, up to h_rows_floats_ of them
+  size_t h_rows_floats_ = 0;
   size_t skinny_floats_ = 0;    // of skinny_ws_, layer-list decoders
   float* skinny_ws_ = nullptr;  // fp32 partial slabs of the decode-step GEMMs
   SkinnyPlan plan_qkv_{}, plan_o_{}, plan_gu_{}, plan_down_{}, plan_head_{};

@@ -602,6 +602,8 @@ int Engine::alloc_runtime_stack() {
   CU(cudaMalloc(&d_step_, step_bytes_));
   CU(cudaMallocHost(&h_step_, step_bytes_));
   CU(cudaMallocHost(&h_sampled_, (size_t)b_cap_ * 4));
+  h_rows_floats_ = std::min<size_t>((size_t)b_cap_ * sd.vocab, 1 << 20);  // (a row per sequence, at most 4 MB)
+  CU(cudaMallocHost(&h_rows_, h_rows_floats_ * 4));
   CU(cudaMallocHost(&kernel_error_, sizeof(int)));
   *kernel_error_ = 0;
   CU(cudaMallocHost(&h_lp_ids_, (size_t)cfg_.max_seqs * HB_MAX_LOGPROBS * 4));
@@ -1621,7 +1623,11 @@ int Engine::seq_step(const hb_seq_feed* entries, int n, float* out, size_t cap, 
   int rc = run_prefill(batch);
   step_driven_ = false;
   if (rc != HB_OK) return rc;  // a CUDA failure is sticky; the sequences keep their records for hb_seq_close
-  if (R > 0) CU(cudaMemcpy(out, all_logits_, (size_t)R * model_.d.vocab * 4, cudaMemcpyDeviceToHost));
+  // Few rows have come with the step's own wait, through pinned memory: the copy to the caller's pageable memory was a second round trip and a
+  // copy by the driver (a turn of 16 sequences, a vocabulary of 4096, 12 tokens each 2445 -> 2374 us)
+  const size_t floats = (size_t)R * model_.d.vocab;
+  if (R > 0 && floats <= h_rows_floats_) memcpy(out, h_rows_, floats * 4);
+  else if (R > 0) CU(cudaMemcpy(out, all_logits_, floats * 4, cudaMemcpyDeviceToHost));
   {
     std::lock_guard<std::mutex> g(mu_);
     for (Request* r : batch) {
