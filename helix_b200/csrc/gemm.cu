@@ -4,9 +4,9 @@
 //   warp 0 lane 0 : TMA producer   (cp.async.bulk.tensor -> 128B-swizzled smem ring, mbarrier tx-count)
 //   warp 1 lane 0 : MMA issuer     (tcgen05.mma cta_group::1, M=128 x N=BLOCK_N x K=16, fp32 accum in TMEM,
 //                                   double-buffered accumulators so tile i+1's MMAs overlap tile i's epilogue)
-//   warps 2..9    : epilogue       (tcgen05.ld -> fused bias / GELU / residual / SwiGLU -> swizzled smem -> TMA store);
-//                                   two groups of four warps (one warp per TMEM lane quadrant) take alternate 64-column
-//                                   chunks with their own staging buffer, so two warps per SM sub-partition hide each
+//   warps 2..     : epilogue       (tcgen05.ld -> fused bias / GELU / residual / SwiGLU -> swizzled smem -> TMA store);
+//                                   two or four groups of four warps (one warp per TMEM lane quadrant) take the 64-column
+//                                   chunks in turn with their own staging buffer, so two warps per SM sub-partition hide each
 //                                   other's TMEM/global latencies and short-K tiles (BERT) are not epilogue-bound
 // M, N, K tails are handled by TMA (zero fill on load, clipping on store).
 #include <math.h>
@@ -28,7 +28,6 @@ namespace {
 constexpr int BLOCK_M = 128;
 constexpr int BLOCK_K = 64;  // 64 bf16 = 128 B = one swizzle span
 constexpr int UMMA_K = 16;
-constexpr int kNumThreads = 320;   // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue (two groups of four)
 constexpr int kEpiThreads = 128;   // per epilogue group
 constexpr int kEpiBarrier = 1;     // named barrier id of group 0 (group 1 uses +1)
 constexpr int kStagingBytes = BLOCK_M * 128;  // one 128-row x 128-byte chunk
@@ -36,12 +35,14 @@ constexpr int kSmemBudget = 227 * 1024;
 
 // CG = CTAs cooperating on one UMMA (cta_group): with CG == 2 a CTA pair (cluster of 2 = one TPC) computes a 256 x BN
 // tile; each CTA stages its own 128 rows of A and HALF of the W tile, so per-SM smem/L2 operand traffic drops by a third.
-template <int BN, int CG = 1>
+// EG = groups of four epilogue warps, a staging buffer each
+template <int BN, int CG = 1, int EG = 2>
 struct Cfg {
+  static constexpr int THREADS = 64 + EG * kEpiThreads;  // warp 0 TMA, warp 1 MMA, then the epilogue
   static constexpr int A_BYTES = BLOCK_M * BLOCK_K * 2;
   static constexpr int B_BYTES = (BN / CG) * BLOCK_K * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int FIXED = 2 * kStagingBytes + 1024 /*align slack*/ + 512 /*barriers*/;
+  static constexpr int FIXED = EG * kStagingBytes + 1024 /*align slack*/ + 512 /*barriers*/;
   static constexpr int STAGES_RAW = (kSmemBudget - FIXED) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 10 ? 10 : STAGES_RAW;
   static constexpr int SMEM = STAGES * STAGE_BYTES + FIXED;
@@ -93,13 +94,13 @@ __device__ __forceinline__ float gelu_tanh_f(float z) {
 }
 __device__ __forceinline__ float silu(float x) { return x / (1.0f + __expf(-x)); }
 
-template <int BN, int EPI, int CG = 1>
-__global__ void __launch_bounds__(kNumThreads, 1)
+template <int BN, int EPI, int CG = 1, int EG = 2>
+__global__ void __launch_bounds__(64 + EG * kEpiThreads, 1)
 gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_r,
                const bf16* __restrict__ bias, int M, int N, int K, int tile_grp, int tile_group_n,
                const __grid_constant__ RopeEpi rope, const int32_t* __restrict__ m_tile_group, float glu_limit, int silu_cols) {
-  using C = Cfg<BN, CG>;
+  using C = Cfg<BN, CG, EG>;
   constexpr int TILE_M = BLOCK_M * CG;  // rows of one UMMA tile (per CTA: BLOCK_M)
   const uint32_t cta_rank = (CG == 2) ? cluster_ctarank() : 0u;
   const bool is_leader = cta_rank == 0;
@@ -121,14 +122,14 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * C::A_BYTES;
-  uint8_t* staging = smem + STAGES * C::STAGE_BYTES;  // 2 x 16 KB, 1024-aligned
-  uint64_t* bars = reinterpret_cast<uint64_t*>(staging + 2 * kStagingBytes);
+  uint8_t* staging = smem + STAGES * C::STAGE_BYTES;  // EG x 16 KB, 1024-aligned
+  uint64_t* bars = reinterpret_cast<uint64_t*>(staging + EG * kStagingBytes);
   uint64_t* full_bar = bars;                    // [STAGES]
   uint64_t* empty_bar = bars + STAGES;          // [STAGES]
   uint64_t* tmem_full = bars + 2 * STAGES;      // [2]
   uint64_t* tmem_empty = bars + 2 * STAGES + 2; // [2]
-  uint64_t* resid_bar = bars + 2 * STAGES + 4;  // [2] one per epilogue group
-  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 6);
+  uint64_t* resid_bar = bars + 2 * STAGES + 4;  // [EG] one per epilogue group
+  uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4 + EG);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -150,10 +151,9 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 8 * CG);  // epilogue warps of BOTH CTAs release the leader's accumulator stage
+      mbar_init(&tmem_empty[i], 4 * EG * CG);  // epilogue warps of BOTH CTAs release the leader's accumulator stage
     }
-    mbar_init(&resid_bar[0], 1);
-    mbar_init(&resid_bar[1], 1);
+    for (int i = 0; i < EG; ++i) mbar_init(&resid_bar[i], 1);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -252,10 +252,10 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     }
   } else {
-    // ===================== epilogue (warps 2..9) =====================
+    // ===================== epilogue (warps 2 and up) =====================
     const int q = warp & 3;               // TMEM lane quadrant this warp may access
     const int row = q * 32 + lane;        // row within the 128-row tile == TMEM lane
-    const int grp = (warp - 2) >> 2;      // epilogue group: chunks c == grp (mod 2), staging buffer `grp`
+    const int grp = (warp - 2) >> 2;      // epilogue group: chunks c == grp (mod EG), staging buffer `grp`
     const bool leader = ((threadIdx.x - 64) & 127) == 0;
     uint8_t* const buf = staging + grp * kStagingBytes;
     uint8_t* const my_row = buf + row * 128;
@@ -295,7 +295,7 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int slot = (row_ok && rope.slots) ? rope.slots[row_g] : -1;
         const int page = slot >= 0 ? slot / rope.page_size : 0, off = slot >= 0 ? slot % rope.page_size : 0;
         bf16* const orow = rope.out + (size_t)(row_ok ? row_g : 0) * rope.ldc;
-        for (int hl = grp; hl < BN / D; hl += 2) {
+        for (int hl = grp; hl < BN / D; hl += EG) {
           const int n_head0 = n_out0 + hl * D;
           const int hidx = n_head0 / D;
           const int kind = hidx < rope.Hq ? 0 : (hidx < rope.Hq + rope.Hkv ? 1 : 2);  // q / k / v
@@ -366,14 +366,14 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         continue;
       }
       int last_c = -1;
-      for (int c = grp; c < NCHUNK; c += 2) last_c = c;
+      for (int c = grp; c < NCHUNK; c += EG) last_c = c;
       if (last_c < 0) {  // this group has no chunk in such a narrow tile: release the accumulator right away
         tc_fence_before();
         __syncwarp();
         if (lane == 0) { if (CG == 2) mbar_arrive_cluster(&tmem_empty[as], 0); else mbar_arrive(&tmem_empty[as]); }
       }
 #pragma unroll 1
-      for (int c = grp; c < NCHUNK; c += 2) {
+      for (int c = grp; c < NCHUNK; c += EG) {
         if (leader) {
           if (!early || c != grp) tma_store_wait_read<0>();  // this group's previous store is done reading `buf`
           if (kResid && (!early || c != grp)) {
@@ -503,9 +503,9 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
 }
 
-template <int BN, int EPI, int CG>
+template <int BN, int EPI, int CG, int EG = 2>
 cudaError_t launch_cfg(cudaStream_t stream, const GemmArgs& g, int num_sms) {
-  using C = Cfg<BN, CG>;
+  using C = Cfg<BN, CG, EG>;
   constexpr bool kF32 = (EPI == EPI_F32);
   constexpr bool kSwiGLU = (EPI == EPI_SWIGLU || EPI == EPI_GEGLU || EPI == EPI_CLAMPGLU);
   constexpr int TILE_M = BLOCK_M * CG;
@@ -525,7 +525,7 @@ cudaError_t launch_cfg(cudaStream_t stream, const GemmArgs& g, int num_sms) {
   } else {
     mr = mc;
   }
-  auto kern = gemm_tn_kernel<BN, EPI, CG>;
+  auto kern = gemm_tn_kernel<BN, EPI, CG, EG>;
   static bool attr_set = false;  // per template instantiation
   if (!attr_set) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
@@ -548,7 +548,7 @@ cudaError_t launch_cfg(cudaStream_t stream, const GemmArgs& g, int num_sms) {
   if (force_gm > 0) { group_n = 0; grp = std::min(force_gm, num_m); }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(workers * CG);
-  cfg.blockDim = dim3(kNumThreads);
+  cfg.blockDim = dim3(C::THREADS);
   cfg.dynamicSmemBytes = C::SMEM;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -576,11 +576,16 @@ bool use_pair() {  // HB_GEMM_2CTA=0 falls back to single-CTA tiles (A/B measure
   return on;
 }
 
+// Epilogues with more to do than scale and store: on tiles of few k blocks four groups of warps work on them, where a stage of operands less costs
+// nothing (us, two groups | four: 7000 x 3072 x 768 gelu 41.8 | 37.8, 13800 61 | 58, 13800 x 768 x 768 residual, 192 columns 30.8 | 27.5; with K = 3072 55 | 59, and
+// without either 13800 x 2304 x 768 42 | 47: those have two)
+constexpr bool deep_epilogue(int epi) { return epi == EPI_BIAS_GELU || epi == EPI_GELU || epi == EPI_RESID || epi == EPI_BIAS_RESID; }
+
 template <int EPI>
 cudaError_t launch_epi(cudaStream_t stream, const GemmArgs& g, int num_sms) {
   constexpr bool kWideOnly = EPI == EPI_SWIGLU || EPI == EPI_GEGLU || EPI == EPI_CLAMPGLU || EPI == EPI_ROPE;
   const bool pairs = use_pair() && !g.m_tile_group;
-  int bn = g.block_n, cg = 1;
+  int bn = g.block_n, cg = 1, eg = 2;
   if (bn == 0) {
     // The tile shape whose waves end first.  Per shape: us per 64-deep k block of one tile, the least a wave takes (its epilogue, when K
     // is short) and the part of a launch that does not depend on K, fitted to runs on random operands:
@@ -598,24 +603,30 @@ cudaError_t launch_epi(cudaStream_t stream, const GemmArgs& g, int num_sms) {
     // four times the products in a pair's 256 x 256, 28 KB for three times in 256 x 192), wide ones leave SMs without a tile.  The rule before,
     // "halve the width until there are two waves", took 128 x 64 for the first, third and seventh line.  Every shape walks K in order: a row's
     // result does not depend on the choice.
-    struct Shape { int bn, cg; double kb, floor, fixed; };
-    static constexpr Shape shapes[] = {{256, 2, 0.36, 5.6, 8.5}, {192, 2, 0.29, 4.8, 8.3}, {128, 2, 0.235, 3.4, 8.0}, {256, 1, 0.42, 6.0, 7.0}, {128, 1, 0.28, 3.9, 6.5}, {64, 1, 0.235, 3.1, 6.0}};
+    struct Shape { int bn, cg, eg; double kb, floor, fixed; };
+    static constexpr Shape shapes[] = {{256, 2, 2, 0.36, 5.6, 8.5}, {256, 2, 4, 0.375, 5.2, 8.5}, {192, 2, 2, 0.29, 4.8, 8.3}, {192, 2, 4, 0.305, 4.3, 8.3}, {128, 2, 2, 0.235, 3.4, 8.0},
+                                       {256, 1, 2, 0.42, 6.0, 7.0}, {128, 1, 2, 0.28, 3.9, 6.5}, {64, 1, 2, 0.235, 3.1, 6.0}};
     const int num_kb = (g.K + BLOCK_K - 1) / BLOCK_K;
     double best = 1e30;
     for (const Shape& t : shapes) {
-      if ((t.cg == 2 && (!pairs || num_sms < 2)) || (kWideOnly && t.bn != 256)) continue;
+      if ((t.cg == 2 && (!pairs || num_sms < 2)) || (kWideOnly && t.bn != 256) || (t.eg != 2 && !deep_epilogue(EPI))) continue;
       const long tiles = (long)((g.M + BLOCK_M * t.cg - 1) / (BLOCK_M * t.cg)) * ((g.N + t.bn - 1) / t.bn);
       const long workers = std::max(1, num_sms / t.cg);
       const double us = (double)((tiles + workers - 1) / workers) * std::max(num_kb * t.kb, t.floor) + t.fixed;
-      if (us < best) { best = us; bn = t.bn; cg = t.cg; }
+      if (us < best) { best = us; bn = t.bn; cg = t.cg; eg = t.eg; }
     }
   } else if (bn == 256 && pairs && (long)((g.M + 255) / 256) * ((g.N + 255) / 256) >= num_sms / 2) {
     cg = 2;  // a width asked for: CTA pairs once the problem has at least a wave of them
   }
   switch (bn * 10 + cg) {
-    case 2562: return launch_cfg<256, EPI, 2>(stream, g, num_sms);
+    case 2562:
+      if constexpr (deep_epilogue(EPI))
+        if (eg == 4) return launch_cfg<256, EPI, 2, 4>(stream, g, num_sms);
+      return launch_cfg<256, EPI, 2>(stream, g, num_sms);
     case 2561: return launch_cfg<256, EPI, 1>(stream, g, num_sms);
     case 1922:
+      if constexpr (deep_epilogue(EPI))
+        if (eg == 4) return launch_cfg<192, EPI, 2, 4>(stream, g, num_sms);
       if constexpr (!kWideOnly) return launch_cfg<192, EPI, 2>(stream, g, num_sms);
       return cudaErrorInvalidValue;
     case 1282:
@@ -634,9 +645,9 @@ cudaError_t launch_epi(cudaStream_t stream, const GemmArgs& g, int num_sms) {
 }  // namespace
 
 namespace {
-template <int BN, int EPI, int CG>
+template <int BN, int EPI, int CG, int EG = 2>
 cudaError_t set_attr() {
-  return cudaFuncSetAttribute(gemm_tn_kernel<BN, EPI, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, CG>::SMEM);
+  return cudaFuncSetAttribute(gemm_tn_kernel<BN, EPI, CG, EG>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN, CG, EG>::SMEM);
 }
 template <int EPI>
 cudaError_t set_attr_epi() {
@@ -645,6 +656,10 @@ cudaError_t set_attr_epi() {
   if ((e = set_attr<256, EPI, 1>()) != cudaSuccess) return e;
   if constexpr (EPI != EPI_SWIGLU && EPI != EPI_GEGLU && EPI != EPI_CLAMPGLU && EPI != EPI_ROPE) {
     if ((e = set_attr<192, EPI, 2>()) != cudaSuccess) return e;
+    if constexpr (deep_epilogue(EPI)) {
+      if ((e = set_attr<256, EPI, 2, 4>()) != cudaSuccess) return e;
+      if ((e = set_attr<192, EPI, 2, 4>()) != cudaSuccess) return e;
+    }
     if ((e = set_attr<128, EPI, 2>()) != cudaSuccess) return e;
     if ((e = set_attr<128, EPI, 1>()) != cudaSuccess) return e;
     return set_attr<64, EPI, 1>();
