@@ -1331,6 +1331,10 @@ cudaError_t stack_ssm_init() {
   return cudaSuccess;
 }
 
+// A row pass launched while a product drains finds the SMs set up for the product's shared memory and keeps that little first-level cache to the end, which
+// costs one of more than a few million entries more than its launch (11k tokens: convolution of 6144 channels 142 us, 123 behind the product; residual step of
+// 2048 columns 62, 49; a step of 8 prompts of 700 to 1500 tokens 1014, 1004; of 16 short ones early is 1.4 % sooner)
+static bool launch_early(long entries, long limit_m) { return entries < limit_m << 20; }
 bool short_conv_fused(const ConvArgs& a) {
   return a.taps <= 4 && a.T <= 65535 && ((a.C | (int)a.ldi | a.off | (int)a.ldo | (int)a.slot_stride | (int)a.tail_off) & 3) == 0 &&
          ((uintptr_t)a.in & 15) == 0 && ((uintptr_t)a.out & 15) == 0 && ((uintptr_t)a.state & 15) == 0;
@@ -1344,7 +1348,7 @@ cudaError_t short_conv(cudaStream_t s, const ConvArgs& a) {
     const bool one = a.single || (long)across * ((a.T + kConvRun - 1) / kConvRun) < 2 * effective_sms(148);
     if (a.slabs.ws && (!a.single || !a.ab || !a.up_out || (a.up.N & 3) || (a.off_dt & 3))) return cudaErrorInvalidValue;
     const dim3 g(across + (a.up_out ? (a.up.N / 4 + 127) / 128 : 0) + (a.ab ? 1 : 0), one ? a.T : (a.T + kConvRun - 1) / kConvRun);
-#define HB_CONV_T(WT, TP) return one ? launch_k(short_conv_run_kernel<WT, TP, 1>, g, dim3(128), 0, s, true, a) : launch_k(short_conv_run_kernel<WT, TP, kConvRun>, g, dim3(128), 0, s, true, a)
+#define HB_CONV_T(WT, TP) return one ? launch_k(short_conv_run_kernel<WT, TP, 1>, g, dim3(128), 0, s, true, a) : launch_k(short_conv_run_kernel<WT, TP, kConvRun>, g, dim3(128), 0, s, launch_early((long)a.T * a.C, 20), a)
 #define HB_CONV(TP) do { if (a.f32) HB_CONV_T(float, TP); else HB_CONV_T(bf16, TP); } while (0)
     if (a.taps == 1) HB_CONV(1);
     if (a.taps == 2) HB_CONV(2);
@@ -1501,7 +1505,7 @@ cudaError_t parallel_step(cudaStream_t s, const float* x, const int32_t* row_ind
                        (uintptr_t)h1b | (uintptr_t)h2 | (uintptr_t)h2b | (uintptr_t)sc.s1 | (uintptr_t)sc.s2 | (uintptr_t)sc.rows;
   if (W % 4 == 0 && W <= 4 * 256 * kParChunks && (al & 15) == 0 && sc.top_k <= kParTop) {
 #define HB_PAR_IN(WT, CH, IN)                                                                                                                  \
-  return launch_k(parallel_step_vec_kernel<WT, CH, IN>, dim3(rows), dim3(256), 0, s, true, x, row_index, y, y2, (const WT*)bias, bias_scale, \
+  return launch_k(parallel_step_vec_kernel<WT, CH, IN>, dim3(rows), dim3(256), 0, s, launch_early((long)rows * W, 8), x, row_index, y, y2, (const WT*)bias, bias_scale, \
                   (const WT*)w1, (const WT*)w2, eps, x_out, h1, h1b, h2, h2b, W, sc)
 #define HB_PAR(WT, CH)                                  \
   do {                                                  \
