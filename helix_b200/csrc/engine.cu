@@ -1367,14 +1367,13 @@ int Engine::run_prefill(std::vector<Request*>& batch) {
     attn_flops_ += 4.0 * (n * s + n * n * 0.5) * d.head_dim * d.heads;  // QK^T + PV over the causal trapezoid
   }
   CU(cudaEventRecord(fwd_a_, stream_));
-  int rc = is_stack() ? forward_stack(T, B, L, step_driven_ ? (const int32_t*)(d_step_ + L.rows) : nullptr, n_extra, all_logits_,
+  rows_on_host_ = step_driven_ && rows_to_host(n_extra);
+  int rc = is_stack() ? forward_stack(T, B, L, step_driven_ ? (const int32_t*)(d_step_ + L.rows) : nullptr, n_extra, rows_on_host_ ? h_rows_ : all_logits_,
                                       !step_driven_)
                       : forward_llama(T, B, true, max_len, L, want_all, paged);
   if (rc != HB_OK) return rc;
   CU(cudaEventRecord(fwd_b_, stream_));
   if (!step_driven_) CU(cudaMemcpyAsync(h_sampled_, sampled_, (size_t)B * 4, cudaMemcpyDeviceToHost, stream_));
-  else if (n_extra > 0 && (size_t)n_extra * d.vocab <= h_rows_floats_)
-    CU(cudaMemcpyAsync(h_rows_, all_logits_, (size_t)n_extra * d.vocab * 4, cudaMemcpyDeviceToHost, stream_));
   CU(cudaStreamSynchronize(stream_));
   if (kernel_error_ && *kernel_error_) {
     *kernel_error_ = 0;

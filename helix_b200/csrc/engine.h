@@ -125,6 +125,7 @@ class Engine {
   int forward_stack(int T, int B, const StepLayout& L, const int32_t* extra_rows, int n_extra, float* extra_out, bool sample);
   // C[M, N] (fp32, row stride ldc) = A . W^T: tcgen05 GEMM when the mode and the strides allow it (A_b16 = bf16 copy of A),
   // CUDA-core fp32 GEMM otherwise
+  bool rows_to_host(int n) const;
   int stack_gemm(const float* A, const bf16* A_b16, int lda, const void* W, int N, int K, float* C, int ldc, int M, const void* bias = nullptr, bf16* relu2 = nullptr, bool* relu2_done = nullptr);
   int take_slot();
   void drop_slot(Request* r);
@@ -245,8 +246,9 @@ class Engine {
   float* rope_cs_ = nullptr;  // [t_cap][head_dim] cos | sin of the current step's positions (EPI_ROPE)
   float* logits_ = nullptr;
   float* dec_ws_ = nullptr;
-  float* h_rows_ = nullptr;     // pinned: a driven step's logits on their way out, up to h_rows_floats_ of them
+  float* h_rows_ = nullptr;     // pinned, written by the head's kernels: a driven step's logits, up to h_rows_floats_ of them
   size_t h_rows_floats_ = 0;
+  bool rows_on_host_ = false;   // this step's are there
   size_t skinny_floats_ = 0;    // of skinny_ws_, layer-list decoders
   float* skinny_ws_ = nullptr;  // fp32 partial slabs of the decode-step GEMMs
   SkinnyPlan plan_qkv_{}, plan_o_{}, plan_gu_{}, plan_down_{}, plan_head_{};

@@ -602,7 +602,7 @@ int Engine::alloc_runtime_stack() {
   CU(cudaMalloc(&d_step_, step_bytes_));
   CU(cudaMallocHost(&h_step_, step_bytes_));
   CU(cudaMallocHost(&h_sampled_, (size_t)b_cap_ * 4));
-  h_rows_floats_ = std::min<size_t>((size_t)b_cap_ * sd.vocab, 1 << 20);  // (a row per sequence, at most 4 MB)
+  h_rows_floats_ = std::min<size_t>((size_t)4 * b_cap_ * sd.vocab, 1 << 20);  // (four rows per sequence, at most 4 MB)
   CU(cudaMallocHost(&h_rows_, h_rows_floats_ * 4));
   CU(cudaMallocHost(&kernel_error_, sizeof(int)));
   *kernel_error_ = 0;
@@ -664,6 +664,13 @@ void Engine::drop_slot(Request* r) {
 static bool few_token_gemm() {  // HB_STACK_SKINNY=0: the tiled GEMM for few tokens too (A/B and bring-up)
   static const bool off = [] { const char* e = getenv("HB_STACK_SKINNY"); return e && atoi(e) == 0; }();
   return !off;
+}
+// Few rows of a driven step: the head's last kernel (a sum of slabs, or the exact mode's product) writes every logit once, by whole lines, to pinned host memory.
+// Not where a softcap or a scale reads them again
+bool Engine::rows_to_host(int n) const {
+  const hb_stack_desc& sd = model_.sd;
+  return n > 0 && n <= 256 && (size_t)n * sd.vocab <= h_rows_floats_ && few_token_gemm() && !(sd.logit_softcap > 0.f) &&
+         (sd.logit_scale == 0.f || sd.logit_scale == 1.f);
 }
 bool Engine::stack_tc(int N, int K, int lda, int ldc) const {
   static const bool simt_only = [] { const char* e = getenv("HB_STACK_SIMT"); return e && atoi(e) != 0; }();
@@ -1623,10 +1630,11 @@ int Engine::seq_step(const hb_seq_feed* entries, int n, float* out, size_t cap, 
   int rc = run_prefill(batch);
   step_driven_ = false;
   if (rc != HB_OK) return rc;  // a CUDA failure is sticky; the sequences keep their records for hb_seq_close
-  // Few rows have come with the step's own wait, through pinned memory: the copy to the caller's pageable memory was a second round trip and a
-  // copy by the driver (a turn of 16 sequences, a vocabulary of 4096, 12 tokens each 2445 -> 2374 us)
+  // Few rows are in pinned memory when the step's own wait is over (run_prefill).  A copy to the caller's pageable memory was a second round trip and a
+  // copy by the driver, one to pinned memory still waited for the copy engine (a turn of 16 sequences, a vocabulary of 4096, 12 tokens each:
+  // 2445, 2370 with the pinned copy, 2285 us; the exact mode, 2 prompts and 2 tokens each 900, 872)
   const size_t floats = (size_t)R * model_.d.vocab;
-  if (R > 0 && floats <= h_rows_floats_) memcpy(out, h_rows_, floats * 4);
+  if (R > 0 && rows_on_host_) memcpy(out, h_rows_, floats * 4);
   else if (R > 0) CU(cudaMemcpy(out, all_logits_, floats * 4, cudaMemcpyDeviceToHost));
   {
     std::lock_guard<std::mutex> g(mu_);
