@@ -8,6 +8,7 @@
 #include "../../include/helix_b200_kernels.h"
 #include "engine.h"
 #include "gguf.h"
+#include "launch.h"
 #include "tma_host.h"
 
 using hb::Engine;
@@ -180,6 +181,23 @@ int hbk_gemm_skinny_finish(const void* X, int ldx, const void* W, int ldw, float
   cudaError_t e2 = cudaDeviceSynchronize();
   cudaFree(ws);
   cudaFree(cnt);
+  return kret(e != cudaSuccess ? e : e2);
+}
+int hbk_gemm_skinny_pair(const void* X, int ldx, const void* W, int ldw, float* out, int ldo, int N, int K, const void* X2, int ldx2, const void* W2,
+                         int ldw2, float* out2, int ldo2, int N2, int K2, int M, int sms) {
+  hb::SmLimitScope scope(sms);
+  hb::SkinnyProduct a{(const hb::bf16*)X, ldx, (const hb::bf16*)W, ldw, nullptr, N, K, {}}, b{(const hb::bf16*)X2, ldx2, (const hb::bf16*)W2, ldw2, nullptr, N2, K2, {}};
+  cudaError_t e = hb::gemm_skinny_plan(N, K, &a.plan);
+  if (e == cudaSuccess) e = hb::gemm_skinny_plan(N2, K2, &b.plan);
+  if (e != cudaSuccess) return kret(e);
+  const size_t first = (hb::gemm_skinny_ws_floats(a.plan, M, N) + 3) / 4 * 4;
+  if ((e = cudaMalloc(&a.ws, (first + hb::gemm_skinny_ws_floats(b.plan, M, N2)) * 4)) != cudaSuccess) return kret(e);
+  b.ws = a.ws + first;
+  e = hb::gemm_skinny_pair(0, a, b, M);
+  if (e == cudaSuccess) e = hb::dec_sum_slabs(0, a.ws, a.plan, out, ldo, M, N);
+  if (e == cudaSuccess) e = hb::dec_sum_slabs(0, b.ws, b.plan, out2, ldo2, M, N2);
+  cudaError_t e2 = cudaDeviceSynchronize();
+  cudaFree(a.ws);
   return kret(e != cudaSuccess ? e : e2);
 }
 int hbk_gemm_naive(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int N, int K) {

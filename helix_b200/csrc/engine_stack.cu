@@ -190,7 +190,8 @@ static bool paired_ok(const Model& m, int i) {
 // fp32 partial slabs of the weight-streaming GEMM that serves steps of <= 256 tokens (every projection it may be given)
 static size_t stack_skinny_floats(const Model& m) {
   size_t f = 0;
-  auto shape = [&](size_t N, size_t K) { f = std::max(f, (size_t)gemm_skinny_max_segs((int)N, (int)K, 148) * 256 * N); };
+  auto slabs = [](size_t N, size_t K) { return (size_t)gemm_skinny_max_segs((int)N, (int)K, 148) * 256 * N; };
+  auto shape = [&](size_t N, size_t K) { f = std::max(f, slabs(N, K)); };
   const size_t W = m.sd.width;
   for (int i = 0; i < m.sd.n_layers; ++i) {
     const hb_layer_desc& l = m.sl[i];
@@ -199,8 +200,8 @@ static size_t stack_skinny_floats(const Model& m) {
     if (l.ff > 0 && l.ff_kind == HB_FF_RELU2) shape(l.ff, W);
     if (paired_ok(m, i)) {
       const int oc = m.sw[i].o_cols ? m.sw[i].o_cols : l.heads * l.vdim;
-      f = std::max(f, gemm_skinny_pair_floats(m.sw[i].n_in, (int)W, l.ff, (int)W, 256, 148));
-      f = std::max(f, gemm_skinny_pair_floats((int)W, oc, (int)W, l.ff, 256, 148));
+      f = std::max(f, slabs(m.sw[i].n_in, W) + slabs(l.ff, W));
+      f = std::max(f, slabs(W, oc) + slabs(W, l.ff));
     }
     if (l.mixer == HB_MIXER_LATENT && l.q_rank > 0) shape((size_t)l.heads * (l.dim + l.rot_dim), l.q_rank);
     if (l.ff > 0) {
@@ -436,10 +437,6 @@ int Engine::alloc_runtime_stack() {
       CU(gemm_skinny_plan(model_.sw[i].n_in, sd.width, &pl));
       CU(gemm_skinny_plan(sd.width, model_.sw[i].o_cols ? model_.sw[i].o_cols : l.heads * l.vdim, &pl));
       if (l.ff > 0 && l.ff_kind == HB_FF_RELU2) CU(gemm_skinny_plan(l.ff, sd.width, &pl));
-      if (paired_ok(model_, i)) {
-        CU(gemm_skinny_pair_plan(model_.sw[i].n_in, sd.width, l.ff, sd.width, &pl));
-        CU(gemm_skinny_pair_plan(sd.width, model_.sw[i].o_cols ? model_.sw[i].o_cols : l.heads * l.vdim, sd.width, l.ff, &pl));
-      }
       if (l.mixer == HB_MIXER_LATENT && l.q_rank > 0) CU(gemm_skinny_plan(l.heads * (l.dim + l.rot_dim), l.q_rank, &pl));
       if (l.ff > 0) {
         CU(gemm_skinny_plan(2 * l.ff, sd.width, &pl));
@@ -1104,22 +1101,21 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       }
       Slabs in_slabs;
       if (paired) {
-        SkinnyPlan plan{};
-        CU(gemm_skinny_pair_plan(w.n_in, W, l.ff, W, &plan));
-        float* up_ws = skinny_ws_ + (size_t)plan.max_segs * T * w.n_in;
-        const SkinnyProduct in{x16, W, (const bf16*)w.w_in, W, skinny_ws_, w.n_in, W}, up{ff_in16, W, (const bf16*)w.w_gu, W, up_ws, l.ff, W};
-        SPAN(4, 2.0 * (T + w.n_in + l.ff) * W + 4.0 * T * (w.n_in + l.ff), gemm_skinny_pair(stream_, plan, in, up, T));
+        SkinnyPlan plan{}, up_plan{};
+        CU(gemm_skinny_plan(w.n_in, W, &plan));
+        CU(gemm_skinny_plan(l.ff, W, &up_plan));
+        float* up_ws = skinny_ws_ + gemm_skinny_ws_floats(plan, T, w.n_in);
+        const SkinnyProduct in{x16, W, (const bf16*)w.w_in, W, skinny_ws_, w.n_in, W, plan}, up{ff_in16, W, (const bf16*)w.w_gu, W, up_ws, l.ff, W, up_plan};
+        SPAN(4, 2.0 * (T + w.n_in + l.ff) * W + 4.0 * T * (w.n_in + l.ff), gemm_skinny_pair(stream_, in, up, T));
         in_slabs = Slabs{skinny_ws_, plan.seg_count, T, w.n_in};
-        const Slabs up_slabs{up_ws, plan.seg_count + plan.n_tiles, T, l.ff};
+        const Slabs up_slabs{up_ws, up_plan.seg_count, T, l.ff};
         if (ca.single && (w.off_a & 3) == 0 && (w.off_g & 3) == 0) {  // its readers take the slabs
           ca.slabs = in_slabs;
           ca.up = up_slabs;
           ca.up_out = k.gu16;
         } else {
-          SkinnyPlan second = plan;
-          second.seg_count += plan.n_tiles;
           SPAN(3, 8.0 * T * w.n_in, dec_sum_slabs(stream_, skinny_ws_, plan, k.p1, k.ld1, T, w.n_in));
-          SPAN(3, 6.0 * T * l.ff, dec_sum_slabs(stream_, up_ws, second, nullptr, 0, T, l.ff, k.gu16));
+          SPAN(3, 6.0 * T * l.ff, dec_sum_slabs(stream_, up_ws, up_plan, nullptr, 0, T, l.ff, k.gu16));
           in_slabs.ws = nullptr;
         }
       }
@@ -1148,15 +1144,16 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
                                                    l.norm_groups, mo_f32, mo16, T, inner, false, nullptr, in_slabs.ws ? &in_slabs : nullptr, w.off_g));
       }
       if (paired) {
-        SkinnyPlan plan{};
-        CU(gemm_skinny_pair_plan(W, ocols, W, l.ff, &plan));
-        float* down_ws = skinny_ws_ + (size_t)plan.max_segs * T * W;
-        const SkinnyProduct o{mo16, ocols, (const bf16*)w.wo, ocols, skinny_ws_, W, ocols}, down{k.gu16, l.ff, (const bf16*)w.w_down, l.ff, down_ws, W, l.ff};
-        SPAN(4, 2.0 * (T + W) * (ocols + l.ff) + 8.0 * T * W, gemm_skinny_pair(stream_, plan, o, down, T));
+        SkinnyPlan plan{}, down_plan{};
+        CU(gemm_skinny_plan(W, ocols, &plan));
+        CU(gemm_skinny_plan(W, l.ff, &down_plan));
+        float* down_ws = skinny_ws_ + gemm_skinny_ws_floats(plan, T, W);
+        const SkinnyProduct o{mo16, ocols, (const bf16*)w.wo, ocols, skinny_ws_, W, ocols, plan}, down{k.gu16, l.ff, (const bf16*)w.w_down, l.ff, down_ws, W, l.ff, down_plan};
+        SPAN(4, 2.0 * (T + W) * (ocols + l.ff) + 8.0 * T * W, gemm_skinny_pair(stream_, o, down, T));
         ParScale scale;
         scale.s1 = w.ls1; scale.s2 = w.ls2; scale.m = sd.resid_mult != 0.f ? sd.resid_mult : 1.f;
         scale.y_slabs = Slabs{skinny_ws_, plan.seg_count, T, W};
-        scale.y2_slabs = Slabs{down_ws, plan.seg_count + plan.n_tiles, T, W};
+        scale.y2_slabs = Slabs{down_ws, down_plan.seg_count, T, W};
         SPAN(3, 5 * rowb, par_step(nullptr, nullptr, w.o_bias, l.mix_scale != 0.f ? l.mix_scale : 1.f, i + 1, &scale));
         continue;
       }

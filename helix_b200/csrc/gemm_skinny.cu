@@ -180,14 +180,15 @@ __device__ __noinline__ void finish_tile(const SkinnyEpi& epi, const uint8_t* __
   }
 }
 
-// A second product behind the first (PAIR): its units follow the first one's in the stream-K line, so two products that wait for
-// nothing of one another (a layer's input and feed-forward projections, its two output projections) cost one launch.  With the
-// readers that sum the slabs and one launch for a token's mixer, thirteen launches of a layer became three: a driven turn of
-// steps 3070 -> 2450 us, one of a single short sequence 2260 -> 1410.
+// A second product behind the first (PAIR), so that two products that wait for nothing of one another (a layer's input and feed-forward
+// projections, its two output projections) cost one launch.  Each is cut as in a launch of its own (the same slabs, the same bits): a CTA walks
+// its range of the first product, then its range of the second, whose ranges go to the last CTAs of the grid, so that products
+// of fewer ranges than SMs lie side by side.
 struct SecondProduct {
   CUtensorMap map_w, map_x;
   float* ws;
   int N, K;
+  int grid1, grid2;  // ranges of the two products
 };
 struct NoSecond {};
 
@@ -217,21 +218,36 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int KB = (K + BLOCK_K - 1) / BLOCK_K;
   const int n_tiles = (N + BLOCK_N - 1) / BLOCK_N;
-  const long long U1 = (long long)n_tiles * KB;
-  long long U = U1;
-  int KB2 = 0;
+  const long long U = (long long)n_tiles * KB;
+  int G = gridDim.x, G2 = 1;
+  if constexpr (PAIR) {
+    G = second.grid1;
+    G2 = second.grid2;
+  }
+  // this CTA's units: [u0, ua) of the first product, then [v0, v0 + u1 - ua) of the second, counted on from ua
+  const int c1 = PAIR ? min((int)blockIdx.x, G) : blockIdx.x;  // (range G is empty)
+  const long long u0 = range_start(c1, U, G), ua = PAIR && c1 == G ? u0 : range_start(c1 + 1, U, G);
+  long long u1 = ua, U2 = 0, v0 = 0;
+  int KB2 = 1, c2 = -1;
   if constexpr (PAIR) {
     KB2 = (second.K + BLOCK_K - 1) / BLOCK_K;
-    U += (long long)((second.N + BLOCK_N - 1) / BLOCK_N) * KB2;
+    U2 = (long long)((second.N + BLOCK_N - 1) / BLOCK_N) * KB2;
+    c2 = (int)blockIdx.x - ((int)gridDim.x - G2);
+    if (c2 >= 0) {
+      v0 = range_start(c2, U2, G2);
+      u1 = ua + range_start(c2 + 1, U2, G2) - v0;
+    }
   }
-  const int G = gridDim.x;
-  // unit u of the line: (second product?, tile, k block)
+  // unit u of this CTA: (second product?, tile, k block)
   struct Unit { bool two; int tile, kb; };
   auto unit = [&](long long u) {
-    if (PAIR && u >= U1) return Unit{true, (int)((u - U1) / KB2), (int)((u - U1) % KB2)};
+    if (PAIR && u >= ua) return Unit{true, (int)((u - ua + v0) / KB2), (int)((u - ua + v0) % KB2)};
     return Unit{false, (int)(u / KB), (int)(u % KB)};
   };
-  auto tile_end = [&](const Unit& x) { return PAIR && x.two ? U1 + (long long)(x.tile + 1) * KB2 : (long long)(x.tile + 1) * KB; };  // behind its tile's last unit
+  // behind the last unit of its tile that this CTA has
+  auto tile_end = [&](const Unit& x) {
+    return PAIR && x.two ? min(u1, (long long)(x.tile + 1) * KB2 - v0 + ua) : min(ua, (long long)(x.tile + 1) * KB);
+  };
   auto load_w = [&](uint8_t* dst, uint64_t* bar, long long u) {
     const Unit x = unit(u);
     if constexpr (PAIR) {
@@ -246,7 +262,6 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     tma_load_2d(dst, &map_x, bar, x.kb * BLOCK_K, 0, kEvictLast);
   };
-  const long long u0 = range_start(blockIdx.x, U, G), u1 = range_start(blockIdx.x + 1, U, G);
 
   pdl_launch_dependents();
   if (blockIdx.x != 0) trace = nullptr;
@@ -329,7 +344,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       int it = 0;
       long long u = u0;
       while (u < u1) {
-        const long long seg_end = min(u1, tile_end(unit(u)));
+        const long long seg_end = tile_end(unit(u));
         const int as = it & 1;
         mbar_wait(&tmem_empty[as], ((it >> 1) & 1) ^ 1);
         tc_fence_after();
@@ -403,8 +418,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     while (u < u1) {
       const Unit at = unit(u);
       const int tile = at.tile;
-      const long long end = tile_end(at), seg_end = min(u1, end);
-      const int seg = blockIdx.x - owner_of(end - (PAIR && at.two ? KB2 : KB), U, G);  // slab index: fixed by the partition
+      const long long seg_end = tile_end(at);
+      // slab index: fixed by the partition
+      const int seg = PAIR && at.two ? c2 - owner_of((long long)tile * KB2, U2, G2) : c1 - owner_of((long long)tile * KB, U, G);
       const int as = it & 1;
       mbar_wait(&tmem_full[as], (it >> 1) & 1);
       tc_fence_after();
@@ -471,24 +487,20 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 }
 
 struct PlanKey {
-  int dev, N, K, N2, K2, sms;
-  bool operator<(const PlanKey& o) const { return std::tie(dev, N, K, N2, K2, sms) < std::tie(o.dev, o.N, o.K, o.N2, o.K2, o.sms); }
+  int dev, N, K, sms;
+  bool operator<(const PlanKey& o) const { return std::tie(dev, N, K, sms) < std::tie(o.dev, o.N, o.K, o.sms); }
 };
-// the stream-K line of one product or of two behind one another: slabs of every 128-column tile
-struct Line {
+// the stream-K line of a product: its ranges, and the slabs of every 128-column tile
+struct Cut {
   int grid = 0;
   std::vector<uint8_t> segs;
-  Line(int N, int K, int N2, int K2, int sms) {
-    const int kb[2] = {(K + BLOCK_K - 1) / BLOCK_K, (K2 + BLOCK_K - 1) / BLOCK_K}, tiles[2] = {(N + BLOCK_N - 1) / BLOCK_N, (N2 + BLOCK_N - 1) / BLOCK_N};
-    const long long U1 = (long long)tiles[0] * kb[0], U = U1 + (long long)tiles[1] * kb[1];
+  Cut(int N, int K, int sms) {
+    const int KB = (K + BLOCK_K - 1) / BLOCK_K, n_tiles = (N + BLOCK_N - 1) / BLOCK_N;
+    const long long U = (long long)n_tiles * KB;
     grid = (int)std::min<long long>(sms, std::max<long long>(1, U / 4));
-    for (int p = 0; p < 2; ++p)
-      for (int t = 0; t < tiles[p]; ++t) {
-        const long long first = (p ? U1 : 0) + (long long)t * kb[p];
-        segs.push_back((uint8_t)(owner_of(first + kb[p] - 1, U, grid) - owner_of(first, U, grid) + 1));
-      }
+    for (long long u = 0; u < U; u += KB) segs.push_back((uint8_t)(owner_of(u + KB - 1, U, grid) - owner_of(u, U, grid) + 1));
   }
-  int most(int from, int to) const { return *std::max_element(segs.begin() + from, segs.begin() + to); }
+  int most() const { return *std::max_element(segs.begin(), segs.end()); }
 };
 std::mutex g_plan_mu;
 std::map<PlanKey, SkinnyPlan> g_plans;
@@ -519,7 +531,7 @@ cudaError_t launch(cudaStream_t stream, const SkinnyPlan& plan, const bf16* X, i
 }
 
 template <int MPAD>
-cudaError_t launch_pair(cudaStream_t stream, const SkinnyPlan& plan, const SkinnyProduct& a, const SkinnyProduct& b, int M) {
+cudaError_t launch_pair(cudaStream_t stream, const SkinnyProduct& a, const SkinnyProduct& b, int M) {
   using C = SCfg<MPAD>;
   CUtensorMap mw, mx;
   SecondProduct second;
@@ -530,8 +542,11 @@ cudaError_t launch_pair(cudaStream_t stream, const SkinnyPlan& plan, const Skinn
   second.ws = b.ws;
   second.N = b.N;
   second.K = b.K;
-  return launch_k(gemm_skinny_kernel<MPAD, true>, dim3(plan.grid), dim3(kThreads), C::SMEM, stream, true, mw, mx, a.ws, M, a.N, a.K, (const int*)nullptr, 0,
-                  (int*)nullptr, 0, a.W, a.ldw, (unsigned long long*)nullptr, SkinnyEpi{}, plan.seg_count, (const int*)nullptr, 0, (int*)nullptr, second);
+  second.grid1 = a.plan.grid;
+  second.grid2 = b.plan.grid;
+  const int grid = std::max({a.plan.grid, b.plan.grid, std::min(a.plan.sms, a.plan.grid + b.plan.grid)});
+  return launch_k(gemm_skinny_kernel<MPAD, true>, dim3(grid), dim3(kThreads), C::SMEM, stream, true, mw, mx, a.ws, M, a.N, a.K, (const int*)nullptr, 0,
+                  (int*)nullptr, 0, a.W, a.ldw, (unsigned long long*)nullptr, SkinnyEpi{}, (const uint8_t*)nullptr, (const int*)nullptr, 0, (int*)nullptr, second);
 }
 
 template <int MPAD>
@@ -550,9 +565,7 @@ cudaError_t gemm_skinny_init() {
   return set_attr<256>();
 }
 
-cudaError_t gemm_skinny_plan(int N, int K, SkinnyPlan* out) { return gemm_skinny_pair_plan(N, K, 0, 0, out); }
-
-cudaError_t gemm_skinny_pair_plan(int N, int K, int N2, int K2, SkinnyPlan* out) {
+cudaError_t gemm_skinny_plan(int N, int K, SkinnyPlan* out) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -560,36 +573,28 @@ cudaError_t gemm_skinny_pair_plan(int N, int K, int N2, int K2, SkinnyPlan* out)
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   sms = effective_sms(sms);  // hb_engine_cfg.sm_budget of the calling engine
   std::lock_guard<std::mutex> g(g_plan_mu);
-  const PlanKey key{dev, N, K, N2, K2, sms};
+  const PlanKey key{dev, N, K, sms};
   auto it = g_plans.find(key);
   if (it != g_plans.end()) {
     *out = it->second;
     return cudaSuccess;
   }
-  const Line line(N, K, N2, K2, sms);
+  const Cut cut(N, K, sms);
   SkinnyPlan p{};
-  p.n_tiles = (N + BLOCK_N - 1) / BLOCK_N;
-  p.grid = line.grid;
-  p.max_segs = line.most(0, p.n_tiles);
-  if (N2 > 0) p.max_segs2 = line.most(p.n_tiles, (int)line.segs.size());
+  p.n_tiles = (int)cut.segs.size();
+  p.grid = cut.grid;
+  p.sms = sms;
+  p.max_segs = cut.most();
   uint8_t* d = nullptr;
-  if ((e = cudaMalloc(&d, line.segs.size())) != cudaSuccess) return e;
-  if ((e = cudaMemcpy(d, line.segs.data(), line.segs.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
+  if ((e = cudaMalloc(&d, cut.segs.size())) != cudaSuccess) return e;
+  if ((e = cudaMemcpy(d, cut.segs.data(), cut.segs.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return e;
   p.seg_count = d;
   g_plans[key] = p;
   *out = p;
   return cudaSuccess;
 }
 
-int gemm_skinny_max_segs(int N, int K, int sms) {
-  const Line line(N, K, 0, 0, sms);
-  return line.most(0, (int)line.segs.size());
-}
-size_t gemm_skinny_pair_floats(int N, int K, int N2, int K2, int M, int sms) {
-  const Line line(N, K, N2, K2, sms);
-  const int n1 = (N + BLOCK_N - 1) / BLOCK_N;
-  return (size_t)M * ((size_t)line.most(0, n1) * N + (size_t)line.most(n1, (int)line.segs.size()) * N2);
-}
+int gemm_skinny_max_segs(int N, int K, int sms) { return Cut(N, K, sms).most(); }
 
 size_t gemm_skinny_ws_floats(const SkinnyPlan& p, int M, int N) { return (size_t)p.max_segs * M * N; }
 
@@ -602,14 +607,14 @@ cudaError_t gemm_skinny(cudaStream_t stream, const SkinnyPlan& plan, const bf16*
   return launch<256>(stream, plan, X, ldx, W, ldw, ws, M, N, K, sig, epi);
 }
 
-cudaError_t gemm_skinny_pair(cudaStream_t stream, const SkinnyPlan& plan, const SkinnyProduct& a, const SkinnyProduct& b, int M) {
-  if (M <= 0 || M > 256 || a.N <= 0 || b.N <= 0) return cudaErrorInvalidValue;
+cudaError_t gemm_skinny_pair(cudaStream_t stream, const SkinnyProduct& a, const SkinnyProduct& b, int M) {
+  if (M <= 0 || M > 256 || a.N <= 0 || b.N <= 0 || a.plan.sms != b.plan.sms) return cudaErrorInvalidValue;
   for (const SkinnyProduct* p : {&a, &b})
     if ((p->K % 8) || (p->ldx % 8) || (p->ldw % 8)) return cudaErrorInvalidValue;
-  if (M <= 32) return launch_pair<32>(stream, plan, a, b, M);
-  if (M <= 64) return launch_pair<64>(stream, plan, a, b, M);
-  if (M <= 128) return launch_pair<128>(stream, plan, a, b, M);
-  return launch_pair<256>(stream, plan, a, b, M);
+  if (M <= 32) return launch_pair<32>(stream, a, b, M);
+  if (M <= 64) return launch_pair<64>(stream, a, b, M);
+  if (M <= 128) return launch_pair<128>(stream, a, b, M);
+  return launch_pair<256>(stream, a, b, M);
 }
 
 }  // namespace hb

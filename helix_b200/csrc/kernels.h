@@ -243,8 +243,8 @@ struct SkinnyPlan {
   int grid;                  // CTAs (== SMs unless the problem is tiny)
   int n_tiles;               // ceil(N/128)
   int max_segs;              // max #slabs any tile is split into
-  const uint8_t* seg_count;  // device [n_tiles]: slabs of each 128-column tile (of two products: the second one's tiles behind the first one's)
-  int max_segs2 = 0;         // the same of a second product
+  const uint8_t* seg_count;  // device [n_tiles]: slabs of each 128-column tile
+  int sms = 0;               // SMs it was cut for
 };
 // Tile finisher of the decode GEMM: the LAST CTA that contributes a slab to an output tile (one counter per tile) sums
 // the tile's slabs in slab order — bit-deterministic whoever finishes — and applies the op that follows the projection
@@ -282,11 +282,9 @@ int gemm_skinny_max_segs(int N, int K, int sms);  // pure host arithmetic (memor
 // ws[seg][m][n] (seg < seg_count[n/128]) = partial sums of X[M,K] . W[N,K]^T
 cudaError_t gemm_skinny(cudaStream_t stream, const SkinnyPlan& plan, const bf16* X, int ldx, const bf16* W, int ldw,
                         float* ws, int M, int N, int K, const StreamSig* sig = nullptr, const SkinnyEpi* epi = nullptr);
-// Two products of the same M rows in one launch, the units of both in one stream-K line; a plan of its own (slabs only)
-struct SkinnyProduct { const bf16* X; int ldx; const bf16* W; int ldw; float* ws; int N, K; };
-cudaError_t gemm_skinny_pair_plan(int N, int K, int N2, int K2, SkinnyPlan* out);
-size_t gemm_skinny_pair_floats(int N, int K, int N2, int K2, int M, int sms);  // of both products' slabs, pure host arithmetic
-cudaError_t gemm_skinny_pair(cudaStream_t stream, const SkinnyPlan& plan, const SkinnyProduct& a, const SkinnyProduct& b, int M);
+// Two products of the same M rows in one launch, each with the plan, and so the slabs, that gemm_skinny gives it
+struct SkinnyProduct { const bf16* X; int ldx; const bf16* W; int ldw; float* ws; int N, K; SkinnyPlan plan; };
+cudaError_t gemm_skinny_pair(cudaStream_t stream, const SkinnyProduct& a, const SkinnyProduct& b, int M);
 // A product's slabs where a kernel takes them instead of the summed rows (it sums a value's slabs in slab order, as dec_sum_slabs does)
 struct Slabs { const float* ws = nullptr; const uint8_t* segs = nullptr; int M = 0, N = 0; };  // N a multiple of four
 // consumers of the slabs (each sums the slabs in fixed order, then applies its fused epilogue)

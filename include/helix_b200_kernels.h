@@ -25,6 +25,9 @@ int hbk_gemm_skinny(const void* X, int ldx, const void* W, int ldw, float* out_f
  * writes out[m, n]); launched `repeats` times back to back: the arrival counters must return to zero by themselves */
 int hbk_gemm_skinny_finish(const void* X, int ldx, const void* W, int ldw, float* out_f32, int ldo, int M, int N, int K,
                            int repeats);
+/* two such products of the same M rows in one launch, cut for `sms` SMs (0 = all): the bits that each has by itself */
+int hbk_gemm_skinny_pair(const void* X, int ldx, const void* W, int ldw, float* out_f32, int ldo, int N, int K, const void* X2, int ldx2,
+                         const void* W2, int ldw2, float* out2_f32, int ldo2, int N2, int K2, int M, int sms);
 int hbk_gemm_naive(const void* A, int lda, const void* W, int ldw, void* C_f32, int ldc, int M, int N, int K);
 
 int hbk_embed_gather(const int32_t* tokens, const void* table, void* x, int T, int H);

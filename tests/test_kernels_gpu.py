@@ -489,3 +489,26 @@ def test_gemm_skinny_stream_k(L, M, N, K):
     out3 = torch.full((M, N), float("nan"), device="cuda")
     ck(L, L.hbk_gemm_skinny_finish(p(X), K, p(W), K, p(out3), N, M, N, K, 3))
     assert torch.equal(out, out3)
+
+
+@pytest.mark.parametrize("M", [1, 32, 33, 100, 129, 256])
+@pytest.mark.parametrize("first,second", [((6272, 1024), (4096, 1024)), ((1024, 2048), (1024, 4096)), ((4112, 512), (2048, 512)), ((392, 128), (1032, 128)),
+                                          ((100, 72), (20, 1000)), ((128, 64), (4100, 3000)), ((30000, 264), (64, 64))])
+@pytest.mark.parametrize("sms", [0, 61])
+def test_gemm_skinny_pair(L, M, first, second, sms):
+    """Two products in one launch are cut as by themselves: the same bits, for ragged columns and k blocks, products of fewer ranges than SMs beside
+    whole ones; with fewer SMs (another cut) against float64."""
+    outs, args, want = [], [], []
+    for i, (N, K) in enumerate((first, second)):
+        X, W, out = rnd(M, K, seed=62 + i), rnd(N, K, scale=K ** -0.5, seed=64 + i), torch.full((M, N), float("nan"), device="cuda")
+        want.append((X, W))
+        outs.append(out)
+        args += [p(X), K, p(W), K, p(out), N, N, K]
+    ck(L, L.hbk_gemm_skinny_pair(*args, M, sms))
+    for out, (X, W) in zip(outs, want):
+        if sms == 0:
+            alone = torch.empty_like(out)
+            ck(L, L.hbk_gemm_skinny(p(X), X.shape[1], p(W), X.shape[1], p(alone), W.shape[0], M, W.shape[0], X.shape[1]))
+            assert torch.equal(out, alone)
+        # fp32 sums, cut to 2^-23 of a partial sum below 8 after every 16 products, then up to 16 slabs
+        assert (out.double() - X.double() @ W.double().T).abs().max() < (X.shape[1] / 16 + 16) * 8 * 2.0 ** -23
