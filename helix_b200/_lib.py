@@ -136,6 +136,8 @@ SIGNATURES = {
     "hbk_gemm_naive": (I, [P, I, P, I, P, I, I, I, I]),
     "hbk_gemm_skinny": (I, [P, I, P, I, P, I, I, I, I]),
     "hbk_gemm_skinny_pair": (I, [P, I, P, I, P, I, I, I, P, I, P, I, P, I, I, I, I, I]),
+    "hbk_gemm_skinny_slabs": (I, [I, I, I]),
+    "hbk_stack_slab_floats": (C.c_int64, [C.POINTER(StackDescC), C.POINTER(LayerDescC), I]),
     "hbk_gemm_skinny_finish": (I, [P, I, P, I, P, I, I, I, I, I]),
     "hbk_embed_gather": (I, [P, P, P, I, I]),
     "hbk_bert_embed_ln": (I, [P, P, P, P, P, P, P, P, I, I, C.c_float]),

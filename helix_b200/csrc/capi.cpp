@@ -200,6 +200,10 @@ int hbk_gemm_skinny_pair(const void* X, int ldx, const void* W, int ldw, float* 
   cudaFree(a.ws);
   return kret(e != cudaSuccess ? e : e2);
 }
+int hbk_gemm_skinny_slabs(int N, int K, int sms) { return N > 0 && K > 0 && sms > 0 ? hb::gemm_skinny_max_segs(N, K, sms) : -1; }
+int64_t hbk_stack_slab_floats(const hb_stack_desc* d, const hb_layer_desc* layers, int sm_budget) {
+  return d && layers && d->n_layers > 0 ? hb::stack_slab_floats(*d, layers, sm_budget) : -1;
+}
 int hbk_gemm_naive(const void* A, int lda, const void* W, int ldw, void* C, int ldc, int M, int N, int K) {
   hb::GemmArgs g{(const hb::bf16*)A, lda, (const hb::bf16*)W, ldw, C, ldc, nullptr, 0, nullptr, M, N, K, hb::EPI_F32, 0};
   return kret(hb::gemm_naive_check(0, g));

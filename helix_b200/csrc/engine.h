@@ -56,6 +56,9 @@ struct StepLayout {
 };
 enum StepFlags : int { STEP_FILTER = 1, STEP_PENALTY = 2, STEP_LOGPROBS = 4, STEP_WIDE_RECORDS = 8 /* of more than two tokens */ };
 
+// fp32 slabs of the few-token products of a layer-list decoder, in an engine with this SM budget (0 = none); host arithmetic, -1: refused description
+int64_t stack_slab_floats(const hb_stack_desc& desc, const hb_layer_desc* layers, int sm_budget);
+
 class Engine {
  public:
   explicit Engine(const hb_engine_cfg& cfg);
@@ -250,6 +253,7 @@ class Engine {
   size_t h_rows_floats_ = 0;
   bool rows_on_host_ = false;   // this step's are there
   size_t skinny_floats_ = 0;    // of skinny_ws_, layer-list decoders
+  std::vector<uint8_t> paired_;  // layers whose products go two to a launch in steps of few tokens
   float* skinny_ws_ = nullptr;  // fp32 partial slabs of the decode-step GEMMs
   SkinnyPlan plan_qkv_{}, plan_o_{}, plan_gu_{}, plan_down_{}, plan_head_{};
   int skinny_max_b_ = 0;

@@ -187,10 +187,15 @@ static bool paired_ok(const Model& m, int i) {
   return !m.sd.compute_f32 && m.sd.norm_place == HB_NORM_PARALLEL && l.mixer == HB_MIXER_MAMBA2 && l.ff > 0 && l.ff_kind == HB_FF_RELU2 &&
          fits(n_in, W) && fits(l.ff, W) && fits(W, ocols) && fits(W, l.ff) && W <= 8192 && inner / l.norm_groups % 4 == 0 && inner / l.norm_groups <= 8192;
 }
-// fp32 partial slabs of the weight-streaming GEMM that serves steps of <= 256 tokens (every projection it may be given)
-static size_t stack_skinny_floats(const Model& m) {
+// fp32 partial slabs of the weight-streaming GEMM that serves steps of <= 256 tokens (every projection it may be given).  Cut for
+// fewer SMs a product can have more slabs (ranges of other lengths straddle more tile ends), so an engine with an SM budget is sized for that
+// cut as well
+static size_t stack_skinny_floats(const Model& m, int sm_budget) {
   size_t f = 0;
-  auto slabs = [](size_t N, size_t K) { return (size_t)gemm_skinny_max_segs((int)N, (int)K, 148) * 256 * N; };
+  auto slabs = [&](size_t N, size_t K) {
+    const int whole = gemm_skinny_max_segs((int)N, (int)K, 148), part = sm_budget > 0 ? gemm_skinny_max_segs((int)N, (int)K, sm_budget) : 0;
+    return (size_t)std::max(whole, part) * 256 * N;
+  };
   auto shape = [&](size_t N, size_t K) { f = std::max(f, slabs(N, K)); };
   const size_t W = m.sd.width;
   for (int i = 0; i < m.sd.n_layers; ++i) {
@@ -409,13 +414,26 @@ size_t Engine::workspace_bytes_stack() const {
   b += al256((size_t)cfg_.max_seqs * 4);                              // sampled
   b += al256(sample_scratch_bytes(cfg_.max_seqs, sd.vocab));
   b += 2 * al256((size_t)cfg_.max_seqs * HB_MAX_LOGPROBS * 4);
-  if (!sd.compute_f32) b += al256(stack_skinny_floats(model_) * 4) + al256(T * (size_t)up8(n2) * 2) + al256(T * (size_t)up8(cx) * 2);
+  if (!sd.compute_f32) b += al256(stack_skinny_floats(model_, cfg_.sm_budget) * 4) + al256(T * (size_t)up8(n2) * 2) + al256(T * (size_t)up8(cx) * 2);
   {
     int qb; size_t rows, keys, rmax, dmax, qa16;
     if (stack_att_caps(model_, &qb, &rows, &keys, &rmax, &dmax, &qa16))
       b += al256(T * qa16 * 2) + al256(keys * dmax * 2) + al256(rmax * keys * 2) + al256(rows * keys * 2) + al256(rows * keys * 4);
   }
   return b;
+}
+
+int64_t stack_slab_floats(const hb_stack_desc& desc, const hb_layer_desc* layers, int sm_budget) {
+  std::vector<hb_layer_desc> lv(layers, layers + desc.n_layers);
+  Model m;
+  std::vector<int> ids;
+  m.sd = desc;
+  if (!unroll_stack(m.sd, lv, ids).empty() || !validate_stack(m.sd, lv.data()).empty()) return -1;
+  m.layer_id = ids;
+  m.sl = lv;
+  m.d.vocab = desc.vocab;
+  layout_stack(m);  // (sizes alone: nothing is behind the addresses)
+  return m.sd.compute_f32 ? 0 : (int64_t)stack_skinny_floats(m, sm_budget);
 }
 
 int Engine::alloc_runtime_stack() {
@@ -429,6 +447,8 @@ int Engine::alloc_runtime_stack() {
   CU(stack_streams_init());
   CU(stack_lightning_init());
   CU(attn_latent_init());
+  paired_.assign(sd.n_layers, 0);
+  skinny_floats_ = sd.compute_f32 ? 0 : stack_skinny_floats(model_, cfg_.sm_budget);
   if (!sd.compute_f32) {  // stream-K plans allocate on first use of a shape: make them now, not inside a graph capture
     SmLimitScope sm_scope(cfg_.sm_budget);
     SkinnyPlan pl{};
@@ -437,6 +457,15 @@ int Engine::alloc_runtime_stack() {
       CU(gemm_skinny_plan(model_.sw[i].n_in, sd.width, &pl));
       CU(gemm_skinny_plan(sd.width, model_.sw[i].o_cols ? model_.sw[i].o_cols : l.heads * l.vdim, &pl));
       if (l.ff > 0 && l.ff_kind == HB_FF_RELU2) CU(gemm_skinny_plan(l.ff, sd.width, &pl));
+      if (paired_ok(model_, i)) {  // asked once, for the most tokens, so that a row's sums do not depend on how many a step has
+        SkinnyPlan in{}, up{}, o{}, down{};
+        CU(gemm_skinny_plan(model_.sw[i].n_in, sd.width, &in));
+        CU(gemm_skinny_plan(l.ff, sd.width, &up));
+        CU(gemm_skinny_plan(sd.width, model_.sw[i].o_cols ? model_.sw[i].o_cols : l.heads * l.vdim, &o));
+        CU(gemm_skinny_plan(sd.width, l.ff, &down));
+        paired_[i] = gemm_skinny_ws_floats(in, 256, model_.sw[i].n_in) + gemm_skinny_ws_floats(up, 256, l.ff) <= skinny_floats_ &&
+                     gemm_skinny_ws_floats(o, 256, sd.width) + gemm_skinny_ws_floats(down, 256, sd.width) <= skinny_floats_;
+      }
       if (l.mixer == HB_MIXER_LATENT && l.q_rank > 0) CU(gemm_skinny_plan(l.heads * (l.dim + l.rot_dim), l.q_rank, &pl));
       if (l.ff > 0) {
         CU(gemm_skinny_plan(2 * l.ff, sd.width, &pl));
@@ -570,7 +599,6 @@ int Engine::alloc_runtime_stack() {
   sample_ws_ = take(sample_scratch_bytes(cfg_.max_seqs, sd.vocab));
   lp_ids_ = (int32_t*)take((size_t)cfg_.max_seqs * HB_MAX_LOGPROBS * 4);
   lp_vals_ = (float*)take((size_t)cfg_.max_seqs * HB_MAX_LOGPROBS * 4);
-  skinny_floats_ = sd.compute_f32 ? 0 : stack_skinny_floats(model_);
   skinny_ws_ = sd.compute_f32 ? nullptr : (float*)take(skinny_floats_ * 4);
   if (!sd.compute_f32) {
     sk_.q16 = (bf16*)take(T * (size_t)sk_.ld2 * 2);
@@ -1072,7 +1100,7 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
     int rc = HB_OK, longest_entry = 0;
     for (const StepEntry& en : step_entries_) longest_entry = std::max(longest_entry, en.n);
     // linear attention over a long portion: bf16 rows, the activations of q | k | v on the accumulators' way out
-    const bool paired = T <= 256 && skinny_ws_ && k.gu16 && paired_ok(model_, i) && stack_tc(w.n_in, W, W, k.ld1) && few_token_gemm();
+    const bool paired = T <= 256 && skinny_ws_ && k.gu16 && paired_[i] && stack_tc(w.n_in, W, W, k.ld1) && few_token_gemm();
     const bool chunked = light_chunk_ok(model_, l) && T > 256 && longest_entry >= kAttDenseMin && k.gu16 && stack_tc(w.n_in, W, W, w.n_in);
     if (chunked) {
       GemmArgs g{x16, W, (const bf16*)w.w_in, W, k.gu16, w.n_in, nullptr, 0, nullptr, T, w.n_in, W, EPI_SILU_COLS, 0};

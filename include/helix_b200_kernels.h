@@ -8,6 +8,8 @@
 #define HELIX_B200_KERNELS_H_
 #include <stddef.h>
 #include <stdint.h>
+
+#include "helix_b200.h"
 #ifdef __cplusplus
 extern "C" {
 #endif
@@ -28,6 +30,11 @@ int hbk_gemm_skinny_finish(const void* X, int ldx, const void* W, int ldw, float
 /* two such products of the same M rows in one launch, cut for `sms` SMs (0 = all): the bits that each has by itself */
 int hbk_gemm_skinny_pair(const void* X, int ldx, const void* W, int ldw, float* out_f32, int ldo, int N, int K, const void* X2, int ldx2,
                          const void* W2, int ldw2, float* out2_f32, int ldo2, int N2, int K2, int M, int sms);
+/* slabs of a 128-column tile at most where such a product is cut for `sms` SMs; no device is asked */
+int hbk_gemm_skinny_slabs(int N, int K, int sms);
+/* floats that an engine with this sm_budget (0 = none) sets aside for such slabs, for steps of up to 256 tokens of a layer-list decoder; -1: a
+ * description that the engine refuses.  No device is asked */
+int64_t hbk_stack_slab_floats(const hb_stack_desc* desc, const hb_layer_desc* layers, int sm_budget);
 int hbk_gemm_naive(const void* A, int lda, const void* W, int ldw, void* C_f32, int ldc, int M, int N, int K);
 
 int hbk_embed_gather(const int32_t* tokens, const void* table, void* x, int T, int H);

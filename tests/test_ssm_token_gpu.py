@@ -38,3 +38,18 @@ def test_single_tokens_have_the_bits_of_portions(heads, groups, ff, seqs):
             got.append(np.concatenate(rows))
     assert launches[0] < launches[-1]  # (another path)
     assert np.isfinite(got[0]).all() and np.array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("budget", [0, 40, 61, 97])
+def test_steps_of_256_tokens_under_an_sm_budget(budget):
+    """Products cut for fewer SMs, with more slabs than on the whole machine: a step of 256 tokens has the bits of the same portions in steps of their own."""
+    layers = [E.LayerDesc(mixer=E.MIXER_MAMBA2, heads=16, vdim=64, dim=128, kv_heads=8, norm_groups=8, conv_taps=4, ff_kind=E.FF_RELU2, ff=2048) for _ in range(2)]
+    d = E.StackDesc(width=512, vocab=4096, layers=layers, norm_eps=1e-5, norm_place=E.NORM_PARALLEL, embed_norm=1, plain_gains=1, tie_head=1)
+    toks = np.random.default_rng(7).integers(0, 4096, (4, 64)).astype(np.int32)
+    want = list(range(64))
+    with hb.Engine(hb.EngineConfig(max_seqs=8, max_ctx=64, max_batched_tokens=256, kv_pool_tokens=512, sm_budget=budget)) as e:
+        e.load_random(d, 5)
+        ids = [e.seq_open() for _ in range(8)]
+        together = e.seq_step([(s, t, want) for s, t in zip(ids, toks)])
+        alone = np.concatenate([e.seq_step([(s, t, want)]) for s, t in zip(ids[4:], toks)])
+    assert np.isfinite(together).all() and np.abs(together).max() > 0 and np.array_equal(together, alone)
