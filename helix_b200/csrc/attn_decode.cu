@@ -86,7 +86,6 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   // lengths (uploaded before the step), all older K/V pages — is immutable during the step, so the TMA ring is filled and
   // the barriers / TMEM are set up while the predecessor is still draining; griddepcontrol.wait sits right in front of
   // the first dependent access of each role.
-  pdl_launch_dependents();
   if (blockIdx.x | blockIdx.y | blockIdx.z) trace = nullptr;
   if (threadIdx.x == 0) trace_ev(trace, 0);
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
@@ -142,6 +141,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   if (warp == 1) {
     tmem_alloc(tmem_ptr, 64);
     tmem_relinquish();
+    pdl_launch_dependents();  // (launch.h; a block without work, above, by its end)
   }
   tc_fence_before();
   __syncthreads();

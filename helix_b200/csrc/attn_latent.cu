@@ -99,7 +99,6 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_con
   const int n_tiles = min(n_total, t_begin + tps) - t_begin;
   const int h0 = hg * NQ, nh = min(NQ, a.H - h0);
   float* ws = a.workspace + (((size_t)tq * gridDim.y + hg) * num_splits + split) * NQ * (R + 2);
-  pdl_launch_dependents();
   if (n_tiles <= 0) {
     pdl_wait();  // the partials may still be read by an earlier launch's combine pass
     for (int i = threadIdx.x; i < NQ * (R + 2); i += kThreads) ws[i] = (i % (R + 2) == R) ? -INFINITY : 0.f;
@@ -127,6 +126,7 @@ latent_decode_kernel(const __grid_constant__ CUtensorMap map_c, const __grid_con
   if (warp == 1) {
     tmem_alloc(tmem_ptr, kCols);
     tmem_relinquish();
+    pdl_launch_dependents();  // (launch.h)
   }
   tc_fence_before();
   __syncthreads();

@@ -263,7 +263,6 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     tma_load_2d(dst, &map_x, bar, x.kb * BLOCK_K, 0, kEvictLast);
   };
 
-  pdl_launch_dependents();
   if (blockIdx.x != 0) trace = nullptr;
   if (threadIdx.x == 0) {
     trace_ev(trace, 0);
@@ -286,6 +285,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   if (warp == 1) {
     tmem_alloc(tmem_ptr, C::TMEM_COLS);
     tmem_relinquish();
+    pdl_launch_dependents();  // (launch.h)
   }
   tc_fence_before();
   __syncthreads();

@@ -1,6 +1,8 @@
 // Launch helper: programmatic dependent launch (PDL) for the decode step's short kernels.
 // A PDL-launched kernel may begin (prologue + anything that touches ONLY static data such as weights)
 // while its predecessor drains; it must execute pdl_wait() before reading or writing any activation.
+// A kernel with tensor memory lets the next one start (pdl_launch_dependents) only once it holds its columns: a block of the next one that
+// finds room on an SM would otherwise take columns first and wait, in pdl_wait, for a block that waits for them.
 #pragma once
 #include <cuda_runtime.h>
 
