@@ -149,6 +149,7 @@ SIGNATURES = {
     "hbk_sample_filtered": (I, [P, I, P, P, P, P, P, I, I]),
     "hbk_apply_penalties": (I, [P, I, P, P, I, I]),
     "hbk_logprob_topk": (I, [P, I, I, P, P, P, P, I, I]),
+    "hbk_embed_step": (I, [P, P, C.c_float, P, P, I, I, I, P, C.c_float, P, P, I, C.c_float, P, P, P, P, P, I, I, I]),
     "hbk_cls_pool_l2": (I, [P, P, P, I, I]),
     "hbk_attn_prefill": (I, [P, I, P, I, P, I, P, I, P, I, I, I, I, I, I, I, C.c_float]),
     "hbk_attn_prefill_paged": (I, [P, I, P, P, P, I, P, P, I, P, I, I, I, I, I, I, I, C.c_float, I]),

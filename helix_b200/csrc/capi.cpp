@@ -294,6 +294,21 @@ int hbk_logprob_topk(const float* logits, int ldl, int V, const int32_t* sampled
                      float* out_lp, int B, int max_width) {
   return kret(hb::logprob_topk(0, logits, ldl, V, sampled, width, out_ids, out_lp, B, max_width, max_width));
 }
+int hbk_embed_step(const int32_t* tokens, const void* table, float scale, const void* pairs, const int32_t* prev, int buckets, int mul_prev,
+                   int mul_cur, const void* w0, float off, const void* w1, const void* w2, int f32, float eps, float* x, float* h1, void* h1b, float* h2,
+                   void* h2b, int T, int W, int parts) {
+  hb::BigramArgs bg;
+  bg.table = pairs; bg.prev = prev; bg.buckets = buckets; bg.mul_prev = mul_prev; bg.mul_cur = mul_cur;
+  if (!parts) {
+    if (!hb::embed_step_ok(table, w0, w1, w2, bg, W)) return kret(cudaErrorInvalidValue);
+    return kret(hb::embed_step(0, tokens, table, scale, bg, w0, off, w1, w2, f32 != 0, eps, x, h1, (hb::bf16*)h1b, h2, (hb::bf16*)h2b, T, W));
+  }
+  cudaError_t e = hb::embed_rows_f32(0, tokens, table, f32 != 0, x, nullptr, T, W, scale, bg);
+  if (e == cudaSuccess) e = hb::norm_rows_f32(0, x, nullptr, w0, f32 != 0, off, eps, x, nullptr, T, W);
+  if (e == cudaSuccess)
+    e = hb::parallel_step(0, x, nullptr, nullptr, nullptr, nullptr, 0.f, w1, w2, f32 != 0, eps, nullptr, h1, (hb::bf16*)h1b, h2, (hb::bf16*)h2b, T, W);
+  return kret(e);
+}
 int hbk_cls_pool_l2(const void* x, const int32_t* first_row, float* out, int B, int H) {
   return kret(hb::cls_pool_l2(0, (const hb::bf16*)x, first_row, out, B, H));
 }

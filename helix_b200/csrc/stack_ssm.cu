@@ -1233,7 +1233,9 @@ __global__ void __launch_bounds__(256) parallel_step_vec_kernel(const float* x, 
 }
 
 // The embedding, its norm and the first layer's norms with the row in registers: three launches passed it through memory (11k tokens x 2048 in
-// 154 us, 47 now), a step of few tokens waited for each of them
+// 154 us, 47 now), a step of few tokens waited for each of them.  The sums of squares are written out in the order that those three's have,
+// so that a row has their bits: sum_of_squares, but for the embedding's norm of fp32 tables, where x^2 is added to y^2's product; the scaled row is
+// rounded before a pair's row joins it
 template <typename WT, int CH>
 __global__ void __launch_bounds__(256) embed_step_kernel(const int32_t* __restrict__ tokens, const WT* __restrict__ table, float scale, BigramArgs bg,
                                                          const WT* __restrict__ w0, float off, const WT* __restrict__ w1, const WT* __restrict__ w2, float eps,
@@ -1260,10 +1262,10 @@ __global__ void __launch_bounds__(256) embed_step_kernel(const int32_t* __restri
     a = make_float4(a.x * scale, a.y * scale, a.z * scale, a.w * scale);
     if (pair) {
       const float4 p = ldf4<WT>(pair + i);
-      a = make_float4(a.x + p.x, a.y + p.y, a.z + p.z, a.w + p.w);
+      a = make_float4(__fadd_rn(a.x, p.x), __fadd_rn(a.y, p.y), __fadd_rn(a.z, p.z), __fadd_rn(a.w, p.w));
     }
     v[c] = a;
-    ss += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+    ss += sizeof(WT) == 4 ? sum_of_squares(make_float4(a.y, a.x, a.z, a.w)) : sum_of_squares(a);
   }
   const float rs0 = 1.f / sqrtf(block_sum(ss, red) / (float)W + eps);
   ss = 0.f;
@@ -1275,7 +1277,7 @@ __global__ void __launch_bounds__(256) embed_step_kernel(const int32_t* __restri
     const float4 a = make_float4(v[c].x * (rs0 * (off + g.x)), v[c].y * (rs0 * (off + g.y)), v[c].z * (rs0 * (off + g.z)), v[c].w * (rs0 * (off + g.w)));
     *reinterpret_cast<float4*>(x + r * W + i) = a;
     v[c] = a;
-    ss += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
+    ss += sum_of_squares(a);
   }
   const float rs = 1.f / sqrtf(block_sum(ss, red) / (float)W + eps);
 #pragma unroll

@@ -60,6 +60,12 @@ int hbk_apply_penalties(float* logits, int ldl, const int32_t* pen_off, const vo
  * descending order (lowest id first on ties).  out_* are [B][max_width]. */
 int hbk_logprob_topk(const float* logits, int ldl, int V, const int32_t* sampled, const int32_t* width, int32_t* out_ids,
                      float* out_lp, int B, int max_width);
+/* The start of a stack with parallel sublayers: x = rms norm (gain off + w0) of scale * table[token] (+ the row of a token pair in `pairs`: buckets + 1 rows,
+ * row (prev mul_prev + token mul_cur) % buckets, the last one where prev < 0; NULL: none), h1 / h2 = rms norms of x with gains w1 / w2 (w2 may be NULL),
+ * fp32 and bf16 (any output of h1, h2 may be NULL).  f32: fp32 weights, else bf16.  parts: three launches instead of one, the same bits. */
+int hbk_embed_step(const int32_t* tokens, const void* table, float scale, const void* pairs, const int32_t* prev, int buckets, int mul_prev,
+                   int mul_cur, const void* w0, float off, const void* w1, const void* w2, int f32, float eps, float* x, float* h1, void* h1_b16,
+                   float* h2, void* h2_b16, int T, int W, int parts);
 int hbk_cls_pool_l2(const void* x, const int32_t* first_row, float* out, int B, int H);
 
 int hbk_attn_prefill(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, void* out, int ldo,
