@@ -55,13 +55,13 @@ struct DCfg {
 template <int D, int G>
 __global__ void __launch_bounds__(kThreads, 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                   const bf16* __restrict__ q, int ldq, const int32_t* __restrict__ page_table, int max_pages,
-                   const int32_t* __restrict__ ctx_lens, float* __restrict__ ws, int Hkv, int num_splits,
+                   const bf16* __restrict__ q, int ldq, const int32_t* page_table, int max_pages,
+                   const int32_t* ctx_lens, float* __restrict__ ws, int Hkv, int num_splits,
                    float scale_log2, bf16* __restrict__ out_direct, int ldo, const int* sig_wait, int sig_wait_count,
                    int* sig_done, int bank_tiles, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache,
                    unsigned long long* trace, const int* dep_wait, int dep_count, int* dep_done,
                    const __grid_constant__ DecodeRope rope, int chunk, int sink, const float* __restrict__ head_gate, int ldg,
-                   int window, float cap_in, float cap_out, const bf16* __restrict__ sink_w) {
+                   int window, float cap_in, float cap_out, const bf16* __restrict__ sink_w, int settled) {
   using C = DCfg<D>;
   constexpr int STAGES = C::STAGES;
   extern __shared__ uint8_t smem_raw[];
@@ -81,11 +81,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
   uint64_t* kv_ready = bars + 2 * STAGES + 7;  // fused RoPE prologue: this CTA's new K/V row is in the cache
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 8);
 
-  // Programmatic dependent launch: only two things here depend on the kernel before this one (RoPE + KV write of the
-  // step's new token): q, and the LAST kv tile (it holds the new position).  Everything else — page table, context
+  // Programmatic dependent launch.  Within an engine's step (settled) only two things here depend on the kernel before this one (RoPE + KV write of
+  // the step's new token): q, and the LAST kv tile (it holds the new position).  Everything else — page table, context
   // lengths (uploaded before the step), all older K/V pages — is immutable during the step, so the TMA ring is filled and
   // the barriers / TMEM are set up while the predecessor is still draining; griddepcontrol.wait sits right in front of
-  // the first dependent access of each role.
+  // the first dependent access of each role.  A caller of the kernel interface may have any of it written by the kernels ahead, however many of them
+  // let the next one start early: there the wait comes first (32 sequences of 2k positions, back to back 39.4 -> 41.7 us; set-up ahead of
+  // the wait measured the same).  No __restrict__ on the two tables: a load that the compiler takes for invariant could move above it.
+  if (!settled) pdl_wait();
   if (blockIdx.x | blockIdx.y | blockIdx.z) trace = nullptr;
   if (threadIdx.x == 0) trace_ev(trace, 0);
   const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
@@ -516,7 +519,7 @@ cudaError_t launch(cudaStream_t stream, const AttnDecodeArgs& a) {
                            a.k_cache, a.v_cache, a.sig.trace, a.sig.dep.wait, a.sig.dep.wait_count, a.sig.dep.done,
                            a.num_splits == 1 ? a.rope : DecodeRope{}, a.block_mask, a.unit_sink, a.head_gate, a.ldg, a.window,
                            a.softcap > 0.f ? 2.f * 1.4426950408889634f * a.scale / a.softcap : 0.f,
-                           a.softcap > 0.f ? a.softcap * 1.4426950408889634f : 0.f, a.sink);
+                           a.softcap > 0.f ? a.softcap * 1.4426950408889634f : 0.f, a.sink, (int)a.settled);
   if (e != cudaSuccess || direct) return e;
   return launch_k(attn_decode_combine_kernel<D>, dim3(a.Hq, a.B), dim3(D / 2), 0, stream, true,
                   (const float*)a.workspace, a.out, a.ldo, a.Hq, a.Hkv, G, a.num_splits, a.unit_sink, a.head_gate, a.ldg, a.sink);

@@ -682,6 +682,7 @@ int Engine::forward_llama(int T, int B, bool prefill, int max_seqlen, const Step
       // token per sequence over its paged context — the HBM-bound decode-attention kernel, not a 128-row prefill q tile each
       const int b0 = prefill ? Bpf : 0, t0 = prefill ? Tpf : 0, nb = prefill ? Bd : B;
       AttnDecodeArgs a{};
+      a.settled = true;  // (kernels.h)
       a.q = qkv_ + (size_t)t0 * QKV; a.ldq = QKV;
       a.k_cache = kc; a.v_cache = vc;
       a.page_table = pt + (size_t)b0 * max_pages_per_seq_; a.max_pages = max_pages_per_seq_;
@@ -822,6 +823,7 @@ int Engine::forward_llama_decode(int B, const StepLayout& L) {
     }
     {
       AttnDecodeArgs a{};
+      a.settled = true;  // (kernels.h)
       a.q = qkv_; a.ldq = QKV;
       a.k_cache = kc; a.v_cache = vc;
       a.page_table = pt; a.max_pages = max_pages_per_seq_;
@@ -942,6 +944,7 @@ int Engine::forward_llama_decode_fused(int B, const StepLayout& L) {
     }
     {
       AttnDecodeArgs a{};
+      a.settled = true;  // (kernels.h)
       a.q = qkv_; a.ldq = QKV;
       a.k_cache = kc; a.v_cache = vc;
       a.page_table = pt; a.max_pages = max_pages_per_seq_;

@@ -1300,6 +1300,7 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
       SPAN(3, 8.0 * T * (H + 2 * G) * Dk, gqa_prep(stream_, pa));
       if (tc_dec) {
         AttnDecodeArgs da{};
+        da.settled = true;  // (kernels.h)
         da.q = k.q16; da.ldq = H * Dk;
         da.k_cache = (const bf16*)kplane; da.v_cache = (const bf16*)vplane;
         da.page_table = pt; da.max_pages = max_pages_per_seq_;

@@ -233,6 +233,9 @@ struct AttnDecodeArgs {
   int window = 0;
   float softcap = 0.f;
   const bf16* sink = nullptr;
+  // No kernel that may still run when this one begins writes the page table, the context lengths or any position but a sequence's last (a step of an
+  // engine that uploads the tables before it and writes one position per sequence): they may be read before the kernels ahead are done
+  bool settled = false;
 };
 cudaError_t attn_decode(cudaStream_t stream, const AttnDecodeArgs& a);
 size_t attn_decode_workspace_floats(int B, int Hq, int D, int num_splits);

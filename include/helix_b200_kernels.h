@@ -89,8 +89,6 @@ int hbk_attn_prefill_plan(int B, int T, int max_seqlen, int Hq, int Hkv, int pag
 int hbk_attn_naive(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, float* out_f32, int ldo,
                    const int32_t* cu_seqlens, int B, int T, int max_seqlen, int Hq, int Hkv, int D, int causal,
                    float scale);
-/* The page table, the context lengths and the tiles before a sequence's last one are read while kernels of this library that were launched right before may
- * still run: those may write the new position (hbk_rope_kv_write, a projection), not the tables or older positions. */
 int hbk_attn_decode(const void* q, int ldq, const void* k_cache, const void* v_cache, const int32_t* page_table,
                     int max_pages, const int32_t* ctx_lens, void* out, int ldo, float* workspace, int B, int Hq, int Hkv,
                     int D, int page_size, int num_splits, float scale, int num_pages);

@@ -473,6 +473,43 @@ def test_attn_prefill_paged_chunks(L, D, Hq, Hkv, causal):
         torch.testing.assert_close(out[cu[b]:cu[b + 1]].float(), want, rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("D,Hq,Hkv,splits", [(128, 32, 8, 1), (64, 32, 8, 2)])
+@pytest.mark.parametrize("between", [0, 1])
+def test_attn_decode_right_behind_what_it_reads(L, D, Hq, Hkv, splits, between):
+    """All positions of a prompt written by kernels right before, with or without a product in between: none is read ahead of them."""
+    page, B, n, K = 64, 4, 704, 512
+    T, N, per = B * n, (Hq + 2 * Hkv) * D, (n + page - 1) // page
+    W, Wm = rnd(N, K, seed=70, scale=K ** -0.5), rnd(4096, N, seed=71, scale=N ** -0.5)
+    inv = (1.0 / (500000.0 ** (torch.arange(0, D, 2, device="cuda").float() / D))).contiguous()
+    pos = torch.arange(n, device="cuda", dtype=torch.int32).repeat(B)
+    table = torch.randperm(B * per, device="cuda").to(torch.int32).view(B, per)
+    slots = (table.repeat_interleave(page, 1)[:, :n] * page + torch.arange(n, device="cuda", dtype=torch.int32) % page).reshape(-1).contiguous()
+    lens = torch.full((B,), n, device="cuda", dtype=torch.int32)
+    qkv, mid = torch.empty(T, N, device="cuda", dtype=BF), torch.empty(T, 4096, device="cuda", dtype=BF)
+    kc, vc = (torch.empty(B * per, Hkv, page, D, device="cuda", dtype=BF) for _ in range(2))
+    ws = torch.empty(L.hbk_attn_decode_workspace_floats(B, Hq, D, splits), device="cuda")
+    out, want = (torch.empty(B, Hq * D, device="cuda", dtype=BF) for _ in range(2))
+
+    def decode(o):
+        ck(L, L.hbk_attn_decode(p(qkv) + (n - 1) * N * 2, n * N, p(kc), p(vc), p(table), per, p(lens), p(o), Hq * D, p(ws), B, Hq, Hkv, D, page, splits,
+                                D ** -0.5, B * per))
+    for r in range(10):
+        A = rnd(T, K, seed=80 + r)
+        kc.fill_(float("nan"))
+        vc.fill_(float("nan"))
+        if between:
+            ck(L, L.hbk_gemm(p(A), K, p(W), K, p(qkv), N, None, 0, None, T, N, K, 0, 0))
+            ck(L, L.hbk_rope_kv_write(p(qkv), p(pos), p(slots), p(inv), p(kc), p(vc), T, Hq, Hkv, D, page))
+            ck(L, L.hbk_gemm(p(qkv), N, p(Wm), N, p(mid), 4096, None, 0, None, T, 4096, N, 0, 0))
+        else:
+            ck(L, L.hbk_gemm_qkv_rope(p(A), K, p(W), K, p(qkv), None, p(pos), p(slots), p(inv), p(kc), p(vc), T, K, Hq, Hkv, D, page))
+        decode(out)
+        torch.cuda.synchronize()
+        decode(want)
+        torch.cuda.synchronize()
+        assert torch.isfinite(want.float()).all() and torch.equal(out, want)
+
+
 @pytest.mark.parametrize("M,N,K", [(32, 6144, 4096), (1, 4096, 4096), (7, 1000, 256), (64, 4096, 14336), (100, 28672, 4096),
                                    (256, 128256, 2048), (200, 512, 64), (33, 128, 4096)])
 def test_gemm_skinny_stream_k(L, M, N, K):
