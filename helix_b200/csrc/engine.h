@@ -126,9 +126,9 @@ class Engine {
   int latent_attention_tc(int T, const StepLayout& L, const hb_layer_desc& l, const StackLayerW& w,
                           const std::vector<std::pair<int, int>>& runs);
   int forward_stack(int T, int B, const StepLayout& L, const int32_t* extra_rows, int n_extra, float* extra_out, bool sample);
+  bool rows_to_host(int n) const;  // the head writes n rows of a driven step's logits to pinned host memory itself
   // C[M, N] (fp32, row stride ldc) = A . W^T: tcgen05 GEMM when the mode and the strides allow it (A_b16 = bf16 copy of A),
   // CUDA-core fp32 GEMM otherwise
-  bool rows_to_host(int n) const;
   int stack_gemm(const float* A, const bf16* A_b16, int lda, const void* W, int N, int K, float* C, int ldc, int M, const void* bias = nullptr, bf16* relu2 = nullptr, bool* relu2_done = nullptr);
   int take_slot();
   void drop_slot(Request* r);

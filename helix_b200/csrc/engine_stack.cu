@@ -694,8 +694,11 @@ static bool few_token_gemm() {  // HB_STACK_SKINNY=0: the tiled GEMM for few tok
 // Not where a softcap or a scale reads them again
 bool Engine::rows_to_host(int n) const {
   const hb_stack_desc& sd = model_.sd;
-  return n > 0 && n <= 256 && (size_t)n * sd.vocab <= h_rows_floats_ && few_token_gemm() && !(sd.logit_softcap > 0.f) &&
-         (sd.logit_scale == 0.f || sd.logit_scale == 1.f);
+  if (n <= 0 || n > 256 || (size_t)n * sd.vocab > h_rows_floats_ || sd.logit_softcap > 0.f || (sd.logit_scale != 0.f && sd.logit_scale != 1.f)) return false;
+  if (sd.compute_f32) return true;
+  SkinnyPlan plan{};  // (what stack_gemm asks)
+  return few_token_gemm() && stack_tc(sd.vocab, sd.width, sd.width, 4) && gemm_skinny_plan(sd.vocab, sd.width, &plan) == cudaSuccess &&
+         gemm_skinny_ws_floats(plan, n, sd.vocab) <= skinny_floats_;
 }
 bool Engine::stack_tc(int N, int K, int lda, int ldc) const {
   static const bool simt_only = [] { const char* e = getenv("HB_STACK_SIMT"); return e && atoi(e) != 0; }();

@@ -53,3 +53,26 @@ def test_steps_of_256_tokens_under_an_sm_budget(budget):
         together = e.seq_step([(s, t, want) for s, t in zip(ids, toks)])
         alone = np.concatenate([e.seq_step([(s, t, want)]) for s, t in zip(ids[4:], toks)])
     assert np.isfinite(together).all() and np.abs(together).max() > 0 and np.array_equal(together, alone)
+
+
+@pytest.mark.parametrize("width,vocab,f32,budget,seqs", [(256, 4096, 0, 0, 2), (256, 4096, 0, 20, 40), (256, 4096, 1, 0, 2), (72, 190, 0, 0, 3), (68, 190, 0, 0, 3),
+                                                         (256, 100003, 0, 0, 8)])
+def test_rows_that_the_head_writes_to_the_host(width, vocab, f32, budget, seqs):
+    """Logits up to the pinned buffer's size (four rows per sequence, 2^20 floats) and one row more, which are copied: the same rows, bit for bit."""
+    layers = [E.LayerDesc(mixer=E.MIXER_MAMBA2, heads=4, vdim=64, dim=128, kv_heads=2, norm_groups=2, conv_taps=4, ff_kind=E.FF_RELU2, ff=1024)]
+    d = E.StackDesc(width=width, vocab=vocab, layers=layers, compute_f32=f32, norm_eps=1e-5, norm_place=E.NORM_PARALLEL, embed_norm=1, plain_gains=1, tie_head=1)
+    limit = min(4 * seqs, 2 ** 20 // vocab)
+    toks = np.random.default_rng(11).integers(0, vocab, 256 // seqs * seqs).astype(np.int32).reshape(seqs, -1)
+    n = toks.shape[1]
+    rows = [(i, j) for i in range(seqs) for j in range(n)]
+    got = []
+    with hb.Engine(hb.EngineConfig(max_seqs=seqs, max_ctx=256, max_batched_tokens=256, kv_pool_tokens=256 * seqs, sm_budget=budget)) as e:
+        e.load_random(d, 5)
+        for count in (limit, limit + 1):
+            ids = [e.seq_open() for _ in range(seqs)]
+            asked = rows[:count]
+            got.append(e.seq_step([(s, t, [j for k, j in asked if k == i]) for i, (s, t) in enumerate(zip(ids, toks))]))
+            for s in ids:
+                e.seq_close(s)
+    assert len(got[0]) == limit and len(got[1]) == limit + 1
+    assert np.isfinite(got[1]).all() and np.abs(got[1]).max() > 0 and np.array_equal(got[0], got[1][:limit])
