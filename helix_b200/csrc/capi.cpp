@@ -150,9 +150,12 @@ int hbk_gemm(const void* A, int lda, const void* W, int ldw, void* C, int ldc, c
                  (const hb::bf16*)bias, M, N, K, (hb::Epi)epi, block_n};
   return kret(hb::gemm_bf16_tn(0, g));
 }
+// The few-token product reads its weights ahead of its dependency wait (an engine's are static); a caller's may be the output of a kernel that still runs
+static cudaError_t weights_settled() { return cudaStreamSynchronize(0); }
 int hbk_gemm_skinny(const void* X, int ldx, const void* W, int ldw, float* out, int ldo, int M, int N, int K) {
   hb::SkinnyPlan plan;
-  cudaError_t e = hb::gemm_skinny_plan(N, K, &plan);
+  cudaError_t e = weights_settled();
+  if (e == cudaSuccess) e = hb::gemm_skinny_plan(N, K, &plan);
   if (e != cudaSuccess) return kret(e);
   float* ws = nullptr;
   if ((e = cudaMalloc(&ws, hb::gemm_skinny_ws_floats(plan, M, N) * 4)) != cudaSuccess) return kret(e);
@@ -164,7 +167,8 @@ int hbk_gemm_skinny(const void* X, int ldx, const void* W, int ldw, float* out, 
 }
 int hbk_gemm_skinny_finish(const void* X, int ldx, const void* W, int ldw, float* out, int ldo, int M, int N, int K, int repeats) {
   hb::SkinnyPlan plan;
-  cudaError_t e = hb::gemm_skinny_plan(N, K, &plan);
+  cudaError_t e = weights_settled();
+  if (e == cudaSuccess) e = hb::gemm_skinny_plan(N, K, &plan);
   if (e != cudaSuccess) return kret(e);
   float* ws = nullptr;
   int* cnt = nullptr;
@@ -187,7 +191,8 @@ int hbk_gemm_skinny_pair(const void* X, int ldx, const void* W, int ldw, float* 
                          int ldw2, float* out2, int ldo2, int N2, int K2, int M, int sms) {
   hb::SmLimitScope scope(sms);
   hb::SkinnyProduct a{(const hb::bf16*)X, ldx, (const hb::bf16*)W, ldw, nullptr, N, K, {}}, b{(const hb::bf16*)X2, ldx2, (const hb::bf16*)W2, ldw2, nullptr, N2, K2, {}};
-  cudaError_t e = hb::gemm_skinny_plan(N, K, &a.plan);
+  cudaError_t e = weights_settled();
+  if (e == cudaSuccess) e = hb::gemm_skinny_plan(N, K, &a.plan);
   if (e == cudaSuccess) e = hb::gemm_skinny_plan(N2, K2, &b.plan);
   if (e != cudaSuccess) return kret(e);
   const size_t first = (hb::gemm_skinny_ws_floats(a.plan, M, N) + 3) / 4 * 4;

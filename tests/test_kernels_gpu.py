@@ -528,6 +528,19 @@ def test_gemm_skinny_stream_k(L, M, N, K):
     assert torch.equal(out, out3)
 
 
+def test_gemm_skinny_right_behind_its_weights(L):
+    """Weights that are the output of the product right before: none is read ahead of it."""
+    M, N, K, J = 32, 8192, 2048, 4096
+    X, B = rnd(M, K, seed=90), rnd(K, J, seed=91, scale=J ** -0.5)
+    W, out, want = torch.empty(N, K, device="cuda", dtype=BF), torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    for r in range(5):
+        A = rnd(N, J, seed=92 + r)
+        ck(L, L.hbk_gemm(p(A), J, p(B), J, p(W), K, None, 0, None, N, K, J, 0, 0))
+        ck(L, L.hbk_gemm_skinny(p(X), K, p(W), K, p(out), N, M, N, K))
+        ck(L, L.hbk_gemm_skinny(p(X), K, p(W), K, p(want), N, M, N, K))
+        assert torch.isfinite(want).all() and torch.equal(out, want)
+
+
 @pytest.mark.parametrize("M", [1, 32, 33, 100, 129, 256])
 @pytest.mark.parametrize("first,second", [((6272, 1024), (4096, 1024)), ((1024, 2048), (1024, 4096)), ((4112, 512), (2048, 512)), ((392, 128), (1032, 128)),
                                           ((100, 72), (20, 1000)), ((128, 64), (4100, 3000)), ((30000, 264), (64, 64))])
