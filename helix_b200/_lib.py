@@ -133,6 +133,7 @@ SIGNATURES = {
     "hbk_init": (I, []),
     "hbk_last_error": (C.c_char_p, []),
     "hbk_gemm": (I, [P, I, P, I, P, I, P, I, P, I, I, I, I, I]),
+    "hbk_gemm_tile": (I, [I, I, I, I, I]),
     "hbk_gemm_naive": (I, [P, I, P, I, P, I, I, I, I]),
     "hbk_gemm_skinny": (I, [P, I, P, I, P, I, I, I, I]),
     "hbk_gemm_skinny_pair": (I, [P, I, P, I, P, I, I, I, P, I, P, I, P, I, I, I, I, I]),

@@ -79,8 +79,8 @@ __device__ int g_attn_trace_n[8];
 enum Order : int { ORDER_PLAIN = 0, ORDER_SPLIT = 1, ORDER_SORTED = 2 };
 // Split walk: the pairs from this one on, those of the last round, are taken as two lone q tiles each, where twice as many of them are no more than
 // there are CTAs (elsewhere the answer is `pairs`): a lone q tile takes about 3/4 of a pair's time, and the SMs that would have had nothing take the other
-// ones.  us, 32 heads over 8 of 128 columns: 777 x 2 rows over 6000 keys 173 -> 163 (64 columns 163 -> 150), 512 over 2500 46 -> 40; 12 heads of their own,
-// 333 x 2 over 4500 71 -> 62
+// ones.  us back to back, pages, with the packings that it makes the better ones and the launches as they are now: 32 heads over 8 of 128 columns, 777 x 2 rows
+// over 6000 keys 173 -> 170 (64 columns 156 -> 142), 512 over 2500 41 -> 33; 12 heads of their own, 333 x 2 over 4500 68 -> 55
 // An instance of its own: the walk's few registers in the plain one cost every other launch 2 % (2048 rows over 7000 191.5 -> 196.5).
 __host__ __device__ inline int first_split(int pairs, int ctas) {
   const int full = (pairs - 1) / ctas * ctas;

@@ -150,6 +150,11 @@ int hbk_gemm(const void* A, int lda, const void* W, int ldw, void* C, int ldc, c
                  (const hb::bf16*)bias, M, N, K, (hb::Epi)epi, block_n};
   return kret(hb::gemm_bf16_tn(0, g));
 }
+int hbk_gemm_tile(int M, int N, int K, int epi, int sms) {
+  if (M <= 0 || N <= 0 || K <= 0 || sms <= 0) return -1;
+  const hb::GemmTile t = hb::gemm_tile(M, N, K, (hb::Epi)epi, sms);
+  return t.bn | t.cg << 12 | t.eg << 16;
+}
 // The few-token product reads its weights ahead of its dependency wait (an engine's are static); a caller's may be the output of a kernel that still runs
 static cudaError_t weights_settled() { return cudaStreamSynchronize(0); }
 int hbk_gemm_skinny(const void* X, int ldx, const void* W, int ldw, float* out, int ldo, int M, int N, int K) {

@@ -175,11 +175,11 @@ int Engine::load_random_stack(const hb_stack_desc& sd, const hb_layer_desc* laye
 
 // ------------------------------------------------------------------ sizing
 // State-space layers with a squared-relu unit beside them (both read the same stream): in steps of up to 256 tokens the two products
-// that read the stream are one launch, and so are the two whose outputs join it.  Where every entry is one token their readers (convolution, gated norm,
-// residual step) sum the slabs themselves: six launches of a layer instead of thirteen, each a link of 4 to 7 us in a chain that nothing else
-// fills (a turn of 16 sequences, 2 layers of width 1024, 12 tokens each: 3070 -> 2560 us, of it about 25 us a step on the host: sizes
-// of the slabs worked out for every product).  The same products in every step of up to 256 tokens, so a row's sums do not
-// depend on whether a portion is among the entries
+// that read the stream are one launch, and so are the two whose outputs join it.  Where every entry is one token their readers sum the slabs
+// themselves: a layer has four launches where one kernel makes all between the products (ssm_token_ok), six where convolution, recurrence and gated norm do,
+// thirteen without any of it, each a link of 4 to 7 us in a chain that nothing else fills (a turn of 16 sequences, 2 layers of width 1024, 12 tokens each,
+// the steps' other changes included: 3065 -> 2290 us).  The same products in every step of up to 256 tokens, so a row's sums do not depend on whether a
+// portion is among the entries
 static bool paired_ok(const Model& m, int i) {
   const hb_layer_desc& l = m.sl[i];
   const int W = m.sd.width, n_in = m.sw[i].n_in, inner = l.heads * l.vdim, ocols = m.sw[i].o_cols ? m.sw[i].o_cols : inner;
@@ -1085,11 +1085,11 @@ int Engine::forward_stack(int T, int B, const StepLayout& L, const int32_t* extr
     SPAN(3, 3 * rowb, embed_step(stream_, tokens, model_.s_embed, sd.embed_scale != 0.f ? sd.embed_scale : 1.f, bigram, model_.s_embed_norm, goff, start.w1,
                                  start.w2, f32, sd.norm_eps, k.x, start.h1, x16, start.h2, f32 ? nullptr : k.x16b, T, W));
   } else {
-  SPAN(3, rowb, embed_rows_f32(stream_, tokens, model_.s_embed, f32, x_emb, pre ? nullptr : x16, T, W, sd.embed_scale != 0.f ? sd.embed_scale : 1.f, bigram));
-  if (sd.embed_norm) SPAN(3, 2 * rowb, norm_rows(x_emb, nullptr, model_.s_embed_norm, x_emb, both || pre ? nullptr : x16, T));
-  if (pre) SPAN(3, preb, pre_step(k.y, nullptr, nullptr, nullptr, 0, 0, nullptr));
-  if (both) SPAN(3, 2 * rowb, norm_rows(k.x, nullptr, model_.sw[0].norm1, k.hn, x16, T));
-  if (par) SPAN(3, 3 * rowb, par_step(nullptr, nullptr, nullptr, 0.f, 0, nullptr));
+    SPAN(3, rowb, embed_rows_f32(stream_, tokens, model_.s_embed, f32, x_emb, pre ? nullptr : x16, T, W, sd.embed_scale != 0.f ? sd.embed_scale : 1.f, bigram));
+    if (sd.embed_norm) SPAN(3, 2 * rowb, norm_rows(x_emb, nullptr, model_.s_embed_norm, x_emb, both || pre ? nullptr : x16, T));
+    if (pre) SPAN(3, preb, pre_step(k.y, nullptr, nullptr, nullptr, 0, 0, nullptr));
+    if (both) SPAN(3, 2 * rowb, norm_rows(k.x, nullptr, model_.sw[0].norm1, k.hn, x16, T));
+    if (par) SPAN(3, 3 * rowb, par_step(nullptr, nullptr, nullptr, 0.f, 0, nullptr));
   }
   for (size_t si = 0; si < k.freq_sets.size(); ++si)  // cos / sin of the step's positions, once per distinct rotation
     SPAN(3, 8.0 * T * k.freq_half[si], stack_rope_table(stream_, positions, k.freq_sets[si], k.freq_half[si], k.rope_cs[si], T, k.freq_mult[si]));

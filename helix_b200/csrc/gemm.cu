@@ -6,8 +6,8 @@
 //                                   double-buffered accumulators so tile i+1's MMAs overlap tile i's epilogue)
 //   warps 2..     : epilogue       (tcgen05.ld -> fused bias / GELU / residual / SwiGLU -> swizzled smem -> TMA store);
 //                                   two or four groups of four warps (one warp per TMEM lane quadrant) take the 64-column
-//                                   chunks in turn with their own staging buffer, so two warps per SM sub-partition hide each
-//                                   other's TMEM/global latencies and short-K tiles (BERT) are not epilogue-bound
+//                                   chunks in turn with their own staging buffer, so the two or four warps per SM sub-partition hide
+//                                   each other's TMEM/global latencies and short-K tiles (BERT) are not epilogue-bound
 // M, N, K tails are handled by TMA (zero fill on load, clipping on store).
 #include <math.h>
 #include <stdio.h>
@@ -169,8 +169,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if constexpr (CG == 2) cluster_sync_all(); else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);  // warp-uniform for the compiler too
-  // Launched while the kernel before it drains (nothing above touches memory that one may write): a product's launch and set-up cost the
-  // one behind it 2.5 us, 512 x 4096 x 14336 65.2 -> 62.6 back to back
+  // Launched while the kernel before it drains (nothing above touches memory that one may write), which hides a product's launch and set-up
+  // behind a kernel ahead of it: 512 x 4096 x 14336 65.2 -> 62.6 us back to back.  A call with nothing ahead of it takes what it took
   pdl_wait();
 
   // The single-thread roles keep the whole warp converged through their loops and barrier waits and predicate only the
@@ -581,12 +581,11 @@ bool use_pair() {  // HB_GEMM_2CTA=0 falls back to single-CTA tiles (A/B measure
 // without either 13800 x 2304 x 768 42 | 47: those have two)
 constexpr bool deep_epilogue(int epi) { return epi == EPI_BIAS_GELU || epi == EPI_GELU || epi == EPI_RESID || epi == EPI_BIAS_RESID; }
 
-template <int EPI>
-cudaError_t launch_epi(cudaStream_t stream, const GemmArgs& g, int num_sms) {
-  constexpr bool kWideOnly = EPI == EPI_SWIGLU || EPI == EPI_GEGLU || EPI == EPI_CLAMPGLU || EPI == EPI_ROPE;
-  const bool pairs = use_pair() && !g.m_tile_group;
-  int bn = g.block_n, cg = 1, eg = 2;
-  if (bn == 0) {
+constexpr bool wide_only(int epi) { return epi == EPI_SWIGLU || epi == EPI_GEGLU || epi == EPI_CLAMPGLU || epi == EPI_ROPE; }
+
+GemmTile tile_of(int M, int N, int K, int epi, int block_n, bool pairs, int num_sms) {
+  GemmTile pick{block_n, 1, 2};
+  if (block_n == 0) {
     // The tile shape whose waves end first.  Per shape: us per 64-deep k block of one tile, the least a wave takes (its epilogue, when K
     // is short) and the part of a launch that does not depend on K, fitted to runs on random operands:
     //                          256 x 256 pair  256 x 192 pair  256 x 128 pair  128 x 256  128 x 128  128 x 64
@@ -606,18 +605,25 @@ cudaError_t launch_epi(cudaStream_t stream, const GemmArgs& g, int num_sms) {
     struct Shape { int bn, cg, eg; double kb, floor, fixed; };
     static constexpr Shape shapes[] = {{256, 2, 2, 0.36, 5.6, 8.5}, {256, 2, 4, 0.375, 5.2, 8.5}, {192, 2, 2, 0.29, 4.8, 8.3}, {192, 2, 4, 0.305, 4.3, 8.3}, {128, 2, 2, 0.235, 3.4, 8.0},
                                        {256, 1, 2, 0.42, 6.0, 7.0}, {128, 1, 2, 0.28, 3.9, 6.5}, {64, 1, 2, 0.235, 3.1, 6.0}};
-    const int num_kb = (g.K + BLOCK_K - 1) / BLOCK_K;
+    const int num_kb = (K + BLOCK_K - 1) / BLOCK_K;
     double best = 1e30;
     for (const Shape& t : shapes) {
-      if ((t.cg == 2 && (!pairs || num_sms < 2)) || (kWideOnly && t.bn != 256) || (t.eg != 2 && !deep_epilogue(EPI))) continue;
-      const long tiles = (long)((g.M + BLOCK_M * t.cg - 1) / (BLOCK_M * t.cg)) * ((g.N + t.bn - 1) / t.bn);
+      if ((t.cg == 2 && (!pairs || num_sms < 2)) || (wide_only(epi) && t.bn != 256) || (t.eg != 2 && !deep_epilogue(epi))) continue;
+      const long tiles = (long)((M + BLOCK_M * t.cg - 1) / (BLOCK_M * t.cg)) * ((N + t.bn - 1) / t.bn);
       const long workers = std::max(1, num_sms / t.cg);
       const double us = (double)((tiles + workers - 1) / workers) * std::max(num_kb * t.kb, t.floor) + t.fixed;
-      if (us < best) { best = us; bn = t.bn; cg = t.cg; eg = t.eg; }
+      if (us < best) { best = us; pick = GemmTile{t.bn, t.cg, t.eg}; }
     }
-  } else if (bn == 256 && pairs && (long)((g.M + 255) / 256) * ((g.N + 255) / 256) >= num_sms / 2) {
-    cg = 2;  // a width asked for: CTA pairs once the problem has at least a wave of them
+  } else if (block_n == 256 && pairs && (long)((M + 255) / 256) * ((N + 255) / 256) >= num_sms / 2) {
+    pick.cg = 2;  // a width asked for: CTA pairs once the problem has at least a wave of them
   }
+  return pick;
+}
+
+template <int EPI>
+cudaError_t launch_epi(cudaStream_t stream, const GemmArgs& g, int num_sms) {
+  constexpr bool kWideOnly = wide_only(EPI);
+  const auto [bn, cg, eg] = tile_of(g.M, g.N, g.K, EPI, g.block_n, use_pair() && !g.m_tile_group, num_sms);
   switch (bn * 10 + cg) {
     case 2562:
       if constexpr (deep_epilogue(EPI))
@@ -654,7 +660,7 @@ cudaError_t set_attr_epi() {
   cudaError_t e;
   if ((e = set_attr<256, EPI, 2>()) != cudaSuccess) return e;
   if ((e = set_attr<256, EPI, 1>()) != cudaSuccess) return e;
-  if constexpr (EPI != EPI_SWIGLU && EPI != EPI_GEGLU && EPI != EPI_CLAMPGLU && EPI != EPI_ROPE) {
+  if constexpr (!wide_only(EPI)) {
     if ((e = set_attr<192, EPI, 2>()) != cudaSuccess) return e;
     if constexpr (deep_epilogue(EPI)) {
       if ((e = set_attr<256, EPI, 2, 4>()) != cudaSuccess) return e;
@@ -742,6 +748,8 @@ cudaError_t gemm_bf16_tn(cudaStream_t stream, const GemmArgs& g) {
   }
   return cudaErrorInvalidValue;
 }
+
+GemmTile gemm_tile(int M, int N, int K, Epi epi, int sms) { return tile_of(M, N, K, epi, 0, use_pair(), sms); }
 
 // ------------------------------------------------------------------ test-only checker
 namespace {

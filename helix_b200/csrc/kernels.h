@@ -68,6 +68,9 @@ struct GemmArgs {
   float glu_limit = 0.f;  // EPI_CLAMPGLU
   int silu_cols = 0;      // EPI_SILU_COLS
 };
+// Tile that gemm_bf16_tn picks: columns, CTAs per tile (128 rows each), groups of four epilogue warps
+struct GemmTile { int bn, cg, eg; };
+GemmTile gemm_tile(int M, int N, int K, Epi epi, int sms);
 cudaError_t gemm_bf16_tn(cudaStream_t stream, const GemmArgs& a);
 // Debug/test-only CUDA-core GEMM (same contract, EPI_NONE/EPI_F32 only); used by tests as an on-device checker.
 cudaError_t gemm_naive_check(cudaStream_t stream, const GemmArgs& a);

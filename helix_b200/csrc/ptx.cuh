@@ -93,6 +93,14 @@ __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+template <int NC, typename T>
+__device__ __forceinline__ T* cluster_ptr(T* p, uint32_t cta) {  // the same shared-memory object in another of the cluster's NC blocks
+  if constexpr (NC == 1) return p;
+  uint64_t r;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t>(p)), "r"(cta));
+  return reinterpret_cast<T*>(r);
+}
+
 // ---------------------------------------------------------------- TMA
 constexpr uint64_t kEvictNormal = 0x1000000000000000ull;
 constexpr uint64_t kEvictFirst = 0x12F0000000000000ull;

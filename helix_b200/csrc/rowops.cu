@@ -411,13 +411,6 @@ __device__ __forceinline__ void voc_sync() {
     cluster_sync_all();
   }
 }
-template <int NC, typename T>
-__device__ __forceinline__ T* cluster_ptr(T* p, uint32_t cta) {  // the same shared-memory object in another block of the cluster
-  if constexpr (NC == 1) return p;
-  uint64_t r;
-  asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t>(p)), "r"(cta));
-  return reinterpret_cast<T*>(r);
-}
 
 // f(i, values, how many of them exist) for every group of four columns i .. i + 3 of a slice of n that a thread keeps; eight groups are
 // in flight per thread (one at a time left the load at the latency of eight round trips)

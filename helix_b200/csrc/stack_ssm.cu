@@ -968,12 +968,6 @@ __global__ void gate_scale_kernel(const float* __restrict__ in, const bf16* __re
 // tokens' make the feed-forward's inner rows.  What bounds it: the state's bytes (read before the products' launch is over) and a chain of
 // two round trips to L2, two cluster barriers and the recurrence; as three launches the same was 15 us of
 // a layer's 33 (16 sequences x 32 heads), 8 now; a turn of 2 such layers and 12 tokens 2520 -> 2450.
-template <typename T>
-__device__ __forceinline__ T* block_of_cluster(T* p, uint32_t cta) {  // the same shared-memory object in another block of the cluster
-  uint64_t r;
-  asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(reinterpret_cast<uint64_t>(p)), "r"(cta));
-  return reinterpret_cast<T*>(r);
-}
 constexpr int kTokDk = 128, kTokDv = 64, kTokTaps = 4;
 template <int HG>
 __global__ void __cluster_dims__(HG, 1, 1) __launch_bounds__(256, 4) ssm_token_kernel(const __grid_constant__ SsmTokenArgs a) {
@@ -1056,7 +1050,7 @@ __global__ void __cluster_dims__(HG, 1, 1) __launch_bounds__(256, 4) ssm_token_k
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   if (conv && !value) {
 #pragma unroll
-    for (int o = 0; o < HG; ++o) *block_of_cluster(reinterpret_cast<float4*>(&kq[shared_at]), o) = made;
+    for (int o = 0; o < HG; ++o) *cluster_ptr<HG>(reinterpret_cast<float4*>(&kq[shared_at]), o) = made;
   }
   __syncwarp();
   cluster_sync_all();
@@ -1079,7 +1073,7 @@ __global__ void __cluster_dims__(HG, 1, 1) __launch_bounds__(256, 4) ssm_token_k
       u = make_float4(y.x * (z.x * s.x), y.y * (z.y * s.y), y.z * (z.z * s.z), y.w * (z.w * s.w));
       const float ss = sum_of_squares(u);
 #pragma unroll
-      for (int o2 = 0; o2 < HG; ++o2) *block_of_cluster(&quads[rank][lane], o2) = ss;
+      for (int o2 = 0; o2 < HG; ++o2) *cluster_ptr<HG>(&quads[rank][lane], o2) = ss;
     }
   }
   __syncwarp();

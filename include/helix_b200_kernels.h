@@ -21,6 +21,8 @@ const char* hbk_last_error(void);
  * 5 swiglu (W packed [128 gate|128 up] per 256 rows, C has N/2 columns), 6 fp32 out). block_n 0 = auto. */
 int hbk_gemm(const void* A, int lda, const void* W, int ldw, void* C, int ldc, const void* R, int ldr, const void* bias,
              int M, int N, int K, int epi, int block_n);
+/* tile that hbk_gemm with block_n 0 picks on `sms` SMs: columns | CTAs of 128 rows << 12 | groups of four epilogue warps << 16; no device is asked */
+int hbk_gemm_tile(int M, int N, int K, int epi, int sms);
 /* decode-step GEMM (M<=256): swap-AB + stream-K partial slabs summed in fixed order -> out fp32 [M,N] */
 int hbk_gemm_skinny(const void* X, int ldx, const void* W, int ldw, float* out_f32, int ldo, int M, int N, int K);
 /* the same GEMM with the fused tile finisher (last-arriving CTA of each output tile sums the slabs in slab order and

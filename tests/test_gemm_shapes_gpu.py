@@ -102,6 +102,27 @@ def test_tiles_of_192_columns(M, N, K, epi):
     """Sizes whose waves end first in 256 x 192: whole and ragged rows and columns, a last tile of a few columns, one k block."""
     l = hb.lib()
     assert l.hbk_init() == 0
+    assert tile(M, N, K, epi) == (192, 2, 4 if epi in (2, 3) and K < 1000 else 2)
+    same_as_narrow_tiles(M, N, K, epi)
+
+
+@pytest.mark.parametrize("M,N,K", [(3000, 3072, 768), (3000, 4104, 72), (4609, 2304, 64), (7000, 2056, 328)])
+@pytest.mark.parametrize("epi", [2, 3])
+def test_four_epilogue_groups_on_256_columns(M, N, K, epi):
+    """Sizes that take tiles of 256 x 256 with four groups of epilogue warps: whole and ragged rows and columns, one k block and several."""
+    l = hb.lib()
+    assert l.hbk_init() == 0
+    assert tile(M, N, K, epi) == (256, 2, 4)
+    same_as_narrow_tiles(M, N, K, epi)
+
+
+def tile(M, N, K, epi):
+    t = hb.lib().hbk_gemm_tile(M, N, K, epi, torch.cuda.get_device_properties(0).multi_processor_count)
+    return t & 4095, t >> 12 & 15, t >> 16
+
+
+def same_as_narrow_tiles(M, N, K, epi):
+    l = hb.lib()
     A, W, R, b = rnd(M, K, seed=6), rnd(N, K, scale=K ** -0.5, seed=7), rnd(M, N, seed=8), rnd(N, seed=9)
     outs = []
     for bn in (0, 64):

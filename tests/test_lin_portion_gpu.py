@@ -78,5 +78,4 @@ def test_longer_portions_on_wide_blocks_equal_single_tokens(kind, heads, dim, vd
 @pytest.mark.parametrize("heads,dim,vdim", [(120, 128, 64), (120, 68, 36)])
 def test_many_blocks_equal_single_tokens(kind, heads, dim, vdim):
     """More blocks than three per SM: eight columns per lane, also with padded channels and columns."""
-    test_portions_equal_single_tokens(kind, heads, dim, vdim)
     test_longer_portions_on_wide_blocks_equal_single_tokens(kind, heads, dim, vdim)
