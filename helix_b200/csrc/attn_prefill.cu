@@ -237,12 +237,6 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   if (warp == 1) {
     tmem_alloc(tmem_ptr, 512);
     tmem_relinquish();
-    // The launch behind may take its places as soon as every block of this one holds its tensor memory (launch.h).  Not behind paged rows with an item a block
-    // at most: those launches run for tens of us on fewer SMs than there are, and a next one that sat down early on the free SMs and
-    // got the rest as they ended ran 6 % longer than one placed at once (128 items a launch, back to back: 891 rows over 2841 keys
-    // 47.4 -> 44.8 us, 700 over 3000 49.8 -> 46.3; with more items than blocks 61.6 both ways).  Packed prompts of that
-    // size end within a few us, where the early start is worth more (6.5 -> 6.2 us).
-    if (!PAGED || max_q_pairs * B * (Hq >> pack) > (int)gridDim.x) pdl_launch_dependents();
   }
   pdl_wait();  // nothing above touches memory that a kernel before this one may write
   // Order of the items (SORTED): rows (q pair, sequence) by falling number of kv tiles, a row's heads side by side (they share keys), dealt
@@ -314,6 +308,12 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // The launch behind may take its places as soon as every block of this one holds its tensor memory (launch.h).  Not behind paged rows with an item a block
+  // at most: those launches run for tens of us on fewer SMs than there are, and a next one that sat down early on the free SMs and
+  // got the rest as they ended ran 6 % longer than one placed at once (128 items a launch, back to back: 891 rows over 2841 keys
+  // 47.4 -> 44.8 us, 700 over 3000 49.8 -> 46.3; with more items than blocks 61.6 both ways).  Packed prompts of that
+  // size end within a few us, where the early start is worth more (6.5 -> 6.2 us).
+  if (!PAGED || max_q_pairs * B * (Hq >> pack) > (int)gridDim.x) pdl_launch_dependents();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);  // warp-uniform for the compiler too
   const int rows = SORTED ? s_rows[0] : -1;
   const int groups = Hq >> pack;  // of heads that an item takes together
